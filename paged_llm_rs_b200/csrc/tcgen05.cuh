@@ -54,6 +54,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     *abort_flag = 1;
     return false;
 }
+// One lane of a converged warp.  A warp that issues tcgen05.mma, a commit or a copy runs its loop with ALL its lanes and
+// puts only the instruction itself under this: addresses and descriptors are then uniform values, which these instructions
+// take as they are.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");

@@ -68,6 +68,8 @@ def lib():
         sig["pllm_attention_prefill_tcgen05"] = [P] * 10 + [c_int] * 7 + [c_float, c_int, P, P]
         sig["pllm_gemm_tcgen05_supports"] = [c_int, c_int, c_int, c_int]
         sig["pllm_gemm_tcgen05"] = [P, P, P, c_int, c_int, c_int, c_int, c_float, P, P]
+        sig["pllm_rows_gemm_supports"] = [c_int, c_int, c_int]
+        sig["pllm_rows_gemm"] = [P, P, P, c_int, c_int, c_int, c_int, c_float, c_int, c_int, P, P]
         sig["pllm_embed_scaled32"] = [c_int, P, P, P, c_int, c_int, c_int, c_float, P, P]
         sig["pllm_sinusoid_add"] = [P, P, P, c_int, c_int, P]
         sig["pllm_round_rows"] = [c_int, P, P, c_ll, P]
@@ -542,8 +544,7 @@ def skinny_gemm_takes(x: torch.Tensor, weight: torch.Tensor, k: Optional[int] = 
 # Measured on a B200 inside a captured step (0.6B shapes, microseconds, skinny / cuBLAS):
 #   rows 1-8:  qkv 3.5-3.8 / 5.0   o 3.1 / 6.4-7.5   gate_up 4.6-4.8 / 5.1   down 3.9-4.2 / 8.9-9.6
 #   rows 64:   qkv 12.3 / 4.9      o 6.3 / 5.4        gate_up 12.6 / 5.3      down 8.4 / 6.6
-# so the kernel (which takes up to 64 rows) is used up to 16, and up to a width where the
-# library's head product is the faster one (151936 x 1024: 66 / 54).
+# so the kernel (which takes up to 64 rows) is used up to 16, for products below ROWS_MIN_WEIGHTS.
 SKINNY_MAX_M = 16
 SKINNY_MAX_N = 32768
 
@@ -592,11 +593,56 @@ def gemm_tcgen05(x: torch.Tensor, weight: torch.Tensor, glu: bool = False, statu
     return out
 
 
+# The rows of a decode step or of a short prompt in bfloat16 with the weights as the tensor cores' 128-row operand
+# (csrc/rows_gemm_tcgen05.cu).  Measured in captured decode steps with ONE product's kernel changed (us a step):
+#   0.6B shape (products of 2 to 6 M weights), 16 rows: the weight-streaming kernel 872, this one 1032; 24 rows: this one 1285,
+#     the library 1561 (its q/k/v 1304 and o 1301 alone would do as well, its gate/up with the activation's pass 1320 not)
+#   8B shape, 8 rows: q/k/v (25 M weights) 714, the weight-streaming kernel 762; gate/up (101 M) 715 / 883; down (50 M) 714 / 851;
+#     o (17 M) 714 / 717; the head 714, the library 738
+#   64 rows: 8B 983, the library 1045; 128 rows, 0.6B shape: 1648, the library and gemm_tcgen05.cu 1507
+# so it takes 17 to 64 rows, and fewer where the product has ROWS_MIN_WEIGHTS or more.
+ROWS_GEMM = True
+ROWS_MAX_M = 64
+ROWS_MIN_WEIGHTS = 16 << 20
+
+
+def rows_gemm_takes(x, weight: torch.Tensor, n_out: int, want: Optional[torch.dtype] = None) -> bool:
+    """Whether ``linear`` / ``linear_glu`` / ``linear_act`` run the product with the weights as the 128-row operand
+    (n_out: columns of the result)."""
+    if not ROWS_GEMM or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous() \
+            or not weight.is_contiguous() or want not in (None, torch.bfloat16, torch.float32) or (x.data_ptr() | weight.data_ptr()) & 15:
+        return False
+    M, K = x.shape[0], weight.shape[1]
+    return M <= ROWS_MAX_M and (M > SKINNY_MAX_M or weight.numel() >= ROWS_MIN_WEIGHTS) and bool(lib().pllm_rows_gemm_supports(M, n_out, K))
+
+
+def rows_gemm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, glu: bool = False,
+              status: Optional[torch.Tensor] = None, act: str = "silu", limit: float = 0.0,
+              out_dtype: torch.dtype = torch.bfloat16, unary: str = "none", splits: int = 0) -> torch.Tensor:
+    """x W^T for up to 64 rows of x (bfloat16, float accumulation); with ``glu`` W is [gate rows; up rows] and the result
+    is act(x Wg^T, x Wu^T).  ``splits``: CTAs that share the sum over k (0: as the sizes ask)."""
+    M, K = x.shape
+    n_out = weight.shape[0] // 2 if glu else weight.shape[0]
+    if weight.shape[1] != K or not lib().pllm_rows_gemm_supports(M, n_out, K):
+        raise KernelError(f"rows_gemm: does not take x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
+    if x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or out_dtype not in (torch.bfloat16, torch.float32):
+        raise KernelError("rows_gemm: bfloat16 operands, a bfloat16 or float32 result")
+    if out is None:
+        out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+    elif out.shape != (M, n_out) or out.dtype != out_dtype:
+        raise KernelError("rows_gemm: out does not fit")
+    _dev(x, weight, out)
+    st = status if status is not None else gemm_status(x.device)
+    _check(lib().pllm_rows_gemm(_ptr(x), _ptr(weight), _ptr(out), M, n_out, K, 1 + _glu(act) if glu else -UNARY_KINDS[unary], float(limit),
+                                1 if out_dtype == torch.float32 else 0, splits, _ptr(st), _stream()), "rows_gemm")
+    return out
+
+
 def skinny_glu_takes(x, weight: torch.Tensor, n_out: int) -> bool:
     """Whether the weight-streaming kernel takes the gate/up product with the activation in its epilogue."""
     if not SKINNY_GEMM or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.dim() != 2:
         return False
-    return n_out <= SKINNY_MAX_N and bool(lib().pllm_skinny_gemm_glu_supports(x.shape[0], n_out, weight.shape[1]))
+    return x.shape[0] <= SKINNY_MAX_M and n_out <= SKINNY_MAX_N and bool(lib().pllm_skinny_gemm_glu_supports(x.shape[0], n_out, weight.shape[1]))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, gated: bool = False,
@@ -623,8 +669,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         act = torch.empty((x.shape[0], K), dtype=x.dtype, device=x.device)
         swiglu(x, act)
         x = act
-    # The widest products (the output head) stay with the library, which is faster there
-    # (measured 54 us against 66 us at 151936 x 1024, batch 8).
+    if rows_gemm_takes(x, weight, N, want) and (out is None or (out.is_contiguous() and not out.data_ptr() & 15)):
+        return rows_gemm(x, weight, out, status=status, out_dtype=want)
     if skinny_gemm_takes(x, weight, K) and N <= SKINNY_MAX_N and want in (torch.bfloat16, torch.float32):
         _dev(x, weight, out)
         M = x.shape[0]
@@ -656,6 +702,8 @@ def linear_glu(x: torch.Tensor, w_gate_up: torch.Tensor, status: Optional[torch.
     inter = two_i // 2
     if x.shape[-1] != K:
         raise KernelError(f"linear_glu: input width {x.shape[-1]} does not fit a weight of {tuple(w_gate_up.shape)}")
+    if FUSE_GLU and rows_gemm_takes(x, w_gate_up, inter):
+        return rows_gemm(x, w_gate_up, glu=True, status=status, act=act, limit=limit)
     if FUSE_GLU and skinny_glu_takes(x, w_gate_up, inter):
         _dev(x, w_gate_up)
         out = torch.empty((x.shape[0], inter), dtype=torch.bfloat16, device=x.device)
@@ -1406,6 +1454,8 @@ def linear_act(x: torch.Tensor, weight: torch.Tensor, act: str, status: Optional
     N, K = weight.shape
     if x.shape[-1] != K:
         raise KernelError(f"linear_act: input width {x.shape[-1]} does not fit a weight of {tuple(weight.shape)}")
+    if rows_gemm_takes(x, weight, N):
+        return rows_gemm(x, weight, status=status, unary=act)
     if skinny_gemm_takes(x, weight, K) and N <= SKINNY_MAX_N:
         _dev(x, weight)
         out = torch.empty((x.shape[0], N), dtype=torch.bfloat16, device=x.device)
