@@ -115,3 +115,16 @@ def test_how_requests_ended_is_remembered_for_a_bounded_number_of_them():
     ids = [eng.submit([1, 2], max_tokens=1) for _ in range(12)]
     eng.run_until_done()
     assert len(eng._finish) == 5 and eng.finish_reason(ids[-1]) == Finish.LENGTH and eng.finish_reason(ids[0]) is None
+
+
+def test_portion_sizes_cover_every_step_and_pad_large_steps_by_a_quarter_at_most():
+    from paged_llm_rs_b200.engine.runner import PADDED_PORTION, portion_sizes
+    for budget in (1, 8, 64, 73, 96, 128, 255, 256, 300, 576, 2048, 5000, 8192):
+        sizes = portion_sizes(budget)
+        assert sizes == sorted(set(sizes)) and sizes[-1] == budget
+        for total in range(1, budget + 1):
+            size = next(n for n in sizes if n >= total)
+            if total > PADDED_PORTION:
+                assert (size - total) * 4 <= size or (size == budget and budget < 2 * PADDED_PORTION)
+            elif size == budget:
+                assert budget < 2 * PADDED_PORTION

@@ -87,3 +87,36 @@ def test_launched_captured_and_prepacked_steps_give_the_same_logits(tmp_path, na
     for k in lens:
         cache.close(k)
     cache.check_invariants()
+
+
+@pytest.mark.parametrize("budget,total,sizes", [(128, 3, [128, 64, 64]), (128, 64, [128, 64, 64]), (128, 65, [128]), (96, 10, [96, 96]),
+                                                (600, 40, [None, 64, 64]), (600, 257, [None, 320, 320]), (600, 590, [600])])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_a_small_portion_step_gives_the_same_logits_launched_and_at_every_captured_size(tmp_path, dtype, budget, total, sizes):
+    from paged_llm_rs_b200.engine.runner import ModelRunner
+    from paged_llm_rs_b200.engine.step import StepEntry
+
+    cfg, seed = CONFIGS["D"]
+    model = write_model(tmp_path, "D", decisive=True)
+    runner = ModelRunner(model, dtype=dtype, page_size=16, num_pages=96, max_requests=8, prefix_cache=False)
+    runner.graph_step_tokens = budget
+    cache, rng = runner.cache, np.random.default_rng(total)
+    toks = rng.integers(0, cfg["vocab_size"], 70 + total).tolist()
+    for r, n in (("a", 70), ("b", 23)):        # a request that decodes beside a portion of another, which has 23 tokens behind it
+        cache.open(r)
+        assert cache.reserve(r, n + total)
+        runner.step([StepEntry(r, toks[:n], [])])
+        cache.commit(r, n)
+    entries = [StepEntry("a", toks[70:71], [0]), StepEntry("b", toks[23:23 + total - 1], [total - 2])]
+    zeros = np.zeros(2, dtype=np.float32)
+    runner.use_graphs = False
+    want = runner.step_and_sample(entries, zeros, zeros)[0].cpu().numpy()
+    runner.use_graphs = True
+    for size in sizes:
+        was = set(runner._graphs)
+        got, tokens = runner.step_and_sample(entries, zeros, zeros)
+        got, tokens = got.cpu().numpy(), tokens.cpu().numpy()
+        runner.check_status()
+        assert {k[0] for k in set(runner._graphs) - was} <= {size} and (size is None) == (runner.tokens_host is None)
+        assert err(got, want) <= (2e-5 if dtype == "float32" else 3e-2) and (tokens[1:] == got.argmax(1)).all()
+    assert {k[0] for k in runner._graphs} == {n for n in sizes if n is not None}
