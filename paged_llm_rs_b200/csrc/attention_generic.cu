@@ -1,7 +1,7 @@
-// Paged attention for any head size (a multiple of 4 floats / 8 bfloat16 up to
-// 256), any number of heads and groups, any page size, with an optional window:
-// the kernel of the true 32-bit path, and of bfloat16 shapes that the tuned
-// kernels do not take.  Arithmetic in float on the CUDA cores.
+// Paged attention for any head size (a multiple of 8 up to 256), any number of
+// heads and groups, any page size, with an optional window: a kernel for bfloat16
+// shapes that the tuned kernels do not take, and below it the kernel of the true
+// 32-bit path.  Arithmetic in float on the CUDA cores.
 //
 // What it computes is the reference's attention
 // (crates/pagedllm/src/model/attention.rs:198-214 and
@@ -161,6 +161,327 @@ __global__ void attention_generic_kernel(
     }
 }
 
+// ---- float32 ------------------------------------------------------------------------------------
+// The same in float32, which is bound by the multiply-adds of a prompt's portion and by its keys and values for decoded
+// tokens.  A CTA of 128 threads holds up to 32 rows (token, head) of an item and takes 64 keys a turn; a turn's keys come
+// in by cp.async while the turn before it is summed, its values while its scores are formed (each buffer is asked for
+// again as soon as it has been read).  More than four rows: a thread makes 4 x 4 scores and then 4 rows x 4 HDV
+// output entries, so that a value read from shared memory serves four sums (the kernel above reads two for each).  Up to
+// four rows (a decoded token): a key belongs to two threads, each taking half of the head, and a row's softmax to a warp.
+// Scores are sums of even and of odd entries (fma.rn.f32x2).  Measured at the 0.6B shape (16 heads over 8 kv heads of 128),
+// 4 requests at 500 beside a portion of 252 tokens: 60 us a layer, the kernel above in its place 136.  It is bound by the
+// latency of its own chains: a warp a scheduler (242 registers a thread), 35% of the issue slots and 37% of the
+// shared-memory pipe in use.
+constexpr int AF_ROWS = 32, AF_BK = 64, AF_THREADS = 128, AF_HEADS = 4;
+
+__device__ __forceinline__ uint32_t af_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void af_copy16(uint32_t dst, const float* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void af_wait_older() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+__device__ __forceinline__ void af_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long af_pack(float lo, float hi) {
+    return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ float af_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float af_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+// A turn's weights times its values: rows ty + 8 a, the head's chunks tx + 16 h.
+template <int HDV, bool GUARD>
+__device__ __forceinline__ void sum_values(const float* p_s, const float* v_s, int hdp, int chunks, int tx, int ty, unsigned long long (&acc)[4][HDV][2]) {
+#pragma unroll 2
+    for (int j = 0; j < AF_BK; j += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int a = 0; a < 4; a++) p[a] = *reinterpret_cast<const float4*>(p_s + (ty + 8 * a) * AF_BK + j);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            ulonglong2 v[HDV];
+#pragma unroll
+            for (int h = 0; h < HDV; h++)
+                v[h] = *reinterpret_cast<const ulonglong2*>(v_s + (j + i) * hdp + ((tx + 16 * h < chunks ? tx + 16 * h : 0) << 2));
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const float pa = i == 0 ? p[a].x : i == 1 ? p[a].y : i == 2 ? p[a].z : p[a].w;
+                const unsigned long long p2 = af_pack(pa, pa);
+                if (!GUARD || pa != 0.f) {
+#pragma unroll
+                    for (int h = 0; h < HDV; h++) {
+                        af_fma2(acc[a][h][0], p2, v[h].x);
+                        af_fma2(acc[a][h][1], p2, v[h].y);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// HDV: 64-entry parts of a head, hd <= 64 HDV.
+template <int HDV>
+__global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_kernel(
+    const float* q, const float* k_pool, const float* v_pool, const int* __restrict__ block_tables,
+    const AttnWork* __restrict__ work, const int* __restrict__ n_work_ptr, float* __restrict__ out, float* __restrict__ part_o,
+    float* __restrict__ part_ml, int nh, int nkv, int hd, int page_size, int n_pages, int table_width, int window, float scale, int* status) {
+    pdl_launch_dependents();
+    // The list of items and the block tables are the host's (the step's packed buffer): what they say is fetched before the wait
+    // for the kernel that makes q and the newest keys.  The CTAs of an item are neighbours in the grid, so that the live ones
+    // are the first and every SM gets one before any gets two.
+    const int ctas = nkv * ((nh / nkv + AF_HEADS - 1) / AF_HEADS), item = blockIdx.x / ctas, part = blockIdx.x % ctas;
+    if (item >= *n_work_ptr) return;
+    const AttnWork w = work[item];
+    const int group = nh / nkv, heads_per_cta = min(group, AF_HEADS), gparts = (group + heads_per_cta - 1) / heads_per_cta;
+    const int kh = part / gparts, head0 = kh * group + (part % gparts) * heads_per_cta;
+    const int n_heads = min(heads_per_cta, kh * group + group - head0);
+    const int rows = min(w.q_count * n_heads, AF_ROWS);
+    const bool few = rows <= 4;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
+    const int hdp = (hd + 31) & ~31, chunks = hd / 4;          // a row of shared memory holds whole groups of eight 16-byte chunks
+
+    extern __shared__ __align__(128) float smem_f[];
+    float* q_s = smem_f;                             // [32][hdp], chunk c of row r at c ^ (r & 7)
+    float* k_s = q_s + AF_ROWS * hdp;                // [64][hdp], likewise
+    float* v_s = k_s + AF_BK * hdp;                  // [64][hdp], as it lies
+    float* p_s = v_s + AF_BK * hdp;                  // scores, then weights: [32][64] (few rows: [64][4])
+    __shared__ long long off_s[2][AF_BK];            // where a key's row of this kv head starts in the pools; -1: nowhere
+    __shared__ float row_s[2][4];                    // few rows: a row's factor for what it holds; at the end its sum
+
+    // rows past the item's are never visible to anything
+    int lo[4], hi[4], my_tok[4], my_head[4];
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        const int r = few ? a : ty + 8 * a;
+        const bool live = r < rows;
+        my_tok[a] = live ? r / n_heads : 0;
+        my_head[a] = live ? head0 + r % n_heads : head0;
+        const int pos = w.q_pos0 + my_tok[a];
+        lo[a] = max(w.kv_begin, window > 0 ? pos - window + 1 : 0);
+        hi[a] = live ? min(w.kv_end, pos + 1) : 0;
+    }
+    const int* table = block_tables + (size_t)w.seg * table_width;
+    auto find = [&](int t) {
+        if (tid < AF_BK) {
+            const int j = w.kv_begin + t * AF_BK + tid;
+            int page = -1;
+            if (j < w.kv_end) {
+                const int b = j / page_size;
+                page = b < table_width ? table[b] : -1;
+                // A freed page of a window layer holds -1 and is never visible to a query of this item; anything else out of range is a fault.
+                if (page >= n_pages) { atomicOr(status, 8); page = -1; }
+            }
+            off_s[t & 1][tid] = page < 0 ? -1 : (((long long)page * nkv + kh) * page_size + j % page_size) * hd;
+        }
+    };
+    // (a thread's rows and chunks: 128 further on is 128 / chunks rows and 128 % chunks chunks further on)
+    const int first_row = tid / chunks, first_chunk = tid % chunks, row_step = AF_THREADS / chunks, chunk_step = AF_THREADS % chunks;
+    auto load = [&](int t, float* dst, const float* pool, bool swizzled) {
+        const uint32_t to = af_smem(dst);
+        int j = first_row, c = first_chunk;
+#pragma unroll 4
+        while (j < AF_BK) {
+            const long long off = off_s[t & 1][j];
+            af_copy16(to + (j * hdp + ((swizzled ? c ^ (j & 7) : c) << 2)) * 4, pool + (off < 0 ? 0 : off + c * 4), off >= 0);
+            j += row_step;
+            c += chunk_step;
+            if (c >= chunks) { c -= chunks; j++; }
+        }
+        af_commit();
+    };
+    float m[4], l[4];
+    unsigned long long acc[4][HDV][2];
+    float acc1[4][(HDV + 1) / 2];                    // few rows: entry tid (+ 128) of each row's output
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        m[a] = -CUDART_INF_F;
+        l[a] = 0.f;
+#pragma unroll
+        for (int h = 0; h < HDV; h++) acc[a][h][0] = acc[a][h][1] = 0ull;
+#pragma unroll
+        for (int h = 0; h < (HDV + 1) / 2; h++) acc1[a][h] = 0.f;
+    }
+    const int turns = (w.kv_end - w.kv_begin + AF_BK - 1) / AF_BK;
+    const int seen_by_all = min(w.kv_end, w.q_pos0 + 1), seen_from = window > 0 ? w.q_pos0 + w.q_count - window : 0;
+    find(0);
+    pdl_wait(KID_ATT_GENERIC);
+    __syncthreads();
+    load(0, k_s, k_pool, true);
+    load(0, v_s, v_pool, false);
+    for (int i = tid; i < AF_ROWS * chunks; i += AF_THREADS) {
+        const int r = i / chunks, c = i % chunks;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < rows) {
+            const float* from = q + ((size_t)(w.q_token0 + r / n_heads) * nh + head0 + r % n_heads) * hd + c * 4;
+            v = make_float4(from[0], from[1], from[2], from[3]);
+        }
+        *reinterpret_cast<float4*>(q_s + r * hdp + ((c ^ (r & 7)) << 2)) = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+    }
+    for (int t = 0; t < turns; t++) {
+        const int kv0 = w.kv_begin + t * AF_BK;
+        af_wait_older();
+        __syncthreads();          // this turn's keys are there
+        if (t + 1 < turns) find(t + 1);
+        float sc[4][4];
+        if (few) {
+            const int j = tid >> 1, half = tid & 1, c0 = half ? (chunks + 1) / 2 : 0, c1 = half ? chunks : (chunks + 1) / 2;
+            unsigned long long s2[4] = {0ull, 0ull, 0ull, 0ull};
+            for (int c = c0; c < c1; c++) {
+                const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k_s + j * hdp + ((c ^ (j & 7)) << 2));
+#pragma unroll
+                for (int a = 0; a < 4; a++) {
+                    const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(q_s + a * hdp + ((c ^ a) << 2));
+                    af_fma2(s2[a], qv.x, kv.x);
+                    af_fma2(s2[a], qv.y, kv.y);
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                float v = af_lo(s2[a]) + af_hi(s2[a]);
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                const int key = kv0 + j;
+                if (half == 0) p_s[j * 4 + a] = key >= lo[a] && key < hi[a] ? v : -CUDART_INF_F;
+            }
+        } else {
+            unsigned long long s2[4][4];
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) s2[a][b] = 0ull;
+#pragma unroll 2
+            for (int c = 0; c < chunks; c++) {
+                ulonglong2 qv[4];
+#pragma unroll
+                for (int a = 0; a < 4; a++) {
+                    const int r = ty + 8 * a;
+                    qv[a] = *reinterpret_cast<const ulonglong2*>(q_s + r * hdp + ((c ^ (r & 7)) << 2));
+                }
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    const int j = tx + 16 * b;
+                    const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k_s + j * hdp + ((c ^ (j & 7)) << 2));
+#pragma unroll
+                    for (int a = 0; a < 4; a++) {
+                        af_fma2(s2[a][b], qv[a].x, kv.x);
+                        af_fma2(s2[a][b], qv[a].y, kv.y);
+                    }
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    const int key = kv0 + tx + 16 * b;
+                    sc[a][b] = key >= lo[a] && key < hi[a] ? af_lo(s2[a][b]) + af_hi(s2[a][b]) : -CUDART_INF_F;
+                }
+        }
+        __syncthreads();          // the keys have been read, the next turn's places are known (few rows: the scores are there)
+        if (t + 1 < turns) load(t + 1, k_s, k_pool, true); else af_commit();
+        if (few) {
+            if (warp < rows) {
+                // row `warp` is this warp's, two keys a lane
+                const float s0 = p_s[lane * 4 + warp], s1 = p_s[(lane + 32) * 4 + warp];
+                const float top = fmaxf(m[0], warp_max(fmaxf(s0, s1)));
+                const float p0 = s0 == -CUDART_INF_F ? 0.f : expf(s0 - top), p1 = s1 == -CUDART_INF_F ? 0.f : expf(s1 - top);
+                const float corr = top == -CUDART_INF_F ? 1.f : expf(m[0] - top);
+                l[0] = l[0] * corr + warp_sum(p0 + p1);
+                m[0] = top;
+                p_s[lane * 4 + warp] = p0;
+                p_s[(lane + 32) * 4 + warp] = p1;
+                if (lane == 0) row_s[0][warp] = corr;
+            } else if (lane == 0) row_s[0][warp] = 1.f;
+        } else {
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                float top = fmaxf(fmaxf(sc[a][0], sc[a][1]), fmaxf(sc[a][2], sc[a][3]));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));     // (the 16 lanes of the row)
+                top = fmaxf(top, m[a]);
+                const float corr = top == -CUDART_INF_F ? 1.f : expf(m[a] - top);
+                float sum = 0.f;
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    const float p = sc[a][b] == -CUDART_INF_F ? 0.f : expf(sc[a][b] - top);
+                    sum += p;
+                    p_s[(ty + 8 * a) * AF_BK + tx + 16 * b] = p;
+                }
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                l[a] = l[a] * corr + sum;
+                m[a] = top;
+                const unsigned long long c2 = af_pack(corr, corr), zero = 0ull;
+#pragma unroll
+                for (int h = 0; h < HDV; h++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        unsigned long long v = zero;
+                        af_fma2(v, acc[a][h][e], c2);
+                        acc[a][h][e] = v;
+                    }
+            }
+        }
+        af_wait_older();
+        __syncthreads();          // this turn's values and weights are there
+        if (few) {
+#pragma unroll
+            for (int h = 0; h < (HDV + 1) / 2; h++) {
+                const int d = tid + 128 * h;
+#pragma unroll
+                for (int a = 0; a < 4; a++) acc1[a][h] *= row_s[0][a];
+                if (d < hd) {
+#pragma unroll 8
+                    for (int j = 0; j < AF_BK; j++) {
+                        const float4 p = *reinterpret_cast<const float4*>(p_s + j * 4);
+                        const float v = v_s[j * hdp + d];
+                        if (p.x != 0.f) acc1[0][h] = fmaf(p.x, v, acc1[0][h]);
+                        if (p.y != 0.f) acc1[1][h] = fmaf(p.y, v, acc1[1][h]);
+                        if (p.z != 0.f) acc1[2][h] = fmaf(p.z, v, acc1[2][h]);
+                        if (p.w != 0.f) acc1[3][h] = fmaf(p.w, v, acc1[3][h]);
+                    }
+                }
+            }
+        } else {
+            // (a key that a row does not see adds nothing, whatever its value holds, since an infinity times zero is no zero:
+            // where a turn has such keys its weights are looked at one by one)
+            if (kv0 + AF_BK <= seen_by_all && kv0 >= seen_from) sum_values<HDV, false>(p_s, v_s, hdp, chunks, tx, ty, acc);
+            else sum_values<HDV, true>(p_s, v_s, hdp, chunks, tx, ty, acc);
+        }
+        __syncthreads();          // the values and weights have been read
+        if (t + 1 < turns) load(t + 1, v_s, v_pool, false); else af_commit();
+    }
+    if (few) {
+        if (lane == 0) { row_s[0][warp] = m[0]; row_s[1][warp] = l[0]; }
+        __syncthreads();
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+            if (a >= rows) break;
+            const float sum = row_s[1][a], inv = w.part_slot >= 0 ? 1.f : sum > 0.f ? 1.0f / sum : 0.f;
+            const size_t pr = (size_t)((w.part_slot >= 0 ? w.part_slot : w.q_token0) + my_tok[a]) * nh + my_head[a];
+            float* o = (w.part_slot >= 0 ? part_o : out) + pr * hd;
+#pragma unroll
+            for (int h = 0; h < (HDV + 1) / 2; h++)
+                if (tid + 128 * h < hd) o[tid + 128 * h] = acc1[a][h] * inv;
+            if (w.part_slot >= 0 && tid == 0) { part_ml[pr * 2] = row_s[0][a]; part_ml[pr * 2 + 1] = sum; }
+        }
+        return;
+    }
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        if (ty + 8 * a >= rows) continue;
+        const float inv = w.part_slot >= 0 ? 1.f : l[a] > 0.f ? 1.0f / l[a] : 0.f;
+        const size_t pr = (size_t)((w.part_slot >= 0 ? w.part_slot : w.q_token0) + my_tok[a]) * nh + my_head[a];
+        float* o = (w.part_slot >= 0 ? part_o : out) + pr * hd;
+#pragma unroll
+        for (int h = 0; h < HDV; h++)
+            if (tx + 16 * h < chunks) {
+                float* to = o + (tx + 16 * h) * 4;
+                to[0] = af_lo(acc[a][h][0]) * inv; to[1] = af_hi(acc[a][h][0]) * inv;
+                to[2] = af_lo(acc[a][h][1]) * inv; to[3] = af_hi(acc[a][h][1]) * inv;
+            }
+        if (w.part_slot >= 0 && tx == 0) { part_ml[pr * 2] = m[a]; part_ml[pr * 2 + 1] = l[a]; }
+    }
+}
+
 // Combine the splits of a token: for entry t,
 // red[t] = {token, first, count, stride}: its parts are first + s * stride, s < count.
 // One CTA per (entry, head), RED_GROUPS groups of hd threads.  The weights exp(m_s - M) are
@@ -282,26 +603,42 @@ PLLM_EXPORT int pllm_attention_generic(int dtype, const void* q, const void* k_p
     if (nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0) return PLLM_ERR_SIZE;
     if (hd <= 0 || hd > ATT_MAX_HD || hd % 8 != 0) return PLLM_ERR_SIZE;
     const int group = nh / nkv;
+    if (dtype == PLLM_F32) {
+        if (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) return PLLM_ERR_ALIGN;
+        const int gparts = (group + AF_HEADS - 1) / AF_HEADS, hdp = (hd + 31) & ~31;
+        const size_t smem = ((size_t)(AF_ROWS + 2 * AF_BK) * hdp + AF_ROWS * AF_BK) * sizeof(float);
+        auto* kernel = hd <= 64 ? attention_f32_kernel<1> : hd <= 128 ? attention_f32_kernel<2> : attention_f32_kernel<4>;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch_chained(kernel, dim3((unsigned)max_work * nkv * gparts), dim3(AF_THREADS), smem, stream, (const float*)q, (const float*)k_pool,
+                       (const float*)v_pool, block_tables, (const AttnWork*)work, n_work_ptr, (float*)out, part_o, part_ml, nh, nkv, hd,
+                       page_size, n_pages, table_width, window, scale, status);
+        return launch_status();
+    }
+    if (dtype != PLLM_BF16) return PLLM_ERR_DTYPE;
     const int heads_per_cta = group < ATT_MAX_ROWS ? group : ATT_MAX_ROWS;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
     const size_t smem = ((size_t)ATT_MAX_ROWS * hd + 2 * (size_t)ATT_BK * (hd + 4)) * sizeof(float);
-    PLLM_DISPATCH_DTYPE(dtype, {
-        cudaFuncSetAttribute(attention_generic_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dim3 grid(max_work, nkv * gparts);
-        launch_chained(attention_generic_kernel<T>, grid, dim3(ATT_MAX_ROWS * 32), smem, stream,
-                       (const T*)q, (const T*)k_pool, (const T*)v_pool, block_tables, (const AttnWork*)work, n_work_ptr,
-                       (T*)out, part_o, part_ml, nh, nkv, hd, page_size, n_pages, table_width, window, scale,
-                       heads_per_cta, status);
-    });
+    typedef bf16 T;
+    cudaFuncSetAttribute(attention_generic_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_chained(attention_generic_kernel<T>, dim3(max_work, nkv * gparts), dim3(ATT_MAX_ROWS * 32), smem, stream,
+                   (const T*)q, (const T*)k_pool, (const T*)v_pool, block_tables, (const AttnWork*)work, n_work_ptr,
+                   (T*)out, part_o, part_ml, nh, nkv, hd, page_size, n_pages, table_width, window, scale,
+                   heads_per_cta, status);
     return launch_status();
 }
 
 // The most query tokens one work item may hold for a given group size, so that
-// the host cuts tiles the kernel accepts.
-PLLM_EXPORT int pllm_attention_generic_tile_tokens(int nh, int nkv) {
+// the host cuts tiles the kernel accepts; and the CTAs that share an item.
+PLLM_EXPORT int pllm_attention_generic_tile_tokens(int dtype, int nh, int nkv) {
     const int group = nh / nkv;
+    if (dtype == PLLM_F32) return AF_ROWS / (group < AF_HEADS ? group : AF_HEADS);
     const int heads_per_cta = group < ATT_MAX_ROWS ? group : ATT_MAX_ROWS;
     return ATT_MAX_ROWS / heads_per_cta;
+}
+
+PLLM_EXPORT int pllm_attention_generic_ctas_per_item(int dtype, int nh, int nkv) {
+    const int heads = dtype == PLLM_F32 ? AF_HEADS : ATT_MAX_ROWS;
+    return nkv * ((nh / nkv + heads - 1) / heads);
 }
 
 // many_splits: the entries have eight splits or more each (a step of very few tokens): four groups of

@@ -213,11 +213,11 @@ static inline void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
-// The same with the CTAs of `cluster_y` consecutive blockIdx.y in one thread-block cluster (they
+// The same with the CTAs of `cluster.y` x `cluster.z` consecutive blockIdx.y and .z in one thread-block cluster (they
 // run at the same time on neighbouring SMs and may read one another's shared memory).
 template <typename... KArgs, typename... Args>
-static inline void launch_chained_cluster_y(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                            int cluster_y, Args... args) {
+static inline void launch_chained_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                          dim3 cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -225,14 +225,19 @@ static inline void launch_chained_cluster_y(void (*kernel)(KArgs...), dim3 grid,
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = (unsigned)cluster_y;
-    attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = cluster.x;
+    attr[0].val.clusterDim.y = cluster.y;
+    attr[0].val.clusterDim.z = cluster.z;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pllm_pdl_enabled ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline void launch_chained_cluster_y(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                            int cluster_y, Args... args) {
+    launch_chained_cluster(kernel, grid, block, smem, stream, dim3(1, (unsigned)cluster_y, 1), args...);
 }
 
 #define PLLM_DISPATCH_DTYPE(dtype, ...)                         \

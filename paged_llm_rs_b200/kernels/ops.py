@@ -43,7 +43,8 @@ def lib():
                                      c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, P],
             "pllm_attention_generic": [c_int, P, P, P, P, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int,
                                        c_int, c_int, c_int, c_float, P, P],
-            "pllm_attention_generic_tile_tokens": [c_int, c_int],
+            "pllm_attention_generic_tile_tokens": [c_int, c_int, c_int],
+            "pllm_attention_generic_ctas_per_item": [c_int, c_int, c_int],
             "pllm_attention_reduce": [c_int, P, P, P, P, c_int, P, c_int, c_int, c_int, P],
             "pllm_sample": [P, c_int, c_int, c_ll, P, P, P, P, P],
             "pllm_sample_scratch_floats": [c_int, c_int],
@@ -68,6 +69,8 @@ def lib():
         sig["pllm_attention_prefill_tcgen05"] = [P] * 10 + [c_int] * 7 + [c_float, c_int, P, P]
         sig["pllm_gemm_tcgen05_supports"] = [c_int, c_int, c_int, c_int]
         sig["pllm_gemm_tcgen05"] = [P, P, P, c_int, c_int, c_int, c_int, c_float, P, P]
+        sig["pllm_gemm_f32_supports"] = [c_int, c_int, c_int]
+        sig["pllm_gemm_f32"] = [P, P, P, c_int, c_int, c_int, c_int, c_int, P]
         sig["pllm_rows_gemm_supports"] = [c_int, c_int, c_int]
         sig["pllm_rows_gemm"] = [P, P, P, c_int, c_int, c_int, c_int, c_float, c_int, c_int, P, P]
         sig["pllm_embed_scaled32"] = [c_int, P, P, P, c_int, c_int, c_int, c_float, P, P]
@@ -343,7 +346,12 @@ def attention_tile_tokens(num_heads: int, num_kv_heads: int, dtype: torch.dtype 
         return lib().pllm_attention_prefill_tcgen05_tile_tokens(num_heads, num_kv_heads)
     if attention_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim):
         return lib().pllm_attention_mma_tile_tokens(num_heads, num_kv_heads)
-    return lib().pllm_attention_generic_tile_tokens(num_heads, num_kv_heads)
+    return lib().pllm_attention_generic_tile_tokens(_code_of(dtype), num_heads, num_kv_heads)
+
+
+def attention_ctas_per_item(num_heads: int, num_kv_heads: int, dtype: torch.dtype) -> int:
+    """CTAs that paged_attention launches for one work item: one for every kv head and every 16 query heads of its group (float32: every 4)."""
+    return lib().pllm_attention_generic_ctas_per_item(_code_of(dtype), num_heads, num_kv_heads)
 
 
 # PAGED_LLM_MIXED_BESIDE=0: in a step of decoded tokens beside prompt portions the tcgen05 kernel takes the
@@ -638,6 +646,47 @@ def rows_gemm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
     return out
 
 
+# True float32 products on the CUDA cores (csrc/gemm_f32.cu) where the library's tiles leave most of the chip idle.
+# Measured back to back on a B200 (us, this kernel / cuBLAS):
+#   rows        4            8            16           32           64           256
+#   4096 x 1024 11.6 / 14.2  11.7 / 27.2  11.8 / 27.3  12.4 / 27.7  21.1 / 28.0  70.5 / 45.4
+#   1024 x 2048 13.0 / 14.6  13.1 / 19.5  12.6 / 20.4  13.2 / 20.1  20.5 / 51.1  36.6 / 47.7   (512: 69.0 / 57.4)
+#   6144 x 1024 12.2 / 15.4  12.4 / 27.4  12.7 / 27.6  24.3 / 28.3  42.3 / 33.8  119 / 73.5
+#   151936 x 1024 182 / 193  185 / 203    188 / 241    320 / 249
+# so it takes 4 to 16 rows, up to 32 but for the widest, and more while the product has 64 tiles of 64 x 64 at most.
+F32_GEMM = True
+F32_MIN_M = 4
+F32_MAX_TILES = 64
+F32_MIN_WEIGHTS = 1 << 18       # (a product of a tiny model's is a launch and nothing else)
+
+
+def gemm_f32_takes(x, weight: torch.Tensor, want: Optional[torch.dtype] = None) -> bool:
+    """Whether ``linear`` runs this library's float32 product (csrc/gemm_f32.cu)."""
+    if not F32_GEMM or x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2 or not x.is_contiguous() \
+            or not weight.is_contiguous() or want not in (None, torch.float32) or (x.data_ptr() | weight.data_ptr()) & 15:
+        return False
+    M, N = x.shape[0], weight.shape[0]
+    if M < F32_MIN_M or weight.numel() < F32_MIN_WEIGHTS or (M > 32 and -(-M // 64) * -(-N // 64) > F32_MAX_TILES) or (M > 16 and N > SKINNY_MAX_N):
+        return False
+    return bool(lib().pllm_gemm_f32_supports(M, *weight.shape))
+
+
+def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, tile: int = 0, splits: int = 0) -> torch.Tensor:
+    """x W^T in float32 on the CUDA cores.  ``tile``: rows of x a tile (16, 32, 128), ``splits``: CTAs that share the sum
+    over k (0: as the sizes ask)."""
+    M, K = x.shape
+    N = weight.shape[0]
+    if weight.shape[1] != K or x.dtype != torch.float32 or weight.dtype != torch.float32 or not lib().pllm_gemm_f32_supports(M, N, K):
+        raise KernelError(f"gemm_f32: does not take x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    elif out.shape != (M, N) or out.dtype != torch.float32:
+        raise KernelError("gemm_f32: out does not fit")
+    _dev(x, weight, out)
+    _check(lib().pllm_gemm_f32(_ptr(x), _ptr(weight), _ptr(out), M, N, K, tile, splits, _stream()), "gemm_f32")
+    return out
+
+
 def skinny_glu_takes(x, weight: torch.Tensor, n_out: int) -> bool:
     """Whether the weight-streaming kernel takes the gate/up product with the activation in its epilogue."""
     if not SKINNY_GEMM or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.dim() != 2:
@@ -681,6 +730,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         _check(lib().pllm_skinny_gemm(_ptr(x), _ptr(weight), _ptr(out), M, N, K,
                                       1 if want == torch.float32 else 0, _stream()), "skinny_gemm")
         return out
+    if gemm_f32_takes(x, weight, want) and (out is None or out.is_contiguous()):
+        return gemm_f32(x, weight, out)
     if TCGEN05_GEMM >= 2 and out is None and want == torch.bfloat16 and x.shape[0] >= TCGEN05_MIN_M \
             and gemm_tcgen05_takes(x, weight, N, False):
         return gemm_tcgen05(x, weight, status=status)

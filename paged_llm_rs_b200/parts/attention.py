@@ -65,10 +65,8 @@ class GQAttention(Mixer):
         return self._need
 
     def plan_wish(self, page_size: int):
-        group = self.nh // self.nkv
         tile = ops.attention_tile_tokens(self.nh, self.nkv, self.rt.dtype, self.hd, page_size, self.window or 0)
-        # CTAs an item: one for every kv head and every 16 query heads of its group
-        return PlanWish(tile, self.nkv * -(-group // 16), self.nh, self.hd)
+        return PlanWish(tile, ops.attention_ctas_per_item(self.nh, self.nkv, self.rt.dtype), self.nh, self.hd)
 
     def forward(self, x, step, cache, writes_cache=True):
         k_pool, v_pool, gi = cache
