@@ -22,10 +22,12 @@
 // cut only by the rounding of the delta rule's pairs of tokens.  Other threads of the CTA fetch the tokens ahead of the
 // recurrence.
 #include "matrix_memory.cuh"
+#include "delta_blocks.cuh"
+#include "mlstm_blocks.cuh"
 
 #define MM_CHUNK 32            // tokens fetched at a time (fewer where keys are so long that shared memory would not hold them)
 #define MM_CHUNK_SMALL 8       // ... in a step of decoded tokens
-#define MM_CONV_TOKENS 64      // tokens a CTA of the convolution
+#define MM_CONV_TOKENS 32      // tokens a CTA of the convolution
 #define MM_MAX_TAPS 16
 
 __device__ __forceinline__ float mm_parts_sum(float v, int parts) {
@@ -47,7 +49,9 @@ __device__ __forceinline__ void mm_parts_sum2(float& a, float& b, int parts) {
 
 // grid (segments, channel blocks of 128, token chunks); u: [tokens, u_width] with the channels at u_off; conv_w [channels, taps],
 // the last tap meets the current token.
-template <typename T>
+// TAPS: taps rounded up (4 or MM_MAX_TAPS).
+#define MM_CONV_RUN 8
+template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) mm_conv_silu_kernel(const T* u, int u_width, int u_off, const T* __restrict__ conv_w,
                                                            const MMSegment* __restrict__ segs, const float* state, long long state_stride,
                                                            long long conv_off, float* __restrict__ c_out, int channels, int taps) {
@@ -58,23 +62,36 @@ __global__ void __launch_bounds__(128) mm_conv_silu_kernel(const T* u, int u_wid
     if (t0 >= s.count) return;
     const int ch = blockIdx.y * 128 + threadIdx.x;
     if (ch >= channels) return;
-    float wt[MM_MAX_TAPS];
+    float wt[TAPS];
 #pragma unroll
-    for (int j = 0; j < MM_MAX_TAPS; j++) wt[j] = j < taps ? to_f32(conv_w[(size_t)ch * taps + j]) : 0.f;
+    for (int j = 0; j < TAPS; j++) wt[j] = j < taps ? to_f32(conv_w[(size_t)ch * taps + j]) : 0.f;
     const float* st = state + (size_t)s.slot * state_stride + conv_off;       // [taps - 1][channels], oldest first
-    const int t1 = min(s.count, t0 + MM_CONV_TOKENS);
-    for (int t = t0; t < t1; t++) {
-        float acc = 0.f;
+    const T* uc = u + (size_t)s.first * u_width + u_off + ch;
+    // the last taps - 1 inputs stay in registers, so that a token costs one load, and eight tokens' loads leave together
+    float win[TAPS - 1];
 #pragma unroll
-        for (int j = 0; j < MM_MAX_TAPS; j++) {
-            if (j >= taps) break;
-            const int r = t - (taps - 1) + j;              // relative to the segment's first token
-            float v;
-            if (r >= 0) v = to_f32(u[(size_t)(s.first + r) * u_width + u_off + ch]);
-            else v = s.before > 0 ? st[(size_t)(taps - 1 + r) * channels + ch] : 0.f;
-            acc = fmaf(wt[j], v, acc);
+    for (int j = 0; j < TAPS - 1; j++) {
+        const int r = t0 - (taps - 1) + j;                 // relative to the segment's first token
+        win[j] = j >= taps - 1 ? 0.f : r >= 0 ? to_f32(uc[(size_t)r * u_width]) : s.before > 0 ? st[(size_t)(taps - 1 + r) * channels + ch] : 0.f;
+    }
+    const int t1 = min(s.count, t0 + MM_CONV_TOKENS);
+    for (int t = t0; t < t1; t += MM_CONV_RUN) {
+        float next[MM_CONV_RUN];
+#pragma unroll
+        for (int j = 0; j < MM_CONV_RUN; j++) next[j] = t + j < t1 ? to_f32(uc[(size_t)(t + j) * u_width]) : 0.f;
+#pragma unroll
+        for (int j = 0; j < MM_CONV_RUN; j++) {
+            float acc = 0.f;
+#pragma unroll
+            for (int k = 0; k < TAPS - 1; k++)
+                if (k < taps - 1) acc = fmaf(wt[k], win[k], acc);
+#pragma unroll
+            for (int k = 0; k < TAPS; k++)
+                if (k == taps - 1) acc = fmaf(wt[k], next[j], acc);
+            if (t + j < t1) c_out[(size_t)(s.first + t + j) * channels + ch] = mm_silu(acc);
+#pragma unroll
+            for (int k = 0; k < TAPS - 1; k++) win[k] = k + 1 < taps - 1 ? win[k + 1 < TAPS - 1 ? k + 1 : k] : k + 1 == taps - 1 ? next[j] : 0.f;
         }
-        c_out[(size_t)(s.first + t) * channels + ch] = mm_silu(acc);
     }
 }
 
@@ -98,7 +115,7 @@ __global__ void __launch_bounds__(256, MINB) delta_scan_kernel(const float* __re
                                                          int u_width, int conv_in_off, const float* __restrict__ a_log,
                                                          const float* __restrict__ dt_bias, const MMSegment* __restrict__ segs, float* state,
                                                          long long state_stride, long long conv_off, float* __restrict__ y, int H, int G,
-                                                         int d, int E, int Ps, int parts, int taps, int ck, int workers, int loaders) {
+                                                         int d, int E, int Ps, int parts, int taps, int ck, int workers, int loaders, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     const int NP = NPT * parts;
     // a buffer: q [ck][NP] | k [ck][NP] | v [ck][Ps] | decay [ck] | beta [ck] | k . q [ck] | k . next k [ck] | k . next q [ck]
@@ -106,7 +123,7 @@ __global__ void __launch_bounds__(256, MINB) delta_scan_kernel(const float* __re
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
     const MMSegment s = segs[blockIdx.x];
-    if (s.count <= 0) return;
+    if (s.count <= 0 || s.count > longest) return;      // (longer segments: delta_blocks.cuh)
     const int h = blockIdx.y, kh = h / (H / G), p0 = blockIdx.z * Ps;
     const bool loader = (int)threadIdx.x >= workers;
     const int ltid = (int)threadIdx.x - workers;
@@ -319,7 +336,7 @@ __global__ void __launch_bounds__(MM_SCAN_THREADS, 1) mlstm_scan_kernel(const T*
                                                                     float cap, const MMSegment* __restrict__ segs, float* state,
                                                                     long long state_stride, float* __restrict__ nm_buf,
                                                                     float* __restrict__ y, float* __restrict__ dn, int H, int d, int E,
-                                                                    int Ps, int parts, int ck) {
+                                                                    int Ps, int parts, int ck, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     constexpr int VEC = MMVec<T>::N;
     const int NP = NPT * parts, C = Ps + 1;
@@ -329,7 +346,7 @@ __global__ void __launch_bounds__(MM_SCAN_THREADS, 1) mlstm_scan_kernel(const T*
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
     const MMSegment s = segs[blockIdx.x];
-    if (s.count <= 0) return;
+    if (s.count <= 0 || s.count > longest) return;      // (longer segments: mlstm_blocks.cuh)
     const int h = blockIdx.y, p0 = blockIdx.z * Ps;
     const int tid = threadIdx.x;
     const int main_threads = Ps * parts, fetch0 = (int)blockDim.x - MM_FETCHERS, side0 = fetch0 - 32;
@@ -495,7 +512,7 @@ __global__ void __launch_bounds__(MM_STEP_THREADS) mlstm_step_kernel(const T* __
                                                                     float cap, const MMSegment* __restrict__ segs, float* state,
                                                                     long long state_stride, float* __restrict__ nm_buf,
                                                                     float* __restrict__ y, float* __restrict__ dn, int H, int d, int E,
-                                                                    int Ps, int parts, int ck) {
+                                                                    int Ps, int parts, int ck, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     constexpr int VEC = MMVec<T>::N;
     const int NP = NPT * parts, C = Ps + 1;
@@ -507,7 +524,7 @@ __global__ void __launch_bounds__(MM_STEP_THREADS) mlstm_step_kernel(const T* __
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
     const MMSegment s = segs[blockIdx.x];
-    if (s.count <= 0) return;
+    if (s.count <= 0 || s.count > longest) return;      // (longer segments: mlstm_blocks.cuh)
     const int h = blockIdx.y, p0 = blockIdx.z * Ps;
     const int tid = threadIdx.x, lane = tid & 31;
     const int main_threads = Ps * parts, side0 = (int)blockDim.x - 32;
@@ -627,11 +644,11 @@ __global__ void __launch_bounds__(MM_STEP_THREADS) mlstm_step_kernel(const T* __
 
 // grid (segments, heads): a head's new normaliser and running maximum from the step's scratch into the request's slot.
 __global__ void __launch_bounds__(128) mlstm_store_nm_kernel(const float* __restrict__ nm_buf, const MMSegment* __restrict__ segs,
-                                                             float* state, long long state_stride, int H, int d, int E) {
+                                                             float* state, long long state_stride, int H, int d, int E, int longest) {
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
     const MMSegment s = segs[blockIdx.x];
-    if (s.count <= 0) return;
+    if (s.count <= 0 || s.count > longest) return;      // (longer segments: mlstm_blocks.cuh)
     const int h = blockIdx.y;
     const float* nm = nm_buf + ((size_t)blockIdx.x * H + h) * (d + 1);
     float* slot = state + (size_t)s.slot * state_stride;
@@ -699,6 +716,13 @@ static inline int mlstm_shape(int n_segs, int H, int d, int E, int max_segment_t
     else if ((npt) == 16) { constexpr int NPT = 16; CALL; } else { constexpr int NPT = 32; CALL; } } while (0)
 
 PLLM_EXPORT long long pllm_mlstm_state_floats(int H, int d, int E) { return (long long)H * d * E + (long long)H * d + H; }
+// Floats of scratch for a step's longer segments (0: the step has none, or its sizes are the recurrence's).
+PLLM_EXPORT long long pllm_mlstm_block_floats(const void* u, int u_width, int n_tokens, int n_segs, int max_segment_tokens, int H, int d, int E) {
+    return mb_takes(u, u_width, d, E, max_segment_tokens) ? mb_floats(n_tokens, n_segs, H, d, E) : 0;
+}
+PLLM_EXPORT long long pllm_delta_block_floats(int n_tokens, int n_segs, int max_segment_tokens, int H, int G, int d, int E) {
+    return db_takes(2 * G * d + H * E, d, E, max_segment_tokens) ? db_floats(n_tokens, n_segs, H, d, E) : 0;
+}
 PLLM_EXPORT long long pllm_delta_state_floats(int H, int G, int d, int E, int taps) {
     return (long long)H * d * E + (long long)(taps - 1) * (2 * G * d + H * E);
 }
@@ -706,13 +730,18 @@ PLLM_EXPORT long long pllm_delta_state_floats(int H, int G, int d, int E, int ta
 // u: [tokens, u_width] of the compute dtype: q (H d) | k (H d) | v (H e) | gate (H e); gates: [tokens, 2 H] float, i_raw | f_raw;
 // gain: H e floats; nm_buf: [n_segs, H, d + 1], dn_buf: [tokens, H, 2] and y_buf: [tokens, H e] float scratch (rows of no
 // segment zero in the last two); out: [tokens, H e] of the compute dtype.  max_segment_tokens bounds a segment's tokens (0: unknown).
+// block_buf: pllm_mlstm_block_floats floats (null: every segment token by token).
 PLLM_EXPORT int pllm_mlstm_mix(int dtype, const void* u, int u_width, const float* gates, const float* i_bias, const float* f_bias,
                                float cap, const float* gain, const int* segs, int n_segs, int max_segment_tokens, float* state,
-                               long long state_stride, float* nm_buf, float* dn_buf, float* y_buf, void* out, int n_tokens, int H, int d,
-                               int E, float eps, cudaStream_t stream) {
+                               long long state_stride, float* nm_buf, float* dn_buf, float* y_buf, float* block_buf, long long block_floats,
+                               void* out, int n_tokens, int H, int d, int E, float eps, cudaStream_t stream) {
     if (n_tokens <= 0 || n_segs <= 0) return PLLM_OK;
     if (H <= 0 || d <= 0 || E <= 0 || !(cap > 0.f) || u_width < 2 * H * d + 2 * H * E) return PLLM_ERR_SIZE;
     if (state_stride < pllm_mlstm_state_floats(H, d, E)) return PLLM_ERR_SIZE;
+    // segments of more than MB_L tokens in blocks where the sizes allow it and the scratch for it was given
+    const bool blocks = block_buf != nullptr && mb_takes(u, u_width, d, E, max_segment_tokens);
+    if (blocks && (block_floats < mb_floats(n_tokens, n_segs, H, d, E) || ((uintptr_t)block_buf & 15))) return PLLM_ERR_SIZE;
+    const int longest = blocks ? MB_L : 0x7fffffff;
     MMShape sh;
     const int rc = mlstm_shape(n_segs, H, d, E, max_segment_tokens, &sh);
     if (rc != PLLM_OK) return rc;
@@ -722,11 +751,14 @@ PLLM_EXPORT int pllm_mlstm_mix(int dtype, const void* u, int u_width, const floa
             if (sh.smem > 48 * 1024) cudaFuncSetAttribute(KERNEL<T, NPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem); \
             launch_chained(KERNEL<T, NPT>, dim3(n_segs, H, sh.slices), dim3(sh.threads), sh.smem, stream, (const T*)u, u_width, \
                            gates, i_bias, f_bias, cap, (const MMSegment*)segs, state, state_stride, nm_buf, y_buf, dn_buf, H, d, E, sh.Ps, \
-                           sh.parts, sh.chunk); } while (0)
+                           sh.parts, sh.chunk, longest); } while (0)
             if (sh.threads == sh.workers + 32) MM_MLSTM_SCAN(mlstm_step_kernel); else MM_MLSTM_SCAN(mlstm_scan_kernel);
         });
         launch_chained(mlstm_store_nm_kernel, dim3(n_segs, H), dim3(128), 0, stream, (const float*)nm_buf, (const MMSegment*)segs, state,
-                       state_stride, H, d, E);
+                       state_stride, H, d, E, longest);
+        if (blocks)
+            launch_mlstm_blocks<T>((const T*)u, u_width, gates, i_bias, f_bias, cap, (const MMSegment*)segs, n_segs, state, state_stride,
+                                   mb_buffers(block_buf, n_tokens, n_segs, H, d, E), y_buf, dn_buf, n_tokens, H, d, E, stream);
         launch_head_norm_gate<T>(y_buf, dn_buf, (const T*)u + 2 * H * d + H * E, u_width, gain, out, n_tokens, H, E, 1, 0, eps, stream);
     });
     return launch_status();
@@ -735,33 +767,46 @@ PLLM_EXPORT int pllm_mlstm_mix(int dtype, const void* u, int u_width, const floa
 // u: [tokens, u_width] of the compute dtype: q (G d) | k (G d) | v (H e) | gate (H e); conv_w: [2 G d + H e, taps] of the same;
 // ba: [tokens, 2 H] float, b_raw | a_raw; a_log, dt_bias: H floats; gain: e floats; c_buf [tokens, 2 G d + H e] and
 // y_buf [tokens, H e] float scratch; out: [tokens, H e] of the compute dtype.
+// block_buf: pllm_delta_block_floats floats (null: every segment token by token).
 PLLM_EXPORT int pllm_delta_mix(int dtype, const void* u, int u_width, const void* conv_w, const float* ba, const float* a_log,
                                const float* dt_bias, const float* gain, const int* segs, int n_segs, int max_segment_tokens,
-                               float* state, long long state_stride, float* c_buf, float* y_buf, void* out, int n_tokens, int H, int G,
-                               int d, int E, int taps, float eps, cudaStream_t stream) {
+                               float* state, long long state_stride, float* c_buf, float* y_buf, float* block_buf, long long block_floats, void* out,
+                               int n_tokens, int H, int G, int d, int E, int taps, float eps, cudaStream_t stream) {
     if (n_tokens <= 0 || n_segs <= 0) return PLLM_OK;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || E <= 0 || taps < 1) return PLLM_ERR_SIZE;
     if (taps > MM_MAX_TAPS) return PLLM_ERR_LIMIT;
     const int channels = 2 * G * d + H * E;
     if (u_width < channels + H * E || state_stride < pllm_delta_state_floats(H, G, d, E, taps)) return PLLM_ERR_SIZE;
     const long long conv_off = (long long)H * d * E;
+    // segments of more than DB_L tokens in blocks where the sizes allow it and the scratch for it was given
+    const bool blocks = block_buf != nullptr && db_takes(channels, d, E, max_segment_tokens);
+    if (blocks && (block_floats < db_floats(n_tokens, n_segs, H, d, E) || (((uintptr_t)block_buf | (uintptr_t)c_buf | (uintptr_t)y_buf) & 15)))
+        return PLLM_ERR_SIZE;
+    const int longest = blocks ? DB_L : 0x7fffffff;
     MMShape sh;
     const int rc = mm_shape(n_segs, H, d, E, 5, max_segment_tokens, &sh);
     if (rc != PLLM_OK) return rc;
     const int chunks = (max_segment_tokens + MM_CONV_TOKENS - 1) / MM_CONV_TOKENS;
     PLLM_DISPATCH_DTYPE(dtype, {
-        launch_chained(mm_conv_silu_kernel<T>, dim3(n_segs, (channels + 127) / 128, chunks > 0 ? chunks : 1), dim3(128), 0, stream,
-                       (const T*)u, u_width, 0, (const T*)conv_w, (const MMSegment*)segs, (const float*)state, state_stride, conv_off,
-                       c_buf, channels, taps);
+        const dim3 conv_grid(n_segs, (channels + 127) / 128, chunks > 0 ? chunks : 1);
+        if (taps <= 4)
+            launch_chained(mm_conv_silu_kernel<T, 4>, conv_grid, dim3(128), 0, stream, (const T*)u, u_width, 0, (const T*)conv_w,
+                           (const MMSegment*)segs, (const float*)state, state_stride, conv_off, c_buf, channels, taps);
+        else
+            launch_chained(mm_conv_silu_kernel<T, MM_MAX_TAPS>, conv_grid, dim3(128), 0, stream, (const T*)u, u_width, 0, (const T*)conv_w,
+                           (const MMSegment*)segs, (const float*)state, state_stride, conv_off, c_buf, channels, taps);
 #define MM_DELTA_SCAN(MINB) do { \
             if (sh.smem > 48 * 1024) \
                 cudaFuncSetAttribute(delta_scan_kernel<T, NPT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem); \
             launch_chained(delta_scan_kernel<T, NPT, MINB>, dim3(n_segs, H, sh.slices), dim3(sh.threads), sh.smem, stream, (const float*)c_buf, \
                            channels, ba, (const T*)u, u_width, 0, a_log, dt_bias, (const MMSegment*)segs, state, state_stride, conv_off, \
-                           y_buf, H, G, d, E, sh.Ps, sh.parts, taps, sh.chunk, sh.workers, sh.threads - sh.workers); } while (0)
+                           y_buf, H, G, d, E, sh.Ps, sh.parts, taps, sh.chunk, sh.workers, sh.threads - sh.workers, longest); } while (0)
         MM_NPT_DISPATCH(sh.npt, {
             if (sh.npt <= 16 && (long long)n_segs * H * sh.slices > sm_count()) MM_DELTA_SCAN(2); else MM_DELTA_SCAN(1);
         });
+        if (blocks)
+            launch_delta_blocks<T>((const float*)c_buf, channels, ba, a_log, dt_bias, (const T*)u, u_width, (const MMSegment*)segs, n_segs, state,
+                                   state_stride, conv_off, taps, db_buffers(block_buf, n_tokens, n_segs, H, d, E), y_buf, n_tokens, H, G, d, E, stream);
         launch_head_norm_gate<T>(y_buf, nullptr, (const T*)u + channels, u_width, gain, out, n_tokens, H, E, 0, 1, eps, stream);
     });
     return launch_status();

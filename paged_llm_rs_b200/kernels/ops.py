@@ -115,8 +115,8 @@ def lib():
         sig["pllm_conv_rope_kv_write"] = [c_int, P, c_int, P, P, c_int, P, c_int, c_int, P, c_ll, P, c_int, P, P, P, P] + [c_int] * 6 + [c_ll, P, P]
         sig["pllm_diff_combine"] = [c_int, P, P, c_int, P] + [c_int] * 4 + [c_float] * 3 + [P]
         sig["pllm_latent_rope_write"] = [c_int, P, c_int, P, c_float, P, c_int, P, P, P, P, P, P, P] + [c_int] * 6 + [c_ll, P, P]
-        sig["pllm_mlstm_mix"] = [c_int, P, c_int, P, P, P, c_float, P, P, c_int, c_int, P, c_ll, P, P, P, P] + [c_int] * 4 + [c_float, P]
-        sig["pllm_delta_mix"] = [c_int, P, c_int, P, P, P, P, P, P, c_int, c_int, P, c_ll, P, P, P] + [c_int] * 6 + [c_float, P]
+        sig["pllm_mlstm_mix"] = [c_int, P, c_int, P, P, P, c_float, P, P, c_int, c_int, P, c_ll, P, P, P, P, c_ll, P] + [c_int] * 4 + [c_float, P]
+        sig["pllm_delta_mix"] = [c_int, P, c_int, P, P, P, P, P, P, c_int, c_int, P, c_ll, P, P, P, c_ll, P] + [c_int] * 6 + [c_float, P]
         sig["pllm_gated_sum_norm32"] = [c_int, P, P, c_int, c_float, P, c_int, c_float, P, c_int, P, P, c_int, P, c_int, P, P, P, P, P, P, P, P, P, P, P,
                                         c_int, P, c_ll, P, c_int, c_int, c_float, P]
         sig["pllm_poly_norm"] = [c_int, P, c_int, P, P, c_int, c_int, c_float, P]
@@ -129,7 +129,7 @@ def lib():
                                          P] + [c_int] * 6 + [c_float, P]
         wide = {"pllm_channel_delta_state_floats": [c_int] * 5, "pllm_channel_delta_record_floats": [c_int] * 4,
                 "pllm_linear_attention_state_floats": [c_int] * 3, "pllm_linear_attention_scratch_floats": [c_int] * 6,
-                "pllm_mlstm_state_floats": [c_int] * 3, "pllm_delta_state_floats": [c_int] * 5}
+                "pllm_mlstm_state_floats": [c_int] * 3, "pllm_mlstm_block_floats": [P] + [c_int] * 7, "pllm_delta_block_floats": [c_int] * 7, "pllm_delta_state_floats": [c_int] * 5}
         for name, args in wide.items():
             fn = getattr(L, name)
             fn.argtypes = args
@@ -1375,6 +1375,9 @@ def _segments_ok(segments: torch.Tensor, what: str):
         raise KernelError(f"{what}: segments must be [n, 4]")
 
 
+MLSTM_BLOCKS = True     # (False: every segment token by token, for comparison)
+
+
 def mlstm_mix(u: torch.Tensor, gates: torch.Tensor, i_bias: torch.Tensor, f_bias: torch.Tensor, cap: float, gain: torch.Tensor,
               segments: torch.Tensor, state: torch.Tensor, out: torch.Tensor, heads: int, dim: int, vdim: int, eps: float,
               max_segment_tokens: int = 0) -> torch.Tensor:
@@ -1396,11 +1399,17 @@ def mlstm_mix(u: torch.Tensor, gates: torch.Tensor, i_bias: torch.Tensor, f_bias
     y_buf = torch.zeros((T, heads * vdim), dtype=torch.float32, device=u.device)     # (rows of no segment stay zero)
     dn_buf = torch.zeros((T, heads, 2), dtype=torch.float32, device=u.device)
     nm_buf = torch.empty((segments.shape[0], heads, dim + 1), dtype=torch.float32, device=u.device)
+    # longer segments run in blocks of tokens (csrc/mlstm_blocks.cuh), four kernels more
+    floats = lib().pllm_mlstm_block_floats(_ptr(u), u.shape[1], T, segments.shape[0], int(max_segment_tokens), heads, dim, vdim) if MLSTM_BLOCKS else 0
+    blocks = torch.empty(floats, dtype=torch.float32, device=u.device) if floats else None
     _check(lib().pllm_mlstm_mix(_code(u), _ptr(u), u.shape[1], _ptr(gates), _ptr(i_bias), _ptr(f_bias), float(cap), _ptr(gain),
                                 _ptr(segments), segments.shape[0], int(max_segment_tokens), _ptr(state), state.stride(0), _ptr(nm_buf),
-                                _ptr(dn_buf), _ptr(y_buf), _ptr(out), T, heads, dim, vdim, float(eps), _stream()),
-           "mlstm_mix", launches=3)
+                                _ptr(dn_buf), _ptr(y_buf), _ptr(blocks), floats, _ptr(out), T, heads, dim, vdim, float(eps), _stream()),
+           "mlstm_mix", launches=7 if floats else 3)
     return out
+
+
+DELTA_BLOCKS = True     # (False: every segment token by token, for comparison)
 
 
 def delta_mix(u: torch.Tensor, conv_w: torch.Tensor, ba: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, gain: torch.Tensor,
@@ -1426,10 +1435,13 @@ def delta_mix(u: torch.Tensor, conv_w: torch.Tensor, ba: torch.Tensor, a_log: to
         raise KernelError("delta_mix: the state slots are too small")
     c_buf = torch.empty((T, channels), dtype=torch.float32, device=u.device)
     y_buf = torch.zeros((T, heads * vdim), dtype=torch.float32, device=u.device)     # (rows of no segment stay zero)
+    # longer segments run in blocks of tokens (csrc/delta_blocks.cuh), three kernels more and one for the convolution's state
+    floats = lib().pllm_delta_block_floats(T, segments.shape[0], int(max_segment_tokens), heads, kv_heads, dim, vdim) if DELTA_BLOCKS else 0
+    blocks = torch.empty(floats, dtype=torch.float32, device=u.device) if floats else None
     _check(lib().pllm_delta_mix(_code(u), _ptr(u), u.shape[1], _ptr(conv_w), _ptr(ba), _ptr(a_log), _ptr(dt_bias), _ptr(gain),
                                 _ptr(segments), segments.shape[0], int(max_segment_tokens), _ptr(state), state.stride(0), _ptr(c_buf),
-                                _ptr(y_buf), _ptr(out), T, heads, kv_heads, dim, vdim, taps, float(eps), _stream()),
-           "delta_mix", launches=3)
+                                _ptr(y_buf), _ptr(blocks), floats, _ptr(out), T, heads, kv_heads, dim, vdim, taps, float(eps), _stream()),
+           "delta_mix", launches=3 if not floats else 7 if taps > 1 else 6)
     return out
 
 
