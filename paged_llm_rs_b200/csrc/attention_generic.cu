@@ -43,12 +43,13 @@ __global__ void attention_generic_kernel(
     int heads_per_cta, int* status) {
     pdl_launch_dependents();
     pdl_wait(KID_ATT_GENERIC);
-    if ((int)blockIdx.x >= *n_work_ptr) return;
-    const AttnWork w = work[blockIdx.x];
     const int group = nh / nkv;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
-    const int kh = blockIdx.y / gparts;
-    const int head0 = kh * group + (blockIdx.y % gparts) * heads_per_cta;       // first q head of this CTA
+    const int item = blockIdx.x / (nkv * gparts), cta = blockIdx.x % (nkv * gparts);     // (an item's CTAs are neighbours in the grid)
+    if (item >= *n_work_ptr) return;
+    const AttnWork w = work[item];
+    const int kh = cta / gparts;
+    const int head0 = kh * group + (cta % gparts) * heads_per_cta;       // first q head of this CTA
     const int n_heads = min(heads_per_cta, kh * group + group - head0);
     const int rows = w.q_count * n_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -620,7 +621,7 @@ PLLM_EXPORT int pllm_attention_generic(int dtype, const void* q, const void* k_p
     const size_t smem = ((size_t)ATT_MAX_ROWS * hd + 2 * (size_t)ATT_BK * (hd + 4)) * sizeof(float);
     typedef bf16 T;
     cudaFuncSetAttribute(attention_generic_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_chained(attention_generic_kernel<T>, dim3(max_work, nkv * gparts), dim3(ATT_MAX_ROWS * 32), smem, stream,
+    launch_chained(attention_generic_kernel<T>, dim3((unsigned)max_work * nkv * gparts), dim3(ATT_MAX_ROWS * 32), smem, stream,
                    (const T*)q, (const T*)k_pool, (const T*)v_pool, block_tables, (const AttnWork*)work, n_work_ptr,
                    (T*)out, part_o, part_ml, nh, nkv, hd, page_size, n_pages, table_width, window, scale,
                    heads_per_cta, status);

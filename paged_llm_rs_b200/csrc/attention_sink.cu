@@ -18,6 +18,8 @@
 //                       before it and the sink; splits leave (max, sum, unnormalised output) for attention_reduce.
 //                       Float arithmetic on the CUDA cores, for any sizes: the true 32-bit path.
 //   attention_sink_mma  the same on the tensor cores for bfloat16 and key / value sizes of 32, 64 or 128.
+#include <type_traits>
+
 #include "common.cuh"
 
 enum : int { KID_ATT_SINK = 70 };
@@ -120,12 +122,15 @@ __global__ void attention_sink_kernel(const T* q,                 // [tokens, nh
                                       int* status) {
     pdl_launch_dependents();
     pdl_wait(KID_ATT_SINK);
-    if ((int)blockIdx.x >= *n_work_ptr) return;
-    const SinkWork w = work[blockIdx.x];
+    // (an item's CTAs are neighbours in the grid: with the items running fastest, a step of 74 of them and 8 kv heads dealt every SM
+    // the same item four times, the longest to some and none to others)
     const int group = nh / nkv;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
-    const int kh = blockIdx.y / gparts;
-    const int head0 = kh * group + (blockIdx.y % gparts) * heads_per_cta;
+    const int item = blockIdx.x / (nkv * gparts), cta = blockIdx.x % (nkv * gparts);
+    if (item >= *n_work_ptr) return;
+    const SinkWork w = work[item];
+    const int kh = cta / gparts;
+    const int head0 = kh * group + (cta % gparts) * heads_per_cta;
     const int n_heads = min(heads_per_cta, kh * group + group - head0);
     const int rows = w.q_count * n_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -281,7 +286,7 @@ PLLM_EXPORT int pllm_attention_sink(int dtype, const void* q, const void* kv_poo
     const size_t smem = ((size_t)SINK_MAX_ROWS * dk + (size_t)SINK_BK * (dk + 4) + (size_t)SINK_BK * (dv + 4)) * sizeof(float);
     PLLM_DISPATCH_DTYPE(dtype, {
         cudaFuncSetAttribute(attention_sink_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dim3 grid(max_work, nkv * gparts);
+        dim3 grid((unsigned)max_work * nkv * gparts);
         launch_chained(attention_sink_kernel<T>, grid, dim3(SINK_MAX_ROWS * 32), smem, stream, (const T*)q, (const T*)kv_pool,
                        block_tables, (const SinkWork*)work, n_work_ptr, (T*)out, part_o, part_ml, sinks, nh, nkv, dk, dv, page_size,
                        n_pages, table_width, window, keep_first, chunk, scale, cap, heads_per_cta, status);
@@ -330,7 +335,7 @@ __device__ __forceinline__ uint32_t sink_pack_bf16(float lo, float hi) {
 }
 
 template <int DK, int DV>
-__global__ void __launch_bounds__(128, (DK + DV <= 192) ? 4 : 3) attention_sink_mma_kernel(const bf16* q, const bf16* kv_pool, const int* __restrict__ block_tables,
+__global__ void __launch_bounds__(128, (DK + DV <= 128) ? 4 : 3) attention_sink_mma_kernel(const bf16* q, const bf16* kv_pool, const int* __restrict__ block_tables,
                                                                  const SinkWork* __restrict__ work, const int* __restrict__ n_work_ptr,
                                                                  bf16* __restrict__ out, float* __restrict__ part_o,
                                                                  float* __restrict__ part_ml, const float* __restrict__ sinks, int nh,
@@ -343,12 +348,15 @@ __global__ void __launch_bounds__(128, (DK + DV <= 192) ? 4 : 3) attention_sink_
     constexpr int TILE = SMMA_BK * (KS + VS);                  // a tile's keys [SMMA_BK][KS], then its values [SMMA_BK][VS]; two tiles
     pdl_launch_dependents();
     pdl_wait(KID_ATT_SINK);
-    if ((int)blockIdx.x >= *n_work_ptr) return;
-    const SinkWork w = work[blockIdx.x];
+    // (an item's CTAs are neighbours in the grid: with the items running fastest, a step of 74 of them and 8 kv heads dealt every SM
+    // the same item four times, the longest to some and none to others)
     const int group = nh / nkv;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
-    const int kh = blockIdx.y / gparts;
-    const int head0 = kh * group + (blockIdx.y % gparts) * heads_per_cta;
+    const int item = blockIdx.x / (nkv * gparts), cta = blockIdx.x % (nkv * gparts);
+    if (item >= *n_work_ptr) return;
+    const SinkWork w = work[item];
+    const int kh = cta / gparts;
+    const int head0 = kh * group + (cta % gparts) * heads_per_cta;
     const int n_heads = min(heads_per_cta, kh * group + group - head0);
     const int rows = w.q_count * n_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -392,22 +400,27 @@ __global__ void __launch_bounds__(128, (DK + DV <= 192) ? 4 : 3) attention_sink_
     // The tiles of the item, in order: those of the kept first tokens before its range (first split only), then its range.
     const int r0_end = first_split && window > 0 ? min(keep_first, w.kv_begin) : 0;
     const int n0 = (r0_end + SMMA_BK - 1) / SMMA_BK, n_tiles = n0 + (max(w.kv_end - w.kv_begin, 0) + SMMA_BK - 1) / SMMA_BK;
-    // Tile i + 1 is on its way (cp.async into the other half of the tiles' place) while tile i is multiplied; a row's
-    // page is looked up by the thread that copies it, a tile ahead, so no lookup stands between a tile and its copy.
-    auto issue = [&](int i) {
+    // Tile i + 1 is on its way (cp.async into the other half of the tiles' place) while tile i is multiplied.  Four threads copy a
+    // row, and look its page up a tile ahead of the copy, so that no copy waits for a lookup.
+    constexpr int PASSES = SMMA_BK / 32;
+    int pages[PASSES];
+    auto look = [&](int i) {
         const int kv0 = i < n0 ? i * SMMA_BK : w.kv_begin + (i - n0) * SMMA_BK, r_end = i < n0 ? r0_end : w.kv_end;
+#pragma unroll
+        for (int pass = 0; pass < PASSES; pass++) {
+            const int key = kv0 + pass * 32 + (threadIdx.x >> 2), b = key / page_size;
+            pages[pass] = i < n_tiles && key < r_end && b < table_width ? __ldg(table + b) : -1;
+        }
+    };
+    auto issue = [&](int i) {
+        const int kv0 = i < n0 ? i * SMMA_BK : w.kv_begin + (i - n0) * SMMA_BK;
         bf16* kb = k_s + (i & 1) * TILE, * vb = kb + SMMA_BK * KS;
-        // four threads a row: the row's page is looked up once, then each copies every fourth 16-byte piece of it
         constexpr int CPR = WROW / 8;
 #pragma unroll
-        for (int pass = 0; pass < SMMA_BK / 32; pass++) {
+        for (int pass = 0; pass < PASSES; pass++) {
             const int j = pass * 32 + (threadIdx.x >> 2), q4 = threadIdx.x & 3;
-            int page = -1;
-            if (kv0 + j < r_end) {
-                const int b = (kv0 + j) / page_size;
-                page = b < table_width ? __ldg(table + b) : -1;
-                if (page >= n_pages) { atomicOr(status, 8); page = -1; }
-            }
+            int page = pages[pass];
+            if (page >= n_pages) { atomicOr(status, 8); page = -1; }
             const bf16* src = kv_pool + (((size_t)max(page, 0) * nkv + kh) * page_size + (kv0 + j) % page_size) * WROW;
             bf16* kd = kb + j * KS;
             bf16* vd = vb + j * VS - DK;
@@ -419,13 +432,91 @@ __global__ void __launch_bounds__(128, (DK + DV <= 192) ? 4 : 3) attention_sink_
         }
         asm volatile("cp.async.commit_group;\n" ::);
     };
-    if (n_tiles > 0) issue(0);
+    // A tile's products for this warp: all its keys for the warp's own rows, or (KSPLIT) the warp's sixteen of them.  Two bodies:
+    // with the choice inside one, every load from shared memory would wait behind a branch (1016 tokens beside 8 decoded ones, 16
+    // heads over 8 of 128, values of 64 / 128: 104 / 96 us with one body, 75 / 87 with two and pages looked up ahead, 54 / 61 with
+    // an item's CTAs neighbours in the grid).
+    auto tile = [&](int kv0, int r_end, const bf16* k_t, const bf16* v_t, auto which) {
+        constexpr bool KSPLIT = decltype(which)::value;
+        constexpr int NJ = KSPLIT ? 2 : SMMA_BK / 8;           // groups of eight keys, from key first on
+        const int first = KSPLIT ? warp * 16 : 0;
+        float sc[NJ][4];
+#pragma unroll
+        for (int j = 0; j < NJ; j++) { sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f; }
+#pragma unroll
+        for (int kk = 0; kk < DK / 16; kk++) {
+#pragma unroll
+            for (int j = 0; j < NJ; j += 2) {
+                uint32_t b[4];
+                sink_ldmatrix_x4(b, sink_smem_u32(k_t + (first + j * 8 + (lane & 7) + (lane >> 4) * 8) * KS + kk * 16 + ((lane >> 3) & 1) * 8));
+                sink_mma_bf16(sc[j], qf[kk], b[0], b[1]);
+                sink_mma_bf16(sc[j + 1], qf[kk], b[2], b[3]);
+            }
+        }
+        // scale, cap, mask; the tile's row maxima
+        float tm0 = -CUDART_INF_F, tm1 = -CUDART_INF_F;
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int key = kv0 + first + j * 8 + t4 * 2 + (e & 1);
+                const int pos = e < 2 ? pos0 : pos1;
+                const bool live = e < 2 ? live0 : live1;
+                const bool seen = live && key < r_end && key <= pos && (key >= (e < 2 ? seen0 : seen1) || key < keep_first);
+                float v = sc[j][e] * scale;
+                // tanh(x) = 1 - 2 / (exp(2x) + 1) with the fast exponential and division: its absolute error (1e-7) is far
+                // below what the bfloat16 operands leave in the score
+                if (cap > 0.f) v = cap * (1.0f - __fdividef(2.0f, __expf(2.0f * v * inv_cap) + 1.0f));
+                v = seen ? v : -CUDART_INF_F;
+                sc[j][e] = v;
+                if (e < 2) tm0 = fmaxf(tm0, v); else tm1 = fmaxf(tm1, v);
+            }
+        }
+        tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 1)); tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 2));
+        tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 1)); tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 2));
+        const float mn0 = fmaxf(m0, tm0), mn1 = fmaxf(m1, tm1);
+        const float c0 = mn0 == -CUDART_INF_F ? 1.f : __expf(m0 - mn0), c1 = mn1 == -CUDART_INF_F ? 1.f : __expf(m1 - mn1);
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            sc[j][0] = mn0 == -CUDART_INF_F ? 0.f : __expf(sc[j][0] - mn0);
+            sc[j][1] = mn0 == -CUDART_INF_F ? 0.f : __expf(sc[j][1] - mn0);
+            sc[j][2] = mn1 == -CUDART_INF_F ? 0.f : __expf(sc[j][2] - mn1);
+            sc[j][3] = mn1 == -CUDART_INF_F ? 0.f : __expf(sc[j][3] - mn1);
+            s0 += sc[j][0] + sc[j][1];
+            s1 += sc[j][2] + sc[j][3];
+        }
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 1); s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, 1); s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+        l0 = l0 * c0 + s0; l1 = l1 * c1 + s1;
+        m0 = mn0; m1 = mn1;
+#pragma unroll
+        for (int j = 0; j < DV / 8; j++) { o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1; }
+        // O += P V
+#pragma unroll
+        for (int kk = 0; kk < NJ / 2; kk++) {
+            uint32_t a[4];
+            a[0] = sink_pack_bf16(sc[2 * kk][0], sc[2 * kk][1]);
+            a[1] = sink_pack_bf16(sc[2 * kk][2], sc[2 * kk][3]);
+            a[2] = sink_pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
+            a[3] = sink_pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]);
+#pragma unroll
+            for (int j = 0; j < DV / 8; j += 2) {
+                uint32_t b[4];
+                sink_ldmatrix_x4_trans(b, sink_smem_u32(v_t + (first + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VS + j * 8 + (lane >> 4) * 8));
+                sink_mma_bf16(o[j], a, b[0], b[1]);
+                sink_mma_bf16(o[j + 1], a, b[2], b[3]);
+            }
+        }
+    };
+    if (n_tiles > 0) { look(0); issue(0); look(1); }
     for (int i = 0; i < n_tiles; i++) {
         const int kv0 = i < n0 ? i * SMMA_BK : w.kv_begin + (i - n0) * SMMA_BK, r_end = i < n0 ? r0_end : w.kv_end;
         const bf16* k_t = k_s + (i & 1) * TILE;
         const bf16* v_t = k_t + SMMA_BK * KS;
         if (i + 1 < n_tiles) {
             issue(i + 1);
+            look(i + 2);
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -438,78 +529,8 @@ __global__ void __launch_bounds__(128, (DK + DV <= 192) ? 4 : 3) attention_sink_
             bool any = warp_live && t_lo <= wpos_hi && t_lo < r_end;
             if (any) any = t_hi >= wseen_lo || t_lo < keep_first;
             if (any) {
-                float sc[SMMA_BK / 8][4];
-#pragma unroll
-                for (int j = 0; j < SMMA_BK / 8; j++) { sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f; }
-#pragma unroll
-                for (int kk = 0; kk < DK / 16; kk++) {
-#pragma unroll
-                    for (int j = 0; j < SMMA_BK / 8; j += 2) {
-                        if (ksplit && j != 2 * warp) continue;
-                        uint32_t b[4];
-                        sink_ldmatrix_x4(b, sink_smem_u32(k_t + (j * 8 + (lane & 7) + (lane >> 4) * 8) * KS + kk * 16 + ((lane >> 3) & 1) * 8));
-                        sink_mma_bf16(sc[j], qf[kk], b[0], b[1]);
-                        sink_mma_bf16(sc[j + 1], qf[kk], b[2], b[3]);
-                    }
-                }
-                // scale, cap, mask; the tile's row maxima
-                float tm0 = -CUDART_INF_F, tm1 = -CUDART_INF_F;
-#pragma unroll
-                for (int j = 0; j < SMMA_BK / 8; j++) {
-                    if (ksplit && (j >> 1) != warp) continue;          // (another warp's keys: left out of everything below)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const int key = kv0 + j * 8 + t4 * 2 + (e & 1);
-                        const int pos = e < 2 ? pos0 : pos1;
-                        const bool live = e < 2 ? live0 : live1;
-                        const bool seen = live && key < r_end && key <= pos && (key >= (e < 2 ? seen0 : seen1) || key < keep_first);
-                        float v = sc[j][e] * scale;
-                        // tanh(x) = 1 - 2 / (exp(2x) + 1) with the fast exponential and division: its absolute error (1e-7) is far
-                        // below what the bfloat16 operands leave in the score
-                        if (cap > 0.f) v = cap * (1.0f - __fdividef(2.0f, __expf(2.0f * v * inv_cap) + 1.0f));
-                        v = seen ? v : -CUDART_INF_F;
-                        sc[j][e] = v;
-                        if (e < 2) tm0 = fmaxf(tm0, v); else tm1 = fmaxf(tm1, v);
-                    }
-                }
-                tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 1)); tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 2));
-                tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 1)); tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 2));
-                const float mn0 = fmaxf(m0, tm0), mn1 = fmaxf(m1, tm1);
-                const float c0 = mn0 == -CUDART_INF_F ? 1.f : __expf(m0 - mn0), c1 = mn1 == -CUDART_INF_F ? 1.f : __expf(m1 - mn1);
-                float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-                for (int j = 0; j < SMMA_BK / 8; j++) {
-                    if (ksplit && (j >> 1) != warp) continue;
-                    sc[j][0] = mn0 == -CUDART_INF_F ? 0.f : __expf(sc[j][0] - mn0);
-                    sc[j][1] = mn0 == -CUDART_INF_F ? 0.f : __expf(sc[j][1] - mn0);
-                    sc[j][2] = mn1 == -CUDART_INF_F ? 0.f : __expf(sc[j][2] - mn1);
-                    sc[j][3] = mn1 == -CUDART_INF_F ? 0.f : __expf(sc[j][3] - mn1);
-                    s0 += sc[j][0] + sc[j][1];
-                    s1 += sc[j][2] + sc[j][3];
-                }
-                s0 += __shfl_xor_sync(0xffffffffu, s0, 1); s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
-                s1 += __shfl_xor_sync(0xffffffffu, s1, 1); s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-                l0 = l0 * c0 + s0; l1 = l1 * c1 + s1;
-                m0 = mn0; m1 = mn1;
-#pragma unroll
-                for (int j = 0; j < DV / 8; j++) { o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1; }
-                // O += P V
-#pragma unroll
-                for (int kk = 0; kk < SMMA_BK / 16; kk++) {
-                    if (ksplit && kk != warp) continue;
-                    uint32_t a[4];
-                    a[0] = sink_pack_bf16(sc[2 * kk][0], sc[2 * kk][1]);
-                    a[1] = sink_pack_bf16(sc[2 * kk][2], sc[2 * kk][3]);
-                    a[2] = sink_pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
-                    a[3] = sink_pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]);
-#pragma unroll
-                    for (int j = 0; j < DV / 8; j += 2) {
-                        uint32_t b[4];
-                        sink_ldmatrix_x4_trans(b, sink_smem_u32(v_t + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * VS + j * 8 + (lane >> 4) * 8));
-                        sink_mma_bf16(o[j], a, b[0], b[1]);
-                        sink_mma_bf16(o[j + 1], a, b[2], b[3]);
-                    }
-                }
+                if (ksplit) tile(kv0, r_end, k_t, v_t, std::true_type());
+                else tile(kv0, r_end, k_t, v_t, std::false_type());
             }
         }
         __syncthreads();                     // before the copy of tile i + 2 overwrites this half
@@ -609,7 +630,7 @@ static int launch_sink_mma(const void* q, const void* kv_pool, const int* block_
     const size_t queries = (size_t)SMMA_ROWS * (DK + SMMA_PAD) * sizeof(bf16);     // (in registers before the first tile lands on them)
     const size_t smem = tiles > queries ? tiles : queries;
     cudaFuncSetAttribute(attention_sink_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_chained(attention_sink_mma_kernel<DK, DV>, dim3(max_work, nkv * gparts), dim3(128), smem, stream, (const bf16*)q,
+    launch_chained(attention_sink_mma_kernel<DK, DV>, dim3((unsigned)max_work * nkv * gparts), dim3(128), smem, stream, (const bf16*)q,
                    (const bf16*)kv_pool, block_tables, (const SinkWork*)work, n_work_ptr, (bf16*)out, part_o, part_ml, sinks, nh, nkv,
                    page_size, n_pages, table_width, window, keep_first, chunk, scale, cap, heads_per_cta, status);
     return launch_status();
