@@ -398,11 +398,50 @@ __global__ void swiglu_bias_kernel(const T* in, const float* __restrict__ bias, 
     }
 }
 
+// Sixteen bytes a thread of each half (the rows in blockIdx.y: no division): 1024 rows of 3072 took 15.4 us an entry at a time
+// (caches cold); 11.2 this way.
+template <typename T>
+__global__ void __launch_bounds__(128) swiglu_bias_vec_kernel(const T* in, const float* __restrict__ bias, T* __restrict__ out, int inter, int n_rows,
+                                                              int rows_a_cta, int act, float limit) {
+    constexpr int N = Vec16<T>::N;
+    const int c = (blockIdx.x * 128 + threadIdx.x) * N;
+    pdl_launch_dependents();
+    if (c >= inter) return;
+    float bg[N], bu[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) { bg[k] = bias[c + k]; bu[k] = bias[inter + c + k]; }
+    pdl_wait(KID_SWIGLU);
+    const int r1 = min(n_rows, ((int)blockIdx.y + 1) * rows_a_cta);
+#pragma unroll 4
+    for (int r = blockIdx.y * rows_a_cta; r < r1; r++) {
+        const T* g = in + (size_t)r * 2 * inter + c;
+        Vec16<T> vg, vu;
+        vg.load(g); vu.load(g + inter);
+        float fg[N], fu[N];
+        vg.unpack(fg); vu.unpack(fu);
+#pragma unroll
+        for (int k = 0; k < N; k++) fg[k] = glu_act(act, limit, fg[k] + bg[k], fu[k] + bu[k]);
+        vg.pack(fg);
+        vg.store(out + (size_t)r * inter + c);
+    }
+}
+
 PLLM_EXPORT int pllm_swiglu_bias(int dtype, const void* in, const float* bias, void* out, int n_rows, int inter, int act, float limit,
                                  cudaStream_t stream) {
     if (n_rows <= 0) return PLLM_OK;
     if (act < GLU_SILU || act > GLU_CLAMPED || inter <= 0 || bias == nullptr) return PLLM_ERR_SIZE;
     PLLM_DISPATCH_DTYPE(dtype, {
+        if (inter % Vec16<T>::N == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0) {
+            // (up to eight rows a CTA where that still makes sixteen CTAs an SM)
+            const int across = (inter / Vec16<T>::N + 127) / 128;
+            int rows = 1;
+            while (rows < 8 && (long long)across * (n_rows / (2 * rows)) >= 16LL * sm_count()) rows *= 2;
+            if ((n_rows + rows - 1) / rows <= 65535) {
+                launch_chained(swiglu_bias_vec_kernel<T>, dim3(across, (n_rows + rows - 1) / rows), dim3(128), 0, stream, (const T*)in, bias, (T*)out,
+                               inter, n_rows, rows, act, limit);
+                return launch_status();
+            }
+        }
         const long long total = (long long)n_rows * inter;
         const int blocks = (int)min((long long)sm_count() * 16, (total + 255) / 256);
         launch_chained(swiglu_bias_kernel<T>, dim3(blocks), dim3(256), 0, stream, (const T*)in, bias, (T*)out, inter, total, act, limit);

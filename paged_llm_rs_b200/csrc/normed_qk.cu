@@ -216,11 +216,36 @@ __global__ void gate_mul_kernel(T* y, const T* g, int g_stride, int width, long 
     }
 }
 
+// Sixteen bytes a thread (a gate an entry, whole vectors, the rows in blockIdx.y): 1024 rows of 2048 took 14.5 us an entry at a time
+// (caches cold); under 5 this way.
+template <typename T>
+__global__ void __launch_bounds__(128) gate_mul_vec_kernel(T* y, const T* g, int g_stride, int width, int kind) {
+    constexpr int N = Vec16<T>::N;
+    const int c = (blockIdx.x * 128 + threadIdx.x) * N;
+    pdl_launch_dependents();
+    if (c >= width) return;
+    pdl_wait(KID_NORMED_QK);
+    T* yr = y + (size_t)blockIdx.y * width + c;
+    Vec16<T> vy, vg;
+    vy.load(yr); vg.load(g + (size_t)blockIdx.y * g_stride + c);
+    float fy[N], fg[N];
+    vy.unpack(fy); vg.unpack(fg);
+#pragma unroll
+    for (int k = 0; k < N; k++) { const float s = nq_sigmoid(fg[k]); fy[k] *= kind == 1 ? fg[k] * s : s; }
+    vy.pack(fy);
+    vy.store(yr);
+}
+
 PLLM_EXPORT int pllm_gate_mul(int dtype, void* y, const void* g, int g_stride, int n_rows, int width, int kind, int per,
                               cudaStream_t stream) {
     if (n_rows <= 0) return PLLM_OK;
     if (width <= 0 || kind < 0 || kind > 1 || per < 1 || width % per) return PLLM_ERR_SIZE;
     PLLM_DISPATCH_DTYPE(dtype, {
+        constexpr int N = Vec16<T>::N;
+        if (per == 1 && width % N == 0 && g_stride % N == 0 && (((uintptr_t)y | (uintptr_t)g) & 15) == 0 && n_rows <= 65535) {
+            launch_chained(gate_mul_vec_kernel<T>, dim3((width / N + 127) / 128, n_rows), dim3(128), 0, stream, (T*)y, (const T*)g, g_stride, width, kind);
+            return launch_status();
+        }
         const long long total = (long long)n_rows * width;
         const int blocks = (int)min((long long)sm_count() * 8, (total + 255) / 256);
         launch_chained(gate_mul_kernel<T>, dim3(blocks), dim3(256), 0, stream, (T*)y, (const T*)g, g_stride, width, total, kind, per);
