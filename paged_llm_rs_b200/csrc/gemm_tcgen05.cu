@@ -46,6 +46,51 @@ __device__ __forceinline__ float glu_act_fast(int kind, float limit, float g, fl
     return __fdividef(g, 1.0f + __expf(-1.702f * g)) * (u + 1.0f);
 }
 
+// A lane's row of an accumulator to its place in y (null: past the last row), 32 columns at a time; ``taken`` is called when the last of
+// them are in registers.
+template <bool GLU, int BN, typename F>
+__device__ __forceinline__ void tile_out(uint32_t acc, bf16* dst, int act, float limit, F taken) {
+    constexpr int OUT_BN = GLU ? BN / 2 : BN;
+#pragma unroll 2
+    for (int c = 0; c < OUT_BN / 32; c++) {
+        uint32_t v[32], out[16];
+        tmem_ld32(acc + c * 32, v);
+        if (GLU) {
+            uint32_t u[32];
+            tmem_ld32(acc + BN / 2 + c * 32, u);
+            tmem_wait_ld();
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                // gate and up rounded as a product of their own would leave them, then the activation
+                const float g0 = round_bf16(__uint_as_float(v[2 * k])), g1 = round_bf16(__uint_as_float(v[2 * k + 1]));
+                const float u0 = round_bf16(__uint_as_float(u[2 * k])), u1 = round_bf16(__uint_as_float(u[2 * k + 1]));
+                // (fast exponential and division: their error is far below the rounding to bfloat16,
+                //  and the epilogue must keep pace with the tensor cores)
+                if (act == GLU_SILU) out[k] = pack2(__fdividef(g0, 1.0f + __expf(-g0)) * u0, __fdividef(g1, 1.0f + __expf(-g1)) * u1);
+                else out[k] = pack2(glu_act_fast(act, limit, g0, u0), glu_act_fast(act, limit, g1, u1));
+            }
+        } else {
+            tmem_wait_ld();
+            if (act == UNARY_NONE) {
+#pragma unroll
+                for (int k = 0; k < 16; k++) out[k] = pack2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
+            } else {
+                // a one-argument activation of the product, rounded first as a product of its own would leave it
+#pragma unroll
+                for (int k = 0; k < 16; k++)
+                    out[k] = pack2(unary_act(act, round_bf16(__uint_as_float(v[2 * k]))),
+                                   unary_act(act, round_bf16(__uint_as_float(v[2 * k + 1]))));
+            }
+        }
+        if (c == OUT_BN / 32 - 1) taken();
+        if (dst) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                *reinterpret_cast<uint4*>(dst + c * 32 + k * 8) = make_uint4(out[4 * k], out[4 * k + 1], out[4 * k + 2], out[4 * k + 3]);
+        }
+    }
+}
+
 // map_a: x [M, K], box 64 x 128.  map_b: W [rows, K], box 64 x BN (plain) or 64 x BN/2 (GLU).
 // y: [M, n_out] bfloat16; n_out = N (plain) or N / 2 (GLU, W = [gate; up] of n_out rows each).
 template <int EPI, int BN>
@@ -168,50 +213,12 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tcgen05_kernel(const __grid
             tc_fence_after();
             const int row = m0 + warp * 32 + lane;
             const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16) + b * BN;
-#pragma unroll 2
-            for (int c = 0; c < OUT_BN / 32; c++) {
-                uint32_t v[32], out[16];
-                tmem_ld32(acc + c * 32, v);
-                if (GLU) {
-                    uint32_t u[32];
-                    tmem_ld32(acc + BN / 2 + c * 32, u);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        // gate and up rounded as a product of their own would leave them, then the activation
-                        const float g0 = round_bf16(__uint_as_float(v[2 * k])), g1 = round_bf16(__uint_as_float(v[2 * k + 1]));
-                        const float u0 = round_bf16(__uint_as_float(u[2 * k])), u1 = round_bf16(__uint_as_float(u[2 * k + 1]));
-                        // (fast exponential and division: their error is far below the rounding to bfloat16,
-                        //  and the epilogue must keep pace with the tensor cores)
-                        if (act == GLU_SILU) out[k] = pack2(__fdividef(g0, 1.0f + __expf(-g0)) * u0, __fdividef(g1, 1.0f + __expf(-g1)) * u1);
-                        else out[k] = pack2(glu_act_fast(act, limit, g0, u0), glu_act_fast(act, limit, g1, u1));
-                    }
-                } else {
-                    tmem_wait_ld();
-                    if (act == UNARY_NONE) {
-#pragma unroll
-                        for (int k = 0; k < 16; k++) out[k] = pack2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-                    } else {
-                        // a one-argument activation of the product, rounded first as a product of its own would leave it
-#pragma unroll
-                        for (int k = 0; k < 16; k++)
-                            out[k] = pack2(unary_act(act, round_bf16(__uint_as_float(v[2 * k]))),
-                                           unary_act(act, round_bf16(__uint_as_float(v[2 * k + 1]))));
-                    }
-                }
-                if (c == OUT_BN / 32 - 1) {
-                    // everything of this accumulator is in registers: the tensor cores may have it back
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty + 8 * b);
-                }
-                if (row < M) {
-                    bf16* dst = y + (size_t)row * n_out + n0 + c * 32;
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        *reinterpret_cast<uint4*>(dst + k * 8) = make_uint4(out[4 * k], out[4 * k + 1], out[4 * k + 2], out[4 * k + 3]);
-                }
-            }
+            tile_out<GLU, BN>(acc, row < M ? y + (size_t)row * n_out + n0 : nullptr, act, limit, [&]() {
+                // everything of this accumulator is in registers: the tensor cores may have it back
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty + 8 * b);
+            });
             i++;
         }
     }
@@ -221,6 +228,129 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tcgen05_kernel(const __grid
     if (warp == 5) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+    }
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(status, 64);
+}
+
+// ---- the same with two CTAs to a tile of 256 x 256 -------------------------------------------------
+// One CTA's product of 128 x 256 reads 12 KB of operands from shared memory for what the tensor cores do in the time of 8; a pair's
+// reads half of W's tile each.  The roles are those above; the loads of both CTAs are counted by the leader's barriers, the
+// leader's sixth warp issues for both, and its commits free the stages and hand over the accumulators in both.  Measured in captured
+// steps with the gated product on pairs (us a step, one CTA a tile / pairs; the results are equal bit for bit): 0.6B shape, 2048 rows
+// 3142 / 3118; 8B shape, 6 layers, 2048 rows 4548 / 4454, 512 rows 1897 / 1856.  The plain products stay with the library: on pairs
+// the 0.6B step of 2048 rows takes 3149 with q/k/v, 3248 with o, 3271 with down (3067 to 3130 with none), the 8B one 4380, 4540 and
+// 4555 (4386 to 4472).  Weights asked for ahead of the wait changed nothing here.
+constexpr int P_STAGE = 2 * G_TILE_A;               // 128 rows of x and 128 of W, 32 KB
+constexpr int P_STAGES = G_SMEM_TILES / P_STAGE;
+
+template <int EPI>
+__global__ void __launch_bounds__(G_THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                                                                 bf16* __restrict__ y, int M, int n_out, int K, int* status, int act, float limit) {
+    constexpr bool GLU = EPI == 1;
+    constexpr int BN = 256, OUT_BN = GLU ? BN / 2 : BN;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t tiles = smem_u32(smem);
+    unsigned char* ctl = smem + P_STAGES * P_STAGE;
+    const uint32_t bars = smem_u32(ctl);                 // full[S] (the leader's), empty[S], acc_full[2], acc_empty[2] (the leader's)
+    const uint32_t acc_full = bars + 8 * 2 * P_STAGES, acc_empty = acc_full + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ctl + 8 * (2 * P_STAGES + 4));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(ctl + 8 * (2 * P_STAGES + 4) + 8);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cluster_rank(), pairs = gridDim.x / 2, pair = blockIdx.x / 2;
+    const int tiles_m = (M + 2 * G_BM - 1) / (2 * G_BM), tiles_n = n_out / OUT_BN, n_tiles = tiles_m * tiles_n;
+    const int k_blocks = (K + G_BK - 1) / G_BK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < P_STAGES; s++) {
+            mbar_init(bars + 8 * s, 1);
+            mbar_init(bars + 8 * (P_STAGES + s), 1);
+        }
+        for (int b = 0; b < 2; b++) {
+            mbar_init(acc_full + 8 * b, 1);
+            mbar_init(acc_empty + 8 * b, 8);     // one arrival from each epilogue warp of both CTAs
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
+        fence_async_smem();
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(2 * BN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+    }
+    tc_fence_before();
+    __syncthreads();
+    pair_sync();                                 // both CTAs' barriers are ready
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 4) {
+        if (lane == 0) {
+            pdl_wait(KID_GEMM_TC, true);         // x comes from the kernel before this one
+            int it = 0;
+            bool ok = true;
+            for (int t = pair; t < n_tiles && ok; t += pairs) {
+                const int m0 = (t % tiles_m) * 2 * G_BM + rank * G_BM, n0 = (t / tiles_m) * OUT_BN;
+                const int w_row = GLU ? rank * n_out + n0 : n0 + rank * (BN / 2);      // (the leader's half: gate rows; its peer's: up rows)
+                for (int kb = 0; kb < k_blocks; kb++, it++) {
+                    const int s = it % P_STAGES;
+                    if (it >= P_STAGES && !mbar_wait(bars + 8 * (P_STAGES + s), ((it / P_STAGES) - 1) & 1, abort_flag)) { ok = false; break; }
+                    const uint32_t dst = tiles + s * P_STAGE, full = leader_addr(bars + 8 * s);
+                    if (rank == 0) mbar_expect_tx(bars + 8 * s, 2 * P_STAGE);
+                    tma_load_2d_pair(dst, &map_a, kb * G_BK, m0, full);
+                    tma_load_2d_pair(dst + G_TILE_A, &map_b, kb * G_BK, w_row, full);
+                }
+            }
+        }
+    } else if (warp == 5) {
+        if (rank == 0 && lane == 0) {
+            constexpr uint32_t idesc = instr_desc(2 * G_BM, BN);
+            int it = 0, i = 0;
+            bool ok = true;
+            for (int t = pair; t < n_tiles && ok; t += pairs) {
+                const int b = i & 1;
+                if (i >= 2 && !mbar_wait(acc_empty + 8 * b, ((i >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                for (int kb = 0; kb < k_blocks; kb++, it++) {
+                    const int s = it % P_STAGES;
+                    if (!mbar_wait(bars + 8 * s, (it / P_STAGES) & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t a_src = tiles + s * P_STAGE, b_src = a_src + G_TILE_A;
+#pragma unroll
+                    for (int j = 0; j < G_BK / 16; j++)
+                        mma_ss_pair(tmem + b * BN, smem_desc(a_src + j * 32), smem_desc(b_src + j * 32), idesc, (kb | j) ? 1u : 0u);
+                    mma_commit_pair(bars + 8 * (P_STAGES + s));
+                }
+                if (ok) mma_commit_pair(acc_full + 8 * b);
+                i++;
+            }
+        }
+    } else {
+        pdl_launch_dependents();
+        int i = 0;
+        for (int t = pair; t < n_tiles; t += pairs) {
+            const int b = i & 1;
+            const int m0 = (t % tiles_m) * 2 * G_BM + rank * G_BM, n0 = (t / tiles_m) * OUT_BN;
+            if (!mbar_wait(acc_full + 8 * b, (i >> 1) & 1, abort_flag)) break;
+            tc_fence_after();
+            const int row = m0 + warp * 32 + lane;
+            const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16) + b * BN;
+            tile_out<GLU, BN>(acc, row < M ? y + (size_t)row * n_out + n0 : nullptr, act, limit, [&]() {
+                // everything of this accumulator is in registers: the tensor cores may have it back
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(leader_addr(acc_empty + 8 * b));
+            });
+            i++;
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    pair_sync();                                 // neither CTA leaves while the other may still signal it, or use its memory
+    if (warp == 5) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(2 * BN));
     }
     if (threadIdx.x == 0 && *abort_flag) atomicOr(status, 64);
 }
@@ -258,6 +388,48 @@ int launch_gemm(const void* x, const void* w, void* y, int M, int n_out, int K, 
     return launch_status();
 }
 
+// Pairs that run at the same time (asked once): a pair sits in one GPC, so that it may be fewer than half of the SMs, and the tiles are
+// dealt to those that do.
+template <int EPI>
+int most_pairs(size_t smem) {
+    static int pairs = 0;
+    if (pairs <= 0) {
+        cudaFuncSetAttribute(gemm_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * (sm_count() / 2));
+        cfg.blockDim = dim3(G_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<EPI>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        pairs = n < sm_count() / 2 ? n : sm_count() / 2;
+    }
+    return pairs;
+}
+
+template <int EPI>
+int launch_pair(const void* x, const void* w, void* y, int M, int n_out, int K, int* status, cudaStream_t stream, int act, float limit) {
+    constexpr bool GLU = EPI == 1;
+    CUtensorMap map_a, map_b;
+    {
+        const long long da[2] = {K, M}, db[2] = {K, GLU ? 2LL * n_out : n_out}, st[1] = {2LL * K};
+        const int box[2] = {G_BK, G_BM};
+        if (tensor_map(x, 2, da, st, box, true, &map_a) != 0) return PLLM_ERR_SIZE;
+        if (tensor_map(w, 2, db, st, box, true, &map_b) != 0) return PLLM_ERR_SIZE;
+    }
+    const size_t smem = (size_t)P_STAGES * P_STAGE + 8 * (2 * P_STAGES + 4) + 16 + 1024;
+    const int n_tiles = ((M + 2 * G_BM - 1) / (2 * G_BM)) * (n_out / (GLU ? 128 : 256)), pairs = most_pairs<EPI>(smem);
+    if (pairs < 1) return PLLM_ERR_SIZE;
+    launch_chained_cluster(gemm_pair_kernel<EPI>, dim3(2 * (n_tiles < pairs ? n_tiles : pairs)), dim3(G_THREADS), smem, stream, dim3(2, 1, 1), map_a,
+                           map_b, (bf16*)y, M, n_out, K, status, act, limit);
+    return launch_status();
+}
+
 }  // namespace
 
 // x: [M, K]; w: [n_out, K], or with glu [2 n_out, K] = gate rows then up rows; y: [M, n_out]; all bfloat16.
@@ -274,6 +446,9 @@ PLLM_EXPORT int pllm_gemm_tcgen05(const void* x, const void* w, void* y, int M, 
     const int tiles_m = (M + G_BM - 1) / G_BM;
     const int unit = glu ? 128 : 256;
     const bool wide = n_out % unit == 0 && (long long)tiles_m * (n_out / unit) >= sm_count();
+    // pairs of CTAs where the tiles of 256 rows are not mostly padding
+    if (wide && (tiles_m % 2 == 0 || tiles_m >= 7))
+        return glu ? launch_pair<1>(x, w, y, M, n_out, K, status, stream, act, limit) : launch_pair<0>(x, w, y, M, n_out, K, status, stream, act, limit);
     if (glu)
         return wide ? launch_gemm<1, 256>(x, w, y, M, n_out, K, status, stream, nullptr, 1, act, limit)
                     : launch_gemm<1, 128>(x, w, y, M, n_out, K, status, stream, nullptr, 1, act, limit);

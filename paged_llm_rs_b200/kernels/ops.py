@@ -563,7 +563,8 @@ SKINNY_MAX_N = 32768
 #   qkv 4096 x 1024   18.5 / 17.7      o 1024 x 2048   17.4 / 10.7      down 1024 x 3072   19.5 / 12.6
 # so the gated product takes it and the plain ones stay with the library (PAGED_LLM_TCGEN05=0: none,
 # =2: the plain ones too).  One CTA's tcgen05.mma reads both operands from shared memory, whose
-# bandwidth bounds a 128 x 256 tile at two thirds of the tensor peak; pairs of CTAs are the next step.
+# bandwidth bounds a 128 x 256 tile at two thirds of the tensor peak: large products take pairs of CTAs
+# (2048 rows, a layer of the 8B shape 12 us less), with which the plain ones are still the library's.
 TCGEN05_GEMM = int(os.environ.get("PAGED_LLM_TCGEN05", "1"))
 TCGEN05_MIN_M = 64     # below this the tiles of 128 rows are mostly padding
 _gemm_status: dict = {}
