@@ -91,12 +91,13 @@ class _DecodeGraph:
                 self._body()
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
-        before = ops.LAUNCHES
         # The step is one captured graph, or, where mixers are not ``graph_safe``, graphs with those
         # mixers between them: ("graph", CUDAGraph) and ("eager", fn, buffer) in the order they run.
-        self.pieces = []
+        # One graph is captured twice, with the reductions of split attention items and without: the host knows
+        # whether a step it packed has any, and a launch with nothing to do is a link of 2 us in the chain, a layer.
         self._ctx = None
         piecewise = not all(getattr(b.mixer, "graph_safe", False) for b in runner.model.blocks)
+        self.variants = {}
         # The collector must not run inside the capture: freeing an older engine's graphs
         # there (they die in reference cycles, at a time of the collector's choosing) is a
         # call the capture forbids, and the capture would be invalidated.
@@ -104,15 +105,30 @@ class _DecodeGraph:
         collecting = gc.isenabled()
         gc.disable()
         try:
-            with torch.no_grad():
-                self._begin_piece()
-                self._body(self._outside if piecewise else None)
-                self._end_piece()
+            plans = [g.plan for g in self.state.groups if g.plan is not None]
+            for reduces in (True, False) if plans and not piecewise else (True,):
+                for plan in plans:
+                    plan.reduces = reduces
+                before = ops.LAUNCHES
+                self.pieces = []
+                with torch.no_grad():
+                    self._begin_piece()
+                    self._body(self._outside if piecewise else None)
+                    self._end_piece()
+                self.variants[reduces] = (self.pieces, self.logits, ops.LAUNCHES - before)
         finally:
             if collecting:
                 gc.enable()
+        self._red_counts = [self.layout[f"g{gi}.n_red"][0] for gi, g in enumerate(self.state.groups) if g.plan is not None]
+        self._use(True)
+
+    def _use(self, reduces: bool) -> None:
+        """Take the captured step with the reductions of split items, or without."""
+        self.pieces, self.logits, self.launches = self.variants.get(reduces, self.variants[True])
         self.graph = self.pieces[0][1] if len(self.pieces) == 1 else None     # (the whole step, when it is one graph)
-        self.launches = ops.LAUNCHES - before
+
+    def _pick(self, packed: np.ndarray) -> None:
+        self._use(any(packed[o] for o in self._red_counts))
 
     def _begin_piece(self):
         # one memory pool for all of this runner's captured steps: they never run at the same time, so
@@ -188,6 +204,7 @@ class _DecodeGraph:
             o = self.layout["uniform"][0]
             self.staging[o:o + n] = np.asarray(uniform, dtype=np.float32).view(np.int32)
         self._before_write()
+        self._pick(self.staging)
         np.copyto(self.pinned_np, self.staging)
         if self.graph is None:
             self.state.host_segments = self._staged_segments
@@ -218,9 +235,11 @@ class _DecodeGraph:
             else:
                 host, _, _ = r.packer.pack(entries, self.caps, self.work_caps, temperature, uniform)
                 self.pinned.numpy()[:] = host
+            self._pick(self.pinned.numpy())
             self._replay()
         else:
             host, _, _ = r.packer.pack(entries, self.caps, self.work_caps, temperature, uniform)
+            self._pick(host)
             i = self._turn
             self._turn = (i + 1) % len(self._pinned)
             if self._copy_pending[i]:

@@ -465,8 +465,9 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                                         num_heads, num_kv_heads, head_dim, page_size, n_pages,
                                         block_tables.shape[-1], int(window), float(scale), _ptr(status), _stream()),
                "paged_attention")
-    _check(L.pllm_attention_reduce(_code(q), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red,
-                                   _ptr(out), num_heads, head_dim, 1 if w.many_splits else 0, _stream()), "attention_reduce")
+    if w.reduces:
+        _check(L.pllm_attention_reduce(_code(q), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red,
+                                       _ptr(out), num_heads, head_dim, 1 if w.many_splits else 0, _stream()), "attention_reduce")
     return out
 
 
@@ -516,8 +517,9 @@ def decode_attention_fused(qkv: torch.Tensor, q_gain, k_gain, eps: float, cos, s
                                              _ptr(part_o), _ptr(part_ml), num_heads, num_kv_heads, head_dim, page_size,
                                              n_pages, block_tables.shape[-1], float(scale), _ptr(status), _stream()),
            "decode_attention_fused")
-    _check(L.pllm_attention_reduce(_code(out), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red,
-                                   _ptr(out), num_heads, head_dim, 1 if w.many_splits else 0, _stream()), "attention_reduce")
+    if w.reduces:
+        _check(L.pllm_attention_reduce(_code(out), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red,
+                                       _ptr(out), num_heads, head_dim, 1 if w.many_splits else 0, _stream()), "attention_reduce")
     return out
 
 
@@ -915,8 +917,9 @@ def latent_attention(q: torch.Tensor, rows: torch.Tensor, block_tables: torch.Te
                                                max_work, _ptr(out), _ptr(part_o), _ptr(part_ml), H, R, page_size, n_pages,
                                                block_tables.shape[-1], float(scale), _ptr(status), _stream()),
                "latent_attention")
-    _check(L.pllm_attention_reduce(_code(q), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red, _ptr(out), H, R,
-                                   1 if (w.many_splits and R * 4 <= 1024) else 0, _stream()), "attention_reduce")
+    if w.reduces:
+        _check(L.pllm_attention_reduce(_code(q), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red, _ptr(out), H, R,
+                                       1 if (w.many_splits and R * 4 <= 1024) else 0, _stream()), "attention_reduce")
     return out
 
 
@@ -1196,8 +1199,9 @@ def attention_sink(q: torch.Tensor, kv_pool: torch.Tensor, block_tables: torch.T
                                      _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(sinks), num_heads, num_kv_heads, dk, dv, page_size,
                                      n_pages, block_tables.shape[-1], int(window), int(keep_first), int(chunk), float(scale), float(cap),
                                      _ptr(status), _stream()), "attention_sink")
-    _check(L.pllm_attention_reduce(_code(q), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red, _ptr(out), num_heads, dv,
-                                   1 if (w.many_splits and dv * 4 <= 1024) else 0, _stream()), "attention_reduce")
+    if w.reduces:
+        _check(L.pllm_attention_reduce(_code(q), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red, _ptr(out), num_heads, dv,
+                                       1 if (w.many_splits and dv * 4 <= 1024) else 0, _stream()), "attention_reduce")
     return out
 
 

@@ -218,6 +218,7 @@ class AttentionWork:
     part_ml: torch.Tensor
     kinds: int = 3              # what the work items are: 1 single tokens only, 2 portions only, 3 both
     many_splits: bool = False   # the step is cut into eight splits a tile or more (the reduction then shares them out)
+    reduces: bool = True        # False: no item is split, and no reduction is launched
 
 
 @dataclass

@@ -120,3 +120,33 @@ def test_a_small_portion_step_gives_the_same_logits_launched_and_at_every_captur
         assert {k[0] for k in set(runner._graphs) - was} <= {size} and (size is None) == (runner.tokens_host is None)
         assert err(got, want) <= (2e-5 if dtype == "float32" else 3e-2) and (tokens[1:] == got.argmax(1)).all()
     assert {k[0] for k in runner._graphs} == {n for n in sizes if n is not None}
+
+
+def test_the_captured_step_without_reductions_is_taken_where_nothing_is_split_and_only_there(tmp_path):
+    from paged_llm_rs_b200.engine.runner import ModelRunner
+    from paged_llm_rs_b200.engine.step import StepEntry
+
+    cfg, seed = CONFIGS["B"]
+    model = write_model(tmp_path, "B", decisive=True)
+    runner = ModelRunner(model, dtype="float32", page_size=16, num_pages=96, max_requests=8, prefix_cache=False)
+    cache, rng = runner.cache, np.random.default_rng(5)
+    toks = rng.integers(0, cfg["vocab_size"], 601).tolist()
+    for r, n in (("short", 40), ("long", 600)):
+        cache.open(r)
+        assert cache.reserve(r, n + 1)
+        runner.step([StepEntry(r, toks[:n], [])])
+        cache.commit(r, n)
+    zero = np.zeros(1, dtype=np.float32)
+    launches = {}
+    for r, n in (("short", 40), ("long", 600), ("short", 40)):
+        entries = [StepEntry(r, [toks[n]], [0])]
+        runner.use_graphs = False
+        want = runner.step_and_sample(entries, zero, zero)[0].cpu().numpy()
+        runner.use_graphs = True
+        got = runner.step_and_sample(entries, zero, zero)[0].cpu().numpy()
+        runner.check_status()
+        assert err(got, want) <= 2e-5
+        launches.setdefault(r, runner.last_launches)
+        assert launches[r] == runner.last_launches
+    assert launches["long"] - launches["short"] == cfg["num_hidden_layers"]      # (one reduction a layer)
+    assert len(runner._graphs) == 1
