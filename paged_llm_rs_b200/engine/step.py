@@ -129,45 +129,29 @@ class StepPacker:
 
         group_parts = []
         planned = {}
+        spans = [(t0, n, p0) for (t0, n, p0, _) in segs]
         for gi, g in enumerate(cache.groups):
-            slots = np.full(Tc, -1, dtype=np.int32)
             width = max((len(rc.tables[gi].blocks) for rc in rcs), default=1)
             W = caps.table_width if caps else max(width, 1)
             if width > W:
                 raise ConfigError("a block table is wider than the step's capacity")
-            tables = np.full((sc, W), -1, dtype=np.int32)
-            for si, (rc, (t0, n, p0, _)) in enumerate(zip(rcs, segs)):
-                tb = rc.tables[gi]
-                if p0 + n > tb.capacity():
+            for rc, (t0, n, p0) in zip(rcs, spans):
+                if p0 + n > rc.tables[gi].capacity():
                     raise CacheError(f"request {rc.request_id!r}: no pages reserved for positions up to {p0 + n - 1}")
-                blocks = tb.array()          # cached; rebuilt only when a page came or went
-                tables[si, :len(blocks)] = blocks
-                if n == 1:
-                    page = int(blocks[p0 // ps])
-                    if page < 0:
-                        raise CacheError(f"request {rc.request_id!r} writes into a page it gave back")
-                    slots[t0] = page * ps + p0 % ps
-                else:
-                    pp = np.arange(p0, p0 + n)
-                    page = blocks[pp // ps].astype(np.int64)
-                    if (page < 0).any():
-                        raise CacheError(f"request {rc.request_id!r} writes into a page it gave back")
-                    slots[t0:t0 + n] = page * ps + pp % ps
             plan = self.plans[gi]
             if plan is None:        # the group's mixers read tables and slots only
-                group_parts.append((slots, tables, None, None, 0, 0, 0, W))
+                group_parts.append((None, None, 0, 0, 0, W))
                 continue
             # groups that cut their work alike (same tile, window, chunk, CTAs an item) share one plan
             key = (plan.tile_tokens, plan.window, plan.ctas_per_item, plan.chunk)
             if key not in planned:
-                planned[key] = attention_plan.plan_attention(
-                    [(t0, n, p0) for (t0, n, p0, _) in segs], plan.tile_tokens, plan.window, plan.ctas_per_item,
-                    self.target_ctas, chunk=plan.chunk)
+                planned[key] = attention_plan.plan_attention(spans, plan.tile_tokens, plan.window, plan.ctas_per_item, self.target_ctas,
+                                                             chunk=plan.chunk)
             work, red, parts = planned[key]
             mw, mr, mp = (work_caps[gi] if work_caps else (len(work), len(red), parts))
             if len(work) > mw or len(red) > mr or parts > mp:
                 raise ConfigError("the step's attention work does not fit the capacities it was given")
-            group_parts.append((slots, tables, work, red, mp, mw, mr, W))
+            group_parts.append((work, red, mp, mw, mr, W))
 
         # layout: offsets in int32 units
         off = 0
@@ -180,42 +164,60 @@ class StepPacker:
 
         take("tokens", Tc); take("positions", Tc); take("logit_rows", max(nc, 1)); take("segments", max(sc, 1) * 4)
         take("temperature", max(nc, 1)); take("uniform", max(nc, 1))
-        for gi, (slots, tables, work, red, parts, mw, mr, W) in enumerate(group_parts):
+        for gi, (work, red, parts, mw, mr, W) in enumerate(group_parts):
             take(f"g{gi}.slots", Tc); take(f"g{gi}.tables", sc * W)
             if work is not None:
                 take(f"g{gi}.n_work", 1); take(f"g{gi}.n_red", 1)
                 take(f"g{gi}.work", max(mw, 1) * 8); take(f"g{gi}.red", max(mr, 1) * 4)
         host = np.zeros(off, dtype=np.int32)
 
-        def put(name, arr):
-            o, _ = layout[name]
-            a = np.asarray(arr, dtype=np.int32).reshape(-1)
-            host[o:o + len(a)] = a
+        def put(name, arr, count):
+            if count:
+                o = layout[name][0]
+                host[o:o + count] = arr
 
-        put("tokens", toks); put("positions", pos); put("logit_rows", rows)
+        put("tokens", toks, T); put("positions", pos, T); put("logit_rows", rows, n_want)
         if temperature is not None:
-            put("temperature", np.asarray(temperature, dtype=np.float32).view(np.int32))
-            put("uniform", np.asarray(uniform, dtype=np.float32).view(np.int32))
-        put("segments", np.asarray(segs, dtype=np.int32).reshape(-1) if segs else [])
-        for gi, (slots, tables, work, red, parts, mw, mr, W) in enumerate(group_parts):
-            put(f"g{gi}.slots", slots); put(f"g{gi}.tables", tables)
+            put("temperature", np.asarray(temperature, dtype=np.float32).view(np.int32), len(temperature))
+            put("uniform", np.asarray(uniform, dtype=np.float32).view(np.int32), len(uniform))
+        put("segments", [x for sg in segs for x in sg], 4 * n_seg)
+        for gi, (work, red, parts, mw, mr, W) in enumerate(group_parts):
+            o_slots, o_tables = layout[f"g{gi}.slots"][0], layout[f"g{gi}.tables"][0]
+            host[o_slots:o_slots + Tc] = -1
+            host[o_tables:o_tables + sc * W] = -1
+            for si, (rc, (t0, n, p0)) in enumerate(zip(rcs, spans)):
+                blocks = rc.tables[gi].array()          # cached; rebuilt only when a page came or went
+                host[o_tables + si * W:o_tables + si * W + len(blocks)] = blocks
+                if n == 1:
+                    page = int(blocks[p0 // ps])
+                    if page < 0:
+                        raise CacheError(f"request {rc.request_id!r} writes into a page it gave back")
+                    host[o_slots + t0] = page * ps + p0 % ps
+                else:
+                    pp = np.arange(p0, p0 + n)
+                    page = blocks[pp // ps].astype(np.int64)
+                    if (page < 0).any():
+                        raise CacheError(f"request {rc.request_id!r} writes into a page it gave back")
+                    host[o_slots + t0:o_slots + t0 + n] = page * ps + pp % ps
             if work is not None:
-                put(f"g{gi}.n_work", [len(work)]); put(f"g{gi}.n_red", [len(red)])
-                put(f"g{gi}.work", work); put(f"g{gi}.red", red)
+                host[layout[f"g{gi}.n_work"][0]], host[layout[f"g{gi}.n_red"][0]] = len(work), len(red)
+                put(f"g{gi}.work", work.reshape(-1), work.size)
+                put(f"g{gi}.red", red.reshape(-1), red.size)
         # What the work items are: bit 0 items of one query token (decoded tokens, but also the
         # last tile of a portion of 33 tokens), bit 1 items of several.  Read off the items, not
         # the segments.  A step packed to capacities is a captured decode step: single tokens only.
         kinds = 0
-        for p in group_parts:
-            if p[2] is None:
-                continue
-            counts = p[2][:, 2] if len(p[2]) else np.zeros(0, np.int32)
-            kinds |= (1 if (counts == 1).any() else 0) | (2 if (counts > 1).any() else 0)
         if caps is not None:
             kinds = caps.kinds      # a captured step launches the same kernels whatever it holds
+        else:
+            for p in group_parts:
+                if p[0] is None or not len(p[0]):
+                    continue
+                counts = p[0][:, 2]
+                kinds |= (1 if (counts == 1).any() else 0) | (2 if (counts > 1).any() else 0)
         singles = bool(segs) and all(n == 1 for (_, n, _, _) in segs)
         sizes = dict(tokens=T, wanted=n_want, segments=n_seg, tokens_cap=Tc, wanted_cap=nc, segments_cap=sc, kinds=kinds,
-                     groups=[dict(planned=p[2] is not None, parts=p[4], max_work=p[5], max_red=p[6], table_width=p[7])
+                     groups=[dict(planned=p[0] is not None, parts=p[2], max_work=p[3], max_red=p[4], table_width=p[5])
                              for p in group_parts],
                      host_segments=segs,
                      # the most tokens a request brings (a captured step: what its capacities allow)

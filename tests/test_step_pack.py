@@ -73,3 +73,25 @@ def test_native_decode_packer_refuses_like_the_python_packer():
         with pytest.raises(ConfigError):
             pack([StepEntry("a", [1], [0])] * 5)       # more requests than the step holds
         pack([StepEntry("a", [999], [0])])
+
+
+@pytest.mark.parametrize("tile,ctas,window,chunk", [(4, 1, None, 0), (16, 2, 300, 0), (64, 8, None, 0), (8, 2, None, 500)])
+def test_a_small_step_planned_number_by_number_is_the_array_plan(monkeypatch, tile, ctas, window, chunk):
+    rng = np.random.default_rng(tile + ctas)
+    small = 0
+    for trial in range(300):
+        segments, at = [], 0
+        for _ in range(int(rng.integers(1, 7))):
+            n, before = int(rng.choice([0, 1, 1, 2, 9, 64, 65, 129])), int(rng.choice([0, 1, 63, 127, 128, 600, 4095, 4200]))
+            segments.append((at, n, before))
+            at += n
+        target = int(rng.choice([1, 40, 296]))
+        got = attention_plan.plan_attention(segments, tile, window, ctas, target, chunk=chunk)
+        small += attention_plan._small_plan(segments, tile, window, ctas, target, attention_plan.MIN_SPLIT_KEYS, attention_plan.MULTI_MIN_SPLIT_KEYS,
+                                            chunk) is not None
+        with monkeypatch.context() as m:
+            m.setattr(attention_plan, "SMALL_PLAN", -1)
+            want = attention_plan.plan_attention(segments, tile, window, ctas, target, chunk=chunk)
+        assert all(np.array_equal(a, b) for a, b in zip(got[:2], want[:2])) and got[2] == want[2]
+        assert got[0].dtype == want[0].dtype
+    assert small > 50
