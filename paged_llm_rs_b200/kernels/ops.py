@@ -721,7 +721,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         act = torch.empty((x.shape[0], K), dtype=x.dtype, device=x.device)
         swiglu(x, act)
         x = act
-    if rows_gemm_takes(x, weight, N, want) and (out is None or (out.is_contiguous() and not out.data_ptr() & 15)):
+    fits = out is None or (out.shape == (x.shape[0], N) and out.dtype == want and out.is_contiguous() and not out.data_ptr() & 15)
+    if fits and rows_gemm_takes(x, weight, N, want):
         return rows_gemm(x, weight, out, status=status, out_dtype=want)
     if skinny_gemm_takes(x, weight, K) and N <= SKINNY_MAX_N and want in (torch.bfloat16, torch.float32):
         _dev(x, weight, out)
@@ -733,7 +734,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         _check(lib().pllm_skinny_gemm(_ptr(x), _ptr(weight), _ptr(out), M, N, K,
                                       1 if want == torch.float32 else 0, _stream()), "skinny_gemm")
         return out
-    if gemm_f32_takes(x, weight, want) and (out is None or out.is_contiguous()):
+    if fits and gemm_f32_takes(x, weight, want):
         return gemm_f32(x, weight, out)
     if TCGEN05_GEMM >= 2 and out is None and want == torch.bfloat16 and x.shape[0] >= TCGEN05_MIN_M \
             and gemm_tcgen05_takes(x, weight, N, False):

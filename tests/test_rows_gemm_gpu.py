@@ -64,3 +64,16 @@ def test_rows_product_is_the_engines_route_and_leaves_the_rest():
                  (torch.randn(24 * 256 + 1, device=DEV).bfloat16()[1:].view(24, 256), w)):
         assert not ops.rows_gemm_takes(a, b, 256)
         torch.testing.assert_close(ops.linear(a, b).float(), a.float() @ b.float().T, atol=3e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_product_into_a_buffer_that_the_kernels_do_not_write_is_the_librarys(dtype):
+    x, w = torch.randn(32, 1024, device="cuda").to(dtype), torch.randn(2048, 1024, device="cuda").to(dtype)
+    want = ops.linear(x, w)
+    wide = torch.zeros(32, 2 * 2048, dtype=dtype, device="cuda")
+    for out in (torch.zeros(32, 2048, dtype=dtype, device="cuda"), wide[:, ::2], torch.zeros(0, dtype=dtype, device="cuda")):
+        got = ops.linear(x, w, out)
+        assert got.data_ptr() == out.data_ptr() and got.shape == (32, 2048)
+        # (two float sums of 1024 products in another order, then one rounding to bfloat16, an ulp apart at most)
+        torch.testing.assert_close(got, want, atol=1e-2 if dtype == torch.bfloat16 else 1e-3, rtol=2 ** -7 if dtype == torch.bfloat16 else 1e-4)
+    assert not wide[:, 1::2].any()
