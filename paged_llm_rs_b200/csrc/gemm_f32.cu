@@ -134,6 +134,8 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(const float* x, 
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     const int live = (M - m0 < BM ? M - m0 : BM) * BN;
     for (int u = rank * F_THREADS + threadIdx.x; u < live; u += splits * F_THREADS) {
+        const int m = m0 + u / BN, n = n0 + u % BN;
+        if (n >= N) continue;          // (nothing is read that is not added and stored)
         float v[8];
 #pragma unroll
         for (int p = 0; p < 8; p++)
@@ -142,11 +144,11 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(const float* x, 
 #pragma unroll
         for (int p = 1; p < 8; p++)
             if (p < splits) s += v[p];
-        const int m = m0 + u / BN, n = n0 + u % BN;
-        if (n < N) y[(size_t)m * N + n] = s;
+        y[(size_t)m * N + n] = s;
     }
-    // a CTA's shared memory stays until its peers have read it
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+    // a CTA's shared memory stays until its peers have read it: an arrival that releases is one behind the reads before it
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 // Whether this kernel takes the product.

@@ -55,8 +55,6 @@ __device__ __forceinline__ float4 ld_cluster16(uint32_t addr) {
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
 }
-// (for a meeting that hands no data over: nobody waits for the stores before it to arrive)
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 
@@ -186,9 +184,10 @@ __global__ void __launch_bounds__(R_THREADS, 2) rows_gemm_kernel(const __grid_co
             for (int h = 0; h < TURN; h++) {
                 const int u = u0 + h * step;
                 const uint32_t at = ring + ((u / UNITS) * R_BM + (u % UNITS) * 4) * 4;
+                const bool in = u < units && row0 + (u % UNITS) * 4 < n_out;      // (nothing is read that is not added and stored)
 #pragma unroll
                 for (int p = 0; p < MAX_SPLITS; p++)
-                    if (p < splits && u < units) {
+                    if (p < splits && in) {
                         const uint32_t from = MAX_SPLITS > 1 ? cluster_addr(at, p) : at;
                         v[h][p] = ld_cluster16(from);
                         if (GLU) w[h][p] = ld_cluster16(from + R_BM * 2);
@@ -221,8 +220,8 @@ __global__ void __launch_bounds__(R_THREADS, 2) rows_gemm_kernel(const __grid_co
             }
         }
     }
-    // a CTA's shared memory stays until its peers have read it (what they read is in their registers: nothing to order)
-    if (splits > 1) { __syncwarp(); cluster_arrive_relaxed(); cluster_wait(); } else __syncthreads();
+    // a CTA's shared memory stays until its peers have read it: an arrival that releases is one behind the reads before it
+    if (splits > 1) { __syncwarp(); cluster_arrive(); cluster_wait(); } else __syncthreads();
     if (warp == 9) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tmem_cols));

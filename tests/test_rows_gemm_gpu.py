@@ -52,6 +52,23 @@ def test_rows_product_with_activations(M, I, K):
         assert ((y.float() - want).abs() / (1 + want)).max().item() < 2e-2
 
 
+@pytest.mark.parametrize("N", [136, 1000, 1992])
+def test_ragged_widths_whose_splits_leave_one_another_at_once(N):
+    # a cluster's CTAs read one another's shared memory; where the last tile is not full, one of them has nothing to add and
+    # store for a column past the width, and must neither read for it nor leave before its peers have read
+    x, w = inputs(40, N, 2048)
+    xf, wf = x.float(), w.float()
+    for splits in (2, 4, 8):
+        first = ops.rows_gemm(x, w, splits=splits, out_dtype=torch.float32), ops.rows_gemm(x, w[: N // 16 * 16], glu=True, splits=splits), \
+            ops.gemm_f32(xf, wf, splits=splits)
+        for _ in range(200):
+            again = ops.rows_gemm(x, w, splits=splits, out_dtype=torch.float32), ops.rows_gemm(x, w[: N // 16 * 16], glu=True, splits=splits), \
+                ops.gemm_f32(xf, wf, splits=splits)
+        assert all(torch.equal(a, b) for a, b in zip(first, again))
+        for y in (first[0], first[2]):       # (the same operands in both: K roundings of the sum of the products' sizes, at most)
+            assert ((y.double() - x.double() @ w.double().T).abs() <= 2048 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all()
+
+
 def test_rows_product_is_the_engines_route_and_leaves_the_rest():
     x, w = inputs(24, 256, 256)
     assert ops.rows_gemm_takes(x, w, 256) and torch.equal(ops.linear(x, w), ops.rows_gemm(x, w))
