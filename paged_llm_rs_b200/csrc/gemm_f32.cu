@@ -146,9 +146,10 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(const float* x, 
             if (p < splits) s += v[p];
         y[(size_t)m * N + n] = s;
     }
-    // a CTA's shared memory stays until its peers have read it: an arrival that releases is one behind the reads before it
+    // A CTA's shared memory stays until its peers have read it.  Every value that a thread read from a peer went into a store to y above, and the
+    // fence keeps those stores ahead of the arrival (rows_gemm_tcgen05.cu says more)
     __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    asm volatile("fence.acq_rel.cta;\nbarrier.cluster.arrive.relaxed.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 // Whether this kernel takes the product.
