@@ -58,7 +58,10 @@ __device__ __forceinline__ void db_unit_rows(const float* src, long long stride,
         if (lane * 4 < dp) *reinterpret_cast<float4*>(dst + t * dp + ((lane ^ (t & 7)) << 2)) = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
     }
 }
-// G of a block's tokens in double and beta, by the CTA's first warp (past nt: the last G, and zero)
+// G of a block's tokens in double and beta, by the CTA's first warp (past nt: the last G, and zero).  A token whose log g is an
+// infinity, or below DB_LEAST, starts anew: the recurrence's factor exp(log g) is zero there.  It counts as DB_LEAST, whose exponential is zero
+// too, so that differences of G between the tokens behind it stay what they are, where infinities would leave none.
+constexpr float DB_LEAST = -1000.f;
 struct DBTokens { double G[DB_L]; float beta[DB_L]; };
 __device__ __forceinline__ void db_tokens(DBTokens& tk, const float* ba, size_t tok0, int nt, int h, int H, float A, float bias) {
     if (threadIdx.x >= 32) return;
@@ -68,7 +71,8 @@ __device__ __forceinline__ void db_tokens(DBTokens& tk, const float* ba, size_t 
     for (int c = 0; c < DB_L; c += 32) {
         const int t = c + lane;
         const float* r = ba + (tok0 + (t < nt ? t : 0)) * 2 * H;
-        double G = t < nt ? (double)(A * mm_softplus(r[H + h] + bias)) : 0.0;
+        const float log_g = A * mm_softplus(r[H + h] + bias);
+        double G = t < nt ? (double)(log_g < DB_LEAST ? DB_LEAST : log_g) : 0.0;      // (a NaN stays one)
         tk.beta[t] = t < nt ? mm_sigmoid(r[h]) : 0.f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {

@@ -160,3 +160,19 @@ def test_a_later_infinite_value_reaches_no_earlier_token_of_the_delta_rule():
     rest = torch.rand(c, taps, generator=g), torch.zeros(H), torch.zeros(H), torch.ones(E)
     a, b = (delta_steps(True, torch.float32, [(100,)], [(x, ba)], *rest, H, G, d, E)[0] for x in (u, bad))
     assert torch.equal(a[:70], b[:70])
+
+
+@pytest.mark.parametrize("gate", [float("inf"), 1e30, 5000.0])
+def test_a_gate_that_resets_the_state_resets_it_in_a_block_too(gate):
+    # tokens whose decay is exactly zero (one at a block's start, two in a row, one in the last block) beside heads without any
+    H, G, d, E, taps = 2, 1, 32, 64, 4
+    g = torch.Generator().manual_seed(3)
+    c = 2 * G * d + H * E
+    u, ba = torch.randn(200, c + H * E, generator=g), torch.randn(200, 2 * H, generator=g)
+    ba[[64, 90, 91, 150], H] = gate
+    conv_w, a_log, dt, gain = torch.rand(c, taps, generator=g), torch.zeros(H), torch.zeros(H), torch.ones(E)
+    want = plain_delta(u, conv_w, ba, a_log, dt, gain, H, G, d, E)
+    for blocks in (True, False):
+        # (the second step starts from the state that the first one left)
+        got = delta_steps(blocks, torch.float32, [(130,), (70,)], [(u, ba)], conv_w, a_log, dt, gain, H, G, d, E)[0]
+        assert float((got.double() - want).norm() / want.norm()) <= 2e-6, blocks
