@@ -786,7 +786,8 @@ PLLM_EXPORT int pllm_delta_mix(int dtype, const void* u, int u_width, const void
     MMShape sh;
     const int rc = mm_shape(n_segs, H, d, E, 5, max_segment_tokens, &sh);
     if (rc != PLLM_OK) return rc;
-    const int chunks = (max_segment_tokens + MM_CONV_TOKENS - 1) / MM_CONV_TOKENS;
+    const int longest_segment = max_segment_tokens > 0 && max_segment_tokens < n_tokens ? max_segment_tokens : n_tokens;
+    const int chunks = (longest_segment + MM_CONV_TOKENS - 1) / MM_CONV_TOKENS;
     PLLM_DISPATCH_DTYPE(dtype, {
         const dim3 conv_grid(n_segs, (channels + 127) / 128, chunks > 0 ? chunks : 1);
         if (taps <= 4)

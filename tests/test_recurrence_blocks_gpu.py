@@ -103,7 +103,7 @@ def plain_delta(u, conv_w, ba, a_log, dt, gain, H, G, d, E):
     return o.reshape(T, H * E) * P.silu(u[:, c:].double())
 
 
-def delta_steps(blocks, dtype, cuts, seqs, conv_w, a_log, dt, gain, H, G, d, E):
+def delta_steps(blocks, dtype, cuts, seqs, conv_w, a_log, dt, gain, H, G, d, E, most=max):
     ops.DELTA_BLOCKS = blocks
     try:
         taps = conv_w.shape[1]
@@ -119,7 +119,7 @@ def delta_steps(blocks, dtype, cuts, seqs, conv_w, a_log, dt, gain, H, G, d, E):
             u, ba = torch.cat(us).to(DEV, dtype).contiguous(), torch.cat(gs).to(DEV).contiguous()
             out = torch.empty(at, H * E, dtype=dtype, device=DEV)
             ops.delta_mix(u, conv_w.to(DEV, dtype), ba, a_log.to(DEV), dt.to(DEV), gain.to(DEV), torch.tensor(segs, dtype=torch.int32, device=DEV),
-                          max(cut), state, out, H, G, d, E, taps, EPS)
+                          most(cut), state, out, H, G, d, E, taps, EPS)
             for r, (a, n, _, _) in enumerate(segs):
                 outs[r].append(out[a:a + n].cpu())
                 done[r] += n
@@ -176,3 +176,16 @@ def test_a_gate_that_resets_the_state_resets_it_in_a_block_too(gate):
         # (the second step starts from the state that the first one left)
         got = delta_steps(blocks, torch.float32, [(130,), (70,)], [(u, ba)], conv_w, a_log, dt, gain, H, G, d, E)[0]
         assert float((got.double() - want).norm() / want.norm()) <= 2e-6, blocks
+
+
+@pytest.mark.parametrize("n", [33, 64, 200])
+def test_the_delta_rule_takes_segments_of_unknown_length(n):
+    # (max_segment_tokens 0: no block path, and every token convolved)
+    H, G, d, E, taps = 2, 1, 16, 24, 4
+    g = torch.Generator().manual_seed(n)
+    c = 2 * G * d + H * E
+    u, ba, rest = torch.randn(n, c + H * E, generator=g), torch.randn(n, 2 * H, generator=g), (torch.zeros(H), torch.zeros(H), torch.ones(E), H, G, d, E)
+    conv_w = torch.rand(c, taps, generator=g)
+    a, b = (delta_steps(False, torch.float32, [(n,)], [(u, ba)], conv_w, *rest, most=most)[0] for most in (lambda cut: 0, max))
+    want = plain_delta(u, conv_w, ba, *rest)
+    assert torch.equal(a, b) and float((a.double() - want).norm() / want.norm()) <= 2e-6
