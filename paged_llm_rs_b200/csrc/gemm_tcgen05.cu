@@ -25,6 +25,8 @@
 //              the tensor cores are on the next tile meanwhile
 // Every wait is bounded: a thread that gives up raises a flag that the others see, the
 // CTA frees its tensor memory and leaves, and the status word says so (bit 64).
+#include <atomic>
+
 #include "tcgen05.cuh"
 
 using namespace tc;
@@ -388,32 +390,45 @@ int launch_gemm(const void* x, const void* w, void* y, int M, int n_out, int K, 
     return launch_status();
 }
 
-// Pairs that run at the same time (asked once): a pair sits in one GPC, so that it may be fewer than half of the SMs, and the tiles are
-// dealt to those that do.
+constexpr size_t P_SMEM = (size_t)P_STAGES * P_STAGE + 8 * (2 * P_STAGES + 4) + 16 + 1024;
+
+// The kernel's shared memory is allowed a device at a time, as every launcher here does it at each launch.
 template <int EPI>
-int most_pairs(size_t smem) {
-    static int pairs = 0;
-    if (pairs <= 0) {
-        cudaFuncSetAttribute(gemm_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * (sm_count() / 2));
-        cfg.blockDim = dim3(G_THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<EPI>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-        pairs = n < sm_count() / 2 ? n : sm_count() / 2;
+bool allow_pair() {
+    return cudaFuncSetAttribute(gemm_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM) == cudaSuccess;
+}
+
+// Pairs that run at the same time on the current device (asked once each): a pair sits in one GPC, so that it may be fewer than half of
+// the SMs, and the tiles are dealt to those that do.  0: none, or not to be known, and the products are the one-CTA kernel's.
+template <int EPI>
+int most_pairs() {
+    constexpr int KNOWN = 64;
+    static std::atomic<int> known[KNOWN];        // 1 + the pairs of each device; 0: not asked yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < KNOWN && known[dev].load() > 0) return known[dev].load() - 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (sm_count() / 2));
+    cfg.blockDim = dim3(G_THREADS);
+    cfg.dynamicSmemBytes = P_SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (!allow_pair<EPI>() || cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<EPI>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;                                // (asked again next time)
     }
-    return pairs;
+    n = n < sm_count() / 2 ? n : sm_count() / 2;
+    if (dev < KNOWN) known[dev].store(n + 1);
+    return n;
 }
 
 template <int EPI>
-int launch_pair(const void* x, const void* w, void* y, int M, int n_out, int K, int* status, cudaStream_t stream, int act, float limit) {
+int launch_pair(const void* x, const void* w, void* y, int M, int n_out, int K, int* status, cudaStream_t stream, int act, float limit, int pairs) {
     constexpr bool GLU = EPI == 1;
     CUtensorMap map_a, map_b;
     {
@@ -422,10 +437,9 @@ int launch_pair(const void* x, const void* w, void* y, int M, int n_out, int K, 
         if (tensor_map(x, 2, da, st, box, true, &map_a) != 0) return PLLM_ERR_SIZE;
         if (tensor_map(w, 2, db, st, box, true, &map_b) != 0) return PLLM_ERR_SIZE;
     }
-    const size_t smem = (size_t)P_STAGES * P_STAGE + 8 * (2 * P_STAGES + 4) + 16 + 1024;
-    const int n_tiles = ((M + 2 * G_BM - 1) / (2 * G_BM)) * (n_out / (GLU ? 128 : 256)), pairs = most_pairs<EPI>(smem);
-    if (pairs < 1) return PLLM_ERR_SIZE;
-    launch_chained_cluster(gemm_pair_kernel<EPI>, dim3(2 * (n_tiles < pairs ? n_tiles : pairs)), dim3(G_THREADS), smem, stream, dim3(2, 1, 1), map_a,
+    const int n_tiles = ((M + 2 * G_BM - 1) / (2 * G_BM)) * (n_out / (GLU ? 128 : 256));
+    allow_pair<EPI>();
+    launch_chained_cluster(gemm_pair_kernel<EPI>, dim3(2 * (n_tiles < pairs ? n_tiles : pairs)), dim3(G_THREADS), P_SMEM, stream, dim3(2, 1, 1), map_a,
                            map_b, (bf16*)y, M, n_out, K, status, act, limit);
     return launch_status();
 }
@@ -446,9 +460,11 @@ PLLM_EXPORT int pllm_gemm_tcgen05(const void* x, const void* w, void* y, int M, 
     const int tiles_m = (M + G_BM - 1) / G_BM;
     const int unit = glu ? 128 : 256;
     const bool wide = n_out % unit == 0 && (long long)tiles_m * (n_out / unit) >= sm_count();
-    // pairs of CTAs where the tiles of 256 rows are not mostly padding
-    if (wide && (tiles_m % 2 == 0 || tiles_m >= 7))
-        return glu ? launch_pair<1>(x, w, y, M, n_out, K, status, stream, act, limit) : launch_pair<0>(x, w, y, M, n_out, K, status, stream, act, limit);
+    // pairs of CTAs where the tiles of 256 rows are not mostly padding and the device has room for a pair
+    const int pairs = wide && (tiles_m % 2 == 0 || tiles_m >= 7) ? (glu ? most_pairs<1>() : most_pairs<0>()) : 0;
+    if (pairs > 0)
+        return glu ? launch_pair<1>(x, w, y, M, n_out, K, status, stream, act, limit, pairs)
+                   : launch_pair<0>(x, w, y, M, n_out, K, status, stream, act, limit, pairs);
     if (glu)
         return wide ? launch_gemm<1, 256>(x, w, y, M, n_out, K, status, stream, nullptr, 1, act, limit)
                     : launch_gemm<1, 128>(x, w, y, M, n_out, K, status, stream, nullptr, 1, act, limit);
