@@ -52,7 +52,8 @@ class _DecodeGraph:
     overwrites; what does not fill the capacities is padding that writes nothing
     (slot -1) and attends to nothing (no work item)."""
 
-    def __init__(self, runner: "ModelRunner", B: int, W: int, segments: Optional[int] = None):
+    def __init__(self, runner: "ModelRunner", B: int, W: int, segments: Optional[int] = None, logits: Optional[torch.Tensor] = None):
+        """``logits``: where the step's logits go, [requests, vocab] float32 (None: a buffer of the step's own)."""
         self.runner, self.B, self.W = runner, B, W
         pk = runner.packer
         self.decode = segments is None
@@ -66,6 +67,8 @@ class _DecodeGraph:
         self.dev = self.pinned.to(runner.device)
         self.nbytes = host.nbytes
         self.state = pk.to_state(self.dev, self.layout, self.sizes, full=True)
+        # (one buffer for both captures of the step, not one in each: 39 MB at 64 requests and a vocabulary of 152 thousand)
+        self.logits = logits if logits is not None else torch.empty((n_seg, runner.vocab_size), dtype=torch.float32, device=runner.device)
         self.tokens = torch.zeros(1 + n_seg, dtype=torch.int32, device=runner.device)
         # the status word and the chosen tokens come back by a copy that is part of the captured step
         self.tokens_host = torch.zeros(1 + n_seg, dtype=torch.int32).pin_memory()
@@ -115,7 +118,7 @@ class _DecodeGraph:
                     self._begin_piece()
                     self._body(self._outside if piecewise else None)
                     self._end_piece()
-                self.variants[reduces] = (self.pieces, self.logits, ops.LAUNCHES - before)
+                self.variants[reduces] = (self.pieces, ops.LAUNCHES - before)
         finally:
             if collecting:
                 gc.enable()
@@ -124,7 +127,7 @@ class _DecodeGraph:
 
     def _use(self, reduces: bool) -> None:
         """Take the captured step with the reductions of split items, or without."""
-        self.pieces, self.logits, self.launches = self.variants.get(reduces, self.variants[True])
+        self.pieces, self.launches = self.variants.get(reduces, self.variants[True])
         self.graph = self.pieces[0][1] if len(self.pieces) == 1 else None     # (the whole step, when it is one graph)
 
     def _pick(self, packed: np.ndarray) -> None:
@@ -168,7 +171,13 @@ class _DecodeGraph:
         r = self.runner
         if self.decode:
             self.dev.copy_(self.pinned, non_blocking=True)  # the step's packed buffer: the graph's first node
-        self.logits = r.model.forward(self.state, r.caches, outside)
+        r.rt.logits_out = self.logits
+        try:
+            made = r.model.forward(self.state, r.caches, outside)
+        finally:
+            r.rt.logits_out = None
+        if made.data_ptr() != self.logits.data_ptr():      # (a head that makes its own)
+            self.logits.copy_(made)
         ops.sample(self.logits, self.state.temperature, self.state.uniform, self.tokens[1:])
         self.tokens[:1].copy_(r.rt.status)
         self.tokens_host.copy_(self.tokens, non_blocking=True)
@@ -336,6 +345,7 @@ class ModelRunner:
         # replayed (None: such steps are launched kernel by kernel)
         self.graph_step_tokens: Optional[int] = None
         self._portions_seen = set()      # (tokens, table width, requests) of smaller portion steps that came once
+        self._portion_logits = {}        # requests: their logits (a caller gets a copy)
         self.bytes_h2d = 0        # bytes the last step copied to the device
         self.tokens_host: Optional[torch.Tensor] = None   # pinned copy of the last step's (status, tokens), valid
                                                           # once the stream is synchronized; None: not made
@@ -365,18 +375,20 @@ class ModelRunner:
         wanted row) by the sampling kernel.  Returns (logits, tokens): tokens is an
         int32 device tensor [1 + wanted] whose first entry is the kernels' status
         word, so one copy brings both back.  A step of single decoded tokens runs
-        as a replayed CUDA graph when graphs are on."""
+        as a replayed CUDA graph when graphs are on, and a step that fills the token budget (or needs its size) likewise: their
+        results lie in the captured step's own buffers until it is replayed.  Every other step's are the caller's."""
         if not entries:
             return torch.zeros((0, self.vocab_size), dtype=torch.float32, device=self.device), None
         self.bytes_h2d = 0
         self.tokens_host = None
         if self.use_graphs and temperature is not None:
             if all(len(e.tokens) == 1 and list(e.want) == [0] for e in entries):
-                g = self._decode_graph(entries)
+                g, lasting = self._decode_graph(entries), False
             else:
-                g = self._portion_graph(entries)
+                g, lasting = self._portion_graph(entries)
             if g is not None:
-                return g.run(entries, temperature, uniform)
+                logits, tokens = g.run(entries, temperature, uniform)
+                return (logits.clone(), tokens.clone()) if lasting else (logits, tokens)
         host, layout, sizes = self.packer.pack(entries, temperature=temperature, uniform=uniform)
         pinned = torch.from_numpy(host).pin_memory()
         dev = pinned.to(self.device, non_blocking=True)
@@ -434,34 +446,40 @@ class ModelRunner:
         rounded up to one of ``portion_sizes``.  The budget's own size is captured when first needed;
         the smaller ones when they are needed again, since a capture takes as long as some ten steps
         launched kernel by kernel.  A first step of a smaller size replays the budget's when that is one
-        of PADDED_PORTION tokens at most, and is launched kernel by kernel when it is larger."""
+        of PADDED_PORTION tokens at most, and is launched kernel by kernel when it is larger.  Returns
+        the captured step (or None) and whether the step's results must outlast its next replay (those of smaller sizes share their buffers)."""
         cap = self.graph_step_tokens
         total = sum(len(e.tokens) for e in entries)
         if not cap or total > cap or len(entries) > self.max_graph_batch:
-            return None
+            return None, False
         S = 1
         while S < len(entries):
             S *= 2
         if sum(len(e.want) for e in entries) > S:
-            return None     # (generation wants one place a request at most; a step that wants more is launched plainly)
+            return None, False     # (generation wants one place a request at most; a step that wants more is launched plainly)
         width = max((len(self.cache.get(e.request_id).tables[gi].blocks) for e in entries
                      for gi in range(len(self.cache.groups))), default=1)
         W = 64
         while W < width:
             W *= 2
         size = next(n for n in portion_sizes(cap) if n >= total)
-        key = (size, W, S)
+        needed, key = size, (size, W, S)
         g = self._graphs.get(key)
         if g is None and size < cap and key not in self._portions_seen:
             self._portions_seen.add(key)
             if cap > PADDED_PORTION:
-                return None
+                return None, False
             size, key = cap, (cap, W, S)
             g = self._graphs.get(key)
         if g is None:
-            g = _DecodeGraph(self, size, W, segments=S)
+            logits = None
+            if size < cap:
+                if S not in self._portion_logits:
+                    self._portion_logits[S] = torch.empty((S, self.vocab_size), dtype=torch.float32, device=self.device)
+                logits = self._portion_logits[S]
+            g = _DecodeGraph(self, size, W, segments=S, logits=logits)
             self._graphs[key] = g
-        return g
+        return g, needed < cap
 
     def capture_ahead(self, max_batch: int, table_width: int = 64) -> int:
         """Capture, before the first request needs them, the steps the engine replays: decode steps of 1, 2, 4, ...

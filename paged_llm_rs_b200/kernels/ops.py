@@ -740,7 +740,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
             and gemm_tcgen05_takes(x, weight, N, False):
         return gemm_tcgen05(x, weight, status=status)
     if want != x.dtype:
-        return torch.mm(x, weight.t(), out_dtype=want)
+        return torch.mm(x, weight.t(), out_dtype=want, out=out) if out is not None else torch.mm(x, weight.t(), out_dtype=want)
     return torch.matmul(x, weight.t(), out=out) if out is not None else torch.matmul(x, weight.t())
 
 

@@ -39,6 +39,8 @@ class Runtime:
     # reference's Trace (crates/pagedllm/src/model/mod.rs:33-80).  Only what a kernel stores
     # can be named: a fused kernel's intermediate values are not.
     trace: Optional[Dict[str, torch.Tensor]] = None
+    # Where the head puts the logits, [rows, vocab] float32 (a captured step's buffer; None: into a tensor of their own).
+    logits_out: Optional[torch.Tensor] = None
 
     def __post_init__(self):
         if self.status is None:

@@ -108,7 +108,7 @@ class LinearHead(Part):
             raise WeightError(f"no {self._name('weight')}, and the config does not tie the embeddings")
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        logits = ops.linear(x, self.weight, out_dtype=torch.float32, status=self.rt.status)
+        logits = ops.linear(x, self.weight, out=self.rt.logits_out, out_dtype=torch.float32, status=self.rt.status)
         if self.scale != 1.0:
             ops.scale32(logits, self.scale)
         if self.softcap:

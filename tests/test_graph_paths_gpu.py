@@ -150,3 +150,46 @@ def test_the_captured_step_without_reductions_is_taken_where_nothing_is_split_an
         assert launches[r] == runner.last_launches
     assert launches["long"] - launches["short"] == cfg["num_hidden_layers"]      # (one reduction a layer)
     assert len(runner._graphs) == 1
+
+
+def portion_runner(tmp_path, budget, requests=8, num_pages=200, dtype="bfloat16"):
+    from paged_llm_rs_b200.engine.runner import ModelRunner
+    runner = ModelRunner(write_model(tmp_path, "D", decisive=True), dtype=dtype, page_size=16, num_pages=num_pages, max_requests=requests, prefix_cache=False)
+    runner.graph_step_tokens = budget
+    return runner, np.random.default_rng(7)
+
+
+def portion_step(runner, rng, total, requests, vocab):
+    """Open ``requests`` requests and give each a portion; ``total`` tokens in all."""
+    from paged_llm_rs_b200.engine.step import StepEntry
+    entries = []
+    for i in range(requests):
+        n = total // requests + (i < total % requests)
+        r = f"r{total}.{requests}.{i}"
+        if not runner.cache.has(r):
+            runner.cache.open(r)
+            assert runner.cache.reserve(r, n)
+        entries.append(StepEntry(r, rng.integers(0, vocab, n).tolist(), [n - 1]))
+    return entries, np.zeros(requests, dtype=np.float32)
+
+
+def close(runner, entries):
+    for e in entries:
+        runner.cache.close(e.request_id)
+
+
+def test_small_portions_results_outlast_the_steps_after_them(tmp_path):
+    # (a step that fills its budget's captured step leaves its results in that step's buffers; a smaller one's are the caller's)
+    runner, rng = portion_runner(tmp_path, 128)
+    V = CONFIGS["D"][0]["vocab_size"]
+    a, zeros = portion_step(runner, rng, 50, 1, V)
+    b, _ = portion_step(runner, rng, 60, 1, V)
+    runner.use_graphs = False
+    want = [runner.step_and_sample(e, zeros, zeros)[0].clone() for e in (a, b)]
+    runner.use_graphs = True
+    assert not torch.equal(*want)
+    for _ in range(3):
+        got = [runner.step_and_sample(e, zeros, zeros) for e in (a, b)]
+        torch.cuda.synchronize()
+        for (logits, tokens), w in zip(got, want):
+            assert err(logits.cpu().numpy(), w.cpu().numpy()) <= 3e-2 and int(tokens[1]) == int(logits[0].argmax())
