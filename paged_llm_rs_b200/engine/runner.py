@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import gc
 import os
+from collections import OrderedDict
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -87,7 +88,10 @@ class _DecodeGraph:
         self._copy_pending = [False for _ in self._pinned]
         self._turn = 0
         # Warm up on a side stream (library handles, workspaces), then capture.
-        side = torch.cuda.Stream()
+        # (one such stream a runner: the library keeps a workspace of 8.5 MB for every stream it has run on)
+        if runner.warm_stream is None:
+            runner.warm_stream = torch.cuda.Stream()
+        side = runner.warm_stream
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side), torch.no_grad():
             for _ in range(2):
@@ -103,8 +107,11 @@ class _DecodeGraph:
         self.variants = {}
         # The collector must not run inside the capture: freeing an older engine's graphs
         # there (they die in reference cycles, at a time of the collector's choosing) is a
-        # call the capture forbids, and the capture would be invalidated.
-        gc.collect()
+        # call the capture forbids, and the capture would be invalidated.  (Collecting takes 37 ms of a capture's 60 to
+        # 75: once a runner, so that a capture while requests run does not pay for it.)
+        if not runner.collected:
+            gc.collect()
+            runner.collected = True
         collecting = gc.isenabled()
         gc.disable()
         try:
@@ -270,6 +277,10 @@ class _DecodeGraph:
 # takes 1.3 ms, at 2048 3.2.
 PADDED_PORTION = 256
 
+# Captured steps of portions below the budget's own size that a runner keeps; the one that was used longest ago goes first.
+# A budget of 2048 has 14 such sizes, one of 8192 has 22, each with up to three request counts up to 64 requests.
+PORTION_CAPTURES = 96
+
 
 def portion_sizes(budget: int) -> List[int]:
     """The sizes (tokens) that portion steps under a token budget are captured at, rising.  Up to 256 tokens a step costs its
@@ -281,6 +292,16 @@ def portion_sizes(budget: int) -> List[int]:
         sizes += [n * 5 // 4, n * 3 // 2, n * 7 // 4, n * 2]
         n *= 2
     return [n for n in sizes if (n * 2 <= budget if n <= 256 else n * 8 <= budget * 7)] + [budget]
+
+
+def portion_requests(n: int) -> int:
+    """The request count that a smaller portion step of ``n`` requests is captured for: 1, 8, 64, then doubling.  What
+    a step pays for rows of logits that nobody asked for is little (of a vocabulary of 152 thousand at width 1024, 64 rows 52 us and one
+    row 48), so that few counts are worth a capture of their own."""
+    S = 1
+    while S < n:
+        S *= 8 if S < 64 else 2
+    return S
 
 
 def group_plans(cache: CacheManager, mixer_of, page_size: int) -> List[Optional[GroupPlanConfig]]:
@@ -341,10 +362,12 @@ class ModelRunner:
         self.max_graph_batch = max_graph_batch
         self._graphs = {}
         self.graph_pool = torch.cuda.graph_pool_handle()
+        self.warm_stream, self.collected = None, False      # (the captures')
         # the engine's token budget a step: steps of prompt portions under it are captured once and
         # replayed (None: such steps are launched kernel by kernel)
         self.graph_step_tokens: Optional[int] = None
         self._portions_seen = set()      # (tokens, table width, requests) of smaller portion steps that came once
+        self._portions = OrderedDict()   # the keys of those that are captured, the one used longest ago first
         self._portion_logits = {}        # requests: their logits (a caller gets a copy)
         self.bytes_h2d = 0        # bytes the last step copied to the device
         self.tokens_host: Optional[torch.Tensor] = None   # pinned copy of the last step's (status, tokens), valid
@@ -442,18 +465,19 @@ class ModelRunner:
 
     def _portion_graph(self, entries):
         """The captured step for portions of prompts (beside decoded tokens), when the engine
-        runs under a token budget: one capture per (tokens, requests, table width), the tokens a step's
+        runs under a token budget: one capture per (tokens, table width, requests), the tokens a step's
         rounded up to one of ``portion_sizes``.  The budget's own size is captured when first needed;
         the smaller ones when they are needed again, since a capture takes as long as some ten steps
-        launched kernel by kernel.  A first step of a smaller size replays the budget's when that is one
-        of PADDED_PORTION tokens at most, and is launched kernel by kernel when it is larger.  Returns
-        the captured step (or None) and whether the step's results must outlast its next replay (those of smaller sizes share their buffers)."""
+        launched kernel by kernel.  A first step of a smaller size replays what is captured already and would
+        be more than half full, or the budget's where that is of PADDED_PORTION tokens at most, and is launched kernel
+        by kernel where there is neither.  Of the smaller ones PORTION_CAPTURES are kept.  Returns the captured step (or None)
+        and whether the step's results must outlast its next replay (those of smaller sizes share their buffers)."""
         cap = self.graph_step_tokens
-        total = sum(len(e.tokens) for e in entries)
-        if not cap or total > cap or len(entries) > self.max_graph_batch:
+        total, n = sum(len(e.tokens) for e in entries), len(entries)
+        if not cap or total > cap or n > self.max_graph_batch:
             return None, False
         S = 1
-        while S < len(entries):
+        while S < n:
             S *= 2
         if sum(len(e.want) for e in entries) > S:
             return None, False     # (generation wants one place a request at most; a step that wants more is launched plainly)
@@ -462,45 +486,78 @@ class ModelRunner:
         W = 64
         while W < width:
             W *= 2
-        size = next(n for n in portion_sizes(cap) if n >= total)
-        needed, key = size, (size, W, S)
-        g = self._graphs.get(key)
-        if g is None and size < cap and key not in self._portions_seen:
+        sizes = portion_sizes(cap)
+        size = next(m for m in sizes if m >= total)
+        if size < cap:
+            R = portion_requests(n)
+            key = (size, W, R)
+            if key in self._portions:
+                return self._smaller(key), True
+            if key in self._portions_seen:
+                return self._capture_smaller(key), True
             self._portions_seen.add(key)
-            if cap > PADDED_PORTION:
+            for m in sizes:
+                if size < m < 2 * total and (m, W, R) in self._portions:
+                    return self._smaller((m, W, R)), True
+            if not ((cap < 2 * total and (cap, W, S) in self._graphs) or cap <= PADDED_PORTION):
                 return None, False
-            size, key = cap, (cap, W, S)
-            g = self._graphs.get(key)
-        if g is None:
-            logits = None
-            if size < cap:
-                if S not in self._portion_logits:
-                    self._portion_logits[S] = torch.empty((S, self.vocab_size), dtype=torch.float32, device=self.device)
-                logits = self._portion_logits[S]
-            g = _DecodeGraph(self, size, W, segments=S, logits=logits)
-            self._graphs[key] = g
-        return g, needed < cap
+        key = (cap, W, S)
+        if key not in self._graphs:
+            self._graphs[key] = _DecodeGraph(self, cap, W, segments=S)
+        return self._graphs[key], size < cap
+
+    def _smaller(self, key):
+        self._portions.move_to_end(key)
+        return self._graphs[key]
+
+    def _capture_smaller(self, key):
+        """Capture a portion step below the budget's own size; of those, the ones used longest ago give way."""
+        size, W, R = key
+        while len(self._portions) >= PORTION_CAPTURES:
+            old, _ = self._portions.popitem(last=False)
+            self._portions_seen.discard(old)      # (it is captured again when it is needed twice again)
+            torch.cuda.synchronize()              # (its last replay may still run)
+            del self._graphs[old]
+        if R not in self._portion_logits:
+            self._portion_logits[R] = torch.empty((R, self.vocab_size), dtype=torch.float32, device=self.device)
+        self._portions_seen.add(key)
+        self._graphs[key] = _DecodeGraph(self, size, W, segments=R, logits=self._portion_logits[R])
+        self._portions[key] = None
+        return self._graphs[key]
 
     def capture_ahead(self, max_batch: int, table_width: int = 64) -> int:
         """Capture, before the first request needs them, the steps the engine replays: decode steps of 1, 2, 4, ...
-        up to ``max_batch`` requests and, under a token budget, the budget's steps of as many requests, for block
+        up to ``max_batch`` requests and, under a token budget, the budget's steps of as many requests and the smaller
+        portion steps (``portion_sizes``) of 1, 8, 64, ... requests, for block
         tables of up to ``table_width`` pages (wider ones are captured when a request first grows that long).
-        A capture takes some 40 ms; without this the first requests pay for them.  Returns how many were made."""
+        A capture takes 20 to 35 ms (the first ones, which load kernels and the library's choices, 150 and more); without this the
+        first requests pay for them.  Returns how many were made."""
         if not self.use_graphs:
             return 0
+        cap = self.graph_step_tokens
+        most = min(max_batch, self.max_graph_batch)
         made, B = 0, 1
         while True:
             b = min(B, self.max_graph_batch)
             if (b, table_width) not in self._graphs:
                 self._graphs[(b, table_width)] = _DecodeGraph(self, b, table_width)
                 made += 1
-            cap = self.graph_step_tokens
             if cap and b <= cap and (cap, table_width, b) not in self._graphs:
                 self._graphs[(cap, table_width, b)] = _DecodeGraph(self, cap, table_width, segments=b)
                 made += 1
             if B >= max_batch or b >= self.max_graph_batch:
-                return made
+                break
             B *= 2
+        R = 1
+        while cap:
+            for size in portion_sizes(cap)[:-1]:
+                if R <= size and (size, table_width, R) not in self._portions and len(self._portions) < PORTION_CAPTURES:
+                    self._capture_smaller((size, table_width, R))
+                    made += 1
+            if R >= most:
+                break
+            R = portion_requests(R + 1)
+        return made
 
     def check_status(self) -> None:
         code = int(self.rt.status.item())

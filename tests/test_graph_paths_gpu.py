@@ -178,6 +178,22 @@ def close(runner, entries):
         runner.cache.close(e.request_id)
 
 
+def test_a_captured_step_has_one_buffer_of_logits_and_those_of_smaller_portions_share_theirs(tmp_path):
+    runner, rng = portion_runner(tmp_path, 1024)
+    V = CONFIGS["D"][0]["vocab_size"]
+    for requests in (1, 2, 5):
+        for total in (40, 100, 300, 600, 1000):
+            entries, zeros = portion_step(runner, rng, total, requests, V)
+            for _ in range(2):
+                runner.step_and_sample(entries, zeros, zeros)
+            close(runner, entries)
+    held = {k: g for k, g in runner._graphs.items() if len(k) == 3}
+    assert {k[0] for k in held} == {64, 128, 320, 640, 1024} and {k[2] for k in held if k[0] < 1024} == {1, 8}
+    below = {g.logits.data_ptr() for k, g in held.items() if k[0] < 1024}
+    assert len(below) == 2 and len({g.logits.data_ptr() for k, g in held.items() if k[0] == 1024} | below) == 2 + 3
+    assert all(len(g.variants) == 2 for g in held.values())
+
+
 def test_small_portions_results_outlast_the_steps_after_them(tmp_path):
     # (a step that fills its budget's captured step leaves its results in that step's buffers; a smaller one's are the caller's)
     runner, rng = portion_runner(tmp_path, 128)
@@ -193,3 +209,51 @@ def test_small_portions_results_outlast_the_steps_after_them(tmp_path):
         torch.cuda.synchronize()
         for (logits, tokens), w in zip(got, want):
             assert err(logits.cpu().numpy(), w.cpu().numpy()) <= 3e-2 and int(tokens[1]) == int(logits[0].argmax())
+
+
+def test_captured_portions_are_bounded_and_the_one_used_longest_ago_gives_way(tmp_path, monkeypatch):
+    from paged_llm_rs_b200.engine import runner as R
+    monkeypatch.setattr(R, "PORTION_CAPTURES", 2)
+    runner, rng = portion_runner(tmp_path, 600)
+    V = CONFIGS["D"][0]["vocab_size"]
+    for total, held in ((40, {64}), (100, {64, 128}), (40, {64, 128}), (200, {64, 256}), (100, {256, 128}), (200, {256, 128})):
+        entries, zeros = portion_step(runner, rng, total, 1, V)
+        runner.use_graphs = False
+        want = runner.step_and_sample(entries, zeros, zeros)[0].cpu().numpy()
+        runner.use_graphs = True
+        for _ in range(3):
+            got = runner.step_and_sample(entries, zeros, zeros)[0]
+            assert err(got.cpu().numpy(), want) <= 3e-2
+        runner.check_status()
+        close(runner, entries)
+        assert {k[0] for k in runner._graphs} == held == {k[0] for k in runner._portions}
+
+
+def test_a_smaller_portion_replays_what_is_captured_before_it_is_captured_itself(tmp_path):
+    runner, rng = portion_runner(tmp_path, 600)
+    V = CONFIGS["D"][0]["vocab_size"]
+    fill, zeros = portion_step(runner, rng, 590, 1, V)
+    runner.step_and_sample(fill, zeros, zeros)
+    assert {k[0] for k in runner._graphs} == {600}
+    close(runner, fill)
+    entries, zeros = portion_step(runner, rng, 310, 1, V)      # (more than half of 600, and 320 is not captured)
+    for held in ({600}, {600, 320}):
+        runner.step_and_sample(entries, zeros, zeros)
+        assert runner.tokens_host is not None and {k[0] for k in runner._graphs} == held
+    small, zeros = portion_step(runner, rng, 130, 1, V)        # (less than half of 320 and of 600: launched)
+    runner.step_and_sample(small, zeros, zeros)
+    assert runner.tokens_host is None and {k[0] for k in runner._graphs} == {600, 320}
+
+
+def test_nothing_is_captured_while_requests_run_after_warming_up(tmp_path):
+    from paged_llm_rs_b200 import Engine
+    cfg, seed = CONFIGS["D"]
+    model = write_model(tmp_path, "D", decisive=True)
+    eng = Engine(model, dtype="bfloat16", block_size=16, blocks=400, chunk=300, max_batch=16, max_prefill_seqs=2)
+    made = eng.warm_up()
+    # 1, 2, 4, 8, 16 requests: decode steps, the budget's; 64 and 128 tokens for 1, 8 and 64 requests
+    assert made == 5 + 5 + 2 * 3 and eng.warm_up() == 0
+    held = set(eng.runner._graphs)
+    rng = np.random.default_rng(3)
+    eng.generate([rng.integers(0, cfg["vocab_size"], n).tolist() for n in (5, 70, 299, 310, 420, 17, 64, 129, 200, 33, 600, 3)], max_tokens=20)
+    assert set(eng.runner._graphs) == held
