@@ -21,7 +21,7 @@
 #include "matrix_memory.cuh"
 #include "mlstm_blocks.cuh"
 
-#define DB_L 64                // tokens a block; longer segments take this path
+#define DB_L 64                // tokens a block
 #define DB_THREADS 256
 #define DB_COLS 16             // columns of S a CTA of delta_states_kernel
 #define DB_C 64                // columns of the outputs a CTA
@@ -34,11 +34,11 @@ struct DBBuffers {
     float* S;                  // [blocks][H][d][E]: what the block starts from
     float* decay;              // [blocks][H]: exp(G_L)
 };
-static inline long long db_floats(int n_tokens, int n_segs, int H, int d, int E) {
-    return mb_blocks(n_tokens, n_segs) * H * (2LL * DB_L * d + (long long)DB_L * E + (long long)d * E + 4) + 16;
+static inline long long db_floats(int n_tokens, int n_segs, int longest, int H, int d, int E) {
+    return mb_blocks(n_tokens, n_segs, longest) * H * (2LL * DB_L * d + (long long)DB_L * E + (long long)d * E + 4) + 16;
 }
-static inline DBBuffers db_buffers(float* at, int n_tokens, int n_segs, int H, int d, int E) {
-    const long long nb = mb_blocks(n_tokens, n_segs) * H;
+static inline DBBuffers db_buffers(float* at, int n_tokens, int n_segs, int longest, int H, int d, int E) {
+    const long long nb = mb_blocks(n_tokens, n_segs, longest) * H;
     DBBuffers b;
     b.W = at;
     b.kd = b.W + nb * DB_L * d;
@@ -113,10 +113,10 @@ __device__ __forceinline__ void db_product(const float* a, const float* b, int d
 // grid (blocks, heads).  c: [tokens, channels] float, q at 0 (G d), k at G d, v at 2 G d (H E); ba: [tokens, 2 H], b_raw | a_raw.
 __global__ void __launch_bounds__(DB_THREADS) delta_solve_kernel(const float* c, int channels, const float* ba, const float* __restrict__ a_log,
                                                                  const float* __restrict__ dt_bias, const MMSegment* __restrict__ segs, int n_segs,
-                                                                 DBBuffers buf, int H, int G, int d, int E) {
+                                                                 DBBuffers buf, int H, int G, int d, int E, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     __shared__ DBTokens tk;
-    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DB_L);
+    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DB_L, longest);
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
     if (b.seg < 0 || b.blocks < 2) return;
@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(DB_THREADS) delta_solve_kernel(const float* c,
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     {
         float kk[4][4];
+    if (s.count <= longest) return;
         db_product(k_s, k_s, dp, d / 4, tx, ty, kk);
 #pragma unroll
         for (int r = 0; r < 4; r++)
@@ -195,14 +196,14 @@ __device__ __forceinline__ void db_fetch16(float* dst, const float* src) {
 // grid (segments, heads, runs of 16 columns).  W S0: thread (token group of four, column group of four, quarter of the key
 // entries); k^T u: thread (key entries of four, column group, half of the tokens); the shares are added in their order.
 __global__ void __launch_bounds__(DB_THREADS) delta_states_kernel(const MMSegment* __restrict__ segs, int n_segs, float* state, long long state_stride,
-                                                                  DBBuffers buf, int H, int d, int E) {
+                                                                  DBBuffers buf, int H, int d, int E, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     const MMSegment s = segs[blockIdx.x];
     int rank = 0;
-    for (int i = 0; i < (int)blockIdx.x; i++) rank += segs[i].count > DB_L ? (segs[i].count + DB_L - 1) / DB_L : 0;
+    for (int i = 0; i < (int)blockIdx.x; i++) rank += segs[i].count > longest ? (segs[i].count + DB_L - 1) / DB_L : 0;
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
-    if (s.count <= DB_L) return;
+    if (s.count <= longest) return;
     const int blocks = (s.count + DB_L - 1) / DB_L, h = blockIdx.y, c0 = blockIdx.z * DB_COLS, tid = threadIdx.x;
     const int wp = d + 4;                        // (a row's pitch: four more, so that neighbouring rows' chunks lie in other banks)
     float* W_s = mm_smem;                        // [2][64][wp]
@@ -320,11 +321,11 @@ __global__ void __launch_bounds__(DB_THREADS) delta_states_kernel(const MMSegmen
 // grid (blocks, heads, column tiles).  A thread has tokens ty + 16 a, and keys tx + 16 b or the columns 4 tx .. 4 tx + 3.
 __global__ void __launch_bounds__(DB_THREADS) delta_outputs_kernel(const float* c, int channels, const float* ba, const float* __restrict__ a_log,
                                                                    const float* __restrict__ dt_bias, const MMSegment* __restrict__ segs, int n_segs,
-                                                                   DBBuffers buf, float* __restrict__ y, int H, int G, int d, int E) {
+                                                                   DBBuffers buf, float* __restrict__ y, int H, int G, int d, int E, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     __shared__ DBTokens tk;
     __shared__ float a_s[DB_L];
-    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DB_L);
+    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DB_L, longest);
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
     if (b.seg < 0 || b.blocks < 2) return;
@@ -350,6 +351,7 @@ __global__ void __launch_bounds__(DB_THREADS) delta_outputs_kernel(const float* 
         for (int r = 0; r < 4; r++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
+    if (s.count <= longest) return;
                 const int t = ty + 16 * r, o = tx + 16 * e;
                 p_s[t * DB_L + o] = o <= t ? mb_exp(tk.G[t] - tk.G[o]) * qk[r][e] : 0.f;
             }
@@ -423,43 +425,44 @@ __global__ void __launch_bounds__(DB_THREADS) delta_outputs_kernel(const float* 
 // convolution of this step has read the ones before.  A longer segment has more tokens than taps.
 template <typename T>
 __global__ void __launch_bounds__(256) delta_conv_state_kernel(const T* u, int u_width, int conv_in_off, const MMSegment* __restrict__ segs, float* state,
-                                                               long long state_stride, long long conv_off, int channels, int taps) {
+                                                               long long state_stride, long long conv_off, int channels, int taps, int longest) {
     const MMSegment s = segs[blockIdx.x];
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
     const int ch = blockIdx.y * 256 + threadIdx.x;
-    if (s.count <= DB_L || ch >= channels) return;
+    if (s.count <= longest || ch >= channels) return;
     float* cs = state + (size_t)s.slot * state_stride + conv_off;
     for (int k = 0; k < taps - 1; k++) cs[(size_t)k * channels + ch] = to_f32(u[(size_t)(s.first + s.count - (taps - 1) + k) * u_width + conv_in_off + ch]);
 }
 
-// Whether segments of more than DB_L tokens take this path: whole vectors of four, and what delta_solve_kernel and
+// Whether segments of more than `longest` tokens take this path: keys of 32 entries or more (with 64 tokens over eight directions U and W S0 nearly
+// cancel, and the writes come out 5 to 17 % further from 64-bit arithmetic than the recurrence's), whole vectors of four, and what delta_solve_kernel and
 // delta_states_kernel keep in shared memory.
 static inline size_t db_solve_smem(int d, int E) { return (size_t)(DB_L * ((d + 31) & ~31) + DB_L * DB_L + DB_L * (d + E)) * sizeof(float); }
 static inline size_t db_states_smem(int d) {
     const int share = 4 * DB_L * DB_COLS > 2 * d * DB_COLS ? 4 * DB_L * DB_COLS : 2 * d * DB_COLS;
     return (size_t)(2 * DB_L * (d + 4) + 2 * DB_L * d + d * DB_COLS + DB_L * DB_COLS + share) * sizeof(float);
 }
-static inline bool db_takes(int channels, int d, int E, int max_segment_tokens) {
-    return max_segment_tokens > DB_L && d % 4 == 0 && d <= DB_MAX_D && E % 4 == 0 && channels % 4 == 0 && db_solve_smem(d, E) <= 200 * 1024;
+static inline bool db_takes(int channels, int d, int E, int max_segment_tokens, int longest) {
+    return longest >= DB_L && max_segment_tokens > longest && d >= 32 && d % 4 == 0 && d <= DB_MAX_D && E % 4 == 0 && channels % 4 == 0 && db_solve_smem(d, E) <= 200 * 1024;
 }
 
 template <typename T>
 static void launch_delta_blocks(const float* c, int channels, const float* ba, const float* a_log, const float* dt_bias, const T* u, int u_width,
                                 const MMSegment* segs, int n_segs, float* state, long long state_stride, long long conv_off, int taps,
-                                const DBBuffers& buf, float* y, int n_tokens, int H, int G, int d, int E, cudaStream_t stream) {
+                                const DBBuffers& buf, float* y, int n_tokens, int H, int G, int d, int E, int longest, cudaStream_t stream) {
     const int dp = (d + 31) & ~31, blocks = n_tokens / DB_L + n_segs;
     const size_t solve = db_solve_smem(d, E), states = db_states_smem(d);
     const size_t outputs = (size_t)(DB_L * dp + (dp > DB_L ? DB_L * dp : DB_L * DB_L) + 2 * DB_L * DB_C) * sizeof(float);
     cudaFuncSetAttribute(delta_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve);
     cudaFuncSetAttribute(delta_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)states);
     cudaFuncSetAttribute(delta_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outputs);
-    launch_chained(delta_solve_kernel, dim3(blocks, H), dim3(DB_THREADS), solve, stream, c, channels, ba, a_log, dt_bias, segs, n_segs, buf, H, G, d, E);
+    launch_chained(delta_solve_kernel, dim3(blocks, H), dim3(DB_THREADS), solve, stream, c, channels, ba, a_log, dt_bias, segs, n_segs, buf, H, G, d, E, longest);
     launch_chained(delta_states_kernel, dim3(n_segs, H, (E + DB_COLS - 1) / DB_COLS), dim3(DB_THREADS), states, stream, segs, n_segs, state, state_stride,
-                   buf, H, d, E);
+                   buf, H, d, E, longest);
     launch_chained(delta_outputs_kernel, dim3(blocks, H, (E + DB_C - 1) / DB_C), dim3(DB_THREADS), outputs, stream, c, channels, ba, a_log, dt_bias, segs,
-                   n_segs, buf, y, H, G, d, E);
+                   n_segs, buf, y, H, G, d, E, longest);
     if (taps > 1)
         launch_chained(delta_conv_state_kernel<T>, dim3(n_segs, (channels + 255) / 256), dim3(256), 0, stream, u, u_width, 0, segs, state, state_stride,
-                       conv_off, channels, taps);
+                       conv_off, channels, taps, longest);
 }

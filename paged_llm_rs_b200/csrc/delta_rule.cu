@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128, 5) delta_prepare_kernel(const T* u, DRSha
     float* g_s = k_s + DR_RUN * dp;
     float* a1_s = g_s + DR_RUN * dp;         // [DR_RUN][padded]
     float* x_s = a1_s + DR_RUN * padded;     // [DR_RUN + taps - 1][128] the convolution's inputs, a channel a thread
-    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DR_RUN);
+    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DR_RUN, DR_RUN);
     if (b.seg < 0) return;
     const MMSegment s = segs[b.seg];
     const int h = blockIdx.y, kh = h / (sh.H / sh.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

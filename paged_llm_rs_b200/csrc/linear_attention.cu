@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256, 2) la_scan_kernel(const T* u, LAShape sh,
     float* y_s = v_s + ck * Ps;                             // [ck][parts][Ps]
     pdl_launch_dependents();
     pdl_wait(KID_LINEAR_ATT);
-    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, L);
+    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, L, L);
     if (b.seg < 0) return;
     const MMSegment s = segs[b.seg];
     const int h = blockIdx.y, p0 = blockIdx.z * Ps, tid = threadIdx.x;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(256) la_block_outputs_kernel(const MMSegment* 
     __shared__ __align__(16) float S_s[LA_TK][LA_TC];
     pdl_launch_dependents();
     pdl_wait(KID_LINEAR_ATT);
-    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, L);
+    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, L, L);
     if (b.seg < 0 || b.tb == 0) return;
     const MMSegment s = segs[b.seg];
     const int h = blockIdx.y / col_tiles, c0 = (blockIdx.y % col_tiles) * LA_TC, t0 = blockIdx.z * LA_TT;

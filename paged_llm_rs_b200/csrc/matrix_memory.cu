@@ -717,11 +717,12 @@ static inline int mlstm_shape(int n_segs, int H, int d, int E, int max_segment_t
 
 PLLM_EXPORT long long pllm_mlstm_state_floats(int H, int d, int E) { return (long long)H * d * E + (long long)H * d + H; }
 // Floats of scratch for a step's longer segments (0: the step has none, or its sizes are the recurrence's).
-PLLM_EXPORT long long pllm_mlstm_block_floats(const void* u, int u_width, int n_tokens, int n_segs, int max_segment_tokens, int H, int d, int E) {
-    return mb_takes(u, u_width, d, E, max_segment_tokens) ? mb_floats(n_tokens, n_segs, H, d, E) : 0;
+PLLM_EXPORT long long pllm_mlstm_block_floats(const void* u, int u_width, int n_tokens, int n_segs, int max_segment_tokens, int longest, int H, int d,
+                                              int E) {
+    return mb_takes(u, u_width, d, E, max_segment_tokens, longest) ? mb_floats(n_tokens, n_segs, longest, H, d, E) : 0;
 }
-PLLM_EXPORT long long pllm_delta_block_floats(int n_tokens, int n_segs, int max_segment_tokens, int H, int G, int d, int E) {
-    return db_takes(2 * G * d + H * E, d, E, max_segment_tokens) ? db_floats(n_tokens, n_segs, H, d, E) : 0;
+PLLM_EXPORT long long pllm_delta_block_floats(int n_tokens, int n_segs, int max_segment_tokens, int longest, int H, int G, int d, int E) {
+    return db_takes(2 * G * d + H * E, d, E, max_segment_tokens, longest) ? db_floats(n_tokens, n_segs, longest, H, d, E) : 0;
 }
 PLLM_EXPORT long long pllm_delta_state_floats(int H, int G, int d, int E, int taps) {
     return (long long)H * d * E + (long long)(taps - 1) * (2 * G * d + H * E);
@@ -730,18 +731,18 @@ PLLM_EXPORT long long pllm_delta_state_floats(int H, int G, int d, int E, int ta
 // u: [tokens, u_width] of the compute dtype: q (H d) | k (H d) | v (H e) | gate (H e); gates: [tokens, 2 H] float, i_raw | f_raw;
 // gain: H e floats; nm_buf: [n_segs, H, d + 1], dn_buf: [tokens, H, 2] and y_buf: [tokens, H e] float scratch (rows of no
 // segment zero in the last two); out: [tokens, H e] of the compute dtype.  max_segment_tokens bounds a segment's tokens (0: unknown).
-// block_buf: pllm_mlstm_block_floats floats (null: every segment token by token).
+// block_buf: pllm_mlstm_block_floats floats for segments of more than `longest` tokens, in blocks (null: every segment token by token).
 PLLM_EXPORT int pllm_mlstm_mix(int dtype, const void* u, int u_width, const float* gates, const float* i_bias, const float* f_bias,
                                float cap, const float* gain, const int* segs, int n_segs, int max_segment_tokens, float* state,
-                               long long state_stride, float* nm_buf, float* dn_buf, float* y_buf, float* block_buf, long long block_floats,
+                               long long state_stride, float* nm_buf, float* dn_buf, float* y_buf, float* block_buf, long long block_floats, int longest,
                                void* out, int n_tokens, int H, int d, int E, float eps, cudaStream_t stream) {
     if (n_tokens <= 0 || n_segs <= 0) return PLLM_OK;
     if (H <= 0 || d <= 0 || E <= 0 || !(cap > 0.f) || u_width < 2 * H * d + 2 * H * E) return PLLM_ERR_SIZE;
     if (state_stride < pllm_mlstm_state_floats(H, d, E)) return PLLM_ERR_SIZE;
-    // segments of more than MB_L tokens in blocks where the sizes allow it and the scratch for it was given
-    const bool blocks = block_buf != nullptr && mb_takes(u, u_width, d, E, max_segment_tokens);
-    if (blocks && (block_floats < mb_floats(n_tokens, n_segs, H, d, E) || ((uintptr_t)block_buf & 15))) return PLLM_ERR_SIZE;
-    const int longest = blocks ? MB_L : 0x7fffffff;
+    // segments of more than `longest` tokens in blocks where the sizes allow it and the scratch for it was given
+    const bool blocks = block_buf != nullptr && mb_takes(u, u_width, d, E, max_segment_tokens, longest);
+    if (blocks && (block_floats < mb_floats(n_tokens, n_segs, longest, H, d, E) || ((uintptr_t)block_buf & 15))) return PLLM_ERR_SIZE;
+    if (!blocks) longest = 0x7fffffff;
     MMShape sh;
     const int rc = mlstm_shape(n_segs, H, d, E, max_segment_tokens, &sh);
     if (rc != PLLM_OK) return rc;
@@ -758,7 +759,7 @@ PLLM_EXPORT int pllm_mlstm_mix(int dtype, const void* u, int u_width, const floa
                        state_stride, H, d, E, longest);
         if (blocks)
             launch_mlstm_blocks<T>((const T*)u, u_width, gates, i_bias, f_bias, cap, (const MMSegment*)segs, n_segs, state, state_stride,
-                                   mb_buffers(block_buf, n_tokens, n_segs, H, d, E), y_buf, dn_buf, n_tokens, H, d, E, stream);
+                                   mb_buffers(block_buf, n_tokens, n_segs, longest, H, d, E), y_buf, dn_buf, n_tokens, H, d, E, longest, stream);
         launch_head_norm_gate<T>(y_buf, dn_buf, (const T*)u + 2 * H * d + H * E, u_width, gain, out, n_tokens, H, E, 1, 0, eps, stream);
     });
     return launch_status();
@@ -766,11 +767,11 @@ PLLM_EXPORT int pllm_mlstm_mix(int dtype, const void* u, int u_width, const floa
 
 // u: [tokens, u_width] of the compute dtype: q (G d) | k (G d) | v (H e) | gate (H e); conv_w: [2 G d + H e, taps] of the same;
 // ba: [tokens, 2 H] float, b_raw | a_raw; a_log, dt_bias: H floats; gain: e floats; c_buf [tokens, 2 G d + H e] and
-// y_buf [tokens, H e] float scratch; out: [tokens, H e] of the compute dtype.
-// block_buf: pllm_delta_block_floats floats (null: every segment token by token).
+// y_buf [tokens, H e] float scratch; out: [tokens, H e] of the compute dtype.  max_segment_tokens bounds a segment's tokens (0: unknown).
+// block_buf: pllm_delta_block_floats floats for segments of more than `longest` tokens, in blocks (null: every segment token by token).
 PLLM_EXPORT int pllm_delta_mix(int dtype, const void* u, int u_width, const void* conv_w, const float* ba, const float* a_log,
                                const float* dt_bias, const float* gain, const int* segs, int n_segs, int max_segment_tokens,
-                               float* state, long long state_stride, float* c_buf, float* y_buf, float* block_buf, long long block_floats, void* out,
+                               float* state, long long state_stride, float* c_buf, float* y_buf, float* block_buf, long long block_floats, int longest, void* out,
                                int n_tokens, int H, int G, int d, int E, int taps, float eps, cudaStream_t stream) {
     if (n_tokens <= 0 || n_segs <= 0) return PLLM_OK;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || E <= 0 || taps < 1) return PLLM_ERR_SIZE;
@@ -778,11 +779,11 @@ PLLM_EXPORT int pllm_delta_mix(int dtype, const void* u, int u_width, const void
     const int channels = 2 * G * d + H * E;
     if (u_width < channels + H * E || state_stride < pllm_delta_state_floats(H, G, d, E, taps)) return PLLM_ERR_SIZE;
     const long long conv_off = (long long)H * d * E;
-    // segments of more than DB_L tokens in blocks where the sizes allow it and the scratch for it was given
-    const bool blocks = block_buf != nullptr && db_takes(channels, d, E, max_segment_tokens);
-    if (blocks && (block_floats < db_floats(n_tokens, n_segs, H, d, E) || (((uintptr_t)block_buf | (uintptr_t)c_buf | (uintptr_t)y_buf) & 15)))
+    // segments of more than `longest` tokens in blocks where the sizes allow it and the scratch for it was given
+    const bool blocks = block_buf != nullptr && db_takes(channels, d, E, max_segment_tokens, longest);
+    if (blocks && (block_floats < db_floats(n_tokens, n_segs, longest, H, d, E) || (((uintptr_t)block_buf | (uintptr_t)c_buf | (uintptr_t)y_buf) & 15)))
         return PLLM_ERR_SIZE;
-    const int longest = blocks ? DB_L : 0x7fffffff;
+    if (!blocks) longest = 0x7fffffff;
     MMShape sh;
     const int rc = mm_shape(n_segs, H, d, E, 5, max_segment_tokens, &sh);
     if (rc != PLLM_OK) return rc;
@@ -807,7 +808,7 @@ PLLM_EXPORT int pllm_delta_mix(int dtype, const void* u, int u_width, const void
         });
         if (blocks)
             launch_delta_blocks<T>((const float*)c_buf, channels, ba, a_log, dt_bias, (const T*)u, u_width, (const MMSegment*)segs, n_segs, state,
-                                   state_stride, conv_off, taps, db_buffers(block_buf, n_tokens, n_segs, H, d, E), y_buf, n_tokens, H, G, d, E, stream);
+                                   state_stride, conv_off, taps, db_buffers(block_buf, n_tokens, n_segs, longest, H, d, E), y_buf, n_tokens, H, G, d, E, longest, stream);
         launch_head_norm_gate<T>(y_buf, nullptr, (const T*)u + channels, u_width, gain, out, n_tokens, H, E, 0, 1, eps, stream);
     });
     return launch_status();

@@ -55,14 +55,15 @@ __device__ __forceinline__ f32x2 mm_fma2(f32x2 a, f32x2 b, f32x2 c) {
 // Block w of the step: the segments' blocks of L tokens one after the other.
 struct MMBlock {
     int seg, tb, blocks;       // segment, which of its blocks, how many it has (seg -1: no such block)
-    int rank;                  // its index among the blocks of segments of several blocks
+    int rank;                  // its index among the blocks of segments of more than `longest` tokens
 };
-__device__ __forceinline__ MMBlock mm_find_block(const MMSegment* __restrict__ segs, int n_segs, int w, int L) {
+// (longest: at least L)
+__device__ __forceinline__ MMBlock mm_find_block(const MMSegment* __restrict__ segs, int n_segs, int w, int L, int longest) {
     const int lane = threadIdx.x & 31;
     int seen = 0, several = 0;
     for (int base = 0; base < n_segs; base += 32) {
         const int c = base + lane < n_segs ? segs[base + lane].count : 0;
-        const int nb = c > 0 ? (c + L - 1) / L : 0, mb = nb > 1 ? nb : 0;
+        const int nb = c > 0 ? (c + L - 1) / L : 0, mb = c > longest ? nb : 0;
         int sum = nb, msum = mb;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {

@@ -19,7 +19,7 @@
 
 #include "matrix_memory.cuh"
 
-#define MB_L 64                // tokens a block; longer segments take this path
+#define MB_L 64                // tokens a block
 #define MB_C 64                // value columns a CTA
 #define MB_THREADS 256
 #define MB_MAX_D 256
@@ -30,15 +30,16 @@ struct MBBuffers {
     float* n;                  // [blocks][H][d], likewise
     float* decay;              // [blocks][H][2]: the block's decay, the m it starts from
 };
-static inline long long mb_blocks(int n_tokens, int n_segs) {
-    const int longer = n_tokens / (MB_L + 1);
+// (longest: the tokens of the longest segment that goes token by token; MB_L at least)
+static inline long long mb_blocks(int n_tokens, int n_segs, int longest) {
+    const int longer = n_tokens / (longest + 1);
     return n_tokens / MB_L + (n_segs < longer ? n_segs : longer) + 1;
 }
-static inline long long mb_floats(int n_tokens, int n_segs, int H, int d, int E) {
-    return mb_blocks(n_tokens, n_segs) * H * ((long long)d * E + d + 4) + 3LL * n_tokens * H + 16;
+static inline long long mb_floats(int n_tokens, int n_segs, int longest, int H, int d, int E) {
+    return mb_blocks(n_tokens, n_segs, longest) * H * ((long long)d * E + d + 4) + 3LL * n_tokens * H + 16;
 }
-static inline MBBuffers mb_buffers(float* at, int n_tokens, int n_segs, int H, int d, int E) {
-    const long long nb = mb_blocks(n_tokens, n_segs);
+static inline MBBuffers mb_buffers(float* at, int n_tokens, int n_segs, int longest, int H, int d, int E) {
+    const long long nb = mb_blocks(n_tokens, n_segs, longest);
     MBBuffers b;
     b.S = at;                                              // (16-byte rows: d and E are multiples of four)
     b.n = b.S + nb * H * d * E;
@@ -50,13 +51,13 @@ static inline MBBuffers mb_buffers(float* at, int n_tokens, int n_segs, int H, i
 // grid (segments, heads)
 __global__ void __launch_bounds__(MB_THREADS) mlstm_gates_kernel(const float* gates, const float* __restrict__ i_bias, const float* __restrict__ f_bias,
                                                                  float cap, const MMSegment* __restrict__ segs, const float* state,
-                                                                 long long state_stride, MBBuffers buf, int H, int d, int E) {
+                                                                 long long state_stride, MBBuffers buf, int H, int d, int E, int longest) {
     // eight warps scan 128 tokens each, then each takes what the warps before it left
     __shared__ double warp_F[MB_THREADS / 32], warp_M[MB_THREADS / 32], carry;
     const MMSegment s = segs[blockIdx.x];
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
-    if (s.count <= MB_L) return;
+    if (s.count <= longest) return;
     const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float bi = i_bias[h], bf = f_bias[h];
     double m = s.before > 0 ? (double)state[(size_t)s.slot * state_stride + (size_t)H * d * E + (size_t)H * d + h] : 0.0;
@@ -150,15 +151,16 @@ __device__ __forceinline__ void mb_rows(const T* src, long long stride, int nt, 
 // grid (blocks, heads, column tiles).  A thread has 4 x 4 entries of the state's change at a time: a chunk of k by a chunk of v.
 template <typename T>
 __global__ void __launch_bounds__(MB_THREADS) mlstm_contributions_kernel(const T* u, int u_width, const MMSegment* __restrict__ segs, int n_segs,
-                                                                         const float* state, long long state_stride, MBBuffers buf, int H, int d, int E) {
+                                                                         const float* state, long long state_stride, MBBuffers buf, int H, int d, int E, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     __shared__ MBTokens tk;
     __shared__ float w_s[MB_L];
-    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, MB_L);
+    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, MB_L, longest);
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
-    if (b.seg < 0 || b.blocks < 2) return;
+    if (b.seg < 0) return;
     const MMSegment s = segs[b.seg];
+    if (s.count <= longest) return;
     const int h = blockIdx.y, c0 = blockIdx.z * MB_C, begin = b.tb * MB_L, nt = min(MB_L, s.count - begin), dp = (d + 31) & ~31;
     const size_t tok0 = (size_t)s.first + begin;
     float* k_s = mm_smem;                        // [64][dp]
@@ -230,13 +232,13 @@ __global__ void __launch_bounds__(MB_THREADS) mlstm_contributions_kernel(const T
 
 // grid (segments, heads, runs of 256 entries of S and n)
 __global__ void __launch_bounds__(256) mlstm_starts_kernel(const MMSegment* __restrict__ segs, int n_segs, float* state, long long state_stride,
-                                                           MBBuffers buf, int H, int d, int E) {
+                                                           MBBuffers buf, int H, int d, int E, int longest) {
     const MMSegment s = segs[blockIdx.x];
     int rank = 0;
-    for (int i = 0; i < (int)blockIdx.x; i++) rank += segs[i].count > MB_L ? (segs[i].count + MB_L - 1) / MB_L : 0;
+    for (int i = 0; i < (int)blockIdx.x; i++) rank += segs[i].count > longest ? (segs[i].count + MB_L - 1) / MB_L : 0;
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
-    if (s.count <= MB_L) return;
+    if (s.count <= longest) return;
     const int blocks = (s.count + MB_L - 1) / MB_L, h = blockIdx.y;
     const long long i = blockIdx.z * 256LL + threadIdx.x, entries = (long long)d * E;
     if (i >= entries + d) return;
@@ -267,15 +269,17 @@ __global__ void __launch_bounds__(256) mlstm_starts_kernel(const MMSegment* __re
 // grid (blocks, heads, column tiles).  A thread has tokens ty + 16 a, and keys tx + 16 b or the columns 4 tx .. 4 tx + 3.
 template <typename T>
 __global__ void __launch_bounds__(MB_THREADS) mlstm_outputs_kernel(const T* u, int u_width, const MMSegment* __restrict__ segs, int n_segs,
-                                                                   MBBuffers buf, float* __restrict__ y, float* __restrict__ dn, int H, int d, int E) {
+                                                                   MBBuffers buf, float* __restrict__ y, float* __restrict__ dn, int H, int d, int E,
+                                                                   int longest) {
     extern __shared__ __align__(16) float mm_smem[];
     __shared__ MBTokens tk;
     __shared__ float a_s[MB_L];
-    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, MB_L);
+    const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, MB_L, longest);
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
-    if (b.seg < 0 || b.blocks < 2) return;
+    if (b.seg < 0) return;
     const MMSegment s = segs[b.seg];
+    if (s.count <= longest) return;
     const int h = blockIdx.y, c0 = blockIdx.z * MB_C, begin = b.tb * MB_L, nt = min(MB_L, s.count - begin), dp = (d + 31) & ~31;
     const size_t tok0 = (size_t)s.first + begin;
     float* q_s = mm_smem;                        // [64][dp]
@@ -409,25 +413,25 @@ __global__ void __launch_bounds__(MB_THREADS) mlstm_outputs_kernel(const T* u, i
     }
 }
 
-// Whether segments of more than MB_L tokens take this path: rows of whole vectors of four, keys that fit shared memory.
-static inline bool mb_takes(const void* u, int u_width, int d, int E, int max_segment_tokens) {
-    return max_segment_tokens > MB_L && d % 4 == 0 && d <= MB_MAX_D && E % 4 == 0 && u_width % 4 == 0 && ((uintptr_t)u & 15) == 0;
+// Whether segments of more than `longest` tokens take this path: rows of whole vectors of four, keys that fit shared memory.
+static inline bool mb_takes(const void* u, int u_width, int d, int E, int max_segment_tokens, int longest) {
+    return longest >= MB_L && max_segment_tokens > longest && d % 4 == 0 && d <= MB_MAX_D && E % 4 == 0 && u_width % 4 == 0 && ((uintptr_t)u & 15) == 0;
 }
 
 template <typename T>
 static void launch_mlstm_blocks(const T* u, int u_width, const float* gates, const float* i_bias, const float* f_bias, float cap,
                                 const MMSegment* segs, int n_segs, float* state, long long state_stride, const MBBuffers& buf, float* y, float* dn,
-                                int n_tokens, int H, int d, int E, cudaStream_t stream) {
+                                int n_tokens, int H, int d, int E, int longest, cudaStream_t stream) {
     const int dp = (d + 31) & ~31, blocks = n_tokens / MB_L + n_segs, tiles = (E + MB_C - 1) / MB_C;
     const size_t smem_c = (size_t)(MB_L * dp + MB_L * MB_C) * sizeof(float);
     const size_t smem_o = (size_t)(2 * MB_L * dp + 2 * MB_L * MB_C) * sizeof(float);
     cudaFuncSetAttribute(mlstm_contributions_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c);
     cudaFuncSetAttribute(mlstm_outputs_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o);
     launch_chained(mlstm_gates_kernel, dim3(n_segs, H), dim3(MB_THREADS), 0, stream, gates, i_bias, f_bias, cap, segs, (const float*)state,
-                   state_stride, buf, H, d, E);
+                   state_stride, buf, H, d, E, longest);
     launch_chained(mlstm_contributions_kernel<T>, dim3(blocks, H, tiles), dim3(MB_THREADS), smem_c, stream, u, u_width, segs, n_segs,
-                   (const float*)state, state_stride, buf, H, d, E);
+                   (const float*)state, state_stride, buf, H, d, E, longest);
     launch_chained(mlstm_starts_kernel, dim3(n_segs, H, (unsigned)(((long long)d * E + d + 255) / 256)), dim3(256), 0, stream, segs, n_segs, state,
-                   state_stride, buf, H, d, E);
-    launch_chained(mlstm_outputs_kernel<T>, dim3(blocks, H, tiles), dim3(MB_THREADS), smem_o, stream, u, u_width, segs, n_segs, buf, y, dn, H, d, E);
+                   state_stride, buf, H, d, E, longest);
+    launch_chained(mlstm_outputs_kernel<T>, dim3(blocks, H, tiles), dim3(MB_THREADS), smem_o, stream, u, u_width, segs, n_segs, buf, y, dn, H, d, E, longest);
 }

@@ -115,8 +115,8 @@ def lib():
         sig["pllm_conv_rope_kv_write"] = [c_int, P, c_int, P, P, c_int, P, c_int, c_int, P, c_ll, P, c_int, P, P, P, P] + [c_int] * 6 + [c_ll, P, P]
         sig["pllm_diff_combine"] = [c_int, P, P, c_int, P] + [c_int] * 4 + [c_float] * 3 + [P]
         sig["pllm_latent_rope_write"] = [c_int, P, c_int, P, c_float, P, c_int, P, P, P, P, P, P, P] + [c_int] * 6 + [c_ll, P, P]
-        sig["pllm_mlstm_mix"] = [c_int, P, c_int, P, P, P, c_float, P, P, c_int, c_int, P, c_ll, P, P, P, P, c_ll, P] + [c_int] * 4 + [c_float, P]
-        sig["pllm_delta_mix"] = [c_int, P, c_int, P, P, P, P, P, P, c_int, c_int, P, c_ll, P, P, P, c_ll, P] + [c_int] * 6 + [c_float, P]
+        sig["pllm_mlstm_mix"] = [c_int, P, c_int, P, P, P, c_float, P, P, c_int, c_int, P, c_ll, P, P, P, P, c_ll, c_int, P] + [c_int] * 4 + [c_float, P]
+        sig["pllm_delta_mix"] = [c_int, P, c_int, P, P, P, P, P, P, c_int, c_int, P, c_ll, P, P, P, c_ll, c_int, P] + [c_int] * 6 + [c_float, P]
         sig["pllm_gated_sum_norm32"] = [c_int, P, P, c_int, c_float, P, c_int, c_float, P, c_int, P, P, c_int, P, c_int, P, P, P, P, P, P, P, P, P, P, P,
                                         c_int, P, c_ll, P, c_int, c_int, c_float, P]
         sig["pllm_poly_norm"] = [c_int, P, c_int, P, P, c_int, c_int, c_float, P]
@@ -129,7 +129,7 @@ def lib():
                                          P] + [c_int] * 6 + [c_float, P]
         wide = {"pllm_channel_delta_state_floats": [c_int] * 5, "pllm_channel_delta_record_floats": [c_int] * 4,
                 "pllm_linear_attention_state_floats": [c_int] * 3, "pllm_linear_attention_scratch_floats": [c_int] * 6,
-                "pllm_mlstm_state_floats": [c_int] * 3, "pllm_mlstm_block_floats": [P] + [c_int] * 7, "pllm_delta_block_floats": [c_int] * 7, "pllm_delta_state_floats": [c_int] * 5}
+                "pllm_mlstm_state_floats": [c_int] * 3, "pllm_mlstm_block_floats": [P] + [c_int] * 8, "pllm_delta_block_floats": [c_int] * 8, "pllm_delta_state_floats": [c_int] * 5}
         for name, args in wide.items():
             fn = getattr(L, name)
             fn.argtypes = args
@@ -1406,11 +1406,11 @@ def mlstm_mix(u: torch.Tensor, gates: torch.Tensor, i_bias: torch.Tensor, f_bias
     dn_buf = torch.zeros((T, heads, 2), dtype=torch.float32, device=u.device)
     nm_buf = torch.empty((segments.shape[0], heads, dim + 1), dtype=torch.float32, device=u.device)
     # longer segments run in blocks of tokens (csrc/mlstm_blocks.cuh), four kernels more
-    floats = lib().pllm_mlstm_block_floats(_ptr(u), u.shape[1], T, segments.shape[0], int(max_segment_tokens), heads, dim, vdim) if MLSTM_BLOCKS else 0
+    floats = lib().pllm_mlstm_block_floats(_ptr(u), u.shape[1], T, segments.shape[0], int(max_segment_tokens), MLSTM_LONGEST, heads, dim, vdim) if MLSTM_BLOCKS else 0
     blocks = torch.empty(floats, dtype=torch.float32, device=u.device) if floats else None
     _check(lib().pllm_mlstm_mix(_code(u), _ptr(u), u.shape[1], _ptr(gates), _ptr(i_bias), _ptr(f_bias), float(cap), _ptr(gain),
                                 _ptr(segments), segments.shape[0], int(max_segment_tokens), _ptr(state), state.stride(0), _ptr(nm_buf),
-                                _ptr(dn_buf), _ptr(y_buf), _ptr(blocks), floats, _ptr(out), T, heads, dim, vdim, float(eps), _stream()),
+                                _ptr(dn_buf), _ptr(y_buf), _ptr(blocks), floats, MLSTM_LONGEST, _ptr(out), T, heads, dim, vdim, float(eps), _stream()),
            "mlstm_mix", launches=7 if floats else 3)
     return out
 
@@ -1428,6 +1428,10 @@ def delta_mix(u: torch.Tensor, conv_w: torch.Tensor, ba: torch.Tensor, a_log: to
     _dev(u, conv_w, ba, a_log, dt_bias, gain, segments, state, out)
     for t, n in ((ba, "ba"), (a_log, "a_log"), (dt_bias, "dt_bias"), (gain, "gain"), (state, "state")):
         _f32(t, n)
+# Tokens of the longest segment that goes token by token: blocks cost four kernels whatever the length.  One segment of 256 / 384 / 512 / 1000
+# tokens on a B200, us token by token and in blocks: 4 heads of 128 x 256 40 / 55 / 70 / 127 and 56 / 57 / 57 / 64, 16 heads 66 / 96 / 123 / 231 and
+# 66 / 94 / 114 / 201; four segments of 512 beside one another, 8 heads: 205 either way, of 384: 158 and 167.
+MLSTM_LONGEST = 512
     _segments_ok(segments, "delta_mix")
     T = u.shape[0]
     channels = 2 * kv_heads * dim + heads * vdim
@@ -1442,11 +1446,11 @@ def delta_mix(u: torch.Tensor, conv_w: torch.Tensor, ba: torch.Tensor, a_log: to
     c_buf = torch.empty((T, channels), dtype=torch.float32, device=u.device)
     y_buf = torch.zeros((T, heads * vdim), dtype=torch.float32, device=u.device)     # (rows of no segment stay zero)
     # longer segments run in blocks of tokens (csrc/delta_blocks.cuh), three kernels more and one for the convolution's state
-    floats = lib().pllm_delta_block_floats(T, segments.shape[0], int(max_segment_tokens), heads, kv_heads, dim, vdim) if DELTA_BLOCKS else 0
+    floats = lib().pllm_delta_block_floats(T, segments.shape[0], int(max_segment_tokens), DELTA_LONGEST, heads, kv_heads, dim, vdim) if DELTA_BLOCKS else 0
     blocks = torch.empty(floats, dtype=torch.float32, device=u.device) if floats else None
     _check(lib().pllm_delta_mix(_code(u), _ptr(u), u.shape[1], _ptr(conv_w), _ptr(ba), _ptr(a_log), _ptr(dt_bias), _ptr(gain),
                                 _ptr(segments), segments.shape[0], int(max_segment_tokens), _ptr(state), state.stride(0), _ptr(c_buf),
-                                _ptr(y_buf), _ptr(blocks), floats, _ptr(out), T, heads, kv_heads, dim, vdim, taps, float(eps), _stream()),
+                                _ptr(y_buf), _ptr(blocks), floats, DELTA_LONGEST, _ptr(out), T, heads, kv_heads, dim, vdim, taps, float(eps), _stream()),
            "delta_mix", launches=3 if not floats else 7 if taps > 1 else 6)
     return out
 
@@ -1462,6 +1466,9 @@ def channel_delta_mix(u: torch.Tensor, conv_w: torch.Tensor, small: torch.Tensor
                       dt_bias: torch.Tensor, g1_off: int, g2: torch.Tensor, gain: torch.Tensor, segments: torch.Tensor,
                       max_segment_tokens: int, state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int,
                       taps: int, eps: float, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+# Likewise: 8 heads of 128 x 128 over 4 key heads 92 / 127 / 162 / 296 token by token and 115 / 125 / 133 / 171 in blocks, 32 over 16 138 / 197 / 255 / 487
+# and 138 / 188 / 226 / 429; four segments of 384 of 16 heads: 384 and 346.
+DELTA_LONGEST = 384
     """From a projection ``u`` [T, width] whose first columns are [q | k | v] (kv_heads dim, kv_heads dim, heads vdim) and a float32
     projection ``small`` [T, width] (step sizes' logits in its first ``heads`` columns, the decays' short vector at a1_off) to the
     output projection's input [T, heads vdim]: convolution and silu, unit q and k, decays exp(-exp(a_log) softplus(a2 a1 + dt_bias))

@@ -37,9 +37,9 @@ def plain(u, gates, ib, fb, gain, H, d, E):
     return out.reshape(T, H * E) * after, ((d + 80) * 2.0 ** -24 * off + 4 * 2.0 ** -24 * out.abs()).reshape(T, H * E) * after.abs()
 
 
-def steps(blocks, dtype, cuts, seqs, ib, fb, gain, H, d, E):
+def steps(blocks, dtype, cuts, seqs, ib, fb, gain, H, d, E, longest=64):
     """Every sequence through ``cuts`` steps: cuts[s] lists the tokens each takes in step s (0: it is not in the step)."""
-    ops.MLSTM_BLOCKS = blocks
+    was, ops.MLSTM_BLOCKS, ops.MLSTM_LONGEST = ops.MLSTM_LONGEST, blocks, longest       # (blocks from the first length that has two)
     try:
         state = torch.full((len(seqs) + 1, ops.mlstm_state_floats(H, d, E)), 7.0, device=DEV)       # (whatever an older request left)
         done, outs = [0] * len(seqs), [[] for _ in seqs]
@@ -59,7 +59,7 @@ def steps(blocks, dtype, cuts, seqs, ib, fb, gain, H, d, E):
                 done[r] += n
         return [torch.cat(o) for o in outs]
     finally:
-        ops.MLSTM_BLOCKS = True
+        ops.MLSTM_BLOCKS, ops.MLSTM_LONGEST = True, was
 
 
 @pytest.mark.parametrize("H,d,E", [(2, 8, 4), (1, 36, 68), (4, 128, 256), (1, 256, 64)])
@@ -103,8 +103,8 @@ def plain_delta(u, conv_w, ba, a_log, dt, gain, H, G, d, E):
     return o.reshape(T, H * E) * P.silu(u[:, c:].double())
 
 
-def delta_steps(blocks, dtype, cuts, seqs, conv_w, a_log, dt, gain, H, G, d, E, most=max):
-    ops.DELTA_BLOCKS = blocks
+def delta_steps(blocks, dtype, cuts, seqs, conv_w, a_log, dt, gain, H, G, d, E, most=max, longest=64):
+    was, ops.DELTA_BLOCKS, ops.DELTA_LONGEST = ops.DELTA_LONGEST, blocks, longest
     try:
         taps = conv_w.shape[1]
         state = torch.full((len(seqs) + 1, ops.delta_state_floats(H, G, d, E, taps)), 7.0, device=DEV)
@@ -125,7 +125,7 @@ def delta_steps(blocks, dtype, cuts, seqs, conv_w, a_log, dt, gain, H, G, d, E, 
                 done[r] += n
         return [torch.cat(o) for o in outs]
     finally:
-        ops.DELTA_BLOCKS = True
+        ops.DELTA_BLOCKS, ops.DELTA_LONGEST = True, was
 
 
 @pytest.mark.parametrize("H,G,d,E,taps", [(2, 1, 8, 4, 4), (1, 1, 36, 68, 3), (8, 4, 128, 128, 4), (2, 2, 64, 200, 6), (1, 1, 16, 16, 1)])
@@ -189,3 +189,32 @@ def test_the_delta_rule_takes_segments_of_unknown_length(n):
     a, b = (delta_steps(False, torch.float32, [(n,)], [(u, ba)], conv_w, *rest, most=most)[0] for most in (lambda cut: 0, max))
     want = plain_delta(u, conv_w, ba, *rest)
     assert torch.equal(a, b) and float((a.double() - want).norm() / want.norm()) <= 2e-6
+
+
+@pytest.mark.parametrize("tokens,longest", [(64, 64), (512, 512), (384, 512)])
+def test_segments_up_to_the_longest_go_token_by_token(tokens, longest):
+    L = ops.lib()
+    assert L.pllm_mlstm_block_floats(None, 4 * 768, 2000, 3, tokens, longest, 4, 128, 256) == 0
+    assert L.pllm_delta_block_floats(2000, 3, tokens, longest, 8, 4, 128, 128) == 0
+    assert L.pllm_mlstm_block_floats(None, 4 * 768, 2000, 3, longest + 1, longest, 4, 128, 256) > 0
+    assert L.pllm_delta_block_floats(2000, 3, longest + 1, longest, 8, 4, 128, 128) > 0
+
+
+@pytest.mark.parametrize("cut", [(70, 300, 90, 512, 40), (513, 100, 640, 385, 3)])
+def test_a_step_of_segments_on_both_sides_of_the_longest(cut):
+    # (at the lengths the engine uses: some go token by token beside others in blocks, and each keeps its own state)
+    H, d, E, G, taps = 2, 32, 64, 2, 4
+    g = torch.Generator().manual_seed(sum(cut))
+    one = torch.zeros(H), torch.zeros(H), torch.ones(H * E)
+    seqs = [(torch.randn(n, H * (2 * d + 2 * E), generator=g), torch.randn(n, 2 * H, generator=g)) for n in cut]
+    was = ops.MLSTM_LONGEST, ops.DELTA_LONGEST
+    assert min(was) >= 384
+    for got, (u, gt) in zip(steps(True, torch.float32, [cut], seqs, *one, H, d, E, longest=was[0]), seqs):
+        want, off = plain(u, gt, *one, H, d, E)
+        assert ((got.double() - want).abs() <= off).all()
+    c = 2 * G * d + H * E
+    seqs = [(torch.randn(n, c + H * E, generator=g), torch.randn(n, 2 * H, generator=g)) for n in cut]
+    conv_w, rest = torch.rand(c, taps, generator=g), (torch.zeros(H), torch.zeros(H), torch.ones(E), H, G, d, E)
+    for got, (u, ba) in zip(delta_steps(True, torch.float32, [cut], seqs, conv_w, *rest, longest=was[1]), seqs):
+        want = plain_delta(u, conv_w, ba, *rest)
+        assert float((got.double() - want).norm() / want.norm()) <= 2e-6
