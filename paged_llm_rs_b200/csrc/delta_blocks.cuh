@@ -11,7 +11,7 @@
 //   delta_states_kernel   a head's 16 columns of S through the blocks of a segment
 //   delta_outputs_kernel  the outputs
 // Sums of log g and their differences are formed in double; everything else is float,
-// as in the recurrence, whose every write the forward substitution repeats in the same order.  No decay is divided by.
+// as in the recurrence, whose every write the forward substitution repeats.  No decay is divided by.
 //
 // What bounds the recurrence is its chain (440 ns a token and head); what bounds the blocks is delta_states_kernel's chain, a few
 // microseconds a block of 64 tokens.  1016 tokens beside 8 decoded ones, 8 heads of 128 x 128 over 4 key heads (us, caches cold): the
@@ -84,25 +84,38 @@ __device__ __forceinline__ void db_tokens(DBTokens& tk, const float* ba, size_t 
         before = __shfl_sync(0xffffffffu, G, 31);
     }
 }
-// acc[r][e] = rows ty + 16 r of a times rows tx + 16 e of b, both [64][dp] swizzled
+// out[r][e] = rows ty + 16 r of a times rows tx + 16 e of b, both [64][dp] swizzled.  A sum is four of every fourth entry, in runs of eight
+// products that are added up when they are complete: one chain over all entries was off by half as much again as the recurrence's warp-wide sums.
 __device__ __forceinline__ void db_product(const float* a, const float* b, int dp, int chunks, int tx, int ty, float (&out)[4][4]) {
     f32x2 acc[4][4];
+    const f32x2 one = mm_pair(1.f, 1.f), zero = mm_pair(0.f, 0.f);
 #pragma unroll
     for (int r = 0; r < 4; r++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc[r][e] = mm_pair(0.f, 0.f);
-#pragma unroll 2
-    for (int c = 0; c < chunks; c++) {
-        ulonglong2 x[4];
+        for (int e = 0; e < 4; e++) acc[r][e] = zero;
+    for (int c0 = 0; c0 < chunks; c0 += 8) {
+        f32x2 lo[4][4], hi[4][4];
 #pragma unroll
-        for (int r = 0; r < 4; r++) { const int t = ty + 16 * r; x[r] = *reinterpret_cast<const ulonglong2*>(a + t * dp + ((c ^ (t & 7)) << 2)); }
+        for (int r = 0; r < 4; r++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int t = tx + 16 * e;
-            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b + t * dp + ((c ^ (t & 7)) << 2));
+            for (int e = 0; e < 4; e++) lo[r][e] = hi[r][e] = zero;
+        const int c1 = min(c0 + 8, chunks);
+        for (int c = c0; c < c1; c++) {
+            ulonglong2 x[4];
 #pragma unroll
-            for (int r = 0; r < 4; r++) { acc[r][e] = mm_fma2(x[r].x, y.x, acc[r][e]); acc[r][e] = mm_fma2(x[r].y, y.y, acc[r][e]); }
+            for (int r = 0; r < 4; r++) { const int t = ty + 16 * r; x[r] = *reinterpret_cast<const ulonglong2*>(a + t * dp + ((c ^ (t & 7)) << 2)); }
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int t = tx + 16 * e;
+                const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b + t * dp + ((c ^ (t & 7)) << 2));
+#pragma unroll
+                for (int r = 0; r < 4; r++) { lo[r][e] = mm_fma2(x[r].x, y.x, lo[r][e]); hi[r][e] = mm_fma2(x[r].y, y.y, hi[r][e]); }
+            }
         }
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[r][e] = mm_fma2(one, mm_fma2(one, lo[r][e], hi[r][e]), acc[r][e]);
     }
 #pragma unroll
     for (int r = 0; r < 4; r++)
@@ -111,7 +124,7 @@ __device__ __forceinline__ void db_product(const float* a, const float* b, int d
 }
 
 // grid (blocks, heads).  c: [tokens, channels] float, q at 0 (G d), k at G d, v at 2 G d (H E); ba: [tokens, 2 H], b_raw | a_raw.
-__global__ void __launch_bounds__(DB_THREADS) delta_solve_kernel(const float* c, int channels, const float* ba, const float* __restrict__ a_log,
+__global__ void __launch_bounds__(DB_THREADS, 2) delta_solve_kernel(const float* c, int channels, const float* ba, const float* __restrict__ a_log,
                                                                  const float* __restrict__ dt_bias, const MMSegment* __restrict__ segs, int n_segs,
                                                                  DBBuffers buf, int H, int G, int d, int E, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
@@ -119,8 +132,9 @@ __global__ void __launch_bounds__(DB_THREADS) delta_solve_kernel(const float* c,
     const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DB_L, longest);
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
-    if (b.seg < 0 || b.blocks < 2) return;
+    if (b.seg < 0) return;
     const MMSegment s = segs[b.seg];
+    if (s.count <= longest) return;
     const int h = blockIdx.y, kh = h / (H / G), begin = b.tb * DB_L, nt = min(DB_L, s.count - begin), dp = (d + 31) & ~31;
     const size_t tok0 = (size_t)s.first + begin;
     const int cols = d + E;
@@ -134,14 +148,13 @@ __global__ void __launch_bounds__(DB_THREADS) delta_solve_kernel(const float* c,
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     {
         float kk[4][4];
-    if (s.count <= longest) return;
         db_product(k_s, k_s, dp, d / 4, tx, ty, kk);
 #pragma unroll
         for (int r = 0; r < 4; r++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const int t = ty + 16 * r, o = tx + 16 * e;
-                A_s[t * DB_L + o] = o < t ? tk.beta[t] * mb_exp(tk.G[t] - tk.G[o]) * kk[r][e] : 0.f;
+                A_s[t * DB_L + o] = o < t ? mb_exp(tk.G[t] - tk.G[o]) * kk[r][e] : 0.f;
             }
     }
     const double GL = tk.G[DB_L - 1];
@@ -149,42 +162,50 @@ __global__ void __launch_bounds__(DB_THREADS) delta_solve_kernel(const float* c,
     for (int i = threadIdx.x; i < DB_L * d; i += DB_THREADS) {
         const int t = i / d, n = i % d;
         const float k = k_s[t * dp + (((n >> 2) ^ (t & 7)) << 2) + (n & 3)];
-        R_s[t * cols + n] = tk.beta[t] * mb_exp(tk.G[t]) * k;
+        R_s[t * cols + n] = mb_exp(tk.G[t]) * k;
         kd[i] = mb_exp(GL - tk.G[t]) * k;
     }
     for (int i = threadIdx.x; i < DB_L * E; i += DB_THREADS) {
         const int t = i / E, e = i % E;
-        R_s[t * cols + d + e] = t < nt ? tk.beta[t] * row[(size_t)t * channels + 2 * (size_t)G * d + (size_t)h * E + e] : 0.f;
+        R_s[t * cols + d + e] = t < nt ? row[(size_t)t * channels + 2 * (size_t)G * d + (size_t)h * E + e] : 0.f;
     }
     if (threadIdx.x == 0) buf.decay[(size_t)b.rank * H + h] = mb_exp(GL);
     __syncthreads();
-    // a thread a column: sixteen rows are solved in registers, then taken off the rows below
+    // A thread a column, sixteen rows at a time: what the rows above them take off, in two sums each (of the even and of the odd rows), then what
+    // they take off one another.  Both are formed apart from the right side, which is rounded once at its own size, as in the recurrence
+    // (taken off one product at a time it was rounded sixteen times); beta comes last.
     float* W = buf.W + ((size_t)b.rank * H + h) * DB_L * d;
     float* U = buf.U + ((size_t)b.rank * H + h) * DB_L * E;
     for (int col = threadIdx.x; col < cols; col += DB_THREADS) {
+        float* out = col < d ? W + col : U + (col - d);
+        const int pitch = col < d ? d : E;
         for (int r0 = 0; r0 < DB_L; r0 += 16) {
+            f32x2 s2[16];
+#pragma unroll
+            for (int t = 0; t < 16; t++) s2[t] = mm_pair(0.f, 0.f);
+            for (int o = 0; o < r0; o += 4) {
+                const f32x2 x0 = mm_pair(R_s[o * cols + col], R_s[(o + 1) * cols + col]), x1 = mm_pair(R_s[(o + 2) * cols + col], R_s[(o + 3) * cols + col]);
+#pragma unroll
+                for (int t = 0; t < 16; t++) {
+                    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(A_s + (r0 + t) * DB_L + o);
+                    s2[t] = mm_fma2(a.x, x0, s2[t]);
+                    s2[t] = mm_fma2(a.y, x1, s2[t]);
+                }
+            }
             float x[16];
 #pragma unroll
             for (int t = 0; t < 16; t++) {
-                float v = R_s[(r0 + t) * cols + col];
+                const float* a = A_s + (r0 + t) * DB_L + r0;
+                float in = 0.f;
 #pragma unroll
                 for (int o = 0; o < 16; o++)
-                    if (o < t) v = fmaf(-A_s[(r0 + t) * DB_L + r0 + o], x[o], v);
-                x[t] = v;
-                if (col < d) W[(r0 + t) * d + col] = v;
-                else U[(r0 + t) * E + col - d] = v;
+                    if (o < t) in = fmaf(a[o], x[o], in);
+                const float2 v = mm_unpair(s2[t]);
+                x[t] = tk.beta[r0 + t] * (R_s[(r0 + t) * cols + col] - ((v.x + v.y) + in));
+                out[(r0 + t) * pitch] = x[t];
             }
-            for (int t = r0 + 16; t < DB_L; t++) {
-                // (four short sums, so that a row is rounded at its own size four times here and not sixteen)
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4* a = reinterpret_cast<const float4*>(A_s + t * DB_L + r0);
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float4 w = a[q];
-                    v.x = fmaf(w.x, x[4 * q], v.x); v.y = fmaf(w.y, x[4 * q + 1], v.y); v.z = fmaf(w.z, x[4 * q + 2], v.z); v.w = fmaf(w.w, x[4 * q + 3], v.w);
-                }
-                R_s[t * cols + col] -= (v.x + v.y) + (v.z + v.w);
-            }
+            for (int t = 0; t < 16; t++) R_s[(r0 + t) * cols + col] = x[t];
         }
     }
 }
@@ -319,7 +340,7 @@ __global__ void __launch_bounds__(DB_THREADS) delta_states_kernel(const MMSegmen
 }
 
 // grid (blocks, heads, column tiles).  A thread has tokens ty + 16 a, and keys tx + 16 b or the columns 4 tx .. 4 tx + 3.
-__global__ void __launch_bounds__(DB_THREADS) delta_outputs_kernel(const float* c, int channels, const float* ba, const float* __restrict__ a_log,
+__global__ void __launch_bounds__(DB_THREADS, 2) delta_outputs_kernel(const float* c, int channels, const float* ba, const float* __restrict__ a_log,
                                                                    const float* __restrict__ dt_bias, const MMSegment* __restrict__ segs, int n_segs,
                                                                    DBBuffers buf, float* __restrict__ y, int H, int G, int d, int E, int longest) {
     extern __shared__ __align__(16) float mm_smem[];
@@ -328,8 +349,9 @@ __global__ void __launch_bounds__(DB_THREADS) delta_outputs_kernel(const float* 
     const MMBlock b = mm_find_block(segs, n_segs, blockIdx.x, DB_L, longest);
     pdl_launch_dependents();
     pdl_wait(KID_MATRIX_MEMORY);
-    if (b.seg < 0 || b.blocks < 2) return;
+    if (b.seg < 0) return;
     const MMSegment s = segs[b.seg];
+    if (s.count <= longest) return;
     const int h = blockIdx.y, kh = h / (H / G), c0 = blockIdx.z * DB_C, begin = b.tb * DB_L, nt = min(DB_L, s.count - begin), dp = (d + 31) & ~31;
     const size_t tok0 = (size_t)s.first + begin;
     float* q_s = mm_smem;                        // [64][dp]
@@ -351,7 +373,6 @@ __global__ void __launch_bounds__(DB_THREADS) delta_outputs_kernel(const float* 
         for (int r = 0; r < 4; r++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-    if (s.count <= longest) return;
                 const int t = ty + 16 * r, o = tx + 16 * e;
                 p_s[t * DB_L + o] = o <= t ? mb_exp(tk.G[t] - tk.G[o]) * qk[r][e] : 0.f;
             }
