@@ -431,7 +431,8 @@ PLLM_EXPORT int pllm_swiglu_bias(int dtype, const void* in, const float* bias, v
     if (n_rows <= 0) return PLLM_OK;
     if (act < GLU_SILU || act > GLU_CLAMPED || inter <= 0 || bias == nullptr) return PLLM_ERR_SIZE;
     PLLM_DISPATCH_DTYPE(dtype, {
-        if (inter % Vec16<T>::N == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0) {
+        // (bfloat16 from some hundred thousand entries on: 64 rows of 1024 take 1.9 us this way and 1.7 an entry at a time, 64 of 2048 1.9 and 2.3)
+        if (inter % Vec16<T>::N == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0 && (sizeof(T) == 4 || (long long)n_rows * inter >= 1 << 17)) {
             // (up to eight rows a CTA where that still makes sixteen CTAs an SM)
             const int across = (inter / Vec16<T>::N + 127) / 128;
             int rows = 1;
