@@ -123,14 +123,14 @@ __global__ void attention_sink_kernel(const T* q,                 // [tokens, nh
     pdl_launch_dependents();
     pdl_wait(KID_ATT_SINK);
     // (an item's CTAs are neighbours in the grid: with the items running fastest, a step of 74 of them and 8 kv heads dealt every SM
-    // the same item four times, the longest to some and none to others)
+    // the same item four times, the longest to some and none to others.  They run along x and the items along y and z: formed by a division,
+    // the item and its CTA cost the loops ten registers, and with them the second CTA of an SM)
     const int group = nh / nkv;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
-    const int item = blockIdx.x / (nkv * gparts), cta = blockIdx.x % (nkv * gparts);
-    if (item >= *n_work_ptr) return;
-    const SinkWork w = work[item];
-    const int kh = cta / gparts;
-    const int head0 = kh * group + (cta % gparts) * heads_per_cta;
+    if ((int)(blockIdx.z * gridDim.y + blockIdx.y) >= *n_work_ptr) return;
+    const SinkWork w = work[blockIdx.z * gridDim.y + blockIdx.y];
+    const int kh = blockIdx.x / gparts;
+    const int head0 = kh * group + (blockIdx.x % gparts) * heads_per_cta;
     const int n_heads = min(heads_per_cta, kh * group + group - head0);
     const int rows = w.q_count * n_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -271,6 +271,11 @@ __global__ void attention_sink_kernel(const T* q,                 // [tokens, nh
     }
 }
 
+// (rows of k_s and v_s start on 16-byte boundaries when dk and dv are multiples of 4; otherwise only scalar reads are made)
+static inline size_t sink_float_smem(int dk, int dv) {
+    return ((size_t)SINK_MAX_ROWS * dk + (size_t)SINK_BK * (dk + 4) + (size_t)SINK_BK * (dv + 4)) * sizeof(float);
+}
+
 PLLM_EXPORT int pllm_attention_sink(int dtype, const void* q, const void* kv_pool, const int* block_tables, const int* work,
                                     const int* n_work_ptr, int max_work, void* out, float* part_o, float* part_ml,
                                     const float* sinks, int nh, int nkv, int dk, int dv, int page_size, int n_pages, int table_width,
@@ -282,11 +287,11 @@ PLLM_EXPORT int pllm_attention_sink(int dtype, const void* q, const void* kv_poo
     const int group = nh / nkv;
     const int heads_per_cta = group < SINK_MAX_ROWS ? group : SINK_MAX_ROWS;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
-    // (rows of k_s and v_s start on 16-byte boundaries when dk and dv are multiples of 4; otherwise only scalar reads are made)
-    const size_t smem = ((size_t)SINK_MAX_ROWS * dk + (size_t)SINK_BK * (dk + 4) + (size_t)SINK_BK * (dv + 4)) * sizeof(float);
+    const size_t smem = sink_float_smem(dk, dv);
     PLLM_DISPATCH_DTYPE(dtype, {
         cudaFuncSetAttribute(attention_sink_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dim3 grid((unsigned)max_work * nkv * gparts);
+        const int across = max_work < 32768 ? max_work : 32768;
+        const dim3 grid(nkv * gparts, across, (max_work + across - 1) / across);
         launch_chained(attention_sink_kernel<T>, grid, dim3(SINK_MAX_ROWS * 32), smem, stream, (const T*)q, (const T*)kv_pool,
                        block_tables, (const SinkWork*)work, n_work_ptr, (T*)out, part_o, part_ml, sinks, nh, nkv, dk, dv, page_size,
                        n_pages, table_width, window, keep_first, chunk, scale, cap, heads_per_cta, status);
@@ -662,3 +667,16 @@ PLLM_EXPORT int pllm_attention_sink_tile_tokens(int nh, int nkv) {
 }
 
 PLLM_TRACE_EXPORT(attention_sink)
+// CTAs of attention_sink_kernel that an SM holds at the same time.
+PLLM_EXPORT int pllm_attention_sink_ctas_per_sm(int dtype, int dk, int dv) {
+    int n = 0;
+    PLLM_DISPATCH_DTYPE(dtype, {
+        cudaFuncSetAttribute(attention_sink_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sink_float_smem(dk, dv));
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attention_sink_kernel<T>, SINK_MAX_ROWS * 32, sink_float_smem(dk, dv)) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+    });
+    return n;
+}
+

@@ -100,6 +100,7 @@ def lib():
         sig["pllm_rope_mix_kv_write"] = [c_int, P, c_int, P, P, c_int, P, P, P, P, c_int, P] + [c_int] * 6 + [c_ll, P, P]
         sig["pllm_attention_sink"] = [c_int, P, P, P, P, P, c_int, P, P, P, P] + [c_int] * 10 + [c_float, c_float, P, P]
         sig["pllm_attention_sink_tile_tokens"] = [c_int, c_int]
+        sig["pllm_attention_sink_ctas_per_sm"] = [c_int, c_int, c_int]
         sig["pllm_attention_sink_mma_supports"] = [c_int] * 5
         sig["pllm_attention_sink_mma_tile_tokens"] = [c_int, c_int]
         sig["pllm_attention_sink_mma"] = [P, P, P, P, P, c_int, P, P, P, P] + [c_int] * 10 + [c_float, c_float, P, P]

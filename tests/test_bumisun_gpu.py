@@ -266,6 +266,13 @@ def test_attention_mixed_batch(dtype, nh, nkv, dk, dv, page, window, keep, cap):
         close(got, want, dtype, f"request {i}", f32=3e-5, bf16=2.5e-2)
 
 
+@pytest.mark.parametrize("code", [0, 1])
+def test_two_ctas_of_the_cuda_core_attention_fit_an_sm(code):
+    # (512 threads each: more than 64 registers a thread leave room for one, which takes nearly twice as long)
+    for dk, dv in ((128, 64), (48, 80), (128, 128)):
+        assert ops_().lib().pllm_attention_sink_ctas_per_sm(code, dk, dv) >= 2
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nh,nkv,dk,dv,window,keep", [(6, 2, 16, 8, 20, 3), (8, 4, 128, 64, 48, 5), (4, 1, 32, 24, 64, 17), (5, 5, 12, 6, 16, 16)])
 def test_one_key_decides_at_every_edge(dtype, nh, nkv, dk, dv, window, keep):
