@@ -339,8 +339,8 @@ __device__ __forceinline__ uint32_t sink_pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template <int DK, int DV>
-__global__ void __launch_bounds__(128, (DK + DV <= 128) ? 4 : 3) attention_sink_mma_kernel(const bf16* q, const bf16* kv_pool, const int* __restrict__ block_tables,
+template <int DK, int DV, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) attention_sink_mma_kernel(const bf16* q, const bf16* kv_pool, const int* __restrict__ block_tables,
                                                                  const SinkWork* __restrict__ work, const int* __restrict__ n_work_ptr,
                                                                  bf16* __restrict__ out, float* __restrict__ part_o,
                                                                  float* __restrict__ part_ml, const float* __restrict__ sinks, int nh,
@@ -625,7 +625,7 @@ PLLM_EXPORT int pllm_attention_sink_mma_tile_tokens(int nh, int nkv) {
 template <int DK, int DV>
 static int launch_sink_mma(const void* q, const void* kv_pool, const int* block_tables, const int* work, const int* n_work_ptr, int max_work,
                            void* out, float* part_o, float* part_ml, const float* sinks, int nh, int nkv, int page_size, int n_pages,
-                           int table_width, int window, int keep_first, int chunk, float scale, float cap, int* status, cudaStream_t stream) {
+                           int table_width, int window, int keep_first, int chunk, int single_ctas, float scale, float cap, int* status, cudaStream_t stream) {
     const int group = nh / nkv;
     const int heads_per_cta = group < SMMA_ROWS ? group : SMMA_ROWS;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
@@ -634,24 +634,32 @@ static int launch_sink_mma(const void* q, const void* kv_pool, const int* block_
     if (tiles < meet) tiles = meet;
     const size_t queries = (size_t)SMMA_ROWS * (DK + SMMA_PAD) * sizeof(bf16);     // (in registers before the first tile lands on them)
     const size_t smem = tiles > queries ? tiles : queries;
-    cudaFuncSetAttribute(attention_sink_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_chained(attention_sink_mma_kernel<DK, DV>, dim3((unsigned)max_work * nkv * gparts), dim3(128), smem, stream, (const bf16*)q,
+    // Keys and values of more than 128 entries in all: three CTAs an SM, whose registers the loop over many keys likes.  Four where that makes
+    // one turn of a step of single tokens that would be two (64 requests over 8 kv heads, 128 / 64: 74 us at context 1024 with three, 56 with four;
+    // a chunk's first token 11.4 and 8.0; of two kv heads, whose 128 CTAs are one turn either way, 21 and 28).
+    constexpr int CTAS = DK + DV <= 128 ? 4 : 3;
+    const int sms = sm_count();
+    auto* kernel = CTAS == 3 && DK == 128 && DV <= 64 && single_ctas > 3 * sms && single_ctas <= 4 * sms ? attention_sink_mma_kernel<DK, DV, 4>
+                                                                                                        : attention_sink_mma_kernel<DK, DV, CTAS>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_chained(kernel, dim3((unsigned)max_work * nkv * gparts), dim3(128), smem, stream, (const bf16*)q,
                    (const bf16*)kv_pool, block_tables, (const SinkWork*)work, n_work_ptr, (bf16*)out, part_o, part_ml, sinks, nh, nkv,
                    page_size, n_pages, table_width, window, keep_first, chunk, scale, cap, heads_per_cta, status);
     return launch_status();
 }
 
+// single_ctas: CTAs of a step of single tokens of which none is split (0: another step).
 PLLM_EXPORT int pllm_attention_sink_mma(const void* q, const void* kv_pool, const int* block_tables, const int* work,
                                         const int* n_work_ptr, int max_work, void* out, float* part_o, float* part_ml,
                                         const float* sinks, int nh, int nkv, int dk, int dv, int page_size, int n_pages, int table_width,
-                                        int window, int keep_first, int chunk, float scale, float cap, int* status, cudaStream_t stream) {
+                                        int window, int keep_first, int chunk, int single_ctas, float scale, float cap, int* status, cudaStream_t stream) {
     if (max_work <= 0) return PLLM_OK;
     if (!pllm_attention_sink_mma_supports(PLLM_BF16, nh, nkv, dk, dv) || page_size <= 0 || window < 0 || keep_first < 0 || chunk < 0 || (chunk && (window || keep_first))) return PLLM_ERR_SIZE;
     if (((uintptr_t)q | (uintptr_t)kv_pool) & 15) return PLLM_ERR_ALIGN;
 #define SINK_MMA_CASE(A, B)                                                                                                     \
     if (dk == A && dv == B)                                                                                                     \
         return launch_sink_mma<A, B>(q, kv_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, sinks, nh, nkv, \
-                                     page_size, n_pages, table_width, window, keep_first, chunk, scale, cap, status, stream);
+                                     page_size, n_pages, table_width, window, keep_first, chunk, single_ctas, scale, cap, status, stream);
     SINK_MMA_CASE(32, 32) SINK_MMA_CASE(32, 64) SINK_MMA_CASE(32, 128)
     SINK_MMA_CASE(64, 32) SINK_MMA_CASE(64, 64) SINK_MMA_CASE(64, 128)
     SINK_MMA_CASE(128, 32) SINK_MMA_CASE(128, 64) SINK_MMA_CASE(128, 128)
@@ -659,14 +667,6 @@ PLLM_EXPORT int pllm_attention_sink_mma(const void* q, const void* kv_pool, cons
     return PLLM_ERR_SIZE;
 }
 
-// The most query tokens one work item may hold for a given group size.
-PLLM_EXPORT int pllm_attention_sink_tile_tokens(int nh, int nkv) {
-    const int group = nh / nkv;
-    const int heads_per_cta = group < SINK_MAX_ROWS ? group : SINK_MAX_ROWS;
-    return SINK_MAX_ROWS / heads_per_cta;
-}
-
-PLLM_TRACE_EXPORT(attention_sink)
 // CTAs of attention_sink_kernel that an SM holds at the same time.
 PLLM_EXPORT int pllm_attention_sink_ctas_per_sm(int dtype, int dk, int dv) {
     int n = 0;
@@ -680,3 +680,11 @@ PLLM_EXPORT int pllm_attention_sink_ctas_per_sm(int dtype, int dk, int dv) {
     return n;
 }
 
+// The most query tokens one work item may hold for a given group size.
+PLLM_EXPORT int pllm_attention_sink_tile_tokens(int nh, int nkv) {
+    const int group = nh / nkv;
+    const int heads_per_cta = group < SINK_MAX_ROWS ? group : SINK_MAX_ROWS;
+    return SINK_MAX_ROWS / heads_per_cta;
+}
+
+PLLM_TRACE_EXPORT(attention_sink)

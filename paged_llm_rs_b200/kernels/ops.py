@@ -103,7 +103,7 @@ def lib():
         sig["pllm_attention_sink_ctas_per_sm"] = [c_int, c_int, c_int]
         sig["pllm_attention_sink_mma_supports"] = [c_int] * 5
         sig["pllm_attention_sink_mma_tile_tokens"] = [c_int, c_int]
-        sig["pllm_attention_sink_mma"] = [P, P, P, P, P, c_int, P, P, P, P] + [c_int] * 10 + [c_float, c_float, P, P]
+        sig["pllm_attention_sink_mma"] = [P, P, P, P, P, c_int, P, P, P, P] + [c_int] * 11 + [c_float, c_float, P, P]
         sig["pllm_mamba2_mix"] = [c_int] + [P] * 8 + [c_int, c_int, P, c_ll, P, P, P] + [c_int] * 7 + [c_float, P]
         sig["pllm_pack_decode_step"] = [P, c_int, c_int, P, P, P, P, P] + [c_int] * 16 + [P, P]
         sig["pllm_sandwich_norm32"] = [c_int, P, P, P, P, P, P, P, c_int, c_int, c_float, P]
@@ -1194,8 +1194,9 @@ def attention_sink(q: torch.Tensor, kv_pool: torch.Tensor, block_tables: torch.T
     if attention_sink_uses_tensor_cores(q.dtype, num_heads, num_kv_heads, dk, dv):
         _check(L.pllm_attention_sink_mma(_ptr(q), _ptr(kv_pool), _ptr(block_tables), _ptr(work), _ptr(n_work), max_work, _ptr(out),
                                          _ptr(part_o), _ptr(part_ml), _ptr(sinks), num_heads, num_kv_heads, dk, dv, page_size, n_pages,
-                                         block_tables.shape[-1], int(window), int(keep_first), int(chunk), float(scale), float(cap), _ptr(status),
-                                         _stream()), "attention_sink (mma)")
+                                         block_tables.shape[-1], int(window), int(keep_first), int(chunk),
+                                         T * num_kv_heads * -(-(num_heads // num_kv_heads) // 64) if w.kinds == 1 else 0, float(scale),
+                                         float(cap), _ptr(status), _stream()), "attention_sink (mma)")
     else:
         _check(L.pllm_attention_sink(_code(q), _ptr(q), _ptr(kv_pool), _ptr(block_tables), _ptr(work), _ptr(n_work), max_work,
                                      _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(sinks), num_heads, num_kv_heads, dk, dv, page_size,

@@ -197,7 +197,7 @@ def test_rotation_value_mixing_and_the_cache_write(dtype, T, nh, nkv, dk, dv, ro
     run_rope_write(dtype, T, nh, nkv, dk, dv, rot, page, mix)
 
 
-def run_attention(dtype, reqs, nh, nkv, dk, dv, page, window, keep, cap, scale=None, craft=None, target_ctas=296, sink=None):
+def run_attention(dtype, reqs, nh, nkv, dk, dv, page, window, keep, cap, scale=None, craft=None, target_ctas=296, sink=None, kinds=3):
     """reqs: (cached tokens before, new tokens).  Random keys and values in shuffled pages; returns per request
     (got [n, nh, dv], want) and the number of reductions."""
     from paged_llm_rs_b200.kernels import attention_plan
@@ -239,7 +239,7 @@ def run_attention(dtype, reqs, nh, nkv, dk, dv, page, window, keep, cap, scale=N
     redd = dev(torch.from_numpy(np.ascontiguousarray(red)).reshape(-1, 4)) if len(red) else torch.zeros(1, 4, dtype=torch.int32, device=DEV)
     w = AttentionWork(workd, dev(torch.tensor([len(work)], dtype=torch.int32)), len(work) + 3, redd,
                       dev(torch.tensor([len(red)], dtype=torch.int32)), len(red),
-                      torch.zeros(max(parts, 1), nh, dv, device=DEV), torch.zeros(max(parts, 1), nh, 2, device=DEV), kinds=3,
+                      torch.zeros(max(parts, 1), nh, dv, device=DEV), torch.zeros(max(parts, 1), nh, 2, device=DEV), kinds=kinds,
                       many_splits=attention_plan.many_splits(len(reqs), ctas, target_ctas))
     qd = dev(torch.cat(qs).contiguous())
     out = torch.zeros(at, nh, dv, dtype=dtype, device=DEV)
@@ -264,6 +264,15 @@ def test_attention_mixed_batch(dtype, nh, nkv, dk, dv, page, window, keep, cap):
     res, _ = run_attention(dtype, reqs, nh, nkv, dk, dv, page, window, keep, cap)
     for i, (got, want) in enumerate(res):
         close(got, want, dtype, f"request {i}", f32=3e-5, bf16=2.5e-2)
+
+
+@pytest.mark.parametrize("nh,nkv,dk,dv,window", [(16, 8, 128, 64, 0), (16, 8, 128, 64, 30), (8, 8, 128, 32, 0), (16, 8, 64, 128, 0)])
+def test_a_step_of_so_many_single_tokens_that_four_ctas_an_sm_are_one_turn(nh, nkv, dk, dv, window):
+    # (60 requests over 8 kv heads: 480 CTAs, between three and four for each of 148 SMs)
+    res, splits = run_attention(torch.bfloat16, [(7 * i % 190, 1) for i in range(60)], nh, nkv, dk, dv, 16, window, 0, 0.0, kinds=1)
+    assert splits == 0
+    for i, (got, want) in enumerate(res):
+        close(got, want, torch.bfloat16, f"request {i}", f32=3e-5, bf16=2.5e-2)
 
 
 @pytest.mark.parametrize("code", [0, 1])
