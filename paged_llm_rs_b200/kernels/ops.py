@@ -1384,6 +1384,10 @@ def _segments_ok(segments: torch.Tensor, what: str):
 
 
 MLSTM_BLOCKS = True     # (False: every segment token by token, for comparison)
+# Tokens of the longest segment that goes token by token: blocks cost four kernels whatever the length.  One segment of 256 / 384 / 512 / 1000
+# tokens on a B200, us token by token and in blocks: 4 heads of 128 x 256 40 / 55 / 70 / 127 and 56 / 57 / 57 / 64, 16 heads 66 / 96 / 123 / 231 and
+# 66 / 94 / 114 / 201; four segments of 512 beside one another, 8 heads: 205 either way, of 384: 158 and 167.
+MLSTM_LONGEST = 512
 
 
 def mlstm_mix(u: torch.Tensor, gates: torch.Tensor, i_bias: torch.Tensor, f_bias: torch.Tensor, cap: float, gain: torch.Tensor,
@@ -1418,6 +1422,9 @@ def mlstm_mix(u: torch.Tensor, gates: torch.Tensor, i_bias: torch.Tensor, f_bias
 
 
 DELTA_BLOCKS = True     # (False: every segment token by token, for comparison)
+# Likewise: 8 heads of 128 x 128 over 4 key heads 92 / 127 / 162 / 296 token by token and 115 / 125 / 133 / 171 in blocks, 32 over 16 138 / 197 / 255 / 487
+# and 138 / 188 / 226 / 429; four segments of 384 of 16 heads: 384 and 346.
+DELTA_LONGEST = 384
 
 
 def delta_mix(u: torch.Tensor, conv_w: torch.Tensor, ba: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, gain: torch.Tensor,
@@ -1430,10 +1437,6 @@ def delta_mix(u: torch.Tensor, conv_w: torch.Tensor, ba: torch.Tensor, a_log: to
     _dev(u, conv_w, ba, a_log, dt_bias, gain, segments, state, out)
     for t, n in ((ba, "ba"), (a_log, "a_log"), (dt_bias, "dt_bias"), (gain, "gain"), (state, "state")):
         _f32(t, n)
-# Tokens of the longest segment that goes token by token: blocks cost four kernels whatever the length.  One segment of 256 / 384 / 512 / 1000
-# tokens on a B200, us token by token and in blocks: 4 heads of 128 x 256 40 / 55 / 70 / 127 and 56 / 57 / 57 / 64, 16 heads 66 / 96 / 123 / 231 and
-# 66 / 94 / 114 / 201; four segments of 512 beside one another, 8 heads: 205 either way, of 384: 158 and 167.
-MLSTM_LONGEST = 512
     _segments_ok(segments, "delta_mix")
     T = u.shape[0]
     channels = 2 * kv_heads * dim + heads * vdim
@@ -1468,9 +1471,6 @@ def channel_delta_mix(u: torch.Tensor, conv_w: torch.Tensor, small: torch.Tensor
                       dt_bias: torch.Tensor, g1_off: int, g2: torch.Tensor, gain: torch.Tensor, segments: torch.Tensor,
                       max_segment_tokens: int, state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int,
                       taps: int, eps: float, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
-# Likewise: 8 heads of 128 x 128 over 4 key heads 92 / 127 / 162 / 296 token by token and 115 / 125 / 133 / 171 in blocks, 32 over 16 138 / 197 / 255 / 487
-# and 138 / 188 / 226 / 429; four segments of 384 of 16 heads: 384 and 346.
-DELTA_LONGEST = 384
     """From a projection ``u`` [T, width] whose first columns are [q | k | v] (kv_heads dim, kv_heads dim, heads vdim) and a float32
     projection ``small`` [T, width] (step sizes' logits in its first ``heads`` columns, the decays' short vector at a1_off) to the
     output projection's input [T, heads vdim]: convolution and silu, unit q and k, decays exp(-exp(a_log) softplus(a2 a1 + dt_bias))
