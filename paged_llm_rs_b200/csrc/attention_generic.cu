@@ -164,16 +164,20 @@ __global__ void attention_generic_kernel(
 
 // ---- float32 ------------------------------------------------------------------------------------
 // The same in float32, which is bound by the multiply-adds of a prompt's portion and by its keys and values for decoded
-// tokens.  A CTA of 128 threads holds up to 32 rows (token, head) of an item and takes 64 keys a turn; a turn's keys come
-// in by cp.async while the turn before it is summed, its values while its scores are formed (each buffer is asked for
-// again as soon as it has been read).  More than four rows: a thread makes 4 x 4 scores and then 4 rows x 4 HDV
+// tokens.  A CTA of 128 threads (256 for heads of more than 128 entries) holds up to 32 rows (token, head) of an item and takes 64 keys a turn;
+// a turn's keys come in by cp.async while the turn before it is summed, its values while its scores are formed (each buffer is asked for
+// again as soon as it has been read).  More than four rows: a thread makes R x 4 scores (R: 4, or 2 of 256 threads) and then R rows x 4 HDV
 // output entries, so that a value read from shared memory serves four sums (the kernel above reads two for each).  Up to
-// four rows (a decoded token): a key belongs to two threads, each taking half of the head, and a row's softmax to a warp.
+// four rows (a decoded token): a key belongs to NT / 64 threads, each taking a share of the head, and a row's softmax to a warp.
 // Scores are sums of even and of odd entries (fma.rn.f32x2).  Measured at the 0.6B shape (16 heads over 8 kv heads of 128),
 // 4 requests at 500 beside a portion of 252 tokens: 60 us a layer, the kernel above in its place 136.  It is bound by the
 // latency of its own chains: a warp a scheduler (242 registers a thread), 35% of the issue slots and 37% of the
-// shared-memory pipe in use.
-constexpr int AF_ROWS = 32, AF_BK = 64, AF_THREADS = 128, AF_HEADS = 4;
+// shared-memory pipe in use.  A turn that is not full leaves out what it does not have: a prompt of 37 tokens takes 11.2 us, the kernel
+// above 12.2.  Heads of more than 128 entries: a CTA with place for 32 rows and 64 keys fills an SM's shared memory, so a step of single
+// tokens takes a kernel with place for four rows and 32 keys, three of which fit (64 requests at 1024, 16 heads over 2 of 256: 187 us, the kernel above 222;
+// 8 over 1: 115 and 126; 8 requests at 2048, 16 over 2: 56 and 51, 8 over 1: 31 and 49.  With the CTA for 32 rows the first two took 260 and 141
+// with the caches cold, the kernel above 229 and 135).
+constexpr int AF_ROWS = 32, AF_BK = 64, AF_HEADS = 4;
 
 __device__ __forceinline__ uint32_t af_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void af_copy16(uint32_t dst, const float* src, bool live) {
@@ -190,14 +194,15 @@ __device__ __forceinline__ unsigned long long af_pack(float lo, float hi) {
 __device__ __forceinline__ float af_lo(unsigned long long v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float af_hi(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
-// A turn's weights times its values: rows ty + 8 a, the head's chunks tx + 16 h.
-template <int HDV, bool GUARD>
-__device__ __forceinline__ void sum_values(const float* p_s, const float* v_s, int hdp, int chunks, int tx, int ty, unsigned long long (&acc)[4][HDV][2]) {
+// The weights of a turn's first `keys` keys (a multiple of four) times their values: rows ty + AF_ROWS / R a, the head's chunks tx + 16 h.
+template <int R, int HDV, bool GUARD>
+__device__ __forceinline__ void sum_values(const float* p_s, const float* v_s, int keys, int hdp, int chunks, int tx, int ty,
+                                           unsigned long long (&acc)[R][HDV][2]) {
 #pragma unroll 2
-    for (int j = 0; j < AF_BK; j += 4) {
-        float4 p[4];
+    for (int j = 0; j < keys; j += 4) {
+        float4 p[R];
 #pragma unroll
-        for (int a = 0; a < 4; a++) p[a] = *reinterpret_cast<const float4*>(p_s + (ty + 8 * a) * AF_BK + j);
+        for (int a = 0; a < R; a++) p[a] = *reinterpret_cast<const float4*>(p_s + (ty + AF_ROWS / R * a) * AF_BK + j);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             ulonglong2 v[HDV];
@@ -205,7 +210,7 @@ __device__ __forceinline__ void sum_values(const float* p_s, const float* v_s, i
             for (int h = 0; h < HDV; h++)
                 v[h] = *reinterpret_cast<const ulonglong2*>(v_s + (j + i) * hdp + ((tx + 16 * h < chunks ? tx + 16 * h : 0) << 2));
 #pragma unroll
-            for (int a = 0; a < 4; a++) {
+            for (int a = 0; a < R; a++) {
                 const float pa = i == 0 ? p[a].x : i == 1 ? p[a].y : i == 2 ? p[a].z : p[a].w;
                 const unsigned long long p2 = af_pack(pa, pa);
                 if (!GUARD || pa != 0.f) {
@@ -220,9 +225,42 @@ __device__ __forceinline__ void sum_values(const float* p_s, const float* v_s, i
     }
 }
 
-// HDV: 64-entry parts of a head, hd <= 64 HDV.
-template <int HDV>
-__global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_kernel(
+// A turn's scores: rows ty + AF_ROWS / R a with keys tx + 16 b, b < B.
+template <int R, int B>
+__device__ __forceinline__ void score_keys(const float* q_s, const float* k_s, int hdp, int chunks, int tx, int ty, float (&sc)[R][4]) {
+    unsigned long long s2[R][B];
+#pragma unroll
+    for (int a = 0; a < R; a++)
+#pragma unroll
+        for (int b = 0; b < B; b++) s2[a][b] = 0ull;
+#pragma unroll 2
+    for (int c = 0; c < chunks; c++) {
+        ulonglong2 qv[R];
+#pragma unroll
+        for (int a = 0; a < R; a++) {
+            const int r = ty + AF_ROWS / R * a;
+            qv[a] = *reinterpret_cast<const ulonglong2*>(q_s + r * hdp + ((c ^ (r & 7)) << 2));
+        }
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            const int j = tx + 16 * b;
+            const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k_s + j * hdp + ((c ^ (j & 7)) << 2));
+#pragma unroll
+            for (int a = 0; a < R; a++) {
+                af_fma2(s2[a][b], qv[a].x, kv.x);
+                af_fma2(s2[a][b], qv[a].y, kv.y);
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < R; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) sc[a][b] = b < B ? af_lo(s2[a][b < B ? b : 0]) + af_hi(s2[a][b < B ? b : 0]) : 0.f;
+}
+
+// HDV: 64-entry parts of a head, hd <= 64 HDV.  NT: threads; R rows each.  BK: keys a turn (64 unless FEW).  FEW: no item has more than four rows.
+template <int HDV, int NT, int BK = AF_BK, bool FEW = false>
+__global__ void __launch_bounds__(NT, FEW ? 3 : HDV <= 2 ? 2 : 1) attention_f32_kernel(
     const float* q, const float* k_pool, const float* v_pool, const int* __restrict__ block_tables,
     const AttnWork* __restrict__ work, const int* __restrict__ n_work_ptr, float* __restrict__ out, float* __restrict__ part_o,
     float* __restrict__ part_ml, int nh, int nkv, int hd, int page_size, int n_pages, int table_width, int window, float scale, int* status) {
@@ -236,25 +274,29 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
     const int group = nh / nkv, heads_per_cta = min(group, AF_HEADS), gparts = (group + heads_per_cta - 1) / heads_per_cta;
     const int kh = part / gparts, head0 = kh * group + (part % gparts) * heads_per_cta;
     const int n_heads = min(heads_per_cta, kh * group + group - head0);
-    const int rows = min(w.q_count * n_heads, AF_ROWS);
-    const bool few = rows <= 4;
+    const int rows = min(w.q_count * n_heads, FEW ? 4 : AF_ROWS);
+    const bool few = FEW || rows <= 4;
+    static_assert(FEW || BK == AF_BK, "many rows take their keys 64 a turn");
+    constexpr int R = AF_ROWS * 16 / NT, RS = AF_ROWS / R;                     // rows ty, ty + RS, ... of a thread
+    constexpr int KT = NT / BK;                                                // few rows: threads that share a key
+    constexpr int DIMS = 64 * HDV, VG = NT > DIMS ? NT / DIMS : 1, VE = NT < DIMS ? DIMS / NT : 1;     // ... groups of keys a value entry, entries a thread
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
     const int hdp = (hd + 31) & ~31, chunks = hd / 4;          // a row of shared memory holds whole groups of eight 16-byte chunks
 
     extern __shared__ __align__(128) float smem_f[];
-    float* q_s = smem_f;                             // [32][hdp], chunk c of row r at c ^ (r & 7)
-    float* k_s = q_s + AF_ROWS * hdp;                // [64][hdp], likewise
-    float* v_s = k_s + AF_BK * hdp;                  // [64][hdp], as it lies
-    float* p_s = v_s + AF_BK * hdp;                  // scores, then weights: [32][64] (few rows: [64][4])
-    __shared__ long long off_s[2][AF_BK];            // where a key's row of this kv head starts in the pools; -1: nowhere
+    float* q_s = smem_f;                             // [32 (FEW: 4)][hdp], chunk c of row r at c ^ (r & 7)
+    float* k_s = q_s + (FEW ? 4 : AF_ROWS) * hdp;    // [BK][hdp], likewise
+    float* v_s = k_s + BK * hdp;                     // [BK][hdp], as it lies
+    float* p_s = v_s + BK * hdp;                     // scores, then weights: [32][64] (few rows: [BK][4])
+    __shared__ long long off_s[2][BK];               // where a key's row of this kv head starts in the pools; -1: nowhere
     __shared__ float row_s[2][4];                    // few rows: a row's factor for what it holds; at the end its sum
 
     // rows past the item's are never visible to anything
-    int lo[4], hi[4], my_tok[4], my_head[4];
+    int lo[4], hi[4], my_tok[4], my_head[4];        // (R of them where the rows are many)
 #pragma unroll
     for (int a = 0; a < 4; a++) {
-        const int r = few ? a : ty + 8 * a;
-        const bool live = r < rows;
+        const int r = few ? a : ty + RS * a;
+        const bool live = r < rows && (few || a < R);
         my_tok[a] = live ? r / n_heads : 0;
         my_head[a] = live ? head0 + r % n_heads : head0;
         const int pos = w.q_pos0 + my_tok[a];
@@ -263,8 +305,8 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
     }
     const int* table = block_tables + (size_t)w.seg * table_width;
     auto find = [&](int t) {
-        if (tid < AF_BK) {
-            const int j = w.kv_begin + t * AF_BK + tid;
+        if (tid < BK) {
+            const int j = w.kv_begin + t * BK + tid;
             int page = -1;
             if (j < w.kv_end) {
                 const int b = j / page_size;
@@ -275,13 +317,13 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
             off_s[t & 1][tid] = page < 0 ? -1 : (((long long)page * nkv + kh) * page_size + j % page_size) * hd;
         }
     };
-    // (a thread's rows and chunks: 128 further on is 128 / chunks rows and 128 % chunks chunks further on)
-    const int first_row = tid / chunks, first_chunk = tid % chunks, row_step = AF_THREADS / chunks, chunk_step = AF_THREADS % chunks;
+    // (a thread's rows and chunks: NT further on is NT / chunks rows and NT % chunks chunks further on)
+    const int first_row = tid / chunks, first_chunk = tid % chunks, row_step = NT / chunks, chunk_step = NT % chunks;
     auto load = [&](int t, float* dst, const float* pool, bool swizzled) {
         const uint32_t to = af_smem(dst);
         int j = first_row, c = first_chunk;
 #pragma unroll 4
-        while (j < AF_BK) {
+        while (j < BK) {
             const long long off = off_s[t & 1][j];
             af_copy16(to + (j * hdp + ((swizzled ? c ^ (j & 7) : c) << 2)) * 4, pool + (off < 0 ? 0 : off + c * 4), off >= 0);
             j += row_step;
@@ -291,25 +333,27 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
         af_commit();
     };
     float m[4], l[4];
-    unsigned long long acc[4][HDV][2];
-    float acc1[4][(HDV + 1) / 2];                    // few rows: entry tid (+ 128) of each row's output
+    unsigned long long acc[R][HDV][2];
+    float acc1[4][VE];                               // few rows: entry tid % DIMS (+ NT) of each row's output, over keys of group tid / DIMS
 #pragma unroll
     for (int a = 0; a < 4; a++) {
         m[a] = -CUDART_INF_F;
         l[a] = 0.f;
 #pragma unroll
-        for (int h = 0; h < HDV; h++) acc[a][h][0] = acc[a][h][1] = 0ull;
-#pragma unroll
-        for (int h = 0; h < (HDV + 1) / 2; h++) acc1[a][h] = 0.f;
+        for (int h = 0; h < VE; h++) acc1[a][h] = 0.f;
     }
-    const int turns = (w.kv_end - w.kv_begin + AF_BK - 1) / AF_BK;
+#pragma unroll
+    for (int a = 0; a < R; a++)
+#pragma unroll
+        for (int h = 0; h < HDV; h++) acc[a][h][0] = acc[a][h][1] = 0ull;
+    const int turns = (w.kv_end - w.kv_begin + BK - 1) / BK;
     const int seen_by_all = min(w.kv_end, w.q_pos0 + 1), seen_from = window > 0 ? w.q_pos0 + w.q_count - window : 0;
     find(0);
     pdl_wait(KID_ATT_GENERIC);
     __syncthreads();
     load(0, k_s, k_pool, true);
     load(0, v_s, v_pool, false);
-    for (int i = tid; i < AF_ROWS * chunks; i += AF_THREADS) {
+    for (int i = tid; i < (FEW ? 4 : AF_ROWS) * chunks; i += NT) {
         const int r = i / chunks, c = i % chunks;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < rows) {
@@ -319,15 +363,17 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
         *reinterpret_cast<float4*>(q_s + r * hdp + ((c ^ (r & 7)) << 2)) = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
     }
     for (int t = 0; t < turns; t++) {
-        const int kv0 = w.kv_begin + t * AF_BK;
+        const int kv0 = w.kv_begin + t * BK, live_keys = min(BK, w.kv_end - kv0);
         af_wait_older();
         __syncthreads();          // this turn's keys are there
         if (t + 1 < turns) find(t + 1);
-        float sc[4][4];
+        float sc[R][4];
         if (few) {
-            const int j = tid >> 1, half = tid & 1, c0 = half ? (chunks + 1) / 2 : 0, c1 = half ? chunks : (chunks + 1) / 2;
+            const int j = tid / KT, share = tid % KT, c0 = chunks * share / KT, c1 = chunks * (share + 1) / KT;
             unsigned long long s2[4] = {0ull, 0ull, 0ull, 0ull};
-            for (int c = c0; c < c1; c++) {
+            // (a key's threads begin at chunks of their own, so that what they read of q lies in other banks)
+            int c = c0 + share < c1 ? c0 + share : c0;
+            for (int i = c0; i < c1; i++) {
                 const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k_s + j * hdp + ((c ^ (j & 7)) << 2));
 #pragma unroll
                 for (int a = 0; a < 4; a++) {
@@ -335,65 +381,48 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
                     af_fma2(s2[a], qv.x, kv.x);
                     af_fma2(s2[a], qv.y, kv.y);
                 }
+                if (++c == c1) c = c0;
             }
 #pragma unroll
             for (int a = 0; a < 4; a++) {
                 float v = af_lo(s2[a]) + af_hi(s2[a]);
-                v += __shfl_xor_sync(0xffffffffu, v, 1);
+#pragma unroll
+                for (int o = 1; o < KT; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
                 const int key = kv0 + j;
-                if (half == 0) p_s[j * 4 + a] = key >= lo[a] && key < hi[a] ? v : -CUDART_INF_F;
+                if (share == 0) p_s[j * 4 + a] = key >= lo[a] && key < hi[a] ? v : -CUDART_INF_F;
             }
         } else {
-            unsigned long long s2[4][4];
+            // (a turn that is not full, a short prompt's only one as a rule, leaves out the sixteens of keys that it does not have)
+            if (live_keys > 48) score_keys<R, 4>(q_s, k_s, hdp, chunks, tx, ty, sc);
+            else if (live_keys > 32) score_keys<R, 3>(q_s, k_s, hdp, chunks, tx, ty, sc);
+            else if (live_keys > 16) score_keys<R, 2>(q_s, k_s, hdp, chunks, tx, ty, sc);
+            else score_keys<R, 1>(q_s, k_s, hdp, chunks, tx, ty, sc);
 #pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) s2[a][b] = 0ull;
-#pragma unroll 2
-            for (int c = 0; c < chunks; c++) {
-                ulonglong2 qv[4];
-#pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    const int r = ty + 8 * a;
-                    qv[a] = *reinterpret_cast<const ulonglong2*>(q_s + r * hdp + ((c ^ (r & 7)) << 2));
-                }
-#pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const int j = tx + 16 * b;
-                    const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(k_s + j * hdp + ((c ^ (j & 7)) << 2));
-#pragma unroll
-                    for (int a = 0; a < 4; a++) {
-                        af_fma2(s2[a][b], qv[a].x, kv.x);
-                        af_fma2(s2[a][b], qv[a].y, kv.y);
-                    }
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < 4; a++)
+            for (int a = 0; a < R; a++)
 #pragma unroll
                 for (int b = 0; b < 4; b++) {
                     const int key = kv0 + tx + 16 * b;
-                    sc[a][b] = key >= lo[a] && key < hi[a] ? af_lo(s2[a][b]) + af_hi(s2[a][b]) : -CUDART_INF_F;
+                    if (key < lo[a] || key >= hi[a]) sc[a][b] = -CUDART_INF_F;
                 }
         }
         __syncthreads();          // the keys have been read, the next turn's places are known (few rows: the scores are there)
         if (t + 1 < turns) load(t + 1, k_s, k_pool, true); else af_commit();
         if (few) {
             if (warp < rows) {
-                // row `warp` is this warp's, two keys a lane
-                const float s0 = p_s[lane * 4 + warp], s1 = p_s[(lane + 32) * 4 + warp];
+                // row `warp` is this warp's, two keys a lane (one of 32)
+                const float s0 = p_s[lane * 4 + warp], s1 = BK > 32 ? p_s[(lane + 32) * 4 + warp] : -CUDART_INF_F;
                 const float top = fmaxf(m[0], warp_max(fmaxf(s0, s1)));
                 const float p0 = s0 == -CUDART_INF_F ? 0.f : expf(s0 - top), p1 = s1 == -CUDART_INF_F ? 0.f : expf(s1 - top);
                 const float corr = top == -CUDART_INF_F ? 1.f : expf(m[0] - top);
                 l[0] = l[0] * corr + warp_sum(p0 + p1);
                 m[0] = top;
                 p_s[lane * 4 + warp] = p0;
-                p_s[(lane + 32) * 4 + warp] = p1;
+                if (BK > 32) p_s[(lane + 32) * 4 + warp] = p1;
                 if (lane == 0) row_s[0][warp] = corr;
-            } else if (lane == 0) row_s[0][warp] = 1.f;
+            } else if (lane == 0 && warp < 4) row_s[0][warp] = 1.f;
         } else {
 #pragma unroll
-            for (int a = 0; a < 4; a++) {
+            for (int a = 0; a < R; a++) {
                 float top = fmaxf(fmaxf(sc[a][0], sc[a][1]), fmaxf(sc[a][2], sc[a][3]));
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));     // (the 16 lanes of the row)
@@ -404,7 +433,7 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
                 for (int b = 0; b < 4; b++) {
                     const float p = sc[a][b] == -CUDART_INF_F ? 0.f : expf(sc[a][b] - top);
                     sum += p;
-                    p_s[(ty + 8 * a) * AF_BK + tx + 16 * b] = p;
+                    p_s[(ty + RS * a) * AF_BK + tx + 16 * b] = p;
                 }
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -424,14 +453,15 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
         af_wait_older();
         __syncthreads();          // this turn's values and weights are there
         if (few) {
+            const int j0 = tid / DIMS * (BK / VG), j1 = min(j0 + BK / VG, live_keys);
 #pragma unroll
-            for (int h = 0; h < (HDV + 1) / 2; h++) {
-                const int d = tid + 128 * h;
+            for (int h = 0; h < VE; h++) {
+                const int d = tid % DIMS + NT * h;
 #pragma unroll
                 for (int a = 0; a < 4; a++) acc1[a][h] *= row_s[0][a];
                 if (d < hd) {
 #pragma unroll 8
-                    for (int j = 0; j < AF_BK; j++) {
+                    for (int j = j0; j < j1; j++) {
                         const float4 p = *reinterpret_cast<const float4*>(p_s + j * 4);
                         const float v = v_s[j * hdp + d];
                         if (p.x != 0.f) acc1[0][h] = fmaf(p.x, v, acc1[0][h]);
@@ -444,15 +474,26 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
         } else {
             // (a key that a row does not see adds nothing, whatever its value holds, since an infinity times zero is no zero:
             // where a turn has such keys its weights are looked at one by one)
-            if (kv0 + AF_BK <= seen_by_all && kv0 >= seen_from) sum_values<HDV, false>(p_s, v_s, hdp, chunks, tx, ty, acc);
-            else sum_values<HDV, true>(p_s, v_s, hdp, chunks, tx, ty, acc);
+            if (kv0 + AF_BK <= seen_by_all && kv0 >= seen_from) sum_values<R, HDV, false>(p_s, v_s, AF_BK, hdp, chunks, tx, ty, acc);
+            else sum_values<R, HDV, true>(p_s, v_s, (live_keys + 3) & ~3, hdp, chunks, tx, ty, acc);
         }
         __syncthreads();          // the values and weights have been read
         if (t + 1 < turns) load(t + 1, v_s, v_pool, false); else af_commit();
     }
     if (few) {
-        if (lane == 0) { row_s[0][warp] = m[0]; row_s[1][warp] = l[0]; }
+        if (lane == 0 && warp < 4) { row_s[0][warp] = m[0]; row_s[1][warp] = l[0]; }
+        if (VG > 1) {
+            // the groups' shares, [group][row][entry] where the keys were, added in the order of the groups
+#pragma unroll
+            for (int a = 0; a < 4; a++) k_s[(tid / DIMS * 4 + a) * DIMS + tid % DIMS] = acc1[a][0];
+        }
         __syncthreads();
+        if (VG > 1) {
+            if (tid >= DIMS) return;
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+                for (int g = 1; g < VG; g++) acc1[a][0] += k_s[(g * 4 + a) * DIMS + tid];
+        }
 #pragma unroll
         for (int a = 0; a < 4; a++) {
             if (a >= rows) break;
@@ -460,15 +501,15 @@ __global__ void __launch_bounds__(AF_THREADS, HDV <= 2 ? 2 : 1) attention_f32_ke
             const size_t pr = (size_t)((w.part_slot >= 0 ? w.part_slot : w.q_token0) + my_tok[a]) * nh + my_head[a];
             float* o = (w.part_slot >= 0 ? part_o : out) + pr * hd;
 #pragma unroll
-            for (int h = 0; h < (HDV + 1) / 2; h++)
-                if (tid + 128 * h < hd) o[tid + 128 * h] = acc1[a][h] * inv;
+            for (int h = 0; h < VE; h++)
+                if (tid + NT * h < hd) o[tid + NT * h] = acc1[a][h] * inv;
             if (w.part_slot >= 0 && tid == 0) { part_ml[pr * 2] = row_s[0][a]; part_ml[pr * 2 + 1] = sum; }
         }
         return;
     }
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-        if (ty + 8 * a >= rows) continue;
+    for (int a = 0; a < R; a++) {
+        if (ty + RS * a >= rows) continue;
         const float inv = w.part_slot >= 0 ? 1.f : l[a] > 0.f ? 1.0f / l[a] : 0.f;
         const size_t pr = (size_t)((w.part_slot >= 0 ? w.part_slot : w.q_token0) + my_tok[a]) * nh + my_head[a];
         float* o = (w.part_slot >= 0 ? part_o : out) + pr * hd;
@@ -599,7 +640,7 @@ PLLM_EXPORT int pllm_attention_generic(int dtype, const void* q, const void* k_p
                                        const int* block_tables, const int* work, const int* n_work_ptr,
                                        int max_work, void* out, float* part_o, float* part_ml, int nh, int nkv,
                                        int hd, int page_size, int n_pages, int table_width, int window,
-                                       float scale, int* status, cudaStream_t stream) {
+                                       int singles, float scale, int* status, cudaStream_t stream) {
     if (max_work <= 0) return PLLM_OK;
     if (nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0) return PLLM_ERR_SIZE;
     if (hd <= 0 || hd > ATT_MAX_HD || hd % 8 != 0) return PLLM_ERR_SIZE;
@@ -607,10 +648,16 @@ PLLM_EXPORT int pllm_attention_generic(int dtype, const void* q, const void* k_p
     if (dtype == PLLM_F32) {
         if (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) return PLLM_ERR_ALIGN;
         const int gparts = (group + AF_HEADS - 1) / AF_HEADS, hdp = (hd + 31) & ~31;
-        const size_t smem = ((size_t)(AF_ROWS + 2 * AF_BK) * hdp + AF_ROWS * AF_BK) * sizeof(float);
-        auto* kernel = hd <= 64 ? attention_f32_kernel<1> : hd <= 128 ? attention_f32_kernel<2> : attention_f32_kernel<4>;
+        // Heads of more than 128 entries: twice the threads, since one CTA fits an SM (a prompt of 37 tokens 16.0 us, the kernel above 19.2; with 128
+        // threads, caches cold, 34.8 and 26.7); and where no item has many rows the kernel without place for them, three of whose CTAs fit.
+        const bool few = singles != 0 && hd > 128;
+        const int threads = hd <= 128 || few ? 128 : 256;
+        const size_t smem = few ? ((size_t)(4 + 2 * 32) * hdp + 4 * 32) * sizeof(float)
+                                : ((size_t)(AF_ROWS + 2 * AF_BK) * hdp + AF_ROWS * AF_BK) * sizeof(float);
+        auto* kernel = few ? attention_f32_kernel<4, 128, 32, true>
+                           : hd <= 64 ? attention_f32_kernel<1, 128> : hd <= 128 ? attention_f32_kernel<2, 128> : attention_f32_kernel<4, 256>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_chained(kernel, dim3((unsigned)max_work * nkv * gparts), dim3(AF_THREADS), smem, stream, (const float*)q, (const float*)k_pool,
+        launch_chained(kernel, dim3((unsigned)max_work * nkv * gparts), dim3(threads), smem, stream, (const float*)q, (const float*)k_pool,
                        (const float*)v_pool, block_tables, (const AttnWork*)work, n_work_ptr, (float*)out, part_o, part_ml, nh, nkv, hd,
                        page_size, n_pages, table_width, window, scale, status);
         return launch_status();

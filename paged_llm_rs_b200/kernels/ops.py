@@ -42,7 +42,7 @@ def lib():
             "pllm_qk_norm_rope_kv": [c_int, P, P, P, P, c_float, P, P, c_int, c_int, P, P, P, P,
                                      c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, P],
             "pllm_attention_generic": [c_int, P, P, P, P, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int,
-                                       c_int, c_int, c_int, c_float, P, P],
+                                       c_int, c_int, c_int, c_int, c_float, P, P],
             "pllm_attention_generic_tile_tokens": [c_int, c_int, c_int],
             "pllm_attention_generic_ctas_per_item": [c_int, c_int, c_int],
             "pllm_attention_reduce": [c_int, P, P, P, P, c_int, P, c_int, c_int, c_int, P],
@@ -464,7 +464,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
         _check(L.pllm_attention_generic(_code(q), _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(block_tables),
                                         _ptr(work), _ptr(n_work), max_work, _ptr(out), _ptr(part_o), _ptr(part_ml),
                                         num_heads, num_kv_heads, head_dim, page_size, n_pages,
-                                        block_tables.shape[-1], int(window), float(scale), _ptr(status), _stream()),
+                                        block_tables.shape[-1], int(window), 1 if kinds == 1 else 0, float(scale), _ptr(status), _stream()),
                "paged_attention")
     if w.reduces:
         _check(L.pllm_attention_reduce(_code(q), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red,

@@ -48,3 +48,20 @@ def test_an_infinite_value_reaches_only_the_rows_that_see_it(nh, nkv, hd):
     for (got, _), (without, want) in zip(res, plain):
         assert torch.isinf(got[-1]).all() and torch.equal(got[:-1], without[:-1])
         torch.testing.assert_close(without, want, **K.tol(torch.float32))
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window", [(8, 1, 256, None), (16, 2, 256, None), (6, 2, 208, 40), (5, 5, 144, None)])
+def test_single_tokens_of_long_heads(nh, nkv, hd, window):
+    # (a step of decoded tokens alone takes a kernel without place for many rows, 32 keys a turn; split items among them)
+    reqs = [(0, 1), (31, 1), (32, 1), (33, 1), (700, 1), (63, 1), (255, 1)]
+    for target in (1, 296):
+        for (got, want) in K.run_attention(torch.float32, reqs, nh, nkv, hd, 16, window, target, kinds=1, idle_items=2)[0]:
+            torch.testing.assert_close(got, want, **K.tol(torch.float32))
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("n", [15, 16, 17, 33, 47, 49, 63, 65])
+def test_turns_that_are_not_full(hd, n):
+    # (a turn of 64 keys leaves out the sixteens that it does not have)
+    for (got, want) in K.run_attention(torch.float32, [(0, n), (40, n)], 8, 4, hd, 16, None, 1)[0]:
+        torch.testing.assert_close(got, want, **K.tol(torch.float32))
