@@ -1,6 +1,6 @@
-// y[M, N] = x[M, K] . W[N, K]^T in true float32 on the CUDA cores: every projection of the float32 path.  The reference
-// calls a library product (crates/pagedllm/src/model/layers.rs:27-35); for the 4 to 300 rows of a step the library's tiles
-// leave most of the chip idle (256 rows, 1024 x 2048: 62 us, 17 of the 74 TFLOP/s).
+// y[M, N] = x[M, K] . W[N, K]^T in true float32 on the CUDA cores: the float32 path's projections of few rows, or of some more into
+// few columns (kernels/ops.py, gemm_f32_sizes).  The reference calls a library product (crates/pagedllm/src/model/layers.rs:27-35),
+// whose tiles leave most of the chip idle there (256 rows, 1024 x 2048: 50 us, 21 of the 74 TFLOP/s).
 //
 // What bounds it: the multiply-adds from some 20 rows on (128 a clock and SM), the bytes of W below.  Hence
 //   - both operands go to shared memory as they lie (K runs along the rows), 32 values of k a stage, three stages by
@@ -189,7 +189,8 @@ int launch_f32(const float* x, const float* w, float* y, int M, int N, int K, in
 PLLM_EXPORT int pllm_gemm_f32(const float* x, const float* w, float* y, int M, int N, int K, int tile, int splits, cudaStream_t stream) {
     if (!pllm_gemm_f32_supports(M, N, K)) return PLLM_ERR_SIZE;
     if (((uintptr_t)x | (uintptr_t)w) & 15) return PLLM_ERR_ALIGN;
-    if (tile == 0) tile = M <= 16 ? 16 : (M <= 32 ? 32 : 128);
+    // (up to 64 rows, and 128 where W has few, two to four tiles of 32 rows rather than one of 128: 1024 x 2048 at 64 rows 22.9 us, 37.4)
+    if (tile == 0) tile = M <= 16 ? 16 : (M <= 64 || (M <= 128 && N <= 1024) ? 32 : 128);
     if (tile == 16) return launch_f32<4, 4, 4, 64>(x, w, y, M, N, K, splits, stream);
     if (tile == 32) return launch_f32<4, 4, 8, 32>(x, w, y, M, N, K, splits, stream);
     if (tile == 128) return launch_f32<8, 4, 16, 16>(x, w, y, M, N, K, splits, stream);

@@ -651,17 +651,43 @@ def rows_gemm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
 
 
 # True float32 products on the CUDA cores (csrc/gemm_f32.cu) where the library's tiles leave most of the chip idle.
-# Measured back to back on a B200 (us, this kernel / cuBLAS):
-#   rows        4            8            16           32           64           256
-#   4096 x 1024 11.6 / 14.2  11.7 / 27.2  11.8 / 27.3  12.4 / 27.7  21.1 / 28.0  70.5 / 45.4
-#   1024 x 2048 13.0 / 14.6  13.1 / 19.5  12.6 / 20.4  13.2 / 20.1  20.5 / 51.1  36.6 / 47.7   (512: 69.0 / 57.4)
-#   6144 x 1024 12.2 / 15.4  12.4 / 27.4  12.7 / 27.6  24.3 / 28.3  42.3 / 33.8  119 / 73.5
-#   151936 x 1024 182 / 193  185 / 203    188 / 241    320 / 249
-# so it takes 4 to 16 rows, up to 32 but for the widest, and more while the product has 64 tiles of 64 x 64 at most.
+# Measured on a B200, a norm and the product behind it (us, this kernel / cuBLAS; - the library's):
+#   rows          4            8            16           32           64           128          256
+#   1024 x 256    - 8.5 / 4.3  - 9.2 / 7.7  - 9.9 / 7.8  - 9.6 / 8.0  - 9.6 / 8.1  - 14.0/ 8.2  - 24.0/ 8.9
+#   1024 x 512    - 8.5 / 7.8  - 9.0 / 7.9  - 9.4 / 8.0  9.0 / 12.1   12.3 / 12.2  - 13.0/ 12.3 - 22.7/ 14.0
+#   2048 x 512    - 8.9 / 8.6  9.4 / 10.7   9.5 / 15.3   9.8 / 15.4   13.0 / 15.8  - 13.4/ 15.9 - 23.4/ 18.2
+#   1024 x 1024   9.2 / 10.8   9.9 / 13.5   9.2 / 10.9   10.2 / 15.4  12.9 / 28.0  17.4 / 26.8  - 29.0/ 27.1
+#   1024 x 2048   14.8 / 15.9  15.7 / 20.8  15.1 / 21.2  17.0 / 20.3  22.9 / 52.6  25.9 / 49.5  42.9 / 50.1
+#   1024 x 4096   26.6 / 28.4  26.7 / 28.6  - 30.9/ 29.3 - 38.1/ 32.5 40.8 / 58.2  56.2 / 95.4  89.5 / 97.6
+#   2048 x 2048   15.4 / 25.6  15.0 / 24.9  19.0 / 25.5  22.9 / 54.0  27.2 / 52.4  43.4 / 51.9  - 71.1/ 60.0
+#   4096 x 1024   12.9 / 15.7  13.0 / 28.5  13.4 / 28.6  17.8 / 28.9  23.2 / 29.1  - 39.2/ 32.9 - 72.7/ 46.7
+#   6144 x 1024   13.4 / 16.8  13.4 / 28.9  13.8 / 29.0  27.6 / 29.4  - 47.6/ 34.6 - 79.8/ 46.7 - 124 / 75.1
+#   32768 x 1024  44.4 / 56.5  45.2 / 57.0  46.2 / 57.9  - 92.9/ 59.2 - 153 / 89.7 - 262 / 161  - 472 / 336
+#   12288 x 4096  - 89.8/ 85.2 - 89.6/ 86.8 99.5 / 134   - 168 / 136  - 260 / 171
+#   4096 x 12288  - 126 / 137  - 126 / 134  126 / 147    152 / 229    222 / 317
 F32_GEMM = True
-F32_MIN_M = 4
-F32_MAX_TILES = 64
-F32_MIN_WEIGHTS = 1 << 18       # (a product of a tiny model's is a launch and nothing else)
+
+
+def gemm_f32_sizes(M: int, N: int, K: int) -> bool:
+    """Whether the float32 product of M rows of x and N of W over K entries is this library's: where the rows are few it has more CTAs to
+    share W out to, until W is so wide, or the rows so many, that the library's larger tiles fill the chip."""
+    if N * K < 1 << 18 or K < 512:         # (a launch and nothing else)
+        return False
+    if M <= 16:
+        # (below six rows of a short K the library reads W by rows; beyond 2^25 weights of long rows, until 12 of them, it is as near the copy
+        # bandwidth; 1024 columns are 32 CTAs at most, which a K of 4096 keeps too long)
+        if K < 1024:
+            return M >= 6 and N * K >= 1 << 20
+        if K >= 4096 and (M > 8 if N <= 1024 else N * K > 1 << 25 and M < 12):
+            return False
+        return M >= 4
+    if M <= 32:
+        return N <= 8192 and not (N <= 1024 and K >= 4096)
+    if M <= 64:
+        return N <= 4096
+    if M <= 128:
+        return (N <= 1024 and K >= 1024) or (N <= 2048 and K >= 2048)
+    return M <= 256 and N <= 1024 and K >= 2048
 
 
 def gemm_f32_takes(x, weight: torch.Tensor, want: Optional[torch.dtype] = None) -> bool:
@@ -669,10 +695,7 @@ def gemm_f32_takes(x, weight: torch.Tensor, want: Optional[torch.dtype] = None) 
     if not F32_GEMM or x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2 or not x.is_contiguous() \
             or not weight.is_contiguous() or want not in (None, torch.float32) or (x.data_ptr() | weight.data_ptr()) & 15:
         return False
-    M, N = x.shape[0], weight.shape[0]
-    if M < F32_MIN_M or weight.numel() < F32_MIN_WEIGHTS or (M > 32 and -(-M // 64) * -(-N // 64) > F32_MAX_TILES) or (M > 16 and N > SKINNY_MAX_N):
-        return False
-    return bool(lib().pllm_gemm_f32_supports(M, *weight.shape))
+    return gemm_f32_sizes(x.shape[0], *weight.shape) and bool(lib().pllm_gemm_f32_supports(x.shape[0], *weight.shape))
 
 
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, tile: int = 0, splits: int = 0) -> torch.Tensor:
