@@ -606,26 +606,39 @@ def gemm_tcgen05(x: torch.Tensor, weight: torch.Tensor, glu: bool = False, statu
 
 
 # The rows of a decode step or of a short prompt in bfloat16 with the weights as the tensor cores' 128-row operand
-# (csrc/rows_gemm_tcgen05.cu).  Measured in captured decode steps with ONE product's kernel changed (us a step):
-#   0.6B shape (products of 2 to 6 M weights), 16 rows: the weight-streaming kernel 872, this one 1032; 24 rows: this one 1285,
-#     the library 1561 (its q/k/v 1304 and o 1301 alone would do as well, its gate/up with the activation's pass 1320 not)
-#   8B shape, 8 rows: q/k/v (25 M weights) 714, the weight-streaming kernel 762; gate/up (101 M) 715 / 883; down (50 M) 714 / 851;
-#     o (17 M) 714 / 717; the head 714, the library 738
-#   64 rows: 8B 983, the library 1045; 128 rows, 0.6B shape: 1648, the library and gemm_tcgen05.cu 1507
-# so it takes 17 to 64 rows, and fewer where the product has ROWS_MIN_WEIGHTS or more.
+# (csrc/rows_gemm_tcgen05.cu).  Measured in captured decode steps at context 512 with ONE product's kernel changed (us a step):
+#   0.6B shape (products of 2 to 6 M weights), 16 rows: the weight-streaming kernel 872, this one 1032
+#     24 rows: this one 1315, the library for q/k/v 1341, o 1344, down 1376, gate/up and its activation's pass 1344
+#     32 rows: 1366, the library 1376, 1389, 1377, 1390;  48 rows: 1679, the library 1683, 1671, 1708, 1718;  64 rows: 1706, 1721, 1690, 1705, 1739
+#   8B shape (6 layers), 8 rows: 722, the library for q/k/v (25 M weights) 740, o (17 M) 753, down (50 M) 805, gate/up (101 M) 879, the head 741;
+#     the weight-streaming kernel 772, 727, 883, 883
+#     32 rows: 866, the library 882, 854, 866, 864, the head 872
+#     48 rows: 968, the library 957, 941, 950, 1034, 964 (for the first three together 947);  64 rows: 973, 967, 942, 948, 1037, 970 (950)
+#   behind a norm alone, 64 rows: 1024 x 256 4.9, the library 3.9; 512 x 1024 5.8 / 4.9; 151936 x 1024 61.8 / 64.7
+# so it takes 17 to 64 rows, and fewer where the product has ROWS_MIN_WEIGHTS or more; but from 33 rows on, of the products without an
+# activation, those between 2^20 and ROWS_MIN_WEIGHTS weights, and the head.
 ROWS_GEMM = True
 ROWS_MAX_M = 64
 ROWS_MIN_WEIGHTS = 16 << 20
 
 
-def rows_gemm_takes(x, weight: torch.Tensor, n_out: int, want: Optional[torch.dtype] = None) -> bool:
+def rows_gemm_sizes(M: int, n_out: int, K: int, weights: int, plain: bool) -> bool:
+    """Whether a bfloat16 product of M rows and so many weights goes with the weights as the 128-row operand (plain: without an activation)."""
+    if M <= SKINNY_MAX_M:
+        return weights >= ROWS_MIN_WEIGHTS
+    if plain and M > 32:
+        return M <= ROWS_MAX_M and (1 << 20 <= weights < ROWS_MIN_WEIGHTS or n_out > SKINNY_MAX_N)
+    return M <= ROWS_MAX_M
+
+
+def rows_gemm_takes(x, weight: torch.Tensor, n_out: int, want: Optional[torch.dtype] = None, plain: bool = False) -> bool:
     """Whether ``linear`` / ``linear_glu`` / ``linear_act`` run the product with the weights as the 128-row operand
-    (n_out: columns of the result)."""
+    (n_out: columns of the result; plain: no activation)."""
     if not ROWS_GEMM or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous() \
             or not weight.is_contiguous() or want not in (None, torch.bfloat16, torch.float32) or (x.data_ptr() | weight.data_ptr()) & 15:
         return False
     M, K = x.shape[0], weight.shape[1]
-    return M <= ROWS_MAX_M and (M > SKINNY_MAX_M or weight.numel() >= ROWS_MIN_WEIGHTS) and bool(lib().pllm_rows_gemm_supports(M, n_out, K))
+    return rows_gemm_sizes(M, n_out, K, weight.numel(), plain) and bool(lib().pllm_rows_gemm_supports(M, n_out, K))
 
 
 def rows_gemm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, glu: bool = False,
@@ -746,7 +759,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         swiglu(x, act)
         x = act
     fits = out is None or (out.shape == (x.shape[0], N) and out.dtype == want and out.is_contiguous() and not out.data_ptr() & 15)
-    if fits and rows_gemm_takes(x, weight, N, want):
+    if fits and rows_gemm_takes(x, weight, N, want, plain=True):
         return rows_gemm(x, weight, out, status=status, out_dtype=want)
     if skinny_gemm_takes(x, weight, K) and N <= SKINNY_MAX_N and want in (torch.bfloat16, torch.float32):
         _dev(x, weight, out)

@@ -1,4 +1,4 @@
-"""Which products are this library's and which cuBLAS's (kernels/ops.py, gemm_f32_sizes): at sizes where one of the
+"""Which products are this library's and which cuBLAS's (kernels/ops.py, gemm_f32_sizes and rows_gemm_sizes): at sizes where one of the
 two was measured to be slower it must not be the one that is taken."""
 
 import pytest
@@ -18,3 +18,14 @@ def test_float32_products_of_the_library(M, N, K):
                                    (16, 12288, 4096), (24, 1024, 512), (16, 2048, 512)])
 def test_float32_products_of_this_library(M, N, K):
     assert ops.gemm_f32_sizes(M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 6144, 4096), (48, 4096, 4096), (64, 4096, 12288), (64, 1024, 256), (48, 512, 1024), (65, 1024, 2048), (16, 4096, 1024)])
+def test_plain_products_of_the_library_or_the_weight_streaming_kernel(M, N, K):
+    assert not ops.rows_gemm_sizes(M, N, K, N * K, True)
+
+
+@pytest.mark.parametrize("M,N,K,rows_of_w,plain", [(8, 6144, 4096, 6144, True), (32, 4096, 12288, 4096, True), (64, 1024, 2048, 1024, True), (17, 256, 256, 256, True),
+                                                   (64, 151936, 1024, 151936, True), (64, 12288, 4096, 24576, False), (48, 512, 1024, 1024, False)])
+def test_products_with_the_weights_as_the_128_row_operand(M, N, K, rows_of_w, plain):
+    assert ops.rows_gemm_sizes(M, N, K, rows_of_w * K, plain)
