@@ -654,8 +654,10 @@ def rows_gemm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
         raise KernelError("rows_gemm: bfloat16 operands, a bfloat16 or float32 result")
     if out is None:
         out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
-    elif out.shape != (M, n_out) or out.dtype != out_dtype:
+    elif out.shape != (M, n_out) or out.dtype != out_dtype or not out.is_contiguous():
         raise KernelError("rows_gemm: out does not fit")
+    if not x.is_contiguous() or not weight.is_contiguous():
+        raise KernelError("rows_gemm: rows that do not lie together")
     _dev(x, weight, out)
     st = status if status is not None else gemm_status(x.device)
     _check(lib().pllm_rows_gemm(_ptr(x), _ptr(weight), _ptr(out), M, n_out, K, 1 + _glu(act) if glu else -UNARY_KINDS[unary], float(limit),
@@ -720,8 +722,10 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
         raise KernelError(f"gemm_f32: does not take x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    elif out.shape != (M, N) or out.dtype != torch.float32:
+    elif out.shape != (M, N) or out.dtype != torch.float32 or not out.is_contiguous():
         raise KernelError("gemm_f32: out does not fit")
+    if not x.is_contiguous() or not weight.is_contiguous():
+        raise KernelError("gemm_f32: rows that do not lie together")
     _dev(x, weight, out)
     _check(lib().pllm_gemm_f32(_ptr(x), _ptr(weight), _ptr(out), M, N, K, tile, splits, _stream()), "gemm_f32")
     return out
@@ -731,15 +735,18 @@ def skinny_glu_takes(x, weight: torch.Tensor, n_out: int) -> bool:
     """Whether the weight-streaming kernel takes the gate/up product with the activation in its epilogue."""
     if not SKINNY_GEMM or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.dim() != 2:
         return False
-    return x.shape[0] <= SKINNY_MAX_M and n_out <= SKINNY_MAX_N and bool(lib().pllm_skinny_gemm_glu_supports(x.shape[0], n_out, weight.shape[1]))
+    return n_out <= SKINNY_MAX_N and bool(lib().pllm_skinny_gemm_glu_supports(x.shape[0], n_out, weight.shape[1]))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, gated: bool = False,
            out_dtype: Optional[torch.dtype] = None, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y = x W^T with W stored [out, in].
 
-    Few rows (a decode step) in bfloat16 run this library's weight-streaming
-    kernel.  With ``gated`` the input is [g | u] of twice W's width and the
+    bfloat16: up to 16 rows (a decode step) run this library's weight-streaming
+    kernel, or with many weights, and up to 64 rows (rows_gemm_sizes), the kernel
+    with the weights as the tensor cores' 128-row operand.  float32: few rows, or
+    some more into few columns (gemm_f32_sizes), run this library's product on the
+    CUDA cores.  With ``gated`` the input is [g | u] of twice W's width and the
     product is taken of silu(g) * u, formed by the activation kernel first.
     Everything else is the library matrix product (cuBLAS through torch), which
     is where the reference uses a library too
@@ -784,9 +791,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
 def linear_glu(x: torch.Tensor, w_gate_up: torch.Tensor, status: Optional[torch.Tensor] = None, act: str = "silu",
                limit: float = 0.0) -> torch.Tensor:
     """act(x Wg^T, x Wu^T), silu(g) * u unless ``act`` says otherwise, for W = [Wg; Wu] stacked [2I, K]: the gated
-    feed-forward's first half (crates/pagedllm/src/model/layers.rs:93-99).  Few
-    rows in bfloat16: one kernel whose CTAs hold the same columns of both halves;
-    many rows: the tcgen05 product with the activation in its epilogue; otherwise
+    feed-forward's first half (crates/pagedllm/src/model/layers.rs:93-99).  Up to
+    16 rows in bfloat16: one kernel whose CTAs hold the same columns of both halves;
+    up to 64 rows, and fewer with many weights: the product with the weights as the 128-row operand;
+    many rows: the tcgen05 product; each with the activation in its epilogue.  Otherwise
     the product, then the activation kernel."""
     two_i, K = w_gate_up.shape
     if two_i % 2:
@@ -1561,8 +1569,8 @@ def unary_act(x: torch.Tensor, act: str) -> torch.Tensor:
 
 def linear_act(x: torch.Tensor, weight: torch.Tensor, act: str, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """act(x W^T) for a one-argument activation: the first half of a feed-forward without a gate.  In bfloat16 the
-    activation sits in the epilogue of the weight-streaming product (few rows) or of the tcgen05 product (many rows);
-    otherwise the product, then the activation in place."""
+    activation sits in the epilogue of the weight-streaming product (few rows), of the one with the weights as the 128-row operand
+    (up to 64) or of the tcgen05 product (many rows); otherwise the product, then the activation in place."""
     if act not in UNARY_KINDS:
         raise KernelError(f"linear_act: activation {act!r} is not known; known: {sorted(UNARY_KINDS)}")
     N, K = weight.shape
