@@ -25,3 +25,24 @@ def test_pairs_of_ctas(M, tiles_n, K, glu):
     assert st.item() == 0 and torch.equal(y, one)
     if not glu:
         torch.testing.assert_close(y.float(), x.float() @ w.float().T, atol=3e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("M", [256, 900])
+@pytest.mark.parametrize("act,limit,f", [("relu", 0.0, lambda g, u: g.clamp(min=0) * u),
+                                         ("clamped", 2.0, lambda g, u: g.clamp(max=2.0) * torch.sigmoid(1.702 * g.clamp(max=2.0)) * (u.clamp(-2.0, 2.0) + 1)),
+                                         ("squared_relu", None, lambda g: g.clamp(min=0).square())])
+def test_pairs_of_ctas_with_the_other_activations(M, act, limit, f):
+    g = torch.Generator(device=DEV).manual_seed(M)
+    K, n_out = 320, 80 * 256
+    glu = limit is not None
+    x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn((2 if glu else 1) * n_out, K, device=DEV, generator=g) * 0.05).bfloat16()
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    run = (lambda r: ops.gemm_tcgen05(r, w, glu=True, status=st, act=act, limit=limit)) if glu else (lambda r: ops.linear_act(r, w, act, status=st))
+    y = run(x)
+    one = torch.cat([run(x[r:r + 128].contiguous()) for r in range(0, M, 128)])
+    assert st.item() == 0 and torch.equal(y, one)
+    h = ops.gemm_tcgen05(x, w, status=st).float()       # (the product as it is rounded before the activation reads it)
+    want = f(h[:, :n_out], h[:, n_out:]) if glu else f(h)
+    # (the activation's result is rounded to bfloat16, and formed with the fast exponential and division)
+    torch.testing.assert_close(y.float(), want, atol=1e-3, rtol=2 ** -7)
