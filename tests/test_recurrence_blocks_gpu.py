@@ -235,3 +235,19 @@ def test_a_step_of_segments_on_both_sides_of_the_longest(cut):
     for got, (u, ba) in zip(delta_steps(True, torch.float32, [cut], seqs, conv_w, *rest, longest=was[1]), seqs):
         want = plain_delta(u, conv_w, ba, *rest)
         assert float((got.double() - want).norm() / want.norm()) <= 2e-6
+
+
+@pytest.mark.parametrize("taps", [1, 2, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_the_delta_rules_convolution_from_step_to_step(dtype, taps):
+    # (a portion shorter than the taps, then single tokens, a step of single tokens alone having a convolution of its own, then a portion again)
+    H, G, d, E = 2, 1, 16, 24
+    g = torch.Generator().manual_seed(taps)
+    c = 2 * G * d + H * E
+    cuts = [(3, 20), (1, 1), (1, 1), (1, 0), (9, 1), (1, 30)]
+    n = [sum(cut[r] for cut in cuts) for r in range(2)]
+    seqs = [(torch.randn(t, c + H * E, generator=g).to(dtype).float(), torch.randn(t, 2 * H, generator=g)) for t in n]
+    conv_w, rest = (torch.randn(c, taps, generator=g) * 0.4).to(dtype).float(), (torch.zeros(H), torch.zeros(H), torch.ones(E), H, G, d, E)
+    for got, (u, ba) in zip(delta_steps(True, dtype, cuts, seqs, conv_w, *rest), seqs):
+        want = plain_delta(u, conv_w, ba, *rest)
+        assert float((got.double() - want).norm() / want.norm()) <= (2e-6 if dtype == torch.float32 else 4e-3)

@@ -94,3 +94,14 @@ def test_a_product_into_a_buffer_that_the_kernels_do_not_write_is_the_librarys(d
         # (two float sums of 1024 products in another order, then one rounding to bfloat16, an ulp apart at most)
         torch.testing.assert_close(got, want, atol=1e-2 if dtype == torch.bfloat16 else 1e-3, rtol=2 ** -7 if dtype == torch.bfloat16 else 1e-4)
     assert not wide[:, 1::2].any()
+
+
+def test_rows_that_do_not_lie_together_are_refused():
+    from paged_llm_rs_b200.errors import KernelError
+    x, w = inputs(24, 256, 512)
+    wide = torch.zeros(24, 512, dtype=torch.bfloat16, device=DEV)
+    for f, a, b, out in ((ops.rows_gemm, x[:, :256], w[:, :256].contiguous(), None), (ops.rows_gemm, x, w.t().contiguous().t(), None),
+                         (ops.rows_gemm, x, w, wide[:, ::2]), (ops.gemm_f32, x.float()[:, :256], w.float()[:, :256].contiguous(), None),
+                         (ops.gemm_f32, x.float(), w.float(), wide.float()[:, ::2])):
+        with pytest.raises(KernelError):
+            f(a, b, out)

@@ -46,7 +46,7 @@ def test_sandwich_norm(dtype, n, W, off):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("off", [0, 1])
-@pytest.mark.parametrize("n,width", [(1, 8), (3, 20), (130, 1024), (1025, 3072), (7, 1032)])
+@pytest.mark.parametrize("n,width", [(1, 8), (3, 20), (130, 1024), (1025, 3072), (7, 1032), (127, 1024), (128, 1032)])
 def test_biased_gated_activation_and_gate(dtype, n, width, off):
     g = torch.Generator(device=DEV).manual_seed(n + width + off)
     gu, bias = at((n, 2 * width), dtype, g, off), at((2 * width,), torch.float32, g, off, 0.3)
