@@ -6,7 +6,8 @@
 // so u = U - W S0, where the rows of U and W solve the same triangular system with beta_t v_t and beta_t exp(G_t) k_t on the right
 // and do not depend on the state: all blocks solve it AT THE SAME TIME.  What goes from block to block is two products,
 //     u = U - W S0,   S <- exp(G_L) S0 + sum_s exp(G_L - G_s) k_s u_s^T
-// and the outputs follow, again for all blocks at once: o_t = exp(G_t) S0^T q_t + sum_{s <= t} exp(G_t - G_s) (q_t . k_s) u_s.
+// (the chunkwise form of the delta rule: Yang et al., "Parallelizing Linear Transformers with the Delta Rule over Sequence Length", 2024, and "Gated Delta
+// Networks", 2024), and the outputs follow, again for all blocks at once: o_t = exp(G_t) S0^T q_t + sum_{s <= t} exp(G_t - G_s) (q_t . k_s) u_s.
 //   delta_solve_kernel    unit vectors, G, the triangular system by forward substitution (16 rows at a time)
 //   delta_states_kernel   a head's 16 columns of S through the blocks of a segment
 //   delta_outputs_kernel  the outputs
@@ -15,7 +16,8 @@
 //
 // What bounds the recurrence is its chain (440 ns a token and head); what bounds the blocks is delta_states_kernel's chain, a few
 // microseconds a block of 64 tokens.  1016 tokens beside 8 decoded ones, 8 heads of 128 x 128 over 4 key heads (us, caches cold): the
-// recurrence 446; these kernels 47 + 74 + 47, and 14 for the decoded tokens.
+// recurrence 446; these kernels 45 + 76 + 49, and 13 for the decoded tokens.  A segment that is not long goes through the recurrence all the same
+// (kernels/ops.py, DELTA_LONGEST).
 #pragma once
 
 #include "matrix_memory.cuh"

@@ -1,6 +1,7 @@
 // The matrix LSTM over a prompt's portion in blocks of 64 tokens that run AT THE SAME TIME (matrix_memory.cu has the recurrence
 // token by token, for decoded tokens and short portions, and says what is computed).
 //
+// (The chunkwise form of the matrix LSTM: Beck et al., "xLSTM: Extended Long Short-Term Memory", 2024, and "Tiled Flash Linear Attention", 2025.)
 // With the running maximum m known for every token, the recurrence is linear: S_t = a_t S_(t-1) + b_t k_t v_t^T with
 // a_t = exp(f_t + m_(t-1) - m_t) and b_t = exp(i_t - m_t), both at most one.  With F the sum of f since a block's start and m0, S0
 // what the block starts from, token t's numerator is
@@ -14,7 +15,8 @@
 //
 // What bounds the recurrence is its chain (240 ns a token and head, 32 CTAs at work for one prompt); what bounds the blocks is
 // the reads from shared memory behind their products.  1016 tokens beside 8 decoded ones, 4 heads of 128 x 256 (us, caches cold): the
-// recurrence 244; these kernels 8 + 17 + 14 + 40, and 11 for the decoded tokens.
+// recurrence 244; these kernels 8 + 17 + 14 + 40, and 11 for the decoded tokens.  A segment that is not long goes through the recurrence
+// all the same (kernels/ops.py, MLSTM_LONGEST).
 #pragma once
 
 #include "matrix_memory.cuh"
