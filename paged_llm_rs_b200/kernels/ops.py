@@ -654,10 +654,8 @@ def rows_gemm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
         raise KernelError("rows_gemm: bfloat16 operands, a bfloat16 or float32 result")
     if out is None:
         out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
-    elif out.shape != (M, n_out) or out.dtype != out_dtype or not out.is_contiguous():
+    elif out.shape != (M, n_out) or out.dtype != out_dtype:
         raise KernelError("rows_gemm: out does not fit")
-    if not x.is_contiguous() or not weight.is_contiguous():
-        raise KernelError("rows_gemm: rows that do not lie together")
     _dev(x, weight, out)
     st = status if status is not None else gemm_status(x.device)
     _check(lib().pllm_rows_gemm(_ptr(x), _ptr(weight), _ptr(out), M, n_out, K, 1 + _glu(act) if glu else -UNARY_KINDS[unary], float(limit),
@@ -722,10 +720,8 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
         raise KernelError(f"gemm_f32: does not take x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    elif out.shape != (M, N) or out.dtype != torch.float32 or not out.is_contiguous():
+    elif out.shape != (M, N) or out.dtype != torch.float32:
         raise KernelError("gemm_f32: out does not fit")
-    if not x.is_contiguous() or not weight.is_contiguous():
-        raise KernelError("gemm_f32: rows that do not lie together")
     _dev(x, weight, out)
     _check(lib().pllm_gemm_f32(_ptr(x), _ptr(weight), _ptr(out), M, N, K, tile, splits, _stream()), "gemm_f32")
     return out
