@@ -84,6 +84,16 @@ __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t desc_a, uint64_
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n"
                  ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
+// The same with descriptors given by their lower halves (desc_lo), whose upper half is a constant: 16 values of k further along are an
+// addition of 2.
+constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);       // stride 1024, version 1, 128-byte swizzle
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr >> 4) & 0x3fff) | (1u << 16); }
+template <bool ACCUMULATE>
+__device__ __forceinline__ void mma_ss_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+    asm volatile("{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.u32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
+                 ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "n"(ACCUMULATE ? 1 : 0), "n"(DESC_HI) : "memory");
+}
 // The same with the A operand in tensor memory: rows are lanes, two 16-bit values of k to a 32-bit column
 // (16 values of k = 8 columns), k ascending from the low half.
 __device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {

@@ -71,6 +71,8 @@ def lib():
         sig["pllm_gemm_tcgen05"] = [P, P, P, c_int, c_int, c_int, c_int, c_float, P, P]
         sig["pllm_gemm_f32_supports"] = [c_int, c_int, c_int]
         sig["pllm_gemm_f32"] = [P, P, P, c_int, c_int, c_int, c_int, c_int, P]
+        sig["pllm_gemm_f32_tcgen05_supports"] = [c_int, c_int, c_int]
+        sig["pllm_gemm_f32_tcgen05"] = [P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P, P]
         sig["pllm_rows_gemm_supports"] = [c_int, c_int, c_int]
         sig["pllm_rows_gemm"] = [P, P, P, c_int, c_int, c_int, c_int, c_float, c_int, c_int, P, P]
         sig["pllm_embed_scaled32"] = [c_int, P, P, P, c_int, c_int, c_int, c_float, P, P]
@@ -727,6 +729,57 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
     return out
 
 
+# float32 products on the tensor cores (csrc/gemm_f32_tcgen05.cu), measured on a B200 (us; what ran before / this with weights that a
+# bfloat16 holds / with any weights, the parts of x made inside):
+#   N x K          32 rows            64                 128                256                512                1024
+#   512 x 1024     - 7.4/ 7.2/ 8.6    - 7.5/ 7.9/ 9.5    - 11.8/ 9.9/11.7   - 19.2/13.3/17.2   - 21.4/13.7/18.0   - 29.5/17.2/23.9
+#   2048 x 512     - 7.5/ 7.0/ 8.4    - 11.1/ 7.9/ 9.8   - 12.4/ 9.6/11.7   - 16.3/12.9/16.9   - 25.0/14.5/18.8   - 44.5/19.0/28.1
+#   1024 x 2048    - 12.7/10.6/13.9   20.6/11.2/15.2     21.2/13.1/18.5     36.7/17.3/25.9     56.3/21.9/36.1     85.2/25.5/44.5
+#   6144 x 1024    - 24.1/14.7/22.4   31.9/16.2/25.0     45.0/18.1/29.8     73.1/23.5/43.2     141/36.4/75.6      248/68.6/144
+#   4096 x 12288   - 110/69.0/125     216/72.1/134       360/80.1/152       489/93.7/209       909/163/399        1800/307/802
+#   24576 x 4096   - 204/162/305      - 280/163/327      546/176/371        972/212/515        1773/333/771       3607/673/1619
+#   32768 x 1024   - 60.0/52.2/91.6   - 89.3/52.0/92.8   158/57.1/104       313/70.4/146       624/141/286        1089/249/511
+# (- stays as it was): what it takes is faster with any weights, and two to five times as fast with weights from a bfloat16 file.  Its
+# error is the smaller one too, against 64 bits, relative to the result: 1.0e-7 to 1.6e-7 for K of 1024 to 12288, before 5.7e-7 to 2.0e-6.
+F32_TENSOR_CORES = True
+
+
+def gemm_f32_tcgen05_sizes(M: int, N: int, K: int) -> bool:
+    """Whether the float32 product of M rows of x and N of W over K entries runs on the tensor cores."""
+    if N * K < 1 << 20 or K < 1024:        # (two launches and little else)
+        return False
+    return M > 64 or (M > 32 and N <= 8192)
+
+
+def gemm_f32_tcgen05_takes(x, weight: torch.Tensor, want: Optional[torch.dtype] = None) -> bool:
+    """Whether ``linear`` runs the float32 product on the tensor cores (csrc/gemm_f32_tcgen05.cu)."""
+    if not F32_TENSOR_CORES or x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2 or not x.is_contiguous() \
+            or not weight.is_contiguous() or want not in (None, torch.float32) or (x.data_ptr() | weight.data_ptr()) & 15:
+        return False
+    return gemm_f32_tcgen05_sizes(x.shape[0], *weight.shape) and bool(lib().pllm_gemm_f32_tcgen05_supports(x.shape[0], *weight.shape))
+
+
+def gemm_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None,
+                     tile: int = 0, splits: int = 0) -> torch.Tensor:
+    """x W^T in float32 on the tensor cores, x and W each as three bfloat16 parts (csrc/gemm_f32_tcgen05.cu).  ``tile``: rows of x
+    a tile (32, 64, 128, 256), ``splits``: CTAs that share the sum over k (0: as the sizes ask)."""
+    M, K = x.shape
+    N = weight.shape[0]
+    if weight.shape[1] != K or x.dtype != torch.float32 or weight.dtype != torch.float32 or not lib().pllm_gemm_f32_tcgen05_supports(M, N, K):
+        raise KernelError(f"gemm_f32_tcgen05: does not take x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    elif out.shape != (M, N) or out.dtype != torch.float32:
+        raise KernelError("gemm_f32_tcgen05: out does not fit")
+    _dev(x, weight, out)
+    parts = torch.empty((3, M, K), dtype=torch.bfloat16, device=x.device)
+    odd_row = torch.empty(M, dtype=torch.int32, device=x.device)
+    st = status if status is not None else gemm_status(x.device)
+    _check(lib().pllm_gemm_f32_tcgen05(_ptr(x), _ptr(weight), _ptr(out), _ptr(parts), _ptr(odd_row), M, N, K, tile, splits, _ptr(st), _stream()),
+           "gemm_f32_tcgen05", 2)
+    return out
+
+
 def skinny_glu_takes(x, weight: torch.Tensor, n_out: int) -> bool:
     """Whether the weight-streaming kernel takes the gate/up product with the activation in its epilogue."""
     if not SKINNY_GEMM or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.dim() != 2:
@@ -740,9 +793,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
 
     bfloat16: up to 16 rows (a decode step) run this library's weight-streaming
     kernel, or with many weights, and up to 64 rows (rows_gemm_sizes), the kernel
-    with the weights as the tensor cores' 128-row operand.  float32: few rows, or
-    some more into few columns (gemm_f32_sizes), run this library's product on the
-    CUDA cores.  With ``gated`` the input is [g | u] of twice W's width and the
+    with the weights as the tensor cores' 128-row operand.  float32: more than 32 rows
+    (gemm_f32_tcgen05_sizes) run on the tensor cores in three bfloat16 parts, fewer
+    (gemm_f32_sizes) this library's product on the CUDA cores.  With ``gated`` the input is [g | u] of twice W's width and the
     product is taken of silu(g) * u, formed by the activation kernel first.
     Everything else is the library matrix product (cuBLAS through torch), which
     is where the reference uses a library too
@@ -774,6 +827,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         _check(lib().pllm_skinny_gemm(_ptr(x), _ptr(weight), _ptr(out), M, N, K,
                                       1 if want == torch.float32 else 0, _stream()), "skinny_gemm")
         return out
+    if fits and gemm_f32_tcgen05_takes(x, weight, want):
+        return gemm_f32_tcgen05(x, weight, out, status)
     if fits and gemm_f32_takes(x, weight, want):
         return gemm_f32(x, weight, out)
     if TCGEN05_GEMM >= 2 and out is None and want == torch.bfloat16 and x.shape[0] >= TCGEN05_MIN_M \
