@@ -47,6 +47,7 @@ class GroupPlanConfig:
     heads: int = 1        # partial results of split items are [rows, heads, head_dim]
     head_dim: int = 1
     chunk: int = 0        # a query reads its own chunk of this many tokens only (0: no chunks)
+    part_keys: int = 0    # keys of a part where a step of several tokens a request is cut (0: by the planner's usual rule)
 
 
 @dataclass
@@ -143,10 +144,10 @@ class StepPacker:
                 group_parts.append((None, None, 0, 0, 0, W))
                 continue
             # groups that cut their work alike (same tile, window, chunk, CTAs an item) share one plan
-            key = (plan.tile_tokens, plan.window, plan.ctas_per_item, plan.chunk)
+            key = (plan.tile_tokens, plan.window, plan.ctas_per_item, plan.chunk, plan.part_keys)
             if key not in planned:
                 planned[key] = attention_plan.plan_attention(spans, plan.tile_tokens, plan.window, plan.ctas_per_item, self.target_ctas,
-                                                             chunk=plan.chunk)
+                                                             chunk=plan.chunk, part_keys=plan.part_keys)
             work, red, parts = planned[key]
             mw, mr, mp = (work_caps[gi] if work_caps else (len(work), len(red), parts))
             if len(work) > mw or len(red) > mr or parts > mp:

@@ -33,16 +33,25 @@ MAX_SPLITS = 128   # the reduce kernel holds the weights of up to 256 splits in 
 # token, 0.6B shape: cut in four from 256 keys on, the attention took 25 us a layer and the reduction 17;
 # whole, see profiles/prefill_2048_tokens.md).
 MULTI_MIN_SPLIT_KEYS = 2048
+# The float32 kernel on the CUDA cores needs some 10 us for 64 keys of its tile of 32 rows, so there a part of few keys is worth its partial
+# results (part_keys below; us a step of the 0.6B shape whole / in parts of 64 / 128 / 192 / 256 keys: 4 decoded tokens beside 252 behind 100
+# 4534 / 4208 / 4207 / 4153 / 4354; 2 beside 60 behind 600 5116 / 2989 / 3051 / 3106 / 3379; 250 alone 3914 / 3709 / 3635 / 3811 / 3909;
+# 4 at 1500 beside 40 2732 / 2791 / 2787 / 2513 / 2619).
+F32_PART_KEYS = 192
 
 
 def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, window: Optional[int],
                    ctas_per_item: int, target_ctas: int,
                    min_split_keys: int = MIN_SPLIT_KEYS,
-                   multi_min_split_keys: int = MULTI_MIN_SPLIT_KEYS, chunk: int = 0) -> Tuple[np.ndarray, np.ndarray, int]:
+                   multi_min_split_keys: int = MULTI_MIN_SPLIT_KEYS, chunk: int = 0, part_keys: int = 0) -> Tuple[np.ndarray, np.ndarray, int]:
     """segments: (first token index, token count, position of the first token) per
-    segment, in step order; ``chunk``: a query reads keys of its own chunk of that many positions only.  Returns (work [n, 8], red [m, 4], partial rows used)."""
+    segment, in step order; ``chunk``: a query reads keys of its own chunk of that many positions only; ``part_keys``: a step with tiles of
+    several tokens is cut into parts of that many keys, or of so many more that they stay within twice the target.
+    Returns (work [n, 8], red [m, 4], partial rows used)."""
+    in_parts = part_keys > 0 and any(c > 1 for _, c, _ in segments)
     if len(segments) <= SMALL_PLAN:
-        small = _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk)
+        small = _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk,
+                            part_keys if in_parts else 0)
         if small is not None:
             return small
     seg_ids, q0s, qns, p0s = [], [], [], []
@@ -70,7 +79,19 @@ def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, w
     keys = kv_end - kv_begin
 
     splits = np.ones(n_tiles, dtype=np.int64)
-    if n_tiles * ctas_per_item < target_ctas:
+    if in_parts:
+        most = 2 * target_ctas // ctas_per_item
+        if n_tiles < most:
+            size = part_keys
+            while int((-(-keys // size)).sum()) > most or int(keys.max()) > MAX_SPLITS * size:
+                size += SPLIT_ALIGN
+            splits = -(-keys // size)
+            # (single tokens are cut as finely as by the rule below where that stays within the bound too)
+            finer = np.where(qn == 1, np.maximum(splits, np.minimum(min(target_ctas // (n_tiles * ctas_per_item), MAX_SPLITS),
+                                                                    keys // min_split_keys)), splits)
+            if int(finer.sum()) <= most:
+                splits = finer
+    elif n_tiles * ctas_per_item < target_ctas:
         # as many splits as keep the launch within the target (one or two full waves of
         # CTAs), rounded down so that the last wave is not a sliver.  A step of single tokens that
         # falls short of the target is cut in two at least; tiles of many tokens are not (their
@@ -111,7 +132,7 @@ def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, w
 SMALL_PLAN = 32        # segments, and tiles, of a step that is planned number by number
 
 
-def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk):
+def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk, part_keys=0):
     """``plan_attention`` for a step of few tiles of which none is split (a prompt's portion, as a rule): the same list without the
     forty array operations that cost such a step more than its work (35 to 80 us).  None when it is not one."""
     items, most = [], 0
@@ -123,6 +144,8 @@ def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_s
         for start in range((count - 1) // tile_tokens * tile_tokens, -1, -tile_tokens):
             n, p = min(tile_tokens, count - start), pos0 + start
             begin = max(0, p - (window - 1)) if window else (p - p % chunk if chunk else 0)
+            if part_keys and p + n - begin > part_keys:
+                return None
             items.append((si, tok0 + start, n, p, begin, p + n, -1, 0))
             most = max(most, n)
     if not items:
@@ -134,7 +157,7 @@ def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_s
         if want > 1:
             for _, _, n, _, begin, end, _, _ in items:
                 if end - begin >= 2 * (max(min_split_keys, multi_min_split_keys) if n > 1 else min_split_keys):
-                    return None
+                    return None       # (in parts, a tile of several tokens has been looked at above)
     return np.array(items, dtype=np.int32), np.zeros((0, 4), np.int32), 0
 
 

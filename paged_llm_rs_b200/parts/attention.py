@@ -14,6 +14,7 @@ import torch
 
 from ..errors import KernelError
 from ..kernels import ops
+from ..kernels.attention_plan import F32_PART_KEYS
 from .base import KVNeed, Mixer, PlanWish, register_mixer
 from .spec import TensorSpec
 
@@ -66,7 +67,8 @@ class GQAttention(Mixer):
 
     def plan_wish(self, page_size: int):
         tile = ops.attention_tile_tokens(self.nh, self.nkv, self.rt.dtype, self.hd, page_size, self.window or 0)
-        return PlanWish(tile, ops.attention_ctas_per_item(self.nh, self.nkv, self.rt.dtype), self.nh, self.hd)
+        return PlanWish(tile, ops.attention_ctas_per_item(self.nh, self.nkv, self.rt.dtype), self.nh, self.hd,
+                        F32_PART_KEYS if self.rt.dtype == torch.float32 else 0)
 
     def forward(self, x, step, cache, writes_cache=True):
         k_pool, v_pool, gi = cache
