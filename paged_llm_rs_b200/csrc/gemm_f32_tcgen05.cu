@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
         } else if (warp == 13) {
             // ---- issue ---------------------------------------------------------------------------------------------
             constexpr uint32_t idesc = instr_desc(S_BM, ROWS);
+            const uint32_t one = elect_one() ? 1 : 0;
             int s = 0;
             uint32_t turn = 0;                         // of the ring
             bool ok = true;
@@ -288,34 +289,31 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
                 const uint32_t acc = tmem + b * ROWS, w_lo = desc_lo(wparts + b * S_PART_W);
                 const uint32_t w2_lo = desc_lo(wparts + 2 * S_PART_W), w3_lo = desc_lo(wparts + 3 * S_PART_W);
                 auto products = [&](uint32_t wl, uint32_t xl, auto first) {      // 16 values of k = 32 bytes along the swizzled row
-                    mma_ss_lo<!decltype(first)::value>(acc, wl, xl, idesc);
+                    mma_ss_lo<!decltype(first)::value>(acc, wl, xl, idesc, one);
 #pragma unroll
-                    for (int j = 1; j < S_BK / 16; j++) mma_ss_lo<true>(acc, wl + 2 * j, xl + 2 * j, idesc);
+                    for (int j = 1; j < S_BK / 16; j++) mma_ss_lo<true>(acc, wl + 2 * j, xl + 2 * j, idesc, one);
                 };
 #pragma unroll
                 for (int p = 2; p >= 0; p--) {
                     if (!__all_sync(0xffffffffu, mbar_wait(xfull + 8 * s, turn, abort_flag))) { ok = false; break; }
                     tc_fence_after();
-                    if (elect_one()) {
-                        const uint32_t x_lo = desc_lo(ring + s * PART_X);
-                        if (p == 2) {
-                            // (the smallest product begins the sum; x3 w3 is left out)
-                            if (has & 2) {
-                                products(w2_lo, x_lo, std::true_type());
-                                products(w_lo, x_lo, std::false_type());
-                            } else products(w_lo, x_lo, std::true_type());
-                        } else {
-                            if (has & 4) products(w3_lo, x_lo, std::false_type());
-                            if (has & 2) products(w2_lo, x_lo, std::false_type());
+                    const uint32_t x_lo = desc_lo(ring + s * PART_X);
+                    if (p == 2) {
+                        // (the smallest product begins the sum; x3 w3 is left out)
+                        if (has & 2) {
+                            products(w2_lo, x_lo, std::true_type());
                             products(w_lo, x_lo, std::false_type());
-                        }
-                        mma_commit(xempty + 8 * s);
-                        if (p == 0) {
-                            mma_commit(wempty + 8 * b);
-                            mma_commit(accfull + 8 * b);
-                        }
+                        } else products(w_lo, x_lo, std::true_type());
+                    } else {
+                        if (has & 4) products(w3_lo, x_lo, std::false_type());
+                        if (has & 2) products(w2_lo, x_lo, std::false_type());
+                        products(w_lo, x_lo, std::false_type());
                     }
-                    __syncwarp();
+                    mma_commit_one(xempty + 8 * s, one);
+                    if (p == 0) {
+                        mma_commit_one(wempty + 8 * b, one);
+                        mma_commit_one(accfull + 8 * b, one);
+                    }
                     if (++s == RING) { s = 0; turn ^= 1; }
                 }
             }

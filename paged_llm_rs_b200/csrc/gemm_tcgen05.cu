@@ -16,10 +16,12 @@
 //   warp 4     producer: waits for a free stage, arms its barrier with the bytes to come and
 //              issues the TMA loads (a 128 x 64 tile of x, a BN x 64 tile of W; GLU: BN/2 rows
 //              of gate and of up)
-//   warp 5     allocates tensor memory (two accumulators of BN columns); one lane waits for
+//   warp 5     allocates tensor memory (two accumulators of BN columns); waits for
 //              a full stage and issues four tcgen05.mma (K = 16 each), then tcgen05.commit,
 //              which frees the stage when those have read it; after a tile's last, a commit
-//              to that accumulator's barrier
+//              to that accumulator's barrier.  All its lanes go through the loop and one of them
+//              executes these instructions (tcgen05.cuh, mma_ss_lo): issued by a thread of its own, the 0.6B
+//              shape's 2048-token step took 3071 us and the 8B shape's 4421, this way 3028 to 3039 and 4315 to 4337
 //   warps 0-3  epilogue: wait for an accumulator, tcgen05.ld their 32 lanes (= rows) 32
 //              columns at a time, convert, (activation,) store, hand the accumulator back;
 //              the tensor cores are on the next tile meanwhile
@@ -177,30 +179,31 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tcgen05_kernel(const __grid
         }
     } else if (warp == 5) {
         // ---- tensor-core issue ------------------------------------------------------------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(G_BM, BN);
-            int it = 0, i = 0;
-            bool ok = true;
-            if (tile_expert) asm volatile("griddepcontrol.wait;\n" ::: "memory");
-            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-                if (tile_expert && tile_expert[t % tiles_m] < 0) continue;
-                const int b = i & 1;
-                // the epilogue must have read this accumulator's last tile out
-                if (i >= 2 && !mbar_wait(acc_empty + 8 * b, ((i >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+        constexpr uint32_t idesc = instr_desc(G_BM, BN);
+        const uint32_t one = elect_one() ? 1 : 0;
+        int i = 0, s = 0;
+        uint32_t turn = 0;
+        bool ok = true;
+        if (tile_expert) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            if (tile_expert && tile_expert[t % tiles_m] < 0) continue;
+            const int b = i & 1;
+            // the epilogue must have read this accumulator's last tile out
+            if (i >= 2 && !__all_sync(0xffffffffu, mbar_wait(acc_empty + 8 * b, ((i >> 1) - 1) & 1, abort_flag))) { ok = false; break; }
+            tc_fence_after();
+            for (int kb = 0; kb < k_blocks; kb++) {
+                if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * s, turn, abort_flag))) { ok = false; break; }
                 tc_fence_after();
-                for (int kb = 0; kb < k_blocks; kb++, it++) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(bars + 8 * s, (it / STAGES) & 1, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a_src = tiles + s * STAGE, b_src = a_src + G_TILE_A;
+                const uint32_t a_lo = desc_lo(tiles + s * STAGE), b_lo = desc_lo(tiles + s * STAGE + G_TILE_A), d = tmem + b * BN;
+                if (kb == 0) mma_ss_lo<false>(d, a_lo, b_lo, idesc, one);
+                else mma_ss_lo<true>(d, a_lo, b_lo, idesc, one);
 #pragma unroll
-                    for (int j = 0; j < G_BK / 16; j++)   // 16 values of k = 32 bytes along the swizzled row
-                        mma_ss(tmem + b * BN, smem_desc(a_src + j * 32), smem_desc(b_src + j * 32), idesc, (kb | j) ? 1u : 0u);
-                    mma_commit(bars + 8 * (STAGES + s));      // the stage is free once these have read it
-                }
-                if (ok) mma_commit(acc_full + 8 * b);         // this tile's accumulator is complete
-                i++;
+                for (int j = 1; j < G_BK / 16; j++) mma_ss_lo<true>(d, a_lo + 2 * j, b_lo + 2 * j, idesc, one);   // 16 values of k = 32 bytes along the swizzled row
+                mma_commit_one(bars + 8 * (STAGES + s), one);      // the stage is free once these have read it
+                if (++s == STAGES) { s = 0; turn ^= 1; }
             }
+            if (ok) mma_commit_one(acc_full + 8 * b, one);         // this tile's accumulator is complete
+            i++;
         }
     } else {
         // ---- epilogue: warp w owns lanes (rows) 32 w .. 32 w + 31 of the accumulators ---------------
@@ -305,25 +308,26 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_pair_kernel(const __grid_co
             }
         }
     } else if (warp == 5) {
-        if (rank == 0 && lane == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = instr_desc(2 * G_BM, BN);
-            int it = 0, i = 0;
+            const uint32_t one = elect_one() ? 1 : 0;
+            int i = 0, s = 0;
+            uint32_t turn = 0;
             bool ok = true;
             for (int t = pair; t < n_tiles && ok; t += pairs) {
                 const int b = i & 1;
-                if (i >= 2 && !mbar_wait(acc_empty + 8 * b, ((i >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+                if (i >= 2 && !__all_sync(0xffffffffu, mbar_wait(acc_empty + 8 * b, ((i >> 1) - 1) & 1, abort_flag))) { ok = false; break; }
                 tc_fence_after();
-                for (int kb = 0; kb < k_blocks; kb++, it++) {
-                    const int s = it % P_STAGES;
-                    if (!mbar_wait(bars + 8 * s, (it / P_STAGES) & 1, abort_flag)) { ok = false; break; }
+                for (int kb = 0; kb < k_blocks; kb++) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * s, turn, abort_flag))) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a_src = tiles + s * P_STAGE, b_src = a_src + G_TILE_A;
+                    const uint64_t a_desc = smem_desc(tiles + s * P_STAGE), b_desc = smem_desc(tiles + s * P_STAGE + G_TILE_A);
 #pragma unroll
-                    for (int j = 0; j < G_BK / 16; j++)
-                        mma_ss_pair(tmem + b * BN, smem_desc(a_src + j * 32), smem_desc(b_src + j * 32), idesc, (kb | j) ? 1u : 0u);
-                    mma_commit_pair(bars + 8 * (P_STAGES + s));
+                    for (int j = 0; j < G_BK / 16; j++) mma_ss_pair(tmem + b * BN, a_desc + 2 * j, b_desc + 2 * j, idesc, (kb | j) ? 1u : 0u, one);
+                    mma_commit_pair(bars + 8 * (P_STAGES + s), one);
+                    if (++s == P_STAGES) { s = 0; turn ^= 1; }
                 }
-                if (ok) mma_commit_pair(acc_full + 8 * b);
+                if (ok) mma_commit_pair(acc_full + 8 * b, one);
                 i++;
             }
         }

@@ -18,8 +18,12 @@
 // products, the activation's own pass and gemm_tcgen05.cu above): 6 layers of the 8B shape with the head, 8 / 16 / 32 / 64
 // requests: 804 / 869 / 920 / 1045 -> 713 / 753 / 856 / 983; the 0.6B shape, 24 / 32 / 64 requests: 1561 / 1586 / 1747 -> 1285 / 1314 / 1713.
 // Alone and back to back: the 8B shape's head (1.24 GB) at 8 rows 189 us (6.6 TB/s), its gate/up 35.0 (5.7), the library's
-// head 213.  Where a product of 4 MB takes its 4 us at 64 rows (clocks of a CTA from the wait's end): 850 until x is there,
-// 16 products 1700, 700 into shared memory, 900 for the cluster's meeting, 1200 to add and store, 800 to leave.
+// head 213.  Where a product of 4 MB takes its 4 us (clocks of a CTA
+// from the wait's end, 37 rows, eight CTAs a cluster): 1240 until x is there, 16 products until 2680, in shared memory at 3350, met at 4000, the
+// peers' 17 KB read by 6530 (shared memory of another SM comes at some 12 bytes a clock), stored at 6770, gone at 7200.  With the warp's one lane
+// issuing by predicate (tcgen05.cuh, mma_ss_lo) and not in a branch the 16 products take 1440 and not 1700: a prompt of 37 tokens 1102 -> 1075 us, 64
+// requests 1720 -> 1687.  Asked for by each CTA from its own memory on, in turn: 0.7 % less, but a row's order of
+// sums would follow its place in the step.  Sent to the CTA that adds them (st.async) instead of read by it: 1112 and 1730, the stores take as long as the reads.
 //
 // Ten warps: 0-7 take the accumulator out of tensor memory (a lane a row of W) and, with 8 and 9, add and store;
 // warp 8 issues the loads, warp 9 owns the tensor memory and issues the tcgen05.mma.  Every wait is bounded: a thread
@@ -138,21 +142,22 @@ __global__ void __launch_bounds__(R_THREADS, 2) rows_gemm_kernel(const __grid_co
             for (int j = i > stages ? i - stages : 0; j < i; j++) mbar_wait(full + 8 * (j % stages), (j / stages) & 1, &ignored);
         }
     } else if (warp == 9) {
-        const uint32_t idesc = instr_desc(R_BM, rows);
+        const uint32_t idesc = instr_desc(R_BM, rows), one = elect_one() ? 1 : 0;
         bool ok = true;
+        int s = 0;
+        uint32_t turn = 0;
         for (int i = 0; i < n_kb; i++) {
-            const int s = i % stages;
-            if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, (i / stages) & 1, abort_flag))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, turn, abort_flag))) { ok = false; break; }
             tc_fence_after();
-            const uint32_t w_src = ring + s * stage, x_src = w_src + 2 * R_TILE_W;
-            if (elect_one()) {
+            const uint32_t w_lo = desc_lo(ring + s * stage), x_lo = desc_lo(ring + s * stage + 2 * R_TILE_W), half = tile_x >> 4;
+            if (i == 0) mma_ss_lo<false>(tmem, w_lo, x_lo, idesc, one);
+            else mma_ss_lo<true>(tmem, w_lo, x_lo, idesc, one);
 #pragma unroll
-                for (int j = 0; j < R_SK / 16; j++) {    // 16 values of k = 32 bytes along the swizzled row
-                    const int h = j / 4, o = (j % 4) * 32;
-                    mma_ss(tmem, smem_desc(w_src + h * R_TILE_W + o), smem_desc(x_src + h * tile_x + o), idesc, (i | j) ? 1u : 0u);
-                }
-                mma_commit(i + 1 < n_kb ? empty + 8 * s : done);
-            }
+            for (int j = 1; j < R_BK / 16; j++) mma_ss_lo<true>(tmem, w_lo + 2 * j, x_lo + 2 * j, idesc, one);     // 16 values of k = 32 bytes along the swizzled row
+#pragma unroll
+            for (int j = 0; j < R_BK / 16; j++) mma_ss_lo<true>(tmem, w_lo + (R_TILE_W >> 4) + 2 * j, x_lo + half + 2 * j, idesc, one);
+            mma_commit_one(i + 1 < n_kb ? empty + 8 * s : done, one);
+            if (++s == stages) { s = 0; turn ^= 1; }
         }
         if (!ok) *abort_flag = 1;
     } else if (mbar_wait(done, 0, abort_flag)) {

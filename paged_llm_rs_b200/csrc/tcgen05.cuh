@@ -85,14 +85,19 @@ __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t desc_a, uint64_
                  ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
 // The same with descriptors given by their lower halves (desc_lo), whose upper half is a constant: 16 values of k further along are an
-// addition of 2.
+// addition of 2.  The whole warp comes here and ``one`` says which lane issues: with no branch around the instruction its operands stay
+// uniform values, where an issuing thread of its own moves each of them into a uniform register first.
 constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);       // stride 1024, version 1, 128-byte swizzle
 __device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr >> 4) & 0x3fff) | (1u << 16); }
 template <bool ACCUMULATE>
-__device__ __forceinline__ void mma_ss_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
-    asm volatile("{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.u32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
-                 ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "n"(ACCUMULATE ? 1 : 0), "n"(DESC_HI) : "memory");
+__device__ __forceinline__ void mma_ss_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t one = 1) {
+    asm volatile("{\n.reg .pred p, q;\n.reg .b64 a, b;\nsetp.ne.u32 p, %4, 0;\nsetp.ne.u32 q, %6, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
+                 ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "n"(ACCUMULATE ? 1 : 0), "n"(DESC_HI), "r"(one) : "memory");
+}
+__device__ __forceinline__ void mma_commit_one(uint32_t bar, uint32_t one) {
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %1, 0;\n@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
+                 ::"r"(bar), "r"(one) : "memory");
 }
 // The same with the A operand in tensor memory: rows are lanes, two 16-bit values of k to a 32-bit column
 // (16 values of k = 8 columns), k ascending from the low half.
@@ -126,15 +131,15 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void mma_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}\n"
-                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+__device__ __forceinline__ void mma_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t one) {
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %4, 0;\nsetp.ne.u32 q, %5, 0;\n@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(one) : "memory");
 }
 // arrives at the barrier of this address in both CTAs when the products issued before are over
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-                 ::"r"(bar), "h"((uint16_t)3) : "memory");
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint32_t one) {
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n"
+                 "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n"
+                 ::"r"(bar), "h"((uint16_t)3), "r"(one) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_bar) : "memory");
