@@ -17,7 +17,7 @@
 // (see qk_norm_rope_kv.cu), which is the layout ldmatrix wants in shared memory,
 // so the slab is copied as it lies.
 //
-// A CTA has four consumer warps and one producer warp.  Tiles of 64 keys go round
+// A CTA has four consumer warps (or two: launch_tma) and one producer warp.  Tiles of 64 (32) keys go round
 // a 3-stage ring; every consumer warp reads every tile in turn (a parity wait tells
 // two phases of a barrier apart and no more, so no warp may run a whole turn of the
 // ring ahead of another: taking tiles in turn keeps them within it).  q.k^T and p.v
@@ -34,7 +34,7 @@
 // cp.async kernel's (attention_mma.cu).
 #include "common.cuh"
 
-#define TD_BK 64
+#define TD_KEYS 16       // keys of a tile for each consumer warp
 #define TD_STAGES 3
 #define TD_CONSUMERS 4
 #define TD_QROWS 64      // query rows (token, head) a CTA may hold
@@ -144,8 +144,8 @@ __device__ __forceinline__ void norm_rope_row(const bf16* src, const float* gain
     }
 }
 
-template <int HD, bool KEYS_AS_ROWS>
-__global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_tma_kernel(
+template <int HD, bool KEYS_AS_ROWS, int CONSUMERS = TD_CONSUMERS>
+__global__ void __launch_bounds__((CONSUMERS + 1) * 32, 8 / CONSUMERS) attention_decode_tma_kernel(
     const bf16* q, const bf16* k_pool, const bf16* v_pool,   // written by the kernels before this one: no __restrict__
     const int* __restrict__ block_tables, const AttnWork* __restrict__ work, const int* __restrict__ n_work_ptr,
     bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
     const AttnWork w = work[blockIdx.y];
     if (!(kinds_mask & (w.q_count == 1 ? 1 : 2))) return;   // another kernel's item
     if (KEYS_AS_ROWS && w.q_count != 1) return;             // (this variant is for single tokens only)
-    if (w.kv_begin & (TD_BK - 1)) {
+    if (w.kv_begin & (TD_KEYS * CONSUMERS - 1)) {
         // slabs and the swizzle need the range to start on a tile boundary
         if (threadIdx.x == 0) atomicOr(status, 32);
         return;
@@ -173,20 +173,21 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
     const int rows = w.q_count * n_heads;          // <= 64: (token, head) pairs
     const bool decode = w.q_count == 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int BK = TD_KEYS * CONSUMERS, QROWS = KEYS_AS_ROWS ? 16 : TD_QROWS;      // keys a tile; rows of q
     constexpr int KSTEPS = HD / 16, DTILES = HD / 8, CH = HD / 8;
-    constexpr int TILE_BYTES = TD_BK * HD * 2;          // keys (or values) of one tile
+    constexpr int TILE_BYTES = BK * HD * 2;          // keys (or values) of one tile
     constexpr int STAGE_BYTES = 2 * TILE_BYTES;
 
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t base = smem_u32(smem);
     const uint32_t q_s = base + TD_STAGES * STAGE_BYTES;
-    const uint32_t bars = q_s + TD_QROWS * HD * 2;       // full[S], empty[S]
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + TD_STAGES * STAGE_BYTES + TD_QROWS * HD * 2 + 16 * TD_STAGES);
+    const uint32_t bars = q_s + QROWS * HD * 2;       // full[S], empty[S]
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + TD_STAGES * STAGE_BYTES + QROWS * HD * 2 + 16 * TD_STAGES);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < TD_STAGES; s++) {
             mbar_init(bars + 8 * s, 1);                      // full: the producer's arrive, plus the bytes
-            mbar_init(bars + 8 * (TD_STAGES + s), TD_CONSUMERS);   // empty: every consumer warp's release
+            mbar_init(bars + 8 * (TD_STAGES + s), CONSUMERS);   // empty: every consumer warp's release
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
@@ -194,12 +195,12 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
     }
     __syncthreads();   // the barriers are set up; the producer goes its own way from here
 
-    const int n_tiles = (w.kv_end - w.kv_begin + TD_BK - 1) / TD_BK;
-    const int slab_rows = page_size < TD_BK ? page_size : TD_BK;
-    const int slabs = TD_BK / slab_rows;          // at most 8 (pages of at least 8 tokens)
+    const int n_tiles = (w.kv_end - w.kv_begin + BK - 1) / BK;
+    const int slab_rows = page_size < BK ? page_size : BK;
+    const int slabs = BK / slab_rows;          // at most 8 (pages of at least 8 tokens)
     const uint32_t slab_bytes = (uint32_t)slab_rows * HD * 2;
 
-    if (warp == TD_CONSUMERS) {
+    if (warp == CONSUMERS) {
         // ---- producer: page slabs into the ring ---------------------------------------------
         const int* table = block_tables + (size_t)w.seg * table_width;
         // the table entries of the key range, 32 at a time, one in each lane: no tile waits for a lookup
@@ -208,11 +209,11 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
         bool waited = false;
         for (int t = 0; t < n_tiles; t++) {
             const int s = t % TD_STAGES;
-            const int kv0 = w.kv_begin + t * TD_BK;
+            const int kv0 = w.kv_begin + t * BK;
             // A decoded token's own key is the only one this step writes for its request; a
             // portion's tiles read keys that other tiles of the portion bring, so they wait first.
-            if (!waited && (!decode || kv0 + TD_BK > w.q_pos0)) { pdl_wait(); waited = true; }
-            if (((kv0 + TD_BK - 1) >> page_shift) >= win0 + 32) {
+            if (!waited && (!decode || kv0 + BK > w.q_pos0)) { pdl_wait(); waited = true; }
+            if (((kv0 + BK - 1) >> page_shift) >= win0 + 32) {
                 win0 = kv0 >> page_shift;
                 tbl = (win0 + lane < table_width) ? table[win0 + lane] : -1;
             }
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
         const int heads_total = nh + 2 * nkv;
         pdl_wait(KID_ATT_TMA);
         const bf16* tok = fq.qkv + (size_t)w.q_token0 * heads_total * HD;
-        for (int row = warp; row < 16; row += TD_CONSUMERS) {
+        for (int row = warp; row < 16; row += CONSUMERS) {
             uint32_t pk[VPL / 2];
 #pragma unroll
             for (int k = 0; k < VPL / 2; k++) pk[k] = 0;
@@ -289,8 +290,8 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
 #pragma unroll
             for (int k = 0; k < VPL / 2; k++) reinterpret_cast<uint32_t*>(dst)[k] = pk[k];
         }
-        if (owns_new && warp >= TD_CONSUMERS - 2) {
-            const bool is_k = warp == TD_CONSUMERS - 2;
+        if (owns_new && warp >= CONSUMERS - 2) {
+            const bool is_k = warp == CONSUMERS - 2;
             float f[VPL];
             norm_rope_row<HD>(tok + (size_t)(nh + (is_k ? 0 : nkv) + kh) * HD, is_k ? fq.k_gain : nullptr, is_k ? cs : nullptr,
                               is_k ? sn : nullptr, fq.eps, lane, f);
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
         }
     } else {
         pdl_wait(KID_ATT_TMA);
-        for (int idx = threadIdx.x; idx < (decode ? 16 : TD_QROWS) * CH; idx += TD_CONSUMERS * 32) {
+        for (int idx = threadIdx.x; idx < (decode ? 16 : QROWS) * CH; idx += CONSUMERS * 32) {
             const int row = idx / CH, chunk = idx % CH;
             uint4 v = make_uint4(0, 0, 0, 0);
             if (row < rows)
@@ -322,10 +323,10 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
             *reinterpret_cast<uint4*>(smem + TD_STAGES * STAGE_BYTES + toff<HD>(row, chunk)) = v;
         }
     }
-    asm volatile("bar.sync 1, %0;\n" ::"n"(TD_CONSUMERS * 32));
+    asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
 
     float* o_s = reinterpret_cast<float*>(smem);          // [4][16][HD], once the ring is no longer read
-    float* ml_s = o_s + TD_CONSUMERS * 16 * HD;           // [4][16][2]
+    float* ml_s = o_s + CONSUMERS * 16 * HD;           // [4][16][2]
     if constexpr (KEYS_AS_ROWS) {
     // ---- consumers, one query token of at most 8 heads: the KEYS are the 16 rows of the score block --------
     // and the heads its 8 columns, S^T = K q^T and O^T = V^T P^T.  A block of 16 keys costs 8 + HD / 16
@@ -352,19 +353,19 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
     for (int t = 0; t < n_tiles; t++) {
         const int s = t % TD_STAGES;
         if (!mbar_wait(bars + 8 * s, (t / TD_STAGES) & 1, abort_flag)) break;
-        const int kv0 = w.kv_begin + t * TD_BK + key_base;
+        const int kv0 = w.kv_begin + t * BK + key_base;
         const uint32_t k_s = base + s * STAGE_BYTES, v_s = k_s + TILE_BYTES;
         if (owns_new && t == n_tiles - 1) {
             // the token's own key and value over what the copy brought for that row (whatever the page held)
-            if (warp >= TD_CONSUMERS - 2) {
-                const int r = w.q_pos0 - (w.kv_begin + t * TD_BK);
-                unsigned char* dst = smem + s * STAGE_BYTES + (warp == TD_CONSUMERS - 2 ? 0 : TILE_BYTES) +
+            if (warp >= CONSUMERS - 2) {
+                const int r = w.q_pos0 - (w.kv_begin + t * BK);
+                unsigned char* dst = smem + s * STAGE_BYTES + (warp == CONSUMERS - 2 ? 0 : TILE_BYTES) +
                                      toff<HD>(r, lane * VPL / 8) + (lane * VPL % 8) * 2;
 #pragma unroll
                 for (int k = 0; k < VPL / 2; k++)
-                    reinterpret_cast<uint32_t*>(dst)[k] = warp == TD_CONSUMERS - 2 ? new_k[k] : new_v[k];
+                    reinterpret_cast<uint32_t*>(dst)[k] = warp == CONSUMERS - 2 ? new_k[k] : new_v[k];
             }
-            asm volatile("bar.sync 1, %0;\n" ::"n"(TD_CONSUMERS * 32));
+            asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
         }
         if (kv0 < hi0) {
             // the warp's 16 keys and values into registers, and the stage goes back to the producer
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
         l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 16);
     }
     pdl_launch_dependents();   // the key tiles are done: the next kernel's CTAs may take their places
-    asm volatile("bar.sync 1, %0;\n" ::"n"(TD_CONSUMERS * 32));
+    asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
     if (*abort_flag) {
         if (threadIdx.x == 0) atomicOr(status, 16);
         return;
@@ -481,24 +482,24 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
     for (int d = 0; d < DTILES; d++) { o_acc[d][0] = o_acc[d][1] = o_acc[d][2] = o_acc[d][3] = 0.f; }
     bool alive = true;
 
-    const int key_base = decode ? warp * (TD_BK / TD_CONSUMERS) : 0;
-    const int np_count = decode ? TD_BK / TD_CONSUMERS / 16 : TD_BK / 16;   // pairs of 8-key score tiles: 1 or 4
+    const int key_base = decode ? warp * (BK / CONSUMERS) : 0;
+    const int np_count = decode ? BK / CONSUMERS / 16 : BK / 16;   // pairs of 8-key score tiles: 1 or 4
     for (int t = 0; t < n_tiles && alive; t++) {
         const int s = t % TD_STAGES;
         if (!mbar_wait(bars + 8 * s, (t / TD_STAGES) & 1, abort_flag)) { alive = false; break; }
-        const int kv0 = w.kv_begin + t * TD_BK + key_base;
+        const int kv0 = w.kv_begin + t * BK + key_base;
         const uint32_t k_s = base + s * STAGE_BYTES, v_s = k_s + TILE_BYTES;
         if (owns_new && t == n_tiles - 1) {
             // the token's own key and value over what the copy brought for that row (whatever the page held)
-            if (warp >= TD_CONSUMERS - 2) {
-                const int r = w.q_pos0 - (w.kv_begin + t * TD_BK);
-                unsigned char* dst = smem + s * STAGE_BYTES + (warp == TD_CONSUMERS - 2 ? 0 : TILE_BYTES) +
+            if (warp >= CONSUMERS - 2) {
+                const int r = w.q_pos0 - (w.kv_begin + t * BK);
+                unsigned char* dst = smem + s * STAGE_BYTES + (warp == CONSUMERS - 2 ? 0 : TILE_BYTES) +
                                      toff<HD>(r, lane * VPL / 8) + (lane * VPL % 8) * 2;
 #pragma unroll
                 for (int k = 0; k < VPL / 2; k++)
-                    reinterpret_cast<uint32_t*>(dst)[k] = warp == TD_CONSUMERS - 2 ? new_k[k] : new_v[k];
+                    reinterpret_cast<uint32_t*>(dst)[k] = warp == CONSUMERS - 2 ? new_k[k] : new_v[k];
             }
-            asm volatile("bar.sync 1, %0;\n" ::"n"(TD_CONSUMERS * 32));
+            asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
         }
         if (kv0 < warp_hi) {   // some key of this warp's share is visible to one of its rows
             float s_acc[8][4];
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
     }
     pdl_launch_dependents();   // the key tiles are done: the next kernel's CTAs may take their places
     // (named barriers from here on: the producer warp has left)
-    asm volatile("bar.sync 1, %0;\n" ::"n"(TD_CONSUMERS * 32));
+    asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
     if (*abort_flag) {   // set before the warp that gave up reached the barrier: all see it alike
         if (threadIdx.x == 0) atomicOr(status, 16);
         return;
@@ -638,15 +639,15 @@ __global__ void __launch_bounds__((TD_CONSUMERS + 1) * 32, 2) attention_decode_t
     }
     }
     if (decode) {
-    asm volatile("bar.sync 1, %0;\n" ::"n"(TD_CONSUMERS * 32));
-    for (int idx = threadIdx.x; idx < rows * HD; idx += TD_CONSUMERS * 32) {
+    asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
+    for (int idx = threadIdx.x; idx < rows * HD; idx += CONSUMERS * 32) {
         const int r = idx / HD, c = idx % HD;
         float M = -CUDART_INF_F;
 #pragma unroll
-        for (int wi = 0; wi < TD_CONSUMERS; wi++) M = fmaxf(M, ml_s[(wi * 16 + r) * 2]);
+        for (int wi = 0; wi < CONSUMERS; wi++) M = fmaxf(M, ml_s[(wi * 16 + r) * 2]);
         float L = 0.f, o = 0.f;
 #pragma unroll
-        for (int wi = 0; wi < TD_CONSUMERS; wi++) {
+        for (int wi = 0; wi < CONSUMERS; wi++) {
             const float mw = ml_s[(wi * 16 + r) * 2];
             const float f = mw == -CUDART_INF_F ? 0.f : exp2f(mw - M);
             L += ml_s[(wi * 16 + r) * 2 + 1] * f;
@@ -674,30 +675,40 @@ PLLM_EXPORT int pllm_attention_decode_tma_supports(int dtype, int nh, int nkv, i
 template <int HD>
 static int launch_tma(const void* q, const void* k_pool, const void* v_pool, const int* block_tables, const int* work,
                       const int* n_work_ptr, int max_work, void* out, float* part_o, float* part_ml, int nh, int nkv,
-                      int page_size, int n_pages, int table_width, float scale, int kinds_mask,
+                      int page_size, int n_pages, int table_width, float scale, int kinds_mask, int singles,
                       FusedQK fq, int* status, cudaStream_t stream) {
     const int group = nh / nkv;
     const int heads_per_cta = group < 16 ? group : 16;
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
     int page_shift = 0;
     while ((1 << page_shift) < page_size) page_shift++;
-    const size_t smem = (size_t)TD_STAGES * 2 * TD_BK * HD * 2 + TD_QROWS * HD * 2 + 16 * TD_STAGES + 16;
+    auto smem_of = [](int consumers, int q_rows) {
+        return (size_t)TD_STAGES * 2 * TD_KEYS * consumers * HD * 2 + (size_t)q_rows * HD * 2 + 16 * TD_STAGES + 16;
+    };
     const float scale_log2 = scale * 1.4426950408889634f;
-    const dim3 block((TD_CONSUMERS + 1) * 32);
     // single tokens of groups of at most 8 heads go to the variant with the keys as rows; what else the
     // caller asked for (several query tokens) to the other, as a launch of its own
     int rest = kinds_mask;
     if (group <= 8 && (kinds_mask & 1)) {
-        cudaFuncSetAttribute(attention_decode_tma_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_chained(attention_decode_tma_kernel<HD, true>, dim3(nkv * gparts, max_work), block, smem,
+        // Two consumer warps and tiles of 32 keys, four CTAs an SM, where a step of single tokens has more CTAs than two an SM: with four warps each and
+        // two CTAs an SM the last turn of them was nearly empty (64 requests over 8 kv heads: 512 CTAs on 296 places).  0.6B shape, us a step of
+        // 64 requests at 60 / 512 / 2500 tokens 1280 / 1730 / 3882 -> 1156 / 1600 / 3590, 48 at 1000 2194 -> 1941, 40 at 300 1425 -> 1325, 33 at 700
+        // 1611 -> 1473; 6 layers of the 8B shape, 64 at 900 1095 -> 1055.  In fewer CTAs the larger ones have twice the bytes under way each.
+        const bool small = singles > 2 * sm_count();
+        auto* kernel = small ? attention_decode_tma_kernel<HD, true, 2> : attention_decode_tma_kernel<HD, true, TD_CONSUMERS>;
+        const int consumers = small ? 2 : TD_CONSUMERS;
+        const size_t smem = smem_of(consumers, 16);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch_chained(kernel, dim3(nkv * gparts, max_work), dim3((consumers + 1) * 32), smem,
                        stream, (const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool, block_tables, (const AttnWork*)work,
                        n_work_ptr, (bf16*)out, part_o, part_ml, nh, nkv, page_size, page_shift, n_pages, table_width,
                        scale_log2, heads_per_cta, 1, fq, status);
         rest &= ~1;
     }
     if (rest) {
+        const size_t smem = smem_of(TD_CONSUMERS, TD_QROWS);
         cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_chained(attention_decode_tma_kernel<HD, false>, dim3(nkv * gparts, max_work), block, smem,
+        launch_chained(attention_decode_tma_kernel<HD, false>, dim3(nkv * gparts, max_work), dim3((TD_CONSUMERS + 1) * 32), smem,
                        stream, (const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool, block_tables, (const AttnWork*)work,
                        n_work_ptr, (bf16*)out, part_o, part_ml, nh, nkv, page_size, page_shift, n_pages, table_width,
                        scale_log2, heads_per_cta, rest, fq, status);
@@ -707,15 +718,16 @@ static int launch_tma(const void* q, const void* k_pool, const void* v_pool, con
 
 static int dispatch_tma(const void* q, const void* k_pool, const void* v_pool, const int* block_tables, const int* work,
                         const int* n_work_ptr, int max_work, void* out, float* part_o, float* part_ml, int nh, int nkv,
-                        int hd, int page_size, int n_pages, int table_width, float scale, int kinds_mask,
+                        int hd, int page_size, int n_pages, int table_width, float scale, int kinds_mask, int single_tokens,
                         FusedQK fq, int* status, cudaStream_t stream) {
     if (max_work <= 0) return PLLM_OK;
     if (!pllm_attention_decode_tma_supports(PLLM_BF16, nh, nkv, hd, page_size, 0)) return PLLM_ERR_SIZE;
+    const int group = nh / nkv, singles = single_tokens * nkv * ((group + 15) / 16);
     if (hd == 128)
         return launch_tma<128>(q, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv,
-                               page_size, n_pages, table_width, scale, kinds_mask, fq, status, stream);
+                               page_size, n_pages, table_width, scale, kinds_mask, singles, fq, status, stream);
     return launch_tma<64>(q, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv,
-                          page_size, n_pages, table_width, scale, kinds_mask, fq, status, stream);
+                          page_size, n_pages, table_width, scale, kinds_mask, singles, fq, status, stream);
 }
 
 PLLM_EXPORT int pllm_attention_decode_tma(const void* q, const void* k_pool, const void* v_pool, const int* block_tables,
@@ -725,22 +737,22 @@ PLLM_EXPORT int pllm_attention_decode_tma(const void* q, const void* k_pool, con
                                           cudaStream_t stream) {
     FusedQK none = {};
     return dispatch_tma(q, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv, hd,
-                        page_size, n_pages, table_width, scale, kinds_mask, none, status, stream);
+                        page_size, n_pages, table_width, scale, kinds_mask, 0, none, status, stream);
 }
 
 // The same for a step of single decoded tokens, straight from the projection's output: the kernel
 // norms and rotates the queries and each token's new key itself and writes key and value to the
-// cache (rotation over the whole head or none; gains and tables may be null).
+// cache (rotation over the whole head or none; gains and tables may be null).  n_tokens: of the step (a captured one: the most it holds).
 PLLM_EXPORT int pllm_attention_decode_tma_fused(const void* qkv, const float* q_gain, const float* k_gain, float eps,
                                                 const float* cos_t, const float* sin_t, int max_pos, void* k_pool,
                                                 void* v_pool, const int* block_tables, const int* work,
                                                 const int* n_work_ptr, int max_work, void* out, float* part_o,
                                                 float* part_ml, int nh, int nkv, int hd, int page_size, int n_pages,
-                                                int table_width, float scale, int* status, cudaStream_t stream) {
+                                                int table_width, float scale, int n_tokens, int* status, cudaStream_t stream) {
     if (qkv == nullptr || ((uintptr_t)qkv & 15)) return PLLM_ERR_ALIGN;
     FusedQK fq = {(const bf16*)qkv, q_gain, k_gain, cos_t, sin_t, (bf16*)k_pool, (bf16*)v_pool, eps, max_pos};
     return dispatch_tma(nullptr, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv, hd,
-                        page_size, n_pages, table_width, scale, 1, fq, status, stream);
+                        page_size, n_pages, table_width, scale, 1, n_tokens, fq, status, stream);
 }
 
 PLLM_TRACE_EXPORT(attention_decode_tma)

@@ -1,0 +1,79 @@
+"""Smaller pieces where a step has too few or too many of the usual ones: gated products in tiles of 32 columns
+(csrc/gemm_tcgen05.cu) and single tokens' attention by CTAs of two consumer warps (csrc/attention_decode_tma.cu)."""
+
+import numpy as np
+import pytest
+import torch
+
+import test_kernels_gpu as K
+from paged_llm_rs_b200.kernels import attention_plan, ops
+from paged_llm_rs_b200.parts.base import AttentionWork
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# one tile, as many tiles as SMs and a few more, an odd number of blocks of k, the last rows of a tile missing
+@pytest.mark.parametrize("M,n_out,k", [(1, 64, 64), (65, 64, 72), (100, 3072, 1024), (128, 4672, 320), (128, 4736, 320), (129, 2304, 136), (255, 2368, 1096)])
+@pytest.mark.parametrize("act", ["silu", "relu", "clamped"])
+def test_gated_products_in_narrow_tiles(M, n_out, k, act):
+    g = torch.Generator(device=DEV).manual_seed(M + n_out + k)
+    x = torch.randn(M, k, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(2 * n_out, k, device=DEV, generator=g) * 0.05).bfloat16()
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    y = ops.gemm_tcgen05(x, w, glu=True, status=st, act=act, limit=2.0 if act == "clamped" else 0.0).float()
+    assert st.item() == 0
+    gate, up = ((x.float() @ h.float().T).bfloat16().float() for h in (w[:n_out], w[n_out:]))
+    if act == "silu":
+        want = gate * torch.sigmoid(gate) * up
+    elif act == "relu":
+        want = gate.clamp(min=0) * up
+    else:
+        c = gate.clamp(max=2.0)
+        want = c * torch.sigmoid(1.702 * c) * (up.clamp(-2.0, 2.0) + 1)
+    # (another order of the sums flips a rounding of gate or up now and then, which the activation scales by the other factor)
+    assert ((y - want).abs() / (1 + gate.abs() + up.abs())).max().item() < 2e-2
+
+
+@pytest.mark.parametrize("nh,nkv,hd,page", [(16, 8, 128, 16), (32, 8, 128, 64), (8, 8, 64, 8), (24, 8, 128, 32), (64, 8, 64, 16)])
+def test_steps_of_many_single_tokens(nh, nkv, hd, page):
+    B = ops.sm_count() * 2 // nkv + 5                        # more CTAs than two an SM
+    rng = np.random.default_rng(nh + page)
+    ctxs = [0, 1, 15, 16, 31, 32, 33, 63, 64, 127, 700] + [int(c) for c in rng.integers(0, 300, B - 11)]
+    width = max(c // page + 1 for c in ctxs)
+    n_pages = sum(c // page + 1 for c in ctxs) + 2
+    order = iter(rng.permutation(n_pages).tolist())
+    tables = np.full((B, width), -1, np.int32)
+    for r, c in enumerate(ctxs):
+        for b in range(c // page + 1):
+            tables[r, b] = next(order)
+    g = torch.Generator(device=DEV).manual_seed(nh)
+    kp, vp = (torch.randn(n_pages, nkv, page, hd, device=DEV, generator=g).bfloat16() for _ in range(2))
+    qkv = torch.randn(B, (nh + 2 * nkv) * hd, device=DEV, generator=g).bfloat16()
+    gain = 1 + 0.1 * torch.randn(hd, device=DEV, generator=g)
+    for target in (1, 10 ** 6):                              # whole; split
+        work, red, parts = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, target, min_split_keys=64)
+        dev = lambda a, n: torch.from_numpy(np.ascontiguousarray(a if len(a) else np.zeros((1, n), np.int32))).to(DEV)
+        w = AttentionWork(dev(work, 8), torch.tensor([len(work)], dtype=torch.int32, device=DEV), len(work), dev(red, 4),
+                          torch.tensor([len(red)], dtype=torch.int32, device=DEV), len(red), torch.zeros(max(parts, 1), nh, hd, device=DEV),
+                          torch.zeros(max(parts, 1), nh, 2, device=DEV), kinds=1)
+        k2, v2, out, st = kp.clone(), vp.clone(), torch.zeros(B, nh * hd, dtype=torch.bfloat16, device=DEV), K.status()
+        ops.decode_attention_fused(qkv, gain, gain, 1e-6, None, None, k2, v2, torch.from_numpy(tables).to(DEV), w, out, nh, nkv, hd, hd ** -0.5, st)
+        assert st.item() == 0
+
+        def rows(pool, r, n):                                # a request's rows as they lie: chunk c of the row at offset o at c ^ (o & 7)
+            t = torch.cat([pool[p] for p in tables[r, :(n - 1) // page + 1]], 1)[:, :n]
+            at = torch.arange(n, device=DEV) % page & 7
+            idx = (torch.arange(hd // 8, device=DEV)[None, :] ^ at[:, None])[None, :, :, None].expand(nkv, n, hd // 8, 8)
+            return t.view(nkv, n, hd // 8, 8).gather(2, idx).reshape(nkv, n, hd).double()
+        norm = lambda x: x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6) * gain.double()
+        for r, c in enumerate(ctxs):
+            f = qkv[r].double().view(nh + 2 * nkv, hd)
+            q, k_new, v_new = norm(f[:nh]), norm(f[nh:nh + nkv]), f[nh + nkv:]
+            k, v = rows(k2, r, c + 1), rows(v2, r, c + 1)
+            assert torch.equal(v[:, c], v_new) and (k[:, c] - k_new).abs().max().item() < 2 ** -7 * (1 + k_new.abs().max().item())
+            assert torch.equal(k[:, :c], rows(kp, r, c + 1)[:, :c])
+            s = torch.einsum("gpd,gnd->gpn", q.view(nkv, nh // nkv, hd).bfloat16().double(), k) * hd ** -0.5
+            want = torch.einsum("gpn,gnd->gpd", torch.softmax(s, -1), v).reshape(-1)
+            # weights rounded to bfloat16 (2^-9 each, of values up to 4.5) and the result once more; q's rounding may differ by an ulp
+            assert (out[r].double() - want).abs().max().item() < 5e-2
