@@ -11,8 +11,10 @@
 //
 // Pages come in with cp.async.bulk (the untiled TMA): a page's rows for one kv head
 // are contiguous in the cache ([pages, kv_heads, page_size, head_dim]), so one
-// elected thread moves a whole page slab (up to 64 rows) with one instruction and
-// an mbarrier counts the bytes.  Nobody computes addresses per 16 bytes.  The
+// thread moves a whole page slab (up to 64 rows) with one instruction and
+// an mbarrier counts the bytes; a tile's slabs go out by as many lanes in one go (issued one after the
+// other by one lane they took it some 280 clocks each, 2200 a tile of pages of 16 tokens, which bounded a CTA: 0.6B shape, us a step, 8 requests at
+// 4096 1317 -> 1240, 16 at 1500 1169 -> 1101, one at 900 721 -> 695).  Nobody computes addresses per 16 bytes.  The
 // cache stores each row's 16-byte chunks XOR-ed with the row's offset in its page
 // (see qk_norm_rope_kv.cu), which is the layout ldmatrix wants in shared memory,
 // so the slab is copied as it lies.
@@ -218,21 +220,12 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, 8 / CONSUMERS) attention
                 tbl = (win0 + lane < table_width) ? table[win0 + lane] : -1;
             }
             if (t >= TD_STAGES && !mbar_wait(bars + 8 * (TD_STAGES + s), ((t / TD_STAGES) - 1) & 1, abort_flag)) break;
-            const uint32_t k_dst = base + s * STAGE_BYTES, v_dst = k_dst + TILE_BYTES;
-            // which slabs exist: a page of the table at or before the range's last key
-            uint32_t have = 0;
-            int pg[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                pg[i] = -1;
-                if (i >= slabs) continue;
-                const int j = kv0 + i * slab_rows;
-                int page = __shfl_sync(0xffffffffu, tbl, ((j >> page_shift) - win0) & 31);
-                if (j >= w.kv_end) page = -1;
-                if (page >= n_pages) { if (lane == 0) atomicOr(status, 8); page = -1; }
-                pg[i] = page;
-                if (page >= 0) have |= 1u << i;
-            }
+            // lane i takes slab i of the keys, lane slabs + i that of the values: its page of the table, at or before the range's last key
+            const int slab = lane & (slabs - 1), j = kv0 + slab * slab_rows;
+            int page = __shfl_sync(0xffffffffu, tbl, ((j >> page_shift) - win0) & 31);
+            if (lane >= 2 * slabs || j >= w.kv_end) page = -1;
+            if (page >= n_pages) { atomicOr(status, 8); page = -1; }
+            const uint32_t have = __ballot_sync(0xffffffffu, page >= 0) & ((1u << slabs) - 1);
             // slabs with no page behind them are zeroed by hand: nothing stale or unset is multiplied
             if (have != (1u << slabs) - 1) {
                 for (int i = 0; i < slabs; i++) {
@@ -245,16 +238,12 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, 8 / CONSUMERS) attention
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // the zeros before the copies
                 __syncwarp();
             }
-            if (lane == 0) {
-                mbar_expect_tx(bars + 8 * s, 2 * slab_bytes * __popc(have));
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (i >= slabs || pg[i] < 0) continue;
-                    const int j = kv0 + i * slab_rows;
-                    const size_t src = (((size_t)pg[i] * nkv + kh) * page_size + (j & (page_size - 1))) * HD;
-                    bulk_copy(k_dst + i * slab_bytes, k_pool + src, slab_bytes, bars + 8 * s);
-                    bulk_copy(v_dst + i * slab_bytes, v_pool + src, slab_bytes, bars + 8 * s);
-                }
+            if (lane == 0) mbar_expect_tx(bars + 8 * s, 2 * slab_bytes * __popc(have));
+            __syncwarp();
+            if (page >= 0) {
+                const size_t src = (((size_t)page * nkv + kh) * page_size + (j & (page_size - 1))) * HD;
+                bulk_copy(base + s * STAGE_BYTES + (lane >= slabs ? TILE_BYTES : 0) + slab * slab_bytes, (lane >= slabs ? v_pool : k_pool) + src, slab_bytes,
+                          bars + 8 * s);
             }
         }
         return;
