@@ -19,7 +19,7 @@
 // (see qk_norm_rope_kv.cu), which is the layout ldmatrix wants in shared memory,
 // so the slab is copied as it lies.
 //
-// A CTA has four consumer warps (or two: launch_tma) and one producer warp.  Tiles of 64 (32) keys go round
+// A CTA has four consumer warps (or two, or eight: launch_tma) and one producer warp.  Tiles of 64 (32, 128) keys go round
 // a 3-stage ring; every consumer warp reads every tile in turn (a parity wait tells
 // two phases of a barrier apart and no more, so no warp may run a whole turn of the
 // ring ahead of another: taking tiles in turn keeps them within it).  q.k^T and p.v
@@ -147,7 +147,7 @@ __device__ __forceinline__ void norm_rope_row(const bf16* src, const float* gain
 }
 
 template <int HD, bool KEYS_AS_ROWS, int CONSUMERS = TD_CONSUMERS>
-__global__ void __launch_bounds__((CONSUMERS + 1) * 32, 8 / CONSUMERS) attention_decode_tma_kernel(
+__global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 / CONSUMERS) attention_decode_tma_kernel(
     const bf16* q, const bf16* k_pool, const bf16* v_pool,   // written by the kernels before this one: no __restrict__
     const int* __restrict__ block_tables, const AttnWork* __restrict__ work, const int* __restrict__ n_work_ptr,
     bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, 8 / CONSUMERS) attention
 
     const int n_tiles = (w.kv_end - w.kv_begin + BK - 1) / BK;
     const int slab_rows = page_size < BK ? page_size : BK;
-    const int slabs = BK / slab_rows;          // at most 8 (pages of at least 8 tokens)
+    const int slabs = BK / slab_rows;          // at most 16 (pages of at least 8 tokens)
     const uint32_t slab_bytes = (uint32_t)slab_rows * HD * 2;
 
     if (warp == CONSUMERS) {
@@ -664,7 +664,7 @@ PLLM_EXPORT int pllm_attention_decode_tma_supports(int dtype, int nh, int nkv, i
 template <int HD>
 static int launch_tma(const void* q, const void* k_pool, const void* v_pool, const int* block_tables, const int* work,
                       const int* n_work_ptr, int max_work, void* out, float* part_o, float* part_ml, int nh, int nkv,
-                      int page_size, int n_pages, int table_width, float scale, int kinds_mask, int singles,
+                      int page_size, int n_pages, int table_width, float scale, int kinds_mask, int singles, int whole,
                       FusedQK fq, int* status, cudaStream_t stream) {
     const int group = nh / nkv;
     const int heads_per_cta = group < 16 ? group : 16;
@@ -684,8 +684,12 @@ static int launch_tma(const void* q, const void* k_pool, const void* v_pool, con
         // 64 requests at 60 / 512 / 2500 tokens 1280 / 1730 / 3882 -> 1156 / 1600 / 3590, 48 at 1000 2194 -> 1941, 40 at 300 1425 -> 1325, 33 at 700
         // 1611 -> 1473; 6 layers of the 8B shape, 64 at 900 1095 -> 1055.  In fewer CTAs the larger ones have twice the bytes under way each.
         const bool small = singles > 2 * sm_count();
-        auto* kernel = small ? attention_decode_tma_kernel<HD, true, 2> : attention_decode_tma_kernel<HD, true, TD_CONSUMERS>;
-        const int consumers = small ? 2 : TD_CONSUMERS;
+        // Eight warps and tiles of 128 keys, one CTA an SM, where no token is split and every CTA gets an SM: half as many turns, and all that fits in
+        // shared memory is on its way before the wait for the projection (whole, four warps / eight, us a step: one request at 250 tokens 623 / 601, at 500
+        // 686 / 634, eight at 500 782 / 743).
+        const bool large = whole && singles > 0 && singles <= sm_count();
+        auto* kernel = small ? attention_decode_tma_kernel<HD, true, 2> : large ? attention_decode_tma_kernel<HD, true, 8> : attention_decode_tma_kernel<HD, true, TD_CONSUMERS>;
+        const int consumers = small ? 2 : large ? 8 : TD_CONSUMERS;
         const size_t smem = smem_of(consumers, 16);
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         launch_chained(kernel, dim3(nkv * gparts, max_work), dim3((consumers + 1) * 32), smem,
@@ -707,16 +711,16 @@ static int launch_tma(const void* q, const void* k_pool, const void* v_pool, con
 
 static int dispatch_tma(const void* q, const void* k_pool, const void* v_pool, const int* block_tables, const int* work,
                         const int* n_work_ptr, int max_work, void* out, float* part_o, float* part_ml, int nh, int nkv,
-                        int hd, int page_size, int n_pages, int table_width, float scale, int kinds_mask, int single_tokens,
+                        int hd, int page_size, int n_pages, int table_width, float scale, int kinds_mask, int single_tokens, int whole,
                         FusedQK fq, int* status, cudaStream_t stream) {
     if (max_work <= 0) return PLLM_OK;
     if (!pllm_attention_decode_tma_supports(PLLM_BF16, nh, nkv, hd, page_size, 0)) return PLLM_ERR_SIZE;
     const int group = nh / nkv, singles = single_tokens * nkv * ((group + 15) / 16);
     if (hd == 128)
         return launch_tma<128>(q, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv,
-                               page_size, n_pages, table_width, scale, kinds_mask, singles, fq, status, stream);
+                               page_size, n_pages, table_width, scale, kinds_mask, singles, whole, fq, status, stream);
     return launch_tma<64>(q, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv,
-                          page_size, n_pages, table_width, scale, kinds_mask, singles, fq, status, stream);
+                          page_size, n_pages, table_width, scale, kinds_mask, singles, whole, fq, status, stream);
 }
 
 PLLM_EXPORT int pllm_attention_decode_tma(const void* q, const void* k_pool, const void* v_pool, const int* block_tables,
@@ -726,22 +730,23 @@ PLLM_EXPORT int pllm_attention_decode_tma(const void* q, const void* k_pool, con
                                           cudaStream_t stream) {
     FusedQK none = {};
     return dispatch_tma(q, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv, hd,
-                        page_size, n_pages, table_width, scale, kinds_mask, 0, none, status, stream);
+                        page_size, n_pages, table_width, scale, kinds_mask, 0, 0, none, status, stream);
 }
 
 // The same for a step of single decoded tokens, straight from the projection's output: the kernel
 // norms and rotates the queries and each token's new key itself and writes key and value to the
-// cache (rotation over the whole head or none; gains and tables may be null).  n_tokens: of the step (a captured one: the most it holds).
+// cache (rotation over the whole head or none; gains and tables may be null).  n_tokens: of the step (a captured one: the most it holds); whole: no item is
+// part of a token's keys.
 PLLM_EXPORT int pllm_attention_decode_tma_fused(const void* qkv, const float* q_gain, const float* k_gain, float eps,
                                                 const float* cos_t, const float* sin_t, int max_pos, void* k_pool,
                                                 void* v_pool, const int* block_tables, const int* work,
                                                 const int* n_work_ptr, int max_work, void* out, float* part_o,
                                                 float* part_ml, int nh, int nkv, int hd, int page_size, int n_pages,
-                                                int table_width, float scale, int n_tokens, int* status, cudaStream_t stream) {
+                                                int table_width, float scale, int n_tokens, int whole, int* status, cudaStream_t stream) {
     if (qkv == nullptr || ((uintptr_t)qkv & 15)) return PLLM_ERR_ALIGN;
     FusedQK fq = {(const bf16*)qkv, q_gain, k_gain, cos_t, sin_t, (bf16*)k_pool, (bf16*)v_pool, eps, max_pos};
     return dispatch_tma(nullptr, k_pool, v_pool, block_tables, work, n_work_ptr, max_work, out, part_o, part_ml, nh, nkv, hd,
-                        page_size, n_pages, table_width, scale, 1, n_tokens, fq, status, stream);
+                        page_size, n_pages, table_width, scale, 1, n_tokens, whole, fq, status, stream);
 }
 
 PLLM_TRACE_EXPORT(attention_decode_tma)

@@ -19,6 +19,7 @@ struct PllmGroupPack {
     int window;                 // 0: every key stays
     int chunk;                  // > 0 (and no window): a query reads its own chunk of this many positions only
     int ctas_per_item;          // CTAs the attention kernel launches per work item
+    int whole;                  // short contexts are not cut (whole_keys)
     int max_work, max_red, max_parts;                                    // capacities of the captured step
     int plans;                  // 0: the group's mixers take no attention work items (the offsets of work and red are unused)
     int off_slots, off_tables, off_n_work, off_n_red, off_work, off_red; // offsets in int32 units
@@ -37,6 +38,8 @@ enum : int {
 static const int SPLIT_ALIGN = 64;
 static const int MAX_SPLITS = 128;
 
+// kernels/attention_plan.py: whole_keys
+static inline int whole_keys(long long ctas, long long target_ctas) { return 8 * ctas >= 3 * target_ctas ? 4096 : (int)(512 + 6 * ctas); }
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // tokens, positions, state_slots, temperature, uniform: one per request (temperature and
@@ -87,6 +90,13 @@ PLLM_EXPORT int pllm_pack_decode_step(int* out, int out_len, int n, const int* t
         if ((long long)n * g.ctas_per_item < target_ctas) {
             want = target_ctas / (n * g.ctas_per_item);
             if (want < 2) want = 2;
+            int most = 0;
+            for (int i = 0; i < n; i++) {
+                const int p0 = positions[i];
+                const int keys = g.window > 0 ? (p0 + 1 < g.window ? p0 + 1 : g.window) : (g.chunk > 0 ? p0 % g.chunk + 1 : p0 + 1);
+                if (keys > most) most = keys;
+            }
+            if (g.whole && most <= whole_keys(n * g.ctas_per_item, target_ctas)) want = 1;
         }
         int n_work = 0, n_red = 0, parts = 0;
         for (int i = 0; i < n; i++) {

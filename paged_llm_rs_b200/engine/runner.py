@@ -314,7 +314,7 @@ def group_plans(cache: CacheManager, mixer_of, page_size: int) -> List[Optional[
         if len(wishes) != 1:
             raise ConfigError(f"the mixers that share a cache group wish for different attention plans: {sorted(map(str, wishes))}")
         w = wishes.pop()
-        plans.append(None if w is None else GroupPlanConfig(w.tile_tokens, w.ctas_per_item, g.window, w.heads, w.head_dim, g.chunk, w.part_keys))
+        plans.append(None if w is None else GroupPlanConfig(w.tile_tokens, w.ctas_per_item, g.window, w.heads, w.head_dim, g.chunk, w.whole, w.part_keys))
     return plans
 
 

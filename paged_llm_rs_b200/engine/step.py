@@ -47,6 +47,7 @@ class GroupPlanConfig:
     heads: int = 1        # partial results of split items are [rows, heads, head_dim]
     head_dim: int = 1
     chunk: int = 0        # a query reads its own chunk of this many tokens only (0: no chunks)
+    whole: bool = False   # short contexts of single tokens are not cut (attention_plan.whole_keys)
     part_keys: int = 0    # keys of a part where a step of several tokens a request is cut (0: by the planner's usual rule)
 
 
@@ -144,10 +145,10 @@ class StepPacker:
                 group_parts.append((None, None, 0, 0, 0, W))
                 continue
             # groups that cut their work alike (same tile, window, chunk, CTAs an item) share one plan
-            key = (plan.tile_tokens, plan.window, plan.ctas_per_item, plan.chunk, plan.part_keys)
+            key = (plan.tile_tokens, plan.window, plan.ctas_per_item, plan.chunk, plan.part_keys, plan.whole)
             if key not in planned:
                 planned[key] = attention_plan.plan_attention(spans, plan.tile_tokens, plan.window, plan.ctas_per_item, self.target_ctas,
-                                                             chunk=plan.chunk, part_keys=plan.part_keys)
+                                                             chunk=plan.chunk, part_keys=plan.part_keys, whole=plan.whole)
             work, red, parts = planned[key]
             mw, mr, mp = (work_caps[gi] if work_caps else (len(work), len(red), parts))
             if len(work) > mw or len(red) > mr or parts > mp:
@@ -246,7 +247,8 @@ class StepPacker:
                                                                            self.target_ctas)
                 plan = AttentionWork(work=view(f"g{gi}.work").view(-1, 8), n_work=view(f"g{gi}.n_work"), max_work=gs["max_work"],
                                      red=view(f"g{gi}.red").view(-1, 4), n_red=view(f"g{gi}.n_red"), max_red=gs["max_red"],
-                                     part_o=part_o, part_ml=part_ml, kinds=sizes["kinds"], many_splits=many)
+                                     part_o=part_o, part_ml=part_ml, kinds=sizes["kinds"], many_splits=many,
+                                     reduces=full or gs["max_red"] > 0)
             groups.append(GroupStep(block_tables=view(f"g{gi}.tables").view(sizes["segments_cap"], gs["table_width"]),
                                     slots=view(f"g{gi}.slots", T), plan=plan))
         state = StepState(n_tokens=T, tokens=view("tokens", T), positions=view("positions", T), groups=groups,
@@ -261,7 +263,7 @@ class StepPacker:
 class _GroupPack(ctypes.Structure):
     """csrc/step_pack.cu: PllmGroupPack."""
     _fields_ = [("tables", ctypes.POINTER(ctypes.c_void_p)), ("table_len", ctypes.POINTER(ctypes.c_int)),
-                ("window", ctypes.c_int), ("chunk", ctypes.c_int), ("ctas_per_item", ctypes.c_int),
+                ("window", ctypes.c_int), ("chunk", ctypes.c_int), ("ctas_per_item", ctypes.c_int), ("whole", ctypes.c_int),
                 ("max_work", ctypes.c_int), ("max_red", ctypes.c_int), ("max_parts", ctypes.c_int),
                 ("plans", ctypes.c_int),
                 ("off_slots", ctypes.c_int), ("off_tables", ctypes.c_int), ("off_n_work", ctypes.c_int),
@@ -307,6 +309,7 @@ class NativeDecodePacker:
             g.plans = 0 if plan is None else 1
             if plan is not None:
                 g.window, g.chunk, g.ctas_per_item = int(plan.window or 0), int(plan.chunk), plan.ctas_per_item
+                g.whole = int(plan.whole)
                 g.max_work, g.max_red, g.max_parts = work_caps[gi]
             for name in ("slots", "tables") + (("n_work", "n_red", "work", "red") if plan is not None else ()):
                 setattr(g, f"off_{name}", layout[f"g{gi}.{name}"][0])

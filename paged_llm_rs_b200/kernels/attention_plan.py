@@ -45,18 +45,33 @@ F32_PART_KEYS = 192
 SINK_PART_KEYS = 256
 
 
+# Single tokens whole (the bulk-copy kernel, csrc/attention_decode_tma.cu, then has eight consumer warps where every CTA gets an SM) or cut and
+# their parts reduced, us a step of the 0.6B shape cut / whole:
+#   requests x 8 CTAs   1: 500 tokens 675 / 635, 620 687 / 682, 700 682 / 699    4: 620 769 / 733, 700 744 / 749, 800 750 / 764
+#   6: 800 828 / 792, 1200 864 / 864                                             8: 900 849 / 825, 1200 882 / 874, 1400 906 / 915
+#   12: 1000 912 / 897, 1500 991 / 983, 2000 1089 / 1104                         16: 300 818 / 791, 1500 1098 / 1069, 4000 1722 / 1670
+#   20: 2000 1731 / 1546, 4000 2466 / 2179                                       32: 300 1171 / 1012, 1200 1559 / 1453, 4000 2847 / 2786
+WHOLE_KEYS, WHOLE_KEYS_A_CTA, WHOLE_KEYS_MANY = 512, 6, 4096
+
+
+def whole_keys(ctas: int, target_ctas: int) -> int:
+    """The most keys of a single token that is left whole in a step of so many CTAs uncut (csrc/step_pack.cu has the same rule)."""
+    return WHOLE_KEYS_MANY if 8 * ctas >= 3 * target_ctas else WHOLE_KEYS + WHOLE_KEYS_A_CTA * ctas
+
+
 def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, window: Optional[int],
                    ctas_per_item: int, target_ctas: int,
                    min_split_keys: int = MIN_SPLIT_KEYS,
-                   multi_min_split_keys: int = MULTI_MIN_SPLIT_KEYS, chunk: int = 0, part_keys: int = 0) -> Tuple[np.ndarray, np.ndarray, int]:
+                   multi_min_split_keys: int = MULTI_MIN_SPLIT_KEYS, chunk: int = 0, part_keys: int = 0, whole: bool = False) -> Tuple[np.ndarray, np.ndarray, int]:
     """segments: (first token index, token count, position of the first token) per
     segment, in step order; ``chunk``: a query reads keys of its own chunk of that many positions only; ``part_keys``: a step with tiles of
-    several tokens is cut into parts of that many keys, or of so many more that they stay within twice the target.
+    several tokens is cut into parts of that many keys, or of so many more that they stay within twice the target; ``whole``: a step of single
+    tokens of which none has more keys than ``whole_keys`` says is not cut.
     Returns (work [n, 8], red [m, 4], partial rows used)."""
     in_parts = part_keys > 0 and any(c > 1 for _, c, _ in segments)
     if len(segments) <= SMALL_PLAN:
         small = _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk,
-                            part_keys if in_parts else 0)
+                            part_keys if in_parts else 0, whole)
         if small is not None:
             return small
     seg_ids, q0s, qns, p0s = [], [], [], []
@@ -105,7 +120,8 @@ def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, w
         if want < 2:
             want = 2 if int(qn.max()) == 1 else 1
         floor = np.where(qn > 1, max(min_split_keys, multi_min_split_keys), min_split_keys)
-        splits = np.clip(np.minimum(want, keys // floor), 1, MAX_SPLITS)
+        if not whole or int(qn.max()) > 1 or int(keys.max()) > whole_keys(n_tiles * ctas_per_item, target_ctas):
+            splits = np.clip(np.minimum(want, keys // floor), 1, MAX_SPLITS)
     if (splits == 1).all():
         work = np.stack([seg, q0, qn, p0, kv_begin, kv_end, np.full(n_tiles, -1), np.zeros(n_tiles, np.int64)], 1)
         return work.astype(np.int32), np.zeros((0, 4), np.int32), 0
@@ -137,7 +153,7 @@ def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, w
 SMALL_PLAN = 32        # segments, and tiles, of a step that is planned number by number
 
 
-def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk, part_keys=0):
+def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk, part_keys=0, whole=False):
     """``plan_attention`` for a step of few tiles of which none is split (a prompt's portion, as a rule): the same list without the
     forty array operations that cost such a step more than its work (35 to 80 us).  None when it is not one."""
     items, most = [], 0
@@ -159,7 +175,8 @@ def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_s
         want = target_ctas // (len(items) * ctas_per_item)
         if want < 2:
             want = 2 if most == 1 else 1
-        if want > 1:
+        if want > 1 and not (whole and most == 1 and max(end - begin for _, _, _, _, begin, end, _, _ in items)
+                             <= whole_keys(len(items) * ctas_per_item, target_ctas)):
             for _, _, n, _, begin, end, _, _ in items:
                 if end - begin >= 2 * (max(min_split_keys, multi_min_split_keys) if n > 1 else min_split_keys):
                     return None       # (in parts, a tile of several tokens has been looked at above)

@@ -63,7 +63,7 @@ def lib():
                                           c_float, c_int, P, P],
         }
         sig["pllm_set_pdl"] = [c_int]
-        sig["pllm_attention_decode_tma_fused"] = [P, P, P, c_float, P, P, c_int, P, P, P, P, P, c_int, P, P, P] + [c_int] * 6 + [c_float, c_int, P, P]
+        sig["pllm_attention_decode_tma_fused"] = [P, P, P, c_float, P, P, c_int, P, P, P, P, P, c_int, P, P, P] + [c_int] * 6 + [c_float, c_int, c_int, P, P]
         sig["pllm_attention_prefill_tcgen05_tile_tokens"] = [c_int, c_int]
         sig["pllm_attention_prefill_tcgen05_supports"] = [c_int] * 6
         sig["pllm_attention_prefill_tcgen05"] = [P] * 10 + [c_int] * 7 + [c_float, c_int, P, P]
@@ -518,7 +518,7 @@ def decode_attention_fused(qkv: torch.Tensor, q_gain, k_gain, eps: float, cos, s
                                              cos.shape[0] if cos is not None else 0, _ptr(k_pool), _ptr(v_pool),
                                              _ptr(block_tables), _ptr(work), _ptr(n_work), max_work, _ptr(out),
                                              _ptr(part_o), _ptr(part_ml), num_heads, num_kv_heads, head_dim, page_size,
-                                             n_pages, block_tables.shape[-1], float(scale), qkv.shape[0], _ptr(status), _stream()),
+                                             n_pages, block_tables.shape[-1], float(scale), qkv.shape[0], 0 if w.reduces else 1, _ptr(status), _stream()),
            "decode_attention_fused")
     if w.reduces:
         _check(L.pllm_attention_reduce(_code(out), _ptr(part_o), _ptr(part_ml), _ptr(red), _ptr(n_red), max_red,

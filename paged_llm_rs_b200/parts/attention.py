@@ -67,8 +67,11 @@ class GQAttention(Mixer):
 
     def plan_wish(self, page_size: int):
         tile = ops.attention_tile_tokens(self.nh, self.nkv, self.rt.dtype, self.hd, page_size, self.window or 0)
-        return PlanWish(tile, ops.attention_ctas_per_item(self.nh, self.nkv, self.rt.dtype), self.nh, self.hd,
-                        F32_PART_KEYS if self.rt.dtype == torch.float32 else 0)
+        swizzled = self.cache_need().swizzled
+        whole = swizzled and self.nh <= 8 * self.nkv and ops.decode_attention_fuses(self.rt.dtype, self.nh, self.nkv, self.hd, page_size,
+                                                                                     self.window or 0, 0, swizzled)
+        return PlanWish(tile, ops.attention_ctas_per_item(self.nh, self.nkv, self.rt.dtype), self.nh, self.hd, whole=whole,
+                        part_keys=F32_PART_KEYS if self.rt.dtype == torch.float32 else 0)
 
     def forward(self, x, step, cache, writes_cache=True):
         k_pool, v_pool, gi = cache

@@ -201,6 +201,7 @@ class PlanWish:
     ctas_per_item: int
     heads: int
     head_dim: int
+    whole: bool = False         # short contexts of single tokens are not cut (attention_plan.whole_keys)
     part_keys: int = 0          # keys of a part where tiles of several tokens are cut (0: by the planner's usual rule)
 
 

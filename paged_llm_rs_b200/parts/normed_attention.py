@@ -136,7 +136,7 @@ class NormedQKAttention(Mixer):
     def plan_wish(self, page_size: int):
         a = (self.nh, self.nkv, self.rt.dtype, self.dk, self.dv)
         return PlanWish(ops.attention_sink_tile_tokens(*a), ops.attention_sink_ctas_per_item(*a), self.nh, self.dv,
-                        SINK_PART_KEYS if ops.attention_sink_uses_tensor_cores(self.rt.dtype, self.nh, self.nkv, self.dk, self.dv) else 0)
+                        part_keys=SINK_PART_KEYS if ops.attention_sink_uses_tensor_cores(self.rt.dtype, self.nh, self.nkv, self.dk, self.dv) else 0)
 
     def forward(self, x, step, cache, writes_cache=True):
         kv_pool, gi = cache

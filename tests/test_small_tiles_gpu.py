@@ -1,5 +1,6 @@
 """Smaller pieces where a step has too few or too many of the usual ones: gated products in tiles of 32 columns
-(csrc/gemm_tcgen05.cu) and single tokens' attention by CTAs of two consumer warps (csrc/attention_decode_tma.cu)."""
+(csrc/gemm_tcgen05.cu) and single tokens' attention by CTAs of two and of eight consumer
+warps (csrc/attention_decode_tma.cu)."""
 
 import numpy as np
 import pytest
@@ -35,11 +36,13 @@ def test_gated_products_in_narrow_tiles(M, n_out, k, act):
     assert ((y - want).abs() / (1 + gate.abs() + up.abs())).max().item() < 2e-2
 
 
-@pytest.mark.parametrize("nh,nkv,hd,page", [(16, 8, 128, 16), (32, 8, 128, 64), (8, 8, 64, 8), (24, 8, 128, 32), (64, 8, 64, 16)])
-def test_steps_of_many_single_tokens(nh, nkv, hd, page):
-    B = ops.sm_count() * 2 // nkv + 5                        # more CTAs than two an SM
+@pytest.mark.parametrize("many", [True, False])
+@pytest.mark.parametrize("nh,nkv,hd,page", [(16, 8, 128, 16), (32, 8, 128, 64), (8, 8, 64, 8), (24, 8, 128, 32), (64, 8, 64, 16), (4, 2, 128, 256)])
+def test_steps_of_single_tokens(nh, nkv, hd, page, many):
+    # more CTAs than two an SM; or one for an SM at most, which take whole items by eight warps
+    B = ops.sm_count() * 2 // nkv + 5 if many else min(ops.sm_count() // nkv, 18)
     rng = np.random.default_rng(nh + page)
-    ctxs = [0, 1, 15, 16, 31, 32, 33, 63, 64, 127, 700] + [int(c) for c in rng.integers(0, 300, B - 11)]
+    ctxs = [0, 1, 15, 16, 31, 32, 33, 63, 64, 127, 700, 128, 129, 511, 383, 1400][:B] + [int(c) for c in rng.integers(0, 300, max(0, B - 16))]
     width = max(c // page + 1 for c in ctxs)
     n_pages = sum(c // page + 1 for c in ctxs) + 2
     order = iter(rng.permutation(n_pages).tolist())
@@ -51,12 +54,12 @@ def test_steps_of_many_single_tokens(nh, nkv, hd, page):
     kp, vp = (torch.randn(n_pages, nkv, page, hd, device=DEV, generator=g).bfloat16() for _ in range(2))
     qkv = torch.randn(B, (nh + 2 * nkv) * hd, device=DEV, generator=g).bfloat16()
     gain = 1 + 0.1 * torch.randn(hd, device=DEV, generator=g)
-    for target in (1, 10 ** 6):                              # whole; split
+    for target in (1, 10 ** 6) if many else (1,):            # whole; split
         work, red, parts = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, target, min_split_keys=64)
         dev = lambda a, n: torch.from_numpy(np.ascontiguousarray(a if len(a) else np.zeros((1, n), np.int32))).to(DEV)
         w = AttentionWork(dev(work, 8), torch.tensor([len(work)], dtype=torch.int32, device=DEV), len(work), dev(red, 4),
                           torch.tensor([len(red)], dtype=torch.int32, device=DEV), len(red), torch.zeros(max(parts, 1), nh, hd, device=DEV),
-                          torch.zeros(max(parts, 1), nh, 2, device=DEV), kinds=1)
+                          torch.zeros(max(parts, 1), nh, 2, device=DEV), kinds=1, reduces=many)
         k2, v2, out, st = kp.clone(), vp.clone(), torch.zeros(B, nh * hd, dtype=torch.bfloat16, device=DEV), K.status()
         ops.decode_attention_fused(qkv, gain, gain, 1e-6, None, None, k2, v2, torch.from_numpy(tables).to(DEV), w, out, nh, nkv, hd, hd ** -0.5, st)
         assert st.item() == 0
