@@ -170,44 +170,39 @@ __global__ void qk_norm_rope_kv_vec_kernel(
     v.store(dst + (c ^ xr) * N);
 }
 
-// The same for the many tokens of a prompt portion: the four warps of a CTA share one token, each
-// taking every fourth run of its heads, 32 / LPH heads at a time, so that the token's rotation
-// angles and the two gains are fetched once a warp and not once a head, four heads' loads are in
-// flight together, and an SM holds some fifty warps (with a warp a token it held fourteen, and the
-// kernel waited on its loads: 15.0 us for the 2048 tokens of the 0.6B shape).
+// The same for the many tokens of a prompt portion: the four warps of a CTA share one token, so that its rotation angles and the two gains are fetched
+// once a warp and not once a head.  What bounds it is its instructions (some hundred for 16 bytes a lane when a lane held one
+// chunk and fetched its rotation's partner by eight shuffles: 8.7 us for 2048 tokens of 16 + 2 x 8 heads of 128).  Here a lane holds chunk c of a head
+// AND its partner, chunk c + LPH / 2: the rotation needs no shuffle and the sum three for sixteen values: 6.9 us.
+// (Warps that walk through the tokens with the next one's loads under way, four CTAs an SM: 11.8.)
 template <typename T, int LPH>
 __global__ void __launch_bounds__(128) qk_norm_rope_kv_token_kernel(
     const T* qkv, T* __restrict__ q_out, const float* __restrict__ q_gain,
     const float* __restrict__ k_gain, float eps, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
     int max_pos, const int* __restrict__ positions, const int* __restrict__ slots, T* __restrict__ k_pool,
     T* __restrict__ v_pool, int n_tokens, int nh, int nkv, int page_size, int n_pages, int swizzle, int* status) {
-    constexpr int N = Vec16<T>::N, HD = LPH * N, HPW = 32 / LPH, UNR = 4;
+    constexpr int N = Vec16<T>::N, HD = LPH * N, LANES = LPH / 2, HPW = 32 / LANES, UNR = 2;
     pdl_launch_dependents();
     // (position, slot, rotation table and gains do not come from the kernel before: they are fetched before the wait for it)
-    const int lane = threadIdx.x & 31, sub = lane / LPH, c = lane % LPH;
+    const int lane = threadIdx.x & 31, sub = lane / LANES, c = lane % LANES;
     const int t = blockIdx.x, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     if (t >= n_tokens) return;
     const int heads = nh + 2 * nkv;
-    float cs[N], sn[N], gq[N], gk[N];
-    const bool upper = c >= LPH / 2;
+    float cs[N], sn[N];
     if (cos_t) {
         int pos = positions[t];
         if (pos < 0 || pos >= max_pos) { if (lane == 0) atomicOr(status, 4); pos = 0; }
         // (N values = 16 or 32 bytes from a multiple of N: vector loads)
-        const size_t o = (size_t)pos * (HD / 2) + (upper ? c - LPH / 2 : c) * N;
+        const size_t o = (size_t)pos * (HD / 2) + c * N;
 #pragma unroll
         for (int k = 0; k < N; k += 4) {
             const float4 a = *reinterpret_cast<const float4*>(cos_t + o + k), b = *reinterpret_cast<const float4*>(sin_t + o + k);
             cs[k] = a.x; cs[k + 1] = a.y; cs[k + 2] = a.z; cs[k + 3] = a.w;
-            sn[k] = upper ? b.x : -b.x; sn[k + 1] = upper ? b.y : -b.y; sn[k + 2] = upper ? b.z : -b.z; sn[k + 3] = upper ? b.w : -b.w;
+            sn[k] = b.x; sn[k + 1] = b.y; sn[k + 2] = b.z; sn[k + 3] = b.w;
         }
-    }
+    } else {
 #pragma unroll
-    for (int k = 0; k < N; k += 4) {
-        const float4 a = q_gain ? *reinterpret_cast<const float4*>(q_gain + c * N + k) : make_float4(1.f, 1.f, 1.f, 1.f);
-        const float4 b = k_gain ? *reinterpret_cast<const float4*>(k_gain + c * N + k) : make_float4(1.f, 1.f, 1.f, 1.f);
-        gq[k] = a.x; gq[k + 1] = a.y; gq[k + 2] = a.z; gq[k + 3] = a.w;
-        gk[k] = b.x; gk[k + 1] = b.y; gk[k + 2] = b.z; gk[k + 3] = b.w;
+        for (int k = 0; k < N; k++) { cs[k] = 1.f; sn[k] = 0.f; }
     }
     // where this token's keys and values go
     const int slot = slots[t];
@@ -221,11 +216,13 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kv_token_kernel(
     const T* src = qkv + (size_t)t * heads * HD + c * N;
     pdl_wait(KID_QK);
     for (int h0 = warp * HPW * UNR; h0 < heads; h0 += warps * HPW * UNR) {
-        Vec16<T> v[UNR];
+        Vec16<T> lo[UNR], hi[UNR];
 #pragma unroll
         for (int u = 0; u < UNR; u++) {
             const int h = h0 + u * HPW + sub;
-            v[u].load(src + (size_t)(h < heads ? h : heads - 1) * HD);
+            const T* from = src + (size_t)(h < heads ? h : heads - 1) * HD;
+            lo[u].load(from);
+            hi[u].load(from + HD / 2);
         }
 #pragma unroll
         for (int u = 0; u < UNR; u++) {
@@ -233,24 +230,32 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kv_token_kernel(
             if (h0 + u * HPW >= heads) break;          // the whole warp is past the last head
             const bool live = h < heads;
             const bool is_q = h < nh, is_k = !is_q && h < nh + nkv;
-            float f[N];
-            v[u].unpack(f);
+            const float* gain = is_q ? q_gain : is_k ? k_gain : nullptr;
+            float f[2][N];
+            lo[u].unpack(f[0]);
+            hi[u].unpack(f[1]);
             float ss = 0.f;
 #pragma unroll
-            for (int k = 0; k < N; k++) ss += f[k] * f[k];
+            for (int k = 0; k < N; k++) ss += f[0][k] * f[0][k] + f[1][k] * f[1][k];
 #pragma unroll
-            for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            if ((is_q && q_gain) || (is_k && k_gain)) {
+            for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (gain) {
                 const float inv = 1.0f / sqrtf(ss / (float)HD + eps);
 #pragma unroll
-                for (int k = 0; k < N; k++) f[k] = f[k] * inv * (is_q ? gq[k] : gk[k]);
+                for (int half = 0; half < 2; half++)
+#pragma unroll
+                    for (int k = 0; k < N; k += 4) {       // (the SM's own cache has the gains)
+                        const float4 g = *reinterpret_cast<const float4*>(gain + half * (HD / 2) + c * N + k);
+                        f[half][k] = f[half][k] * inv * g.x; f[half][k + 1] = f[half][k + 1] * inv * g.y;
+                        f[half][k + 2] = f[half][k + 2] * inv * g.z; f[half][k + 3] = f[half][k + 3] * inv * g.w;
+                    }
             }
-            if (cos_t) {
+            if (cos_t && (is_q || is_k)) {
 #pragma unroll
                 for (int k = 0; k < N; k++) {
-                    const float other = __shfl_xor_sync(0xffffffffu, f[k], LPH / 2);
-                    // upper half: x cos + partner sin; lower half: x cos - partner sin (the sign is in sn)
-                    if (is_q || is_k) f[k] = f[k] * cs[k] + other * sn[k];
+                    const float a = f[0][k], b = f[1][k];
+                    f[0][k] = a * cs[k] - b * sn[k];
+                    f[1][k] = b * cs[k] + a * sn[k];
                 }
             }
             if (!live) continue;
@@ -265,15 +270,18 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kv_token_kernel(
                 x = xr;
             }
             Vec16<T> o;
-            o.pack(f);
+            o.pack(f[0]);
             o.store(dst + (c ^ x) * N);
+            o.pack(f[1]);
+            o.store(dst + ((c + LANES) ^ x) * N);
         }
     }
 }
 
 // From how many tokens on a CTA takes a whole token (a setter for tuning runs).  Measured back to back in a
 // captured loop, 16 + 2 x 8 heads of 128, microseconds a CTA a token / a warp a pair of heads: 128 tokens
-// 3.6 / 3.2, 256: 4.2 / 4.5, 512: 4.4 / 5.0, 1024: 5.7 / 7.5, 2048: 9.8 / 12.1, 4096: 17.8 / 21.8.
+// 2.4 / 2.5, 256: 2.8 / 2.8, 512: 3.0 / 4.8, 1024: 3.6 / 7.7, 2048: 6.9 / 13.8, 4096: 12.3 / 26.1; 32 + 2 x 8 heads, 192: 4.0 / 2.8, 256: 3.8 / 4.0,
+// 512: 4.1 / 6.3, 2048: 9.8 / 19.8.
 static int g_qk_token_threshold = 256;
 PLLM_EXPORT int pllm_qk_set_token_threshold(int n) {
     const int was = g_qk_token_threshold;

@@ -80,3 +80,50 @@ def test_steps_of_single_tokens(nh, nkv, hd, page, many):
             want = torch.einsum("gpn,gnd->gpd", torch.softmax(s, -1), v).reshape(-1)
             # weights rounded to bfloat16 (2^-9 each, of values up to 4.5) and the result once more; q's rounding may differ by an ulp
             assert (out[r].double() - want).abs().max().item() < 5e-2
+
+
+# (a lane holds a chunk of a head and its rotation's partner: heads of 8, 16 and 32 chunks, numbers of heads that leave lanes and warps without one)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 8, 128), (5, 1, 64), (3, 3, 256), (33, 11, 128), (1, 1, 32)])
+@pytest.mark.parametrize("rope,norm", [(True, True), (False, True), (True, False)])
+def test_norm_and_rotation_of_many_tokens(dtype, nh, nkv, hd, rope, norm):
+    T, page = 300, 16
+    chunks = hd * (4 if dtype == torch.float32 else 2) // 16
+    swizzled = chunks % 8 == 0
+    g = torch.Generator(device=DEV).manual_seed(nh + hd)
+    qkv = torch.randn(T, (nh + 2 * nkv) * hd, device=DEV, generator=g).to(dtype)
+    qg, kg = (1 + 0.1 * torch.randn(hd, device=DEV, generator=g) for _ in range(2)) if norm else (None, None)
+    cos, sin = (torch.randn(400, hd // 2, device=DEV, generator=g) for _ in range(2)) if rope else (None, None)
+    pos = torch.randperm(400, device=DEV, generator=g)[:T].to(torch.int32)
+    slots = torch.randperm(20 * page, device=DEV, generator=g)[:T].to(torch.int32)
+    slots[7] = -1
+    pools = [torch.zeros(20, nkv, page, hd, device=DEV, dtype=dtype) for _ in range(2)]
+    q, st = torch.empty(T, nh * hd, device=DEV, dtype=dtype), K.status()
+    ops.qk_norm_rope_kv(qkv, q, qg, kg, 1e-6, cos, sin, hd if rope else 0, pos, slots, *pools, nh, nkv, hd, st, swizzled=swizzled)
+    assert st.item() == 0
+    x = qkv.double().view(T, nh + 2 * nkv, hd)
+
+    def made(y, gain):
+        if gain is not None:
+            y = y * torch.rsqrt((y * y).mean(-1, keepdim=True) + 1e-6) * gain.double()
+        if rope:
+            c, s = cos.double()[pos.long()][:, None], sin.double()[pos.long()][:, None]
+            a, b = y[..., :hd // 2], y[..., hd // 2:]
+            y = torch.cat([a * c - b * s, b * c + a * s], -1)
+        return y
+    want_q, want_k, want_v = made(x[:, :nh], qg), made(x[:, nh:nh + nkv], kg), x[:, nh + nkv:]
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21          # one rounding, and some of float's before it
+    near = lambda a, b: ((a.double() - b).abs() <= eps * (1 + b.abs().amax(-1, keepdim=True))).all()
+    assert near(q.view(T, nh, hd), want_q)
+    for pool, want in zip(pools, (want_k, want_v)):
+        rows = pool.transpose(1, 2).reshape(20 * page, nkv, hd)
+        got = rows[slots.long().clamp(min=0)]
+        if swizzled:
+            at = slots.clamp(min=0) % page & 7
+            idx = (torch.arange(chunks, device=DEV)[None, :] ^ at[:, None])[:, None, :, None].expand(T, nkv, chunks, hd // chunks)
+            got = got.view(T, nkv, chunks, -1).gather(2, idx.long()).reshape(T, nkv, hd)
+        keep = slots >= 0
+        assert near(got[keep], want[keep])
+        untouched = torch.ones(20 * page, dtype=torch.bool, device=DEV)
+        untouched[slots[keep].long()] = False
+        assert not rows[untouched].any()
