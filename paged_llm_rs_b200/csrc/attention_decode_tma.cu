@@ -118,30 +118,59 @@ struct FusedQK {
     int max_pos;
 };
 
-// One head's row, hd / 32 values a lane (lane l: dims l * VPL ..): the norm over the row, then the
-// rotation of dim d with d +- hd / 2 (16 lanes away), in float; the arithmetic of qk_norm_rope_kv.cu.
+// What a head's row is made with, hd / 32 values a lane (lane l: dims l * VPL ..): the gain and the token's rotation, by vector loads where
+// they lie on such boundaries.
 template <int HD>
-__device__ __forceinline__ void norm_rope_row(const bf16* src, const float* gain, const float* cs, const float* sn, float eps,
-                                              int lane, float (&f)[HD / 32]) {
-    constexpr int VPL = HD / 32;
+struct RowConsts {
+    static constexpr int VPL = HD / 32;      // 2 or 4
+    float g[VPL], c[VPL], s[VPL];
+    __device__ __forceinline__ static void load(const float* p, float (&f)[VPL]) {
+        if ((uintptr_t)p & (4 * VPL - 1)) {
 #pragma unroll
-    for (int k = 0; k < VPL; k++) f[k] = __bfloat162float(src[lane * VPL + k]);
-    if (gain) {
+            for (int k = 0; k < VPL; k++) f[k] = p[k];
+        } else if constexpr (VPL == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(p);
+            f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+        } else {
+            const float2 v = *reinterpret_cast<const float2*>(p);
+            f[0] = v.x; f[1] = v.y;
+        }
+    }
+    __device__ __forceinline__ void gain(const float* gain, int lane) { if (gain) load(gain + lane * VPL, g); }
+    __device__ __forceinline__ void rotation(const float* cs, const float* sn, int lane) {
+        if (cs) { load(cs + (lane & 15) * VPL, c); load(sn + (lane & 15) * VPL, s); }
+    }
+};
+template <int HD>
+__device__ __forceinline__ void row_values(const bf16* src, int lane, float (&f)[HD / 32]) {
+    if constexpr (HD == 128) {
+        const uint2 v = *reinterpret_cast<const uint2*>(src + lane * 4);
+        f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+        f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+    } else {
+        const uint32_t v = *reinterpret_cast<const uint32_t*>(src + lane * 2);
+        f[0] = __uint_as_float(v << 16); f[1] = __uint_as_float(v & 0xffff0000u);
+    }
+}
+// A head's row: the norm over it, then the rotation of dim d with d +- hd / 2 (16 lanes away), in float; the arithmetic of qk_norm_rope_kv.cu.
+template <int HD>
+__device__ __forceinline__ void norm_rope_row(const RowConsts<HD>& with, bool norm, bool rotate, float eps, int lane, float (&f)[HD / 32]) {
+    constexpr int VPL = HD / 32;
+    if (norm) {
         float ss = 0.f;
 #pragma unroll
         for (int k = 0; k < VPL; k++) ss += f[k] * f[k];
         ss = warp_sum(ss);
         const float inv = 1.0f / sqrtf(ss / (float)HD + eps);
 #pragma unroll
-        for (int k = 0; k < VPL; k++) f[k] = f[k] * inv * gain[lane * VPL + k];
+        for (int k = 0; k < VPL; k++) f[k] = f[k] * inv * with.g[k];
     }
-    if (cs) {
+    if (rotate) {
         const bool upper = lane >= 16;
 #pragma unroll
         for (int k = 0; k < VPL; k++) {
             const float other = __shfl_xor_sync(0xffffffffu, f[k], 16);
-            const int i = (lane & 15) * VPL + k;
-            f[k] = upper ? f[k] * cs[i] + other * sn[i] : f[k] * cs[i] - other * sn[i];
+            f[k] = upper ? f[k] * with.c[k] + other * with.s[k] : f[k] * with.c[k] - other * with.s[k];
         }
     }
 }
@@ -262,6 +291,15 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
         const float* cs = fq.cos_t ? fq.cos_t + (size_t)pos * (HD / 2) : nullptr;
         const float* sn = fq.sin_t ? fq.sin_t + (size_t)pos * (HD / 2) : nullptr;
         const int heads_total = nh + 2 * nkv;
+        // (gains, rotation and the page of the token's own row are there before the projection is: fetched ahead of the wait.  0.6B shape, us a step, one
+        // request at 300 tokens 609 -> 599, 64 at 512 1580 -> 1548)
+        RowConsts<HD> rc;
+        rc.gain(fq.q_gain, lane);
+        rc.rotation(cs, sn, lane);
+        const bool is_k = warp == CONSUMERS - 2, makes_row = owns_new && warp >= CONSUMERS - 2;
+        RowConsts<HD> rk = rc;
+        if (makes_row && is_k) rk.gain(fq.k_gain, lane);
+        const int page = makes_row ? block_tables[(size_t)w.seg * table_width + (w.q_pos0 >> page_shift)] : 0;
         pdl_wait(KID_ATT_TMA);
         const bf16* tok = fq.qkv + (size_t)w.q_token0 * heads_total * HD;
         for (int row = warp; row < 16; row += CONSUMERS) {
@@ -270,7 +308,8 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
             for (int k = 0; k < VPL / 2; k++) pk[k] = 0;
             if (row < n_heads) {
                 float f[VPL];
-                norm_rope_row<HD>(tok + (size_t)(head0 + row) * HD, fq.q_gain, cs, sn, fq.eps, lane, f);
+                row_values<HD>(tok + (size_t)(head0 + row) * HD, lane, f);
+                norm_rope_row<HD>(rc, fq.q_gain != nullptr, cs != nullptr, fq.eps, lane, f);
 #pragma unroll
                 for (int k = 0; k < VPL / 2; k++) pk[k] = pack2(f[2 * k], f[2 * k + 1]);
             }
@@ -279,16 +318,14 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
 #pragma unroll
             for (int k = 0; k < VPL / 2; k++) reinterpret_cast<uint32_t*>(dst)[k] = pk[k];
         }
-        if (owns_new && warp >= CONSUMERS - 2) {
-            const bool is_k = warp == CONSUMERS - 2;
+        if (makes_row) {
             float f[VPL];
-            norm_rope_row<HD>(tok + (size_t)(nh + (is_k ? 0 : nkv) + kh) * HD, is_k ? fq.k_gain : nullptr, is_k ? cs : nullptr,
-                              is_k ? sn : nullptr, fq.eps, lane, f);
+            row_values<HD>(tok + (size_t)(nh + (is_k ? 0 : nkv) + kh) * HD, lane, f);
+            norm_rope_row<HD>(rk, is_k && fq.k_gain, is_k && cs, fq.eps, lane, f);
             uint32_t pk[VPL / 2];
 #pragma unroll
             for (int k = 0; k < VPL / 2; k++) pk[k] = pack2(f[2 * k], f[2 * k + 1]);
             // into the cache, chunk c at c ^ (offset in page & 7), for the steps to come
-            const int page = block_tables[(size_t)w.seg * table_width + (w.q_pos0 >> page_shift)];
             const int off = w.q_pos0 & (page_size - 1);
             if (page >= 0 && page < n_pages) {
                 bf16* row_w = (is_k ? fq.k_pool : fq.v_pool) + (((size_t)page * nkv + kh) * page_size + off) * HD;

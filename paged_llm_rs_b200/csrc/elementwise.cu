@@ -398,8 +398,8 @@ __global__ void swiglu_bias_kernel(const T* in, const float* __restrict__ bias, 
     }
 }
 
-// Sixteen bytes a thread of each half (the rows in blockIdx.y: no division): 1024 rows of 3072 took 15.4 us an entry at a time
-// (caches cold); 11.2 this way.
+// Sixteen bytes a thread of each half (the rows in blockIdx.y: no division): 1024 rows of 3072 take 5.3 us, 512 3.6, 128 2.4; 8.7, 5.9 and 3.3 with the
+// biases fetched one by one, which were then most of the kernel's loads.
 template <typename T>
 __global__ void __launch_bounds__(128) swiglu_bias_vec_kernel(const T* in, const float* __restrict__ bias, T* __restrict__ out, int inter, int n_rows,
                                                               int rows_a_cta, int act, float limit) {
@@ -409,7 +409,11 @@ __global__ void __launch_bounds__(128) swiglu_bias_vec_kernel(const T* in, const
     if (c >= inter) return;
     float bg[N], bu[N];
 #pragma unroll
-    for (int k = 0; k < N; k++) { bg[k] = bias[c + k]; bu[k] = bias[inter + c + k]; }
+    for (int k = 0; k < N; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(bias + c + k), b = *reinterpret_cast<const float4*>(bias + inter + c + k);
+        bg[k] = a.x; bg[k + 1] = a.y; bg[k + 2] = a.z; bg[k + 3] = a.w;
+        bu[k] = b.x; bu[k + 1] = b.y; bu[k + 2] = b.z; bu[k + 3] = b.w;
+    }
     pdl_wait(KID_SWIGLU);
     const int r1 = min(n_rows, ((int)blockIdx.y + 1) * rows_a_cta);
 #pragma unroll 4
@@ -432,7 +436,7 @@ PLLM_EXPORT int pllm_swiglu_bias(int dtype, const void* in, const float* bias, v
     if (act < GLU_SILU || act > GLU_CLAMPED || inter <= 0 || bias == nullptr) return PLLM_ERR_SIZE;
     PLLM_DISPATCH_DTYPE(dtype, {
         // (bfloat16 from some hundred thousand entries on: 64 rows of 1024 take 1.9 us this way and 1.7 an entry at a time, 64 of 2048 1.9 and 2.3)
-        if (inter % Vec16<T>::N == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0 && (sizeof(T) == 4 || (long long)n_rows * inter >= 1 << 17)) {
+        if (inter % Vec16<T>::N == 0 && (((uintptr_t)in | (uintptr_t)out | (uintptr_t)bias) & 15) == 0 && (sizeof(T) == 4 || (long long)n_rows * inter >= 1 << 17)) {
             // (up to eight rows a CTA where that still makes sixteen CTAs an SM)
             const int across = (inter / Vec16<T>::N + 127) / 128;
             int rows = 1;

@@ -123,11 +123,18 @@ __global__ void qk_norm_rope_kv_vec_kernel(
         if (pos < 0 || pos >= max_pos) { if (c == 0 && live) atomicOr(status, 4); pos = 0; }
         const size_t o = (size_t)pos * HALF + (upper ? c - LPH / 2 : c) * N;
 #pragma unroll
-        for (int k = 0; k < N; k++) { cs[k] = cos_t[o + k]; sn[k] = sin_t[o + k]; }
+        for (int k = 0; k < N; k += 4) {          // (N values = 16 or 32 bytes from a multiple of N: vector loads)
+            const float4 a = *reinterpret_cast<const float4*>(cos_t + o + k), b = *reinterpret_cast<const float4*>(sin_t + o + k);
+            cs[k] = a.x; cs[k + 1] = a.y; cs[k + 2] = a.z; cs[k + 3] = a.w;
+            sn[k] = b.x; sn[k + 1] = b.y; sn[k + 2] = b.z; sn[k + 3] = b.w;
+        }
     }
     if (gain) {
 #pragma unroll
-        for (int k = 0; k < N; k++) gn[k] = gain[c * N + k];
+        for (int k = 0; k < N; k += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(gain + c * N + k);
+            gn[k] = a.x; gn[k + 1] = a.y; gn[k + 2] = a.z; gn[k + 3] = a.w;
+        }
     }
     const int slot = (live && !is_q && k_pool) ? slots[t] : -1;
     pdl_wait(KID_QK);
@@ -321,7 +328,8 @@ PLLM_EXPORT int pllm_qk_norm_rope_kv(int dtype, const void* qkv, void* q_out, co
     // sixteen bytes a lane where the head is 8, 16 or 32 chunks wide and rotated over its whole width
     const int chunks = hd * (dtype == PLLM_F32 ? 4 : 2) / 16;
     if ((dtype == PLLM_F32 || dtype == PLLM_BF16) && (chunks == 8 || chunks == 16 || chunks == 32) &&
-        hd * (dtype == PLLM_F32 ? 4 : 2) % 16 == 0 && (!cos_t || rotary_dim == hd)) {
+        hd * (dtype == PLLM_F32 ? 4 : 2) % 16 == 0 && (!cos_t || rotary_dim == hd) &&
+        (((uintptr_t)q_gain | (uintptr_t)k_gain | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0) {
 #define PLLM_QK_VEC(T, LPH)                                                                                        \
     launch_qk_vec<T, LPH>(qkv, q_out, q_gain, k_gain, eps, cos_t, sin_t, max_pos, positions, slots, k_pool, v_pool, \
                           n_tokens, nh, nkv, page_size, n_pages, swizzle, status, stream)

@@ -127,3 +127,34 @@ def test_norm_and_rotation_of_many_tokens(dtype, nh, nkv, hd, rope, norm):
         untouched = torch.ones(20 * page, dtype=torch.bool, device=DEV)
         untouched[slots[keep].long()] = False
         assert not rows[untouched].any()
+
+
+def test_gains_and_tables_off_sixteen_bytes():
+    # (the vector loads ask for such boundaries: elsewhere the values are fetched one by one)
+    nh, nkv, hd, page, T = 8, 4, 128, 16, 300
+    g = torch.Generator(device=DEV).manual_seed(3)
+    off = lambda t: torch.cat([torch.zeros(1, device=DEV), t.reshape(-1)])[1:].view(t.shape)
+    qkv = torch.randn(T, (nh + 2 * nkv) * hd, device=DEV, generator=g).bfloat16()
+    qg, kg, cos, sin = (torch.randn(*s, device=DEV, generator=g) for s in ((hd,), (hd,), (T, hd // 2), (T, hd // 2)))
+    pos = torch.arange(T, device=DEV, dtype=torch.int32)
+    got = []
+    for f in (lambda t: t, off):
+        for n in (40, T):
+            pools = [torch.zeros(T // page + 1, nkv, page, hd, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+            q, st = torch.empty(n, nh * hd, device=DEV, dtype=torch.bfloat16), K.status()
+            ops.qk_norm_rope_kv(qkv[:n], q, f(qg), f(kg), 1e-6, f(cos), f(sin), hd, pos[:n], pos[:n], *pools, nh, nkv, hd, st, swizzled=True)
+            got.append((q, *pools))
+        work, red, parts = attention_plan.plan_attention([(r, 1, 0) for r in range(9)], 1, None, nkv, 1)
+        w = AttentionWork(torch.from_numpy(work).to(DEV), torch.tensor([9], dtype=torch.int32, device=DEV), 9, torch.zeros(1, 4, dtype=torch.int32, device=DEV),
+                          torch.zeros(1, dtype=torch.int32, device=DEV), 0, torch.zeros(1, nh, hd, device=DEV), torch.zeros(1, nh, 2, device=DEV), kinds=1)
+        pools = [torch.zeros(9, nkv, page, hd, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+        out, st = torch.zeros(9, nh * hd, dtype=torch.bfloat16, device=DEV), K.status()
+        ops.decode_attention_fused(qkv[:9], f(qg), f(kg), 1e-6, f(cos), f(sin), *pools, torch.arange(9, dtype=torch.int32, device=DEV).view(9, 1), w, out,
+                                   nh, nkv, hd, hd ** -0.5, st)
+        got.append((out, *pools))
+        gu = torch.randn(200, 2048, device=DEV, generator=torch.Generator(device=DEV).manual_seed(9)).bfloat16()
+        got.append((ops.swiglu_bias(gu, f(qg.repeat(16)), torch.empty(200, 1024, dtype=torch.bfloat16, device=DEV)),))
+    for a, b in zip(got[:4], got[4:]):
+        for x, y in zip(a, b):
+            # another order of a row's sum flips a rounding now and then: an ulp of bfloat16
+            torch.testing.assert_close(x.float(), y.float(), atol=1e-2, rtol=2 ** -7)
