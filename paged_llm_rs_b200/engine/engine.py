@@ -175,7 +175,7 @@ class Engine:
             self.bytes_d2h = 0
             return []
         if back is not None:     # a captured step copies them to pinned memory itself
-            torch.cuda.current_stream().synchronize()
+            ops.current_stream().synchronize()
         else:
             back = tokens_dev.cpu()
         self.bytes_d2h = back.numel() * 4

@@ -237,7 +237,7 @@ class _DecodeGraph:
 
     def _replay(self):
         self.replay()
-        self._replayed.record()
+        self._replayed.record(ops.current_stream())
         self._pending = True
 
     def run(self, entries, temperature, uniform):
@@ -262,7 +262,7 @@ class _DecodeGraph:
                 self._copied[i].synchronize()               # the copy that last read this buffer (long done, as a rule)
             self._pinned[i].numpy()[:] = host
             self.dev.copy_(self._pinned[i], non_blocking=True)
-            self._copied[i].record()
+            self._copied[i].record(ops.current_stream())
             self._copy_pending[i] = True
             self.replay()
         r.bytes_h2d = self.nbytes

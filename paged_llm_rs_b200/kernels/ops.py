@@ -183,8 +183,13 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+def current_stream() -> "torch.cuda.Stream":
+    """torch's current stream, asked for by the device's number: without one the call looks its device up in Python, 4 us against 1."""
+    return torch.cuda.current_stream(torch.cuda.current_device())
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return current_stream().cuda_stream
 
 
 def _i32(t: Optional[torch.Tensor], name: str):
@@ -427,7 +432,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
             # the single tokens' long key ranges no longer queue behind tiles of 128 rows with two of them live.
             global MIXED_BESIDE_CALLS
             MIXED_BESIDE_CALLS += 1
-            main, side = torch.cuda.current_stream(), _side_stream(q.device)
+            main, side = current_stream(), _side_stream(q.device)
             side.wait_stream(main)
             with torch.cuda.stream(side):
                 _check(L.pllm_attention_decode_tma(_ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(block_tables), _ptr(work),
@@ -443,7 +448,7 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                                                     _ptr(status), _stream()),
                    "paged_attention (tcgen05)")
             if beside:
-                torch.cuda.current_stream().wait_stream(_side_stream(q.device))
+                current_stream().wait_stream(_side_stream(q.device))
             # (else) beside portions it takes the single decoded tokens too: one launch a layer, not two
             kinds = 0 if kinds == 3 else kinds & ~2
         take = (kinds & TMA_KINDS) if tma_ok else 0
