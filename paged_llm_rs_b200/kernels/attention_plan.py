@@ -38,11 +38,6 @@ MULTI_MIN_SPLIT_KEYS = 2048
 # 4534 / 4208 / 4207 / 4153 / 4354; 2 beside 60 behind 600 5116 / 2989 / 3051 / 3106 / 3379; 250 alone 3914 / 3709 / 3635 / 3811 / 3909;
 # 4 at 1500 beside 40 2732 / 2791 / 2787 / 2513 / 2619).
 F32_PART_KEYS = 192
-# The mma.sync kernel of attention with joined rows (csrc/attention_sink.cu) needs some 5 us for 64 keys of its tile of 64 rows, whatever runs beside
-# it, and a prompt's last tile has all of them (Pamarax, 4 layers, us a step whole / in parts of 192 / 256 / 384 / 448 / 640 keys: 1016 tokens beside 8
-# 863 / 834 / 835 / 834 / 834 / 838; 1024 alone 826 / 799 / 799 / 776 / 779 / 792; 100 behind 600 beside 4 493 / 442 / 449 / 465 / 448 / 482; 60 behind 500
-# beside 2 419 / 389 / 391 / 398 / 400 / 420; 400 alone 587 / 582 / 583 / 595 / 588 / 587).
-SINK_PART_KEYS = 256
 
 
 # Single tokens whole (the bulk-copy kernel, csrc/attention_decode_tma.cu, then has eight consumer warps where every CTA gets an SM) or cut and

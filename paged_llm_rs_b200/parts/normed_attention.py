@@ -34,7 +34,6 @@ import torch
 
 from ..errors import KernelError
 from ..kernels import ops
-from ..kernels.attention_plan import SINK_PART_KEYS
 from .base import JoinedKVNeed, Mixer, PlanWish, register_mixer, stack_rows
 from .position import rotary_frequencies
 from .spec import TensorSpec
@@ -135,8 +134,7 @@ class NormedQKAttention(Mixer):
 
     def plan_wish(self, page_size: int):
         a = (self.nh, self.nkv, self.rt.dtype, self.dk, self.dv)
-        return PlanWish(ops.attention_sink_tile_tokens(*a), ops.attention_sink_ctas_per_item(*a), self.nh, self.dv,
-                        part_keys=SINK_PART_KEYS if ops.attention_sink_uses_tensor_cores(self.rt.dtype, self.nh, self.nkv, self.dk, self.dv) else 0)
+        return PlanWish(ops.attention_sink_tile_tokens(*a), ops.attention_sink_ctas_per_item(*a), self.nh, self.dv)
 
     def forward(self, x, step, cache, writes_cache=True):
         kv_pool, gi = cache
