@@ -175,7 +175,7 @@ __device__ __forceinline__ void norm_rope_row(const RowConsts<HD>& with, bool no
     }
 }
 
-template <int HD, bool KEYS_AS_ROWS, int CONSUMERS = TD_CONSUMERS>
+template <int HD, bool KEYS_AS_ROWS, int CONSUMERS = TD_CONSUMERS, int STAGES = TD_STAGES>
 __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 / CONSUMERS) attention_decode_tma_kernel(
     const bf16* q, const bf16* k_pool, const bf16* v_pool,   // written by the kernels before this one: no __restrict__
     const int* __restrict__ block_tables, const AttnWork* __restrict__ work, const int* __restrict__ n_work_ptr,
@@ -211,14 +211,14 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
 
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t base = smem_u32(smem);
-    const uint32_t q_s = base + TD_STAGES * STAGE_BYTES;
+    const uint32_t q_s = base + STAGES * STAGE_BYTES;
     const uint32_t bars = q_s + QROWS * HD * 2;       // full[S], empty[S]
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + TD_STAGES * STAGE_BYTES + QROWS * HD * 2 + 16 * TD_STAGES);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + STAGES * STAGE_BYTES + QROWS * HD * 2 + 16 * STAGES);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < TD_STAGES; s++) {
+        for (int s = 0; s < STAGES; s++) {
             mbar_init(bars + 8 * s, 1);                      // full: the producer's arrive, plus the bytes
-            mbar_init(bars + 8 * (TD_STAGES + s), CONSUMERS);   // empty: every consumer warp's release
+            mbar_init(bars + 8 * (STAGES + s), CONSUMERS);   // empty: every consumer warp's release
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
         int tbl = (win0 + lane < table_width) ? table[win0 + lane] : -1;
         bool waited = false;
         for (int t = 0; t < n_tiles; t++) {
-            const int s = t % TD_STAGES;
+            const int s = t % STAGES;
             const int kv0 = w.kv_begin + t * BK;
             // A decoded token's own key is the only one this step writes for its request; a
             // portion's tiles read keys that other tiles of the portion bring, so they wait first.
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
                 win0 = kv0 >> page_shift;
                 tbl = (win0 + lane < table_width) ? table[win0 + lane] : -1;
             }
-            if (t >= TD_STAGES && !mbar_wait(bars + 8 * (TD_STAGES + s), ((t / TD_STAGES) - 1) & 1, abort_flag)) break;
+            if (t >= STAGES && !mbar_wait(bars + 8 * (STAGES + s), ((t / STAGES) - 1) & 1, abort_flag)) break;
             // lane i takes slab i of the keys, lane slabs + i that of the values: its page of the table, at or before the range's last key
             const int slab = lane & (slabs - 1), j = kv0 + slab * slab_rows;
             int page = __shfl_sync(0xffffffffu, tbl, ((j >> page_shift) - win0) & 31);
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
                 for (int k = 0; k < VPL / 2; k++) pk[k] = pack2(f[2 * k], f[2 * k + 1]);
             }
             // lane l's values are dims l * VPL ..: chunk (l * VPL) / 8 of the row, (l * VPL) % 8 values in
-            unsigned char* dst = smem + TD_STAGES * STAGE_BYTES + toff<HD>(row, lane * VPL / 8) + (lane * VPL % 8) * 2;
+            unsigned char* dst = smem + STAGES * STAGE_BYTES + toff<HD>(row, lane * VPL / 8) + (lane * VPL % 8) * 2;
 #pragma unroll
             for (int k = 0; k < VPL / 2; k++) reinterpret_cast<uint32_t*>(dst)[k] = pk[k];
         }
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
             uint4 v = make_uint4(0, 0, 0, 0);
             if (row < rows)
                 v = *reinterpret_cast<const uint4*>(q + ((size_t)(w.q_token0 + row / n_heads) * nh + head0 + row % n_heads) * HD + chunk * 8);
-            *reinterpret_cast<uint4*>(smem + TD_STAGES * STAGE_BYTES + toff<HD>(row, chunk)) = v;
+            *reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + toff<HD>(row, chunk)) = v;
         }
     }
     asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
@@ -377,8 +377,8 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
     const int key_base = warp * 16;
     const int mat = lane >> 3;
     for (int t = 0; t < n_tiles; t++) {
-        const int s = t % TD_STAGES;
-        if (!mbar_wait(bars + 8 * s, (t / TD_STAGES) & 1, abort_flag)) break;
+        const int s = t % STAGES;
+        if (!mbar_wait(bars + 8 * s, (t / STAGES) & 1, abort_flag)) break;
         const int kv0 = w.kv_begin + t * BK + key_base;
         const uint32_t k_s = base + s * STAGE_BYTES, v_s = k_s + TILE_BYTES;
         if (owns_new && t == n_tiles - 1) {
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
 #pragma unroll
             for (int d = 0; d < MT; d++) ldsm4_t(vf[d], v_s + toff<HD>(vkey, d * 2 + (mat & 1)));
             __syncwarp();
-            if (lane == 0) mbar_arrive(bars + 8 * (TD_STAGES + s));
+            if (lane == 0) mbar_arrive(bars + 8 * (STAGES + s));
             // two chains of mma over the k-steps, added at the end
             float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
             for (int d = 0; d < MT; d++) mma(o_acc[d], vf[d], pb0, pb1);
         } else {
             __syncwarp();
-            if (lane == 0) mbar_arrive(bars + 8 * (TD_STAGES + s));
+            if (lane == 0) mbar_arrive(bars + 8 * (STAGES + s));
         }
     }
 #pragma unroll
@@ -511,8 +511,8 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
     const int key_base = decode ? warp * (BK / CONSUMERS) : 0;
     const int np_count = decode ? BK / CONSUMERS / 16 : BK / 16;   // pairs of 8-key score tiles: 1 or 4
     for (int t = 0; t < n_tiles && alive; t++) {
-        const int s = t % TD_STAGES;
-        if (!mbar_wait(bars + 8 * s, (t / TD_STAGES) & 1, abort_flag)) { alive = false; break; }
+        const int s = t % STAGES;
+        if (!mbar_wait(bars + 8 * s, (t / STAGES) & 1, abort_flag)) { alive = false; break; }
         const int kv0 = w.kv_begin + t * BK + key_base;
         const uint32_t k_s = base + s * STAGE_BYTES, v_s = k_s + TILE_BYTES;
         if (owns_new && t == n_tiles - 1) {
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
             }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(bars + 8 * (TD_STAGES + s));   // this warp is done with the stage
+        if (lane == 0) mbar_arrive(bars + 8 * (STAGES + s));   // this warp is done with the stage
     }
 #pragma unroll
     for (int i = 0; i < 2; i++) {
@@ -708,8 +708,8 @@ static int launch_tma(const void* q, const void* k_pool, const void* v_pool, con
     const int gparts = (group + heads_per_cta - 1) / heads_per_cta;
     int page_shift = 0;
     while ((1 << page_shift) < page_size) page_shift++;
-    auto smem_of = [](int consumers, int q_rows) {
-        return (size_t)TD_STAGES * 2 * TD_KEYS * consumers * HD * 2 + (size_t)q_rows * HD * 2 + 16 * TD_STAGES + 16;
+    auto smem_of = [](int consumers, int stages, int q_rows) {
+        return (size_t)stages * 2 * TD_KEYS * consumers * HD * 2 + (size_t)q_rows * HD * 2 + 16 * stages + 16;
     };
     const float scale_log2 = scale * 1.4426950408889634f;
     // single tokens of groups of at most 8 heads go to the variant with the keys as rows; what else the
@@ -721,13 +721,15 @@ static int launch_tma(const void* q, const void* k_pool, const void* v_pool, con
         // 64 requests at 60 / 512 / 2500 tokens 1280 / 1730 / 3882 -> 1156 / 1600 / 3590, 48 at 1000 2194 -> 1941, 40 at 300 1425 -> 1325, 33 at 700
         // 1611 -> 1473; 6 layers of the 8B shape, 64 at 900 1095 -> 1055.  In fewer CTAs the larger ones have twice the bytes under way each.
         const bool small = singles > 2 * sm_count();
-        // Eight warps and tiles of 128 keys, one CTA an SM, where no token is split and every CTA gets an SM: half as many turns, and all that fits in
-        // shared memory is on its way before the wait for the projection (whole, four warps / eight, us a step: one request at 250 tokens 623 / 601, at 500
-        // 686 / 634, eight at 500 782 / 743).
-        const bool large = whole && singles > 0 && singles <= sm_count();
-        auto* kernel = small ? attention_decode_tma_kernel<HD, true, 2> : large ? attention_decode_tma_kernel<HD, true, 8> : attention_decode_tma_kernel<HD, true, TD_CONSUMERS>;
-        const int consumers = small ? 2 : large ? 8 : TD_CONSUMERS;
-        const size_t smem = smem_of(consumers, 16);
+        // Eight warps and tiles of 128 keys where no token is split and every CTA gets an SM: half as many turns, and what fits in
+        // shared memory is on its way before the wait for the projection.  A ring of two stages leaves the projection's CTAs room on the same SM, so that
+        // these can be there before it is over; three where a CTA meets one on few SMs (us a step, three / two stages / four warps: 12 requests at 141
+        // tokens 836 / 723 / 737, 16 at 500 862 / 797, eight at 100 677 / 653 / 671 and at 500 743 / 734 / 782, one at 300 609 / 630).
+        const bool large = whole && singles > 0 && singles <= sm_count(), deep = large && 8 * singles <= sm_count();
+        auto* kernel = small ? attention_decode_tma_kernel<HD, true, 2> : deep ? attention_decode_tma_kernel<HD, true, 8, 3>
+                     : large ? attention_decode_tma_kernel<HD, true, 8, 2> : attention_decode_tma_kernel<HD, true, TD_CONSUMERS>;
+        const int consumers = small ? 2 : large ? 8 : TD_CONSUMERS, stages = large && !deep ? 2 : TD_STAGES;
+        const size_t smem = smem_of(consumers, stages, 16);
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         launch_chained(kernel, dim3(nkv * gparts, max_work), dim3((consumers + 1) * 32), smem,
                        stream, (const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool, block_tables, (const AttnWork*)work,
@@ -736,7 +738,7 @@ static int launch_tma(const void* q, const void* k_pool, const void* v_pool, con
         rest &= ~1;
     }
     if (rest) {
-        const size_t smem = smem_of(TD_CONSUMERS, TD_QROWS);
+        const size_t smem = smem_of(TD_CONSUMERS, TD_STAGES, TD_QROWS);
         cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         launch_chained(attention_decode_tma_kernel<HD, false>, dim3(nkv * gparts, max_work), dim3((TD_CONSUMERS + 1) * 32), smem,
                        stream, (const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool, block_tables, (const AttnWork*)work,
