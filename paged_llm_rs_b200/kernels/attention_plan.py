@@ -40,7 +40,7 @@ MULTI_MIN_SPLIT_KEYS = 2048
 F32_PART_KEYS = 192
 
 
-# Single tokens whole (the bulk-copy kernel, csrc/attention_decode_tma.cu, then has eight consumer warps where every CTA gets an SM) or cut and
+# Single tokens whole (the bulk-copy kernel, csrc/attention_decode_tma.cu, then has eight consumer warps where every CTA gets an SM, here with a ring of three stages) or cut and
 # their parts reduced, us a step of the 0.6B shape cut / whole:
 #   requests x 8 CTAs   1: 500 tokens 675 / 635, 620 687 / 682, 700 682 / 699    4: 620 769 / 733, 700 744 / 749, 800 750 / 764
 #   6: 800 828 / 792, 1200 864 / 864                                             8: 900 849 / 825, 1200 882 / 874, 1400 906 / 915
