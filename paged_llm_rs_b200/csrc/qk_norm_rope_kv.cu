@@ -157,7 +157,8 @@ __global__ void qk_norm_rope_kv_vec_kernel(
 #pragma unroll
         for (int k = 0; k < N; k++) {
             const float other = __shfl_xor_sync(0xffffffffu, f[k], LPH / 2);
-            if (is_q || is_k) f[k] = upper ? f[k] * cs[k] + other * sn[k] : f[k] * cs[k] - other * sn[k];
+            // (which of the two products is rounded is said here and in the kernel below, or the compiler might choose one in each)
+            if (is_q || is_k) f[k] = fmaf(f[k], cs[k], upper ? __fmul_rn(other, sn[k]) : -__fmul_rn(other, sn[k]));
         }
     }
     if (!live) return;
@@ -241,9 +242,12 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kv_token_kernel(
             float f[2][N];
             lo[u].unpack(f[0]);
             hi[u].unpack(f[1]);
-            float ss = 0.f;
+            // The squares in the order of the kernel above, a sum a chunk and the two added, and the rotation with its roundings: a token's key and queries
+            // do not depend on how many others a step brings (another order moved the logits of 28 layers by a hundredth)
+            float ss = 0.f, ss_hi = 0.f;
 #pragma unroll
-            for (int k = 0; k < N; k++) ss += f[0][k] * f[0][k] + f[1][k] * f[1][k];
+            for (int k = 0; k < N; k++) { ss += f[0][k] * f[0][k]; ss_hi += f[1][k] * f[1][k]; }
+            ss += ss_hi;
 #pragma unroll
             for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
             if (gain) {
@@ -261,8 +265,8 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kv_token_kernel(
 #pragma unroll
                 for (int k = 0; k < N; k++) {
                     const float a = f[0][k], b = f[1][k];
-                    f[0][k] = a * cs[k] - b * sn[k];
-                    f[1][k] = b * cs[k] + a * sn[k];
+                    f[0][k] = fmaf(a, cs[k], -__fmul_rn(b, sn[k]));
+                    f[1][k] = fmaf(b, cs[k], __fmul_rn(a, sn[k]));
                 }
             }
             if (!live) continue;

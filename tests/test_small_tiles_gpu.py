@@ -158,3 +158,27 @@ def test_gains_and_tables_off_sixteen_bytes():
         for x, y in zip(a, b):
             # another order of a row's sum flips a rounding now and then: an ulp of bfloat16
             torch.testing.assert_close(x.float(), y.float(), atol=1e-2, rtol=2 ** -7)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 8, 128), (5, 1, 64), (33, 11, 128), (1, 1, 32), (6, 2, 256)])
+def test_many_tokens_get_the_same_bits_as_few(dtype, nh, nkv, hd):
+    # a CTA a token (from 256 tokens on) and some lanes a head (below): the same sums in the same order, so that a token's key does not
+    # depend on how many others its step brings
+    T, page = 300, 16
+    g = torch.Generator(device=DEV).manual_seed(nh * hd)
+    qkv = (torch.randn(T, (nh + 2 * nkv) * hd, device=DEV, generator=g) * 3).to(dtype)
+    qg, kg = (1 + 0.1 * torch.randn(hd, device=DEV, generator=g) for _ in range(2))
+    angle = torch.rand(T, hd // 2, device=DEV, generator=g) * 6.3
+    pos = torch.arange(T, device=DEV, dtype=torch.int32)
+
+    def made(rows):
+        pools = [torch.zeros(T // page + 1, nkv, page, hd, device=DEV, dtype=dtype) for _ in range(2)]
+        q, st = torch.empty(T, nh * hd, device=DEV, dtype=dtype), K.status()
+        for a in range(0, T, rows):
+            b = slice(a, min(T, a + rows))
+            ops.qk_norm_rope_kv(qkv[b], q[b], qg, kg, 1e-6, angle.cos(), angle.sin(), hd, pos[b], pos[b], *pools, nh, nkv, hd, st)
+        assert st.item() == 0
+        return (q, *pools)
+    for many, few in zip(made(T), made(100)):
+        assert torch.equal(many, few)
