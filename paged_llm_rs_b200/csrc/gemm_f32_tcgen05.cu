@@ -358,34 +358,39 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
     tc_fence_before();
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     else __syncthreads();
-    {
-        // ---- this CTA's share of the tile: four columns of a row of y a thread and turn, all splits' values asked for at once ----
-        constexpr int UNITS = S_BM / 4;
-        bool odd_tile = false;
-        for (int p = 0; p < splits; p++) odd_tile |= s_ld_cluster_int(s_cluster_addr(smem_u32(&odd_w), p)) != 0;
-        const int live = (M - m0 < ROWS ? M - m0 : ROWS) * UNITS;
-        for (int u = rank * S_THREADS + threadIdx.x; u < live; u += splits * S_THREADS) {
-            const int m = m0 + u / UNITS, n = n0 + (u % UNITS) * 4;
-            if (n >= N) continue;                      // (nothing is read that is not added and stored)
-            float4 v[MAX_SPLITS];
+    // ---- this CTA's share of the tile: four columns of a row of y a thread and turn, all splits' values asked for at once ----
+    constexpr int UNITS = S_BM / 4;
+    // (a thread asks for a CTA's flag, and all wait for what these got: a read whose value nobody uses could be under way when that CTA leaves)
+    const bool odd_tile = __syncthreads_or(threadIdx.x < splits && s_ld_cluster_int(s_cluster_addr(smem_u32(&odd_w), threadIdx.x)) != 0);
+    const int live = (M - m0 < ROWS ? M - m0 : ROWS) * UNITS;
+    bool again = odd_tile;
+    for (int u = rank * S_THREADS + threadIdx.x; u < live; u += splits * S_THREADS) {
+        const int m = m0 + u / UNITS, n = n0 + (u % UNITS) * 4;
+        if (n >= N) continue;                          // (nothing is read that is not added and stored)
+        float4 v[MAX_SPLITS];
 #pragma unroll
-            for (int p = 0; p < MAX_SPLITS; p++)
-                if (p < splits) v[p] = s_ld_cluster16(s_cluster_addr(wparts + u * 16, p));
-            float4 s = v[0];
+        for (int p = 0; p < MAX_SPLITS; p++)
+            if (p < splits) v[p] = s_ld_cluster16(s_cluster_addr(wparts + u * 16, p));
+        float4 s = v[0];
 #pragma unroll
-            for (int p = 1; p < MAX_SPLITS; p++)
-                if (p < splits) { s.x += v[p].x; s.y += v[p].y; s.z += v[p].z; s.w += v[p].w; }
-            float* dst = y + (size_t)m * N + n;
-            *reinterpret_cast<float4*>(dst) = s;
-            if (odd_tile || odd_row[m])
-#pragma unroll 1
-                for (int e = 0; e < 4; e++) dst[e] = plain_dot(x + (size_t)m * K, w + (size_t)(n + e) * K, K);
-        }
+        for (int p = 1; p < MAX_SPLITS; p++)
+            if (p < splits) { s.x += v[p].x; s.y += v[p].y; s.z += v[p].z; s.w += v[p].w; }
+        *reinterpret_cast<float4*>(y + (size_t)m * N + n) = s;
+        again |= odd_row[m] != 0;
     }
     __syncwarp();
-    // A CTA's shared memory stays until its peers have read it.  Every value that a thread read from a peer went into a store to y above or into
-    // a branch, and the fence keeps those ahead of the arrival (rows_gemm_tcgen05.cu says more)
-    if (splits > 1) asm volatile("fence.acq_rel.cta;\nbarrier.cluster.arrive.relaxed.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    // A CTA's shared memory stays until its peers have read it.  Every sum that a thread read from a peer went into a store to y above, every flag
+    // into the barrier that told the threads of them, and the fence keeps those ahead of the arrival (rows_gemm_tcgen05.cu says more)
+    if (splits > 1) asm volatile("fence.acq_rel.cta;\nbarrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+    if (again)                                         // (behind the arrival: of what cannot be summed in parts the peers need nothing)
+        for (int u = rank * S_THREADS + threadIdx.x; u < live; u += splits * S_THREADS) {
+            const int m = m0 + u / UNITS, n = n0 + (u % UNITS) * 4;
+            if (n < N && (odd_tile || odd_row[m]))
+#pragma unroll 1
+                for (int e = 0; e < 4; e++) y[(size_t)m * N + n + e] = plain_dot(x + (size_t)m * K, w + (size_t)(n + e) * K, K);
+        }
+    __syncwarp();
+    if (splits > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     else __syncthreads();
     if (warp == 13) {
         tc_fence_after();

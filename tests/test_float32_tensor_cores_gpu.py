@@ -66,3 +66,19 @@ def test_the_route_and_what_it_leaves():
     for a, b in ((x[:32], w), (x, w[:512]), (x[:, :1020].contiguous(), w[:, :1020].contiguous()), (x, w[:2047]), (odd, w), (x[:, ::2], w[:, ::2])):
         assert not ops.gemm_f32_tcgen05_takes(a, b)
         torch.testing.assert_close(ops.linear(a, b), (a.double() @ b.double().T).float(), atol=1e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("at", [0, 700, 1031])
+@pytest.mark.parametrize("M,tile,splits", [(1, 32, 8), (33, 64, 8), (33, 64, 5), (200, 256, 8)])
+def test_every_cta_of_a_cluster_learns_of_a_value_that_cannot_be_split(M, tile, splits, at):
+    # (33 rows in eight CTAs: the last five have no entries of the tile to add, and leave as the others do)
+    g = torch.Generator(device=DEV).manual_seed(M + at)
+    x, w = torch.randn(M, 1032, device=DEV, generator=g), torch.randn(264, 1032, device=DEV, generator=g)
+    w[77, at], w[262, at] = float("inf"), 3.4028e38
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for _ in range(20):
+        got = ops.gemm_f32_tcgen05(x, w, status=st, tile=tile, splits=splits)
+    want = x.double() @ w.double().T
+    assert st.item() == 0 and torch.equal(torch.isinf(got), torch.isinf(want.float())) and not got.isnan().any()
+    live = torch.isfinite(want.float())
+    assert ((got.double() - want).abs() <= _bound(x, w))[live].all()
