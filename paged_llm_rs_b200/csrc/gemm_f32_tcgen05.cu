@@ -9,9 +9,13 @@
 //   Sums: the tensor cores add in float but cut off where a rounding would be, so a long sum there drifts towards zero.  A block of 64
 // values of k therefore starts from zero, takes the small parts' products first and x1 w1 last (four instructions), and is then
 // taken out of tensor memory and added in registers with rounding.
-//   Not finite, or so large that a part would be infinite: the rows of x (a flag each) and the tiles of W that hold such a value
-// are computed again by fused multiply-adds, entry by entry, as float arithmetic has them; so are rows of x without a value of 2^-100
-// or more, whose third parts would lose bits.
+//   Not finite, or so large that a part would be infinite: the entries of such a row of x or of W (a flag each) are computed again by fused
+// multiply-adds, as float arithmetic has them; so are those of a row with no value of 2^-100 or more, whose third parts
+// would lose bits (what is below 2^-110 has some below bfloat16's least, 2^-133), and those whose sum is not finite: a first part is rounded up, and 1.9999 2^100
+// by 2^27 is in float's range where the product of the first parts is not.  (A row of W of nothing but bfloat16's subnormal numbers is its own first part and stays: up to
+// six bits fewer of its products are kept, as the tensor cores line them up by their leading zeros.)  Of W the splitting warps say which rows have values that three parts do not
+// hold, and those are looked at once more, whole, behind the product (looked at by the splitting warps, which bound a product of few rows, 4096 x 12288 at 33 rows took
+// 77 us and not 63).
 //
 // What bounds it: for many rows the bytes of x's parts on their way from L2 (6 a value and tile of W, against 8 instructions of
 // tensor-core time), for few rows W's bytes and their splitting.  Hence tiles of 128 rows of W (the tensor cores' 128-row operand) by up to 256 rows
@@ -39,7 +43,7 @@ constexpr int S_TILE_W = S_BM * S_BK * 4;            // 32 KB: a block of W as i
 constexpr int S_THREADS = 512;
 constexpr int S_MAX_RING = 8, S_MAX_W = 3;
 constexpr float S_LARGEST = 3.3895313e38f;           // the largest bfloat16: beyond it a part would be infinite
-constexpr float S_SMALLEST = 7.8886091e-31f;         // 2^-100: the third part of what is below 2^-110 has lost bits (below 2^-133)
+constexpr float S_SMALLEST = 7.8886091e-31f;         // 2^-100: what a third part loses (below 2^-133) of the values beside one of this size is nothing to a float
 
 __device__ __forceinline__ uint32_t s_cluster_addr(uint32_t addr, uint32_t rank) {
     uint32_t r;
@@ -107,13 +111,28 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* x, bf16* _
     if (threadIdx.x == 0) odd_row[row] = any_odd || (any && !any_large);
 }
 
-// The entry as float arithmetic has it, for values that cannot be split.
-__device__ __forceinline__ float plain_dot(const float* x, const float* w, int K) {
+// The entry as float arithmetic has it, for values that cannot be split: by a warp (K is a multiple of eight).
+__device__ __forceinline__ float plain_dot(const float* x, const float* w, int K, int lane) {
     float s = 0.f;
 #pragma unroll 1
-    for (int k = 0; k < K; k++) s = fmaf(x[k], w[k], s);
-    return s;
+    for (int k = lane * 4; k < K; k += 128) {
+        const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+        s = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+    }
+    return warp_sum(s);
 }
+// Whether three parts of a row are not the row: it has a value that no part can hold, or none beside which a lost bit is nothing.
+__device__ __forceinline__ bool row_is_odd(const float* row, int K, int lane) {
+    bool odd = false, large = false;
+#pragma unroll 1
+    for (int k = lane * 4; k < K; k += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(row + k);
+        odd |= too_large(v.x) | too_large(v.y) | too_large(v.z) | too_large(v.w);
+        large |= fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))) >= S_SMALLEST;
+    }
+    return __any_sync(0xffffffffu, odd) || !__any_sync(0xffffffffu, large);
+}
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= CUDART_MAX_NORMAL_F; }
 
 }  // namespace
 
@@ -132,7 +151,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
     const uint32_t wparts = smem_u32(smem), wring = wparts + S_W, ring = wring + WRING * S_TILE_W;
     __shared__ __align__(8) unsigned long long bar_mem[2 * S_MAX_RING + 2 * S_MAX_W + 8];
     __shared__ uint32_t tmem_slot;
-    __shared__ int abort_mem, odd_w;
+    __shared__ int abort_mem;
+    __shared__ uint32_t odd_w[S_BM / 32], odd_all[S_BM / 32];      // the rows of W that three parts do not hold, a bit each: here, and in any share of k
     __shared__ volatile int need[2][4];                // which parts of a block of W hold anything (a warp's rows each): bit 1 the second, bit 2 the third
     volatile int* abort_flag = &abort_mem;
     const uint32_t xfull = smem_u32(bar_mem), xempty = xfull + 8 * S_MAX_RING, wfull = xempty + 8 * S_MAX_RING, wempty = wfull + 16,
@@ -159,7 +179,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
             mbar_init(accempty + 8 * b, 8);
         }
         abort_mem = 0;
-        odd_w = 0;
+        for (int c = 0; c < S_BM / 32; c++) odd_w[c] = odd_all[c] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
         fence_async_smem();
     }
@@ -183,6 +203,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
             const uint32_t lane_row = (cw * 32 + (lane & 7)) * 128;
             const uint32_t from = lane_row + (((lane >> 3) * 2 ^ (lane & 7)) << 4);               // (the chunk behind it: ^ 16)
             const uint32_t to0 = lane_row + (((lane >> 3) ^ (lane & 7)) << 4), to1 = to0 ^ 64;    // (values 0 to 31 of the block, and 32 to 63)
+            uint32_t lost = 0;                         // turns of which three parts leave something
             uint32_t filled = 0xfu;                    // turns (eight rows each) whose second and third part are not known to be zero
             for (int i = 0; i < n_kb; i++) {
                 const int b = i & 1, ss = i % WRING;
@@ -217,13 +238,11 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
                     if (any || (filled >> g & 1)) {
                         if (!alone && i >= 1) ok = __all_sync(0xffffffffu, mbar_wait(wempty + 8 * (b ^ 1), ((i - 1) >> 1) & 1, abort_flag));
                         alone = true;
-#pragma unroll
-                        for (int e = 0; e < 4; e++)    // (a value that is not finite, or too large for a part, leaves one that is not finite)
-                            if (too_large(a[e].x) || too_large(a[e].y) || too_large(a[e].z) || too_large(a[e].w)) odd_w = 1;
                         if (left) has |= 2;
                         store(wparts + 2 * S_PART_W);
                         if (left) has |= 4;
                         store(wparts + 3 * S_PART_W);
+                        if (left) lost |= 1u << g;     // (so does what is not finite, and what is too large for a part)
                         filled = any ? filled | 1u << g : filled & ~(1u << g);
                     }
                 }
@@ -237,6 +256,11 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
                 }
                 if (!ok) break;
             }
+            uint32_t rows = 0;
+#pragma unroll
+            for (int g = 0; g < 4; g++) rows |= (lost >> g & 1) << (g * 8 + (lane & 7));
+            rows = __reduce_or_sync(0xffffffffu, rows);
+            if (lane == 0) odd_w[cw] = rows;
         } else if (warp == 12) {
             // ---- x's parts, the smallest first ---------------------------------------------------------------------
             pdl_wait(KID_GEMM_TC, lane == 0);
@@ -360,10 +384,13 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
     else __syncthreads();
     // ---- this CTA's share of the tile: four columns of a row of y a thread and turn, all splits' values asked for at once ----
     constexpr int UNITS = S_BM / 4;
-    // (a thread asks for a CTA's flag, and all wait for what these got: a read whose value nobody uses could be under way when that CTA leaves)
-    const bool odd_tile = __syncthreads_or(threadIdx.x < splits && s_ld_cluster_int(s_cluster_addr(smem_u32(&odd_w), threadIdx.x)) != 0);
+    // (a thread asks for 32 rows' flags, and all wait for what these got: a read whose value nobody uses could be under way when that CTA leaves)
+    uint32_t flags = 0;
+    if (threadIdx.x < splits * (S_BM / 32)) flags = s_ld_cluster_int(s_cluster_addr(smem_u32(odd_w + threadIdx.x % (S_BM / 32)), threadIdx.x / (S_BM / 32)));
+    if (flags) atomicOr(odd_all + threadIdx.x % (S_BM / 32), flags);
+    const bool flagged = __syncthreads_or(flags != 0);
+    bool again = flagged;
     const int live = (M - m0 < ROWS ? M - m0 : ROWS) * UNITS;
-    bool again = odd_tile;
     for (int u = rank * S_THREADS + threadIdx.x; u < live; u += splits * S_THREADS) {
         const int m = m0 + u / UNITS, n = n0 + (u % UNITS) * 4;
         if (n >= N) continue;                          // (nothing is read that is not added and stored)
@@ -376,18 +403,35 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_f32_tcgen05_kernel(const __
         for (int p = 1; p < MAX_SPLITS; p++)
             if (p < splits) { s.x += v[p].x; s.y += v[p].y; s.z += v[p].z; s.w += v[p].w; }
         *reinterpret_cast<float4*>(y + (size_t)m * N + n) = s;
-        again |= odd_row[m] != 0;
+        again |= odd_row[m] != 0 || !(finite(s.x) && finite(s.y) && finite(s.z) && finite(s.w));
     }
     __syncwarp();
     // A CTA's shared memory stays until its peers have read it.  Every sum that a thread read from a peer went into a store to y above, every flag
     // into the barrier that told the threads of them, and the fence keeps those ahead of the arrival (rows_gemm_tcgen05.cu says more)
     if (splits > 1) asm volatile("fence.acq_rel.cta;\nbarrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
-    if (again)                                         // (behind the arrival: of what cannot be summed in parts the peers need nothing)
-        for (int u = rank * S_THREADS + threadIdx.x; u < live; u += splits * S_THREADS) {
-            const int m = m0 + u / UNITS, n = n0 + (u % UNITS) * 4;
-            if (n < N && (odd_tile || odd_row[m]))
+    // Behind the arrival (the peers need nothing more): the entries that cannot be summed in parts.  A warp's units are a row of x each turn.
+    if (flagged) {
+        for (int r = warp; r < S_BM; r += S_THREADS / 32)
+            if ((odd_all[r / 32] >> (r % 32) & 1) && !row_is_odd(w + (size_t)(n0 + r) * K, K, lane) && lane == 0) atomicAnd(odd_all + r / 32, ~(1u << (r % 32)));
+        __syncthreads();
+    }
+    if (__any_sync(0xffffffffu, again))
 #pragma unroll 1
-                for (int e = 0; e < 4; e++) y[(size_t)m * N + n + e] = plain_dot(x + (size_t)m * K, w + (size_t)(n + e) * K, K);
+        for (int u = rank * S_THREADS + threadIdx.x; u < live; u += splits * S_THREADS) {
+            const int m = m0 + u / UNITS, n = n0 + lane * 4;
+            uint32_t which = 0;
+            if (n < N) {
+                const float4 s = *reinterpret_cast<const float4*>(y + (size_t)m * N + n);
+                which = odd_row[m] ? 0xfu : (odd_all[lane / 8] >> (lane % 8 * 4) & 0xfu) | !finite(s.x) | !finite(s.y) << 1 | !finite(s.z) << 2 | !finite(s.w) << 3;
+            }
+#pragma unroll 1
+            for (int e = 0; e < 4; e++)
+#pragma unroll 1
+                for (uint32_t todo = __ballot_sync(0xffffffffu, which >> e & 1); todo; todo &= todo - 1) {
+                    const int owner = __ffs(todo) - 1, at = n0 + owner * 4 + e;
+                    const float v = plain_dot(x + (size_t)m * K, w + (size_t)at * K, K, lane);
+                    if (lane == owner) y[(size_t)m * N + at] = v;
+                }
         }
     __syncwarp();
     if (splits > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");

@@ -82,3 +82,48 @@ def test_every_cta_of_a_cluster_learns_of_a_value_that_cannot_be_split(M, tile, 
     assert st.item() == 0 and torch.equal(torch.isinf(got), torch.isinf(want.float())) and not got.isnan().any()
     live = torch.isfinite(want.float())
     assert ((got.double() - want).abs() <= _bound(x, w))[live].all()
+
+
+@pytest.mark.parametrize("K,splits", [(192, 1), (1032, 1), (192, 2), (1032, 8)])
+@pytest.mark.parametrize("M,tile", [(1, 32), (40, 64), (130, 256)])
+def test_small_weights(M, tile, K, splits):
+    # what is below 2^-110 keeps fewer than 24 bits in three parts: rows of W that hold nothing larger, wholly or in some CTA's share of k
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    x, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(264, K, device=DEV, generator=g)
+    small = [5, 31, 32, 127, 128, 200, 263]
+    w[small] *= torch.tensor([1e-36, 1e-35, 1e-34, 1e-36, 1e-37, 1e-33, 1e-36], device=DEV)[:, None]
+    w[40, :K // 2] *= 1e-37
+    w[41, K - 70:] *= 1e-37
+    w[42] = (w[42] * 1e-36).bfloat16().float()
+    got, want = ops.gemm_f32_tcgen05(x, w, tile=tile, splits=splits).double(), x.double() @ w.double().T
+    norm = (x.double().norm(dim=1)[:, None] * w.double().norm(dim=1)).clamp(min=1e-300)
+    # (as _bound, of the row's own size: K products of it at most)
+    assert ((got - want).abs() / norm).max().item() < 2.0 ** -20
+
+
+@pytest.mark.parametrize("splits", [1, 2])
+def test_sums_that_leave_the_range_on_their_way(splits):
+    # a first part is rounded up and may take a product out of float's range that is in it; what the further parts bring then has the other sign
+    g = torch.Generator(device=DEV).manual_seed(8)
+    x, w = torch.randn(40, 192, device=DEV, generator=g) * 0.1, torch.randn(264, 192, device=DEV, generator=g)
+    x[:, 7], w[:, 7], x[:, 150], w[:, 150] = 0.0, 0.0, 0.0, 0.0
+    x[4, 7], w[9, 7], w[130, 7] = 1.9999 * 2.0 ** 100, 2.0 ** 27, -2.0 ** 120
+    x[39, 150], w[263, 150] = -1.9999 * 2.0 ** 90, 2.0 ** 37
+    got, want = ops.gemm_f32_tcgen05(x, w, splits=splits), (x.double() @ w.double().T).float()
+    assert want[4, 9].isfinite() and want[4, 130] == -float("inf") and want[39, 263].isfinite()
+    assert torch.equal(torch.isinf(got), torch.isinf(want)) and not got.isnan().any()
+    live = torch.isfinite(want)
+    assert ((got.double() - want.double()).abs() <= _bound(x, w))[live].all()
+
+
+def test_few_tiny_weights_beside_others():
+    # A weight that decays: tiny in every row beside weights of the usual size, where what its third part loses is nothing.  Rows of bfloat16's
+    # least numbers are their own first part; a product of such a number is cut off by where its leading zeros stand, six bits earlier
+    g = torch.Generator(device=DEV).manual_seed(11)
+    x, w = torch.randn(70, 512, device=DEV, generator=g), torch.randn(140, 512, device=DEV, generator=g) * 0.02
+    w[:, 100] *= 1e-37
+    w[50] = 3 * 2.0 ** -133
+    x[:, 7] *= 2.0 ** 60
+    got, want, bound = ops.gemm_f32_tcgen05(x, w).double(), x.double() @ w.double().T, _bound(x, w)
+    bound[:, 50] *= 2 ** 6
+    assert ((got - want).abs() <= bound).all() and (bound[:, 50] < 2e-4 * want[:, 50].abs()).all()
