@@ -189,10 +189,12 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
     // a key of this step; the consumers wait before they read the queries.
     if ((int)blockIdx.y >= *n_work_ptr) return;
     const AttnWork w = work[blockIdx.y];
+    // rows of a slab at most: a range may begin at any multiple of 64 (a chunk's start), of which a page of 128 tokens or more need not hold a whole tile
+    constexpr int SLAB = TD_KEYS * CONSUMERS < 64 ? TD_KEYS * CONSUMERS : 64;
     if (!(kinds_mask & (w.q_count == 1 ? 1 : 2))) return;   // another kernel's item
     if (KEYS_AS_ROWS && w.q_count != 1) return;             // (this variant is for single tokens only)
-    if (w.kv_begin & (TD_KEYS * CONSUMERS - 1)) {
-        // slabs and the swizzle need the range to start on a tile boundary
+    if (w.kv_begin & (SLAB - 1)) {
+        // slabs and the swizzle need the range to start on a slab's boundary
         if (threadIdx.x == 0) atomicOr(status, 32);
         return;
     }
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
     __syncthreads();   // the barriers are set up; the producer goes its own way from here
 
     const int n_tiles = (w.kv_end - w.kv_begin + BK - 1) / BK;
-    const int slab_rows = page_size < BK ? page_size : BK;
+    const int slab_rows = page_size < SLAB ? page_size : SLAB;
     const int slabs = BK / slab_rows;          // at most 16 (pages of at least 8 tokens)
     const uint32_t slab_bytes = (uint32_t)slab_rows * HD * 2;
 

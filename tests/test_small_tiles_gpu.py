@@ -182,3 +182,58 @@ def test_many_tokens_get_the_same_bits_as_few(dtype, nh, nkv, hd):
         return (q, *pools)
     for many, few in zip(made(T), made(100)):
         assert torch.equal(many, few)
+
+
+def _single_tokens(ctxs, work, nh, nkv, hd, page, rope):
+    """A step of single tokens whose items are not cut, of which item r begins at its own first key, against 64 bits."""
+    B, total, last = len(ctxs), nh + 2 * nkv, max(ctxs)
+    rng = np.random.default_rng(B * hd + page)
+    n_pages = sum(c // page + 1 for c in ctxs) + 2
+    order = iter(rng.permutation(n_pages).tolist())
+    tables = np.full((B, last // page + 1), -1, np.int32)
+    for r, c in enumerate(ctxs):
+        for b in range(c // page + 1):
+            tables[r, b] = next(order)
+    g = torch.Generator(device=DEV).manual_seed(nh + last)
+    kp, vp = (torch.randn(n_pages, nkv, page, hd, device=DEV, generator=g).bfloat16() for _ in range(2))
+    qkv = torch.randn(B, total * hd, device=DEV, generator=g).bfloat16()
+    qg, kg = (1 + 0.1 * torch.randn(hd, device=DEV, generator=g) for _ in range(2))
+    angle = torch.rand(last + 1, hd // 2, device=DEV, generator=g) * 6.3
+    cos, sin = (angle.cos(), angle.sin()) if rope else (None, None)
+    one = torch.zeros(1, dtype=torch.int32, device=DEV)
+    w = AttentionWork(torch.from_numpy(work).to(DEV), one + B, B, torch.zeros(1, 4, dtype=torch.int32, device=DEV), one, 0,
+                      torch.zeros(1, nh, hd, device=DEV), torch.zeros(1, nh, 2, device=DEV), kinds=1, reduces=False)
+    out, st = torch.zeros(B, nh * hd, dtype=torch.bfloat16, device=DEV), K.status()
+    ops.decode_attention_fused(qkv, qg, kg, 1e-6, cos, sin, kp, vp, torch.from_numpy(tables).to(DEV), w, out, nh, nkv, hd, hd ** -0.5, st)
+    assert st.item() == 0
+
+    def made(x, gain, c):
+        x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6) * gain.double()
+        if rope:
+            a, b, co, si = x[..., :hd // 2], x[..., hd // 2:], cos[c].double(), sin[c].double()
+            x = torch.cat([a * co - b * si, b * co + a * si], -1)
+        return x.bfloat16().double()
+    for r, c in enumerate(ctxs):
+        f = qkv[r].double().view(total, hd)
+        begin, n = int(work[r, 4]), c + 1
+        at = torch.arange(n, device=DEV) % page & 7
+        idx = (torch.arange(hd // 8, device=DEV)[None, :] ^ at[:, None])[None, :, :, None].expand(nkv, n, hd // 8, 8)
+        k, v = (torch.cat([p[i] for i in tables[r, :c // page + 1]], 1)[:, :n].reshape(nkv, n, hd // 8, 8).gather(2, idx).reshape(nkv, n, hd).double()
+                for p in (kp, vp))                           # (the step has written its own key and value)
+        near = (k[:, c] - made(f[nh:nh + nkv], kg, c)).abs()
+        assert near.max().item() < 2 ** -6 and torch.equal(v[:, c], f[nh + nkv:])
+        s = torch.einsum("gpd,gnd->gpn", made(f[:nh], qg, c).view(nkv, nh // nkv, hd), k[:, begin:]) * hd ** -0.5
+        want = torch.einsum("gpn,gnd->gpd", torch.softmax(s, -1), v[:, begin:]).reshape(-1)
+        # weights rounded to bfloat16 (2^-9 each, of values up to 4.5) and the result once more; q's rounding may differ by an ulp
+        assert (out[r].double() - want).abs().max().item() < 5e-2, (r, c)
+
+
+# A key range may begin at any multiple of 64, whichever kernel takes it (the eight warps' tiles have 128 keys; pages of 128 tokens and more do
+# not hold a whole tile that begins in their middle)
+@pytest.mark.parametrize("nh,nkv,hd,page", [(16, 8, 128, 16), (8, 2, 64, 64), (16, 8, 128, 128), (4, 1, 128, 256)])
+@pytest.mark.parametrize("chunk", [64, 192])
+@pytest.mark.parametrize("ctxs", [[64, 700], [70, 127, 191, 192, 200, 383, 384, 447, 511, 1000]])
+def test_key_ranges_that_begin_within_a_tile(nh, nkv, hd, page, chunk, ctxs):
+    work, _, parts = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, 1, chunk=chunk)
+    assert parts == 0 and (work[:, 4] % 128 == 64).any()
+    _single_tokens(ctxs, work, nh, nkv, hd, page, True)
