@@ -2,6 +2,7 @@
 
 import random
 
+import numpy as np
 import pytest
 
 from paged_llm_rs_b200.kernels import attention_plan as P
@@ -45,3 +46,28 @@ def test_single_tokens_alone_are_cut_as_before():
     a = P.plan_attention(segments, 16, None, 8, 296)
     b = P.plan_attention(segments, 16, None, 8, 296, part_keys=P.F32_PART_KEYS)
     assert (a[0] == b[0]).all() and (a[1] == b[1]).all() and a[2] == b[2]
+
+
+@pytest.mark.parametrize("most", [5, 37, 148, 592])
+def test_a_part_is_the_smallest_that_leaves_few_enough(most):
+    rng = random.Random(most)
+    for _ in range(300):
+        keys = np.array([rng.choice([1, rng.randint(1, 300), rng.randint(1, 40000)]) for _ in range(rng.randint(1, most - 1))])
+        part = rng.choice([64, P.F32_PART_KEYS, 1000])
+        size = P.part_size(keys, part, most)
+
+        def fits(n):
+            return int((-(-keys // n)).sum()) <= most and int(keys.max()) <= P.MAX_SPLITS * n
+        assert size >= part and (size - part) % P.SPLIT_ALIGN == 0 and fits(size) and (size == part or not fits(size - P.SPLIT_ALIGN))
+
+
+def test_long_ranges_are_planned_without_trying_every_size():
+    # (a portion behind 30 000 tokens: counted, as a time says little on a busy machine)
+    sums = []
+
+    class Counted(np.ndarray):
+        def sum(self, *a, **k):
+            sums.append(1)
+            return np.asarray(self).sum(*a, **k)
+    P.part_size(np.arange(30000, 30256, 2).view(Counted), P.F32_PART_KEYS, 148)
+    assert len(sums) <= 20             # (of some 470 sizes: two logarithms of that, and the sum of the keys)
