@@ -14,7 +14,8 @@ from __future__ import annotations
 import gc
 import os
 from collections import OrderedDict
-from typing import List, Optional, Sequence
+from dataclasses import replace
+from typing import Collection, List, Optional, Sequence
 
 import numpy as np
 import torch
@@ -304,16 +305,24 @@ def portion_requests(n: int) -> int:
     return S
 
 
-def group_plans(cache: CacheManager, mixer_of, page_size: int) -> List[Optional[GroupPlanConfig]]:
-    """Per cache group how its attention is cut into work items: what its mixers wish (those of one group alike; a group
+def group_plans(cache: CacheManager, mixer_of, page_size: int, lenders: Collection[int] = ()) -> List[Optional[GroupPlanConfig]]:
+    """Per cache group how its attention is cut into work items: what its mixers wish (those of one group alike, but for how the key ranges are
+    cut, which is by the planner's usual rule unless all wish for another; a group
     whose mixers wish for nothing gets tables and slots only).  ``mixer_of(cell)`` gives the mixer a cache of the group
-    belongs to (``CacheGroup.cells``: a schedule entry, or (entry, part, ...) for a piece of a CompositeNeed)."""
+    belongs to (``CacheGroup.cells``: a schedule entry, or (entry, part, ...) for a piece of a CompositeNeed).  ``lenders``: the schedule entries
+    whose cache a later entry reads, which writes none and so runs kernels that gain nothing by whole contexts."""
     plans = []
     for g in cache.groups:
-        wishes = {mixer_of(cell).plan_wish(page_size) for cell in g.cells}
+        asked = {mixer_of(cell).plan_wish(page_size) for cell in g.cells}
+        cuts = {(w.whole, w.part_keys) for w in asked if w is not None}
+        wishes = {w if w is None else replace(w, whole=False, part_keys=0) for w in asked}
         if len(wishes) != 1:
             raise ConfigError(f"the mixers that share a cache group wish for different attention plans: {sorted(map(str, wishes))}")
         w = wishes.pop()
+        if w is not None:
+            lent = any((cell[0] if isinstance(cell, tuple) else cell) in lenders for cell in g.cells)
+            parts = {part for _, part in cuts}
+            w = replace(w, whole=not lent and all(whole for whole, _ in cuts), part_keys=parts.pop() if len(parts) == 1 else 0)
         plans.append(None if w is None else GroupPlanConfig(w.tile_tokens, w.ctas_per_item, g.window, w.heads, w.head_dim, g.chunk, w.whole, w.part_keys))
     return plans
 
@@ -350,7 +359,8 @@ class ModelRunner:
         self.cache = CacheManager(needs, page_size, num_pages, max_requests, self.dtype, self.device,
                                   prefix_cache=prefix_cache)
         self.caches = self.cache.layer_caches()
-        plans = group_plans(self.cache, self._mixer_of, page_size)
+        plans = group_plans(self.cache, self._mixer_of, page_size,
+                            {e.reads_cache_of for e in self.model.schedule if e.reads_cache_of is not None})
         # CTAs an attention launch should have before splits stop: one full wave at two CTAs an SM
         self.packer = StepPacker(self.cache, plans, 2 * ops.sm_count(), self.spec.vocab_size, self.spec.max_positions,
                                  self.device)

@@ -67,19 +67,23 @@ class GQAttention(Mixer):
 
     def plan_wish(self, page_size: int):
         tile = ops.attention_tile_tokens(self.nh, self.nkv, self.rt.dtype, self.hd, page_size, self.window or 0)
+        # whole where a step of single tokens runs as one kernel, as forward() decides it
         swizzled = self.cache_need().swizzled
         whole = swizzled and self.nh <= 8 * self.nkv and ops.decode_attention_fuses(self.rt.dtype, self.nh, self.nkv, self.hd, page_size,
-                                                                                     self.window or 0, 0, swizzled)
+                                                                                     self.window or 0, self._rotary()[2], swizzled)
         return PlanWish(tile, ops.attention_ctas_per_item(self.nh, self.nkv, self.rt.dtype), self.nh, self.hd, whole=whole,
                         part_keys=F32_PART_KEYS if self.rt.dtype == torch.float32 else 0)
+
+    def _rotary(self):
+        rot = self.position.rotary() if self.position is not None else None
+        return rot if rot is not None else (None, None, 0)
 
     def forward(self, x, step, cache, writes_cache=True):
         k_pool, v_pool, gi = cache
         g = step.groups[gi]
         w = g.plan
         T = x.shape[0]
-        rot = self.position.rotary() if self.position is not None else None
-        cos, sin, rdim = rot if rot is not None else (None, None, 0)
+        cos, sin, rdim = self._rotary()
         swizzled = self.cache_need().swizzled
         qkv = ops.linear(x, self.w_qkv, status=self.rt.status)
         if writes_cache and w.kinds == 1 and ops.decode_attention_fuses(x.dtype, self.nh, self.nkv, self.hd, k_pool.shape[2],

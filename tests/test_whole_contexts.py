@@ -1,12 +1,20 @@
 """Steps of single tokens with short contexts, which are not cut (attention_plan.whole_keys): the native packer and the array planner
 keep one rule."""
 
+from types import SimpleNamespace
+
 import numpy as np
 import pytest
+import torch
 
 from paged_llm_rs_b200.cache.manager import CacheManager
+from paged_llm_rs_b200.engine.runner import group_plans
 from paged_llm_rs_b200.engine.step import GroupPlanConfig, StepEntry
+from paged_llm_rs_b200.errors import ConfigError
 from paged_llm_rs_b200.kernels import attention_plan as P
+from paged_llm_rs_b200.parts.attention import GQAttention
+from paged_llm_rs_b200.parts.base import PlanWish
+from paged_llm_rs_b200.parts.spec import PartSpec
 from test_step_pack import FULL, WIN, setup
 
 
@@ -52,3 +60,33 @@ def test_only_short_contexts_of_single_tokens_are_left_whole():
     mixed = [(0, 1, 600), (1, 9, 30)]
     a, b = (P.plan_attention(mixed, 8, None, 2, 296, whole=w) for w in (False, True))
     assert (a[0] == b[0]).all() and (a[1] == b[1]).all()
+
+
+def _mixer(rotary, head_dim=128):
+    """An attention layer as the planner sees it (no device is touched); ``rotary``: entries of a head that turn, None without an encoding."""
+    rt = SimpleNamespace(device=torch.device("cuda"), dtype=torch.bfloat16, trace=None, status=None)
+    turn = SimpleNamespace(rotary=lambda: (None, None, rotary) if rotary else None)
+    params = dict(hidden_size=256, num_heads=16, num_kv_heads=8, head_dim=head_dim, scale=1.0, **({} if rotary is None else dict(position_encoding="p")))
+    return GQAttention(PartSpec("gqa_attention", params, "m"), rt, {"p": turn})
+
+
+def test_contexts_are_left_whole_for_the_kernel_that_gains_by_it():
+    # (a rotation of part of a head: forward() norms and rotates by a kernel of its own, and the attention has four warps)
+    assert [_mixer(r).plan_wish(16).whole for r in (None, 0, 128, 64)] == [True, True, True, False]
+
+
+def test_layers_of_one_group_that_differ_in_how_ranges_are_cut():
+    whole, cut = _mixer(128), _mixer(64)
+    of = lambda *mixers: (CacheManager([m.cache_need() for m in mixers], 16, 10, 4, torch.bfloat16, "cpu", allocate_device=False), list(mixers).__getitem__)
+    for mixers, lenders, want in (((whole, whole), (), True), ((whole, cut), (), False), ((whole, whole), {1}, False), ((cut,), (), False)):
+        plan, = group_plans(*of(*mixers), 16, lenders)
+        assert plan.whole == want and plan.part_keys == 0
+    # a mixer of a caller's own beside them says nothing about it
+    wish = whole.plan_wish(16)
+    own = SimpleNamespace(cache_need=whole.cache_need, plan_wish=lambda page: PlanWish(wish.tile_tokens, wish.ctas_per_item, wish.heads, wish.head_dim))
+    assert not group_plans(*of(whole, own), 16)[0].whole
+    parts = lambda n: SimpleNamespace(cache_need=whole.cache_need, plan_wish=lambda page: PlanWish(8, 2, 16, 128, part_keys=n))
+    assert group_plans(*of(parts(192), parts(192)), 16)[0].part_keys == 192 and group_plans(*of(parts(192), parts(0)), 16)[0].part_keys == 0
+    other = SimpleNamespace(cache_need=whole.cache_need, plan_wish=lambda page: PlanWish(7, 2, 16, 128))
+    with pytest.raises(ConfigError):
+        group_plans(*of(parts(0), other), 16)
