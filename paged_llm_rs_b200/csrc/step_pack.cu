@@ -19,7 +19,7 @@ struct PllmGroupPack {
     int window;                 // 0: every key stays
     int chunk;                  // > 0 (and no window): a query reads its own chunk of this many positions only
     int ctas_per_item;          // CTAs the attention kernel launches per work item
-    int whole;                  // short contexts are not cut (whole_keys)
+    int whole;                  // short contexts of like lengths are not cut (whole_keys, even_enough)
     int max_work, max_red, max_parts;                                    // capacities of the captured step
     int plans;                  // 0: the group's mixers take no attention work items (the offsets of work and red are unused)
     int off_slots, off_tables, off_n_work, off_n_red, off_work, off_red; // offsets in int32 units
@@ -40,6 +40,12 @@ static const int MAX_SPLITS = 128;
 
 // kernels/attention_plan.py: whole_keys
 static inline int whole_keys(long long ctas, long long target_ctas) { return 8 * ctas >= 3 * target_ctas ? 4096 : (int)(512 + 6 * ctas); }
+// kernels/attention_plan.py: even_enough
+static inline bool even_enough(long long longest, long long total, long long items, long long ctas, long long target_ctas) {
+    const int fifths = 16 * ctas <= 7 * target_ctas ? 4 : (target_ctas < 2 * ctas && 9 * ctas <= 8 * target_ctas ? 6 : 5);
+    const int keys = fifths == 4 ? 480 : (fifths == 6 ? 320 : 192);
+    return 5 * items * longest - fifths * total <= 5 * items * keys;
+}
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // tokens, positions, state_slots, temperature, uniform: one per request (temperature and
@@ -91,12 +97,14 @@ PLLM_EXPORT int pllm_pack_decode_step(int* out, int out_len, int n, const int* t
             want = target_ctas / (n * g.ctas_per_item);
             if (want < 2) want = 2;
             int most = 0;
+            long long total = 0;
             for (int i = 0; i < n; i++) {
                 const int p0 = positions[i];
                 const int keys = g.window > 0 ? (p0 + 1 < g.window ? p0 + 1 : g.window) : (g.chunk > 0 ? p0 % g.chunk + 1 : p0 + 1);
                 if (keys > most) most = keys;
+                total += keys;
             }
-            if (g.whole && most <= whole_keys(n * g.ctas_per_item, target_ctas)) want = 1;
+            if (g.whole && most <= whole_keys(n * g.ctas_per_item, target_ctas) && even_enough(most, total, n, n * g.ctas_per_item, target_ctas)) want = 1;
         }
         int n_work = 0, n_red = 0, parts = 0;
         for (int i = 0; i < n; i++) {

@@ -148,7 +148,7 @@ class StepPacker:
             key = (plan.tile_tokens, plan.window, plan.ctas_per_item, plan.chunk, plan.part_keys, plan.whole)
             if key not in planned:
                 planned[key] = attention_plan.plan_attention(spans, plan.tile_tokens, plan.window, plan.ctas_per_item, self.target_ctas,
-                                                             chunk=plan.chunk, part_keys=plan.part_keys, whole=plan.whole)
+                                                             chunk=plan.chunk, part_keys=plan.part_keys, whole=plan.whole, even=True)
             work, red, parts = planned[key]
             mw, mr, mp = (work_caps[gi] if work_caps else (len(work), len(red), parts))
             if len(work) > mw or len(red) > mr or parts > mp:

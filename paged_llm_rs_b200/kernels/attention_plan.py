@@ -54,6 +54,26 @@ def whole_keys(ctas: int, target_ctas: int) -> int:
     return WHOLE_KEYS_MANY if 8 * ctas >= 3 * target_ctas else WHOLE_KEYS + WHOLE_KEYS_A_CTA * ctas
 
 
+# Contexts of very different lengths: the longest one's CTAs walk on alone when the others have left, where cut in two they walk half as far.  A step
+# whole / cut (0.6B shape, 8 CTAs a request; lengths from the longest down by a quarter | a half | nine tenths | one long, the rest an eighth of it):
+#   requests  8: 520 tokens .97 .98 1.00 1.02, 760 1.00 1.01 1.01 1.02             12: 640 .96 .97 1.01 1.00, 900 .99 1.01 1.03 1.10
+#            16: 640 .95 .95 .97 .95, 1200 .98 .98 1.01 1.06, 4000 .98 1.03 1.10 1.18   (eight warps to a CTA, each CTA an SM)
+#            18: 300 .94 .94 .97 .99, 640 .97 .99 1.01 1.04, 1600 .98 1.02 1.07 1.12, 4000 1.03 1.09 1.24 1.30
+#            20: 420 .89 .90 .98 1.01, 1200 .88 .92 1.02 1.07, 4000 .87 1.01 1.17 1.30   (cut, its CTAs are more than the SMs have places for)
+#            28: 420 .89 .88 .88 1.00, 1200 .91 .93 .96 1.07, 4000 .99 1.05 1.13 1.33    32: 420 .92 .90 .90 1.01, 2200 .95 .98 1.02 1.19
+#            36: 300 .98 .99 .98 1.01, 900 .96 1.01 1.03 1.12, 4000 1.01 1.05 1.16 1.32  (small CTAs, for which the cut ones have places again)
+# So the longest may be longer than a share of the mean (in fifths) by so many keys: what is then left whole takes .86 to 1.03 of its time cut, and before there was
+# this bound 4000 tokens beside 60 took up to 1.39.
+EVEN_LARGE, EVEN_CROWDED, EVEN = (4, 480), (6, 320), (5, 192)
+
+
+def even_enough(longest: int, total: int, items: int, ctas: int, target_ctas: int) -> bool:
+    """Whether the contexts of a step of ``items`` single tokens (``total`` keys in all, in ``ctas`` CTAs uncut) are near enough to one another
+    to be left whole (csrc/step_pack.cu has the same rule)."""
+    fifths, keys = EVEN_LARGE if 16 * ctas <= 7 * target_ctas else EVEN_CROWDED if target_ctas < 2 * ctas and 9 * ctas <= 8 * target_ctas else EVEN
+    return 5 * items * longest - fifths * total <= 5 * items * keys
+
+
 def part_size(keys: np.ndarray, part_keys: int, most: int) -> int:
     """The least of ``part_keys``, ``part_keys`` + 64, .. that cuts key ranges ``keys`` (fewer than ``most``) into ``most`` parts at most and none into
     more than MAX_SPLITS.  From the size that their sum and the longest ask for on, by steps that double and then by halves: tried one
@@ -76,16 +96,16 @@ def part_size(keys: np.ndarray, part_keys: int, most: int) -> int:
 def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, window: Optional[int],
                    ctas_per_item: int, target_ctas: int,
                    min_split_keys: int = MIN_SPLIT_KEYS,
-                   multi_min_split_keys: int = MULTI_MIN_SPLIT_KEYS, chunk: int = 0, part_keys: int = 0, whole: bool = False) -> Tuple[np.ndarray, np.ndarray, int]:
+                   multi_min_split_keys: int = MULTI_MIN_SPLIT_KEYS, chunk: int = 0, part_keys: int = 0, whole: bool = False, even: bool = False) -> Tuple[np.ndarray, np.ndarray, int]:
     """segments: (first token index, token count, position of the first token) per
     segment, in step order; ``chunk``: a query reads keys of its own chunk of that many positions only; ``part_keys``: a step with tiles of
     several tokens is cut into parts of that many keys, or of so many more that they stay within twice the target; ``whole``: a step of single
-    tokens of which none has more keys than ``whole_keys`` says is not cut.
+    tokens of which none has more keys than ``whole_keys`` says is not cut; ``even``: nor more than ``even_enough`` allows beside the others.
     Returns (work [n, 8], red [m, 4], partial rows used)."""
     in_parts = part_keys > 0 and any(c > 1 for _, c, _ in segments)
     if len(segments) <= SMALL_PLAN:
         small = _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk,
-                            part_keys if in_parts else 0, whole)
+                            part_keys if in_parts else 0, whole, even)
         if small is not None:
             return small
     seg_ids, q0s, qns, p0s = [], [], [], []
@@ -131,7 +151,8 @@ def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, w
         if want < 2:
             want = 2 if int(qn.max()) == 1 else 1
         floor = np.where(qn > 1, max(min_split_keys, multi_min_split_keys), min_split_keys)
-        if not whole or int(qn.max()) > 1 or int(keys.max()) > whole_keys(n_tiles * ctas_per_item, target_ctas):
+        if not whole or int(qn.max()) > 1 or int(keys.max()) > whole_keys(n_tiles * ctas_per_item, target_ctas) or \
+                even and not even_enough(int(keys.max()), int(keys.sum()), n_tiles, n_tiles * ctas_per_item, target_ctas):
             splits = np.clip(np.minimum(want, keys // floor), 1, MAX_SPLITS)
     if (splits == 1).all():
         work = np.stack([seg, q0, qn, p0, kv_begin, kv_end, np.full(n_tiles, -1), np.zeros(n_tiles, np.int64)], 1)
@@ -164,7 +185,7 @@ def plan_attention(segments: Sequence[Tuple[int, int, int]], tile_tokens: int, w
 SMALL_PLAN = 32        # segments, and tiles, of a step that is planned number by number
 
 
-def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk, part_keys=0, whole=False):
+def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_split_keys, multi_min_split_keys, chunk, part_keys=0, whole=False, even=False):
     """``plan_attention`` for a step of few tiles of which none is split (a prompt's portion, as a rule): the same list without the
     forty array operations that cost such a step more than its work (35 to 80 us).  None when it is not one."""
     items, most = [], 0
@@ -186,8 +207,11 @@ def _small_plan(segments, tile_tokens, window, ctas_per_item, target_ctas, min_s
         want = target_ctas // (len(items) * ctas_per_item)
         if want < 2:
             want = 2 if most == 1 else 1
-        if want > 1 and not (whole and most == 1 and max(end - begin for _, _, _, _, begin, end, _, _ in items)
-                             <= whole_keys(len(items) * ctas_per_item, target_ctas)):
+        if want > 1 and whole and most == 1:
+            keys, ctas = [end - begin for _, _, _, _, begin, end, _, _ in items], len(items) * ctas_per_item
+            if max(keys) <= whole_keys(ctas, target_ctas) and (not even or even_enough(max(keys), sum(keys), len(items), ctas, target_ctas)):
+                want = 1
+        if want > 1:
             for _, _, n, _, begin, end, _, _ in items:
                 if end - begin >= 2 * (max(min_split_keys, multi_min_split_keys) if n > 1 else min_split_keys):
                     return None       # (in parts, a tile of several tokens has been looked at above)
