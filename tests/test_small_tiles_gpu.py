@@ -237,3 +237,26 @@ def test_key_ranges_that_begin_within_a_tile(nh, nkv, hd, page, chunk, ctxs):
     work, _, parts = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, 1, chunk=chunk)
     assert parts == 0 and (work[:, 4] % 128 == 64).any()
     _single_tokens(ctxs, work, nh, nkv, hd, page, True)
+
+
+# One or two requests (eight consumer warps, a ring of three stages of 128 keys) and some more (a ring of two): the edges of a tile, of the ring's
+# first turn and of the second, the token's own key in each place of the ring
+@pytest.mark.parametrize("rope", [True, False])
+@pytest.mark.parametrize("nh,nkv,hd,page", [(16, 8, 128, 16), (32, 8, 64, 64), (6, 1, 128, 8), (2, 2, 64, 256)])
+@pytest.mark.parametrize("ctxs", [[0, 1], [126, 127], [128, 129], [255, 256], [383, 384], [385, 511], [767, 768], [900, 15],
+                                  [0, 127, 128, 255, 256, 257, 384, 511, 512, 640, 1000]])
+def test_whole_contexts_by_eight_warps(nh, nkv, hd, page, rope, ctxs):
+    if nkv * len(ctxs) > ops.sm_count():
+        pytest.skip("more CTAs than SMs: other kernels")
+    work, _, parts = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, 1)
+    assert parts == 0
+    _single_tokens(ctxs, work, nh, nkv, hd, page, rope)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,page", [(16, 8, 128, 16), (8, 4, 64, 32)])
+def test_many_requests_with_a_rotation(nh, nkv, hd, page):
+    # (more CTAs than two an SM: two consumer warps and tiles of 32 keys)
+    ctxs = [(37 * r) % 300 for r in range(2 * ops.sm_count() // nkv + 5)]
+    work, _, parts = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, 1)
+    assert parts == 0
+    _single_tokens(ctxs, work, nh, nkv, hd, page, True)
