@@ -320,7 +320,7 @@ def mixed_point(runner, decoding, context, portion, behind, vocab, steps, warmup
     runner.graph_step_tokens = decoding + portion
     try:
         runner.step_and_sample(entries, zeros, zeros)
-        graph = runner._portion_graph(entries)
+        graph, _ = runner._portion_graph(entries)
         assert graph is not None, "the mixed step does not run as a captured step"
         ms, span, spread = time_on_device(graph.replay, steps, warmup, repeats)
     finally:
@@ -1636,7 +1636,7 @@ def timeline(runner, batch, context, layers, prefill_tokens=0, vocab=1000, mixed
         zeros = np.zeros(batch, dtype=np.float32)
         runner.graph_step_tokens = batch + mixed_tokens
         runner.step_and_sample(entries, zeros, zeros)
-        graph = runner._portion_graph(entries)
+        graph, _ = runner._portion_graph(entries)
         assert graph is not None, "the mixed step does not run as a captured step"
     elif prefill_tokens:
         prompt = np.random.default_rng(0).integers(0, vocab, prefill_tokens).tolist()
@@ -1645,7 +1645,7 @@ def timeline(runner, batch, context, layers, prefill_tokens=0, vocab=1000, mixed
         entries = [StepEntry("tp", prompt, [prefill_tokens - 1])]
         zeros = np.zeros(1, dtype=np.float32)
         runner.step_and_sample(entries, zeros, zeros)
-        graph = runner._portion_graph(entries)
+        graph, _ = runner._portion_graph(entries)
         assert graph is not None, "the portion does not run as a captured step"
     else:
         ids = [f"t{b}" for b in range(batch)]

@@ -7,6 +7,7 @@ import json
 import os
 import subprocess
 import sys
+from types import SimpleNamespace
 
 import pytest
 
@@ -49,3 +50,13 @@ def test_the_long_prompt_mode_times_every_portion():
     first, last = out["portion_at_0"], out["portion_at_4096"]
     assert 0 < first["bf16_frac"] < 1.2 and 0 < last["bf16_frac"] < 1.2
     assert last["attention_share_of_flops"] > first["attention_share_of_flops"]
+
+
+def test_a_mixed_point_times_the_captured_step(tmp_path):
+    sys.path.insert(0, ROOT)
+    import bench
+    from paged_llm_rs_b200.engine.runner import ModelRunner
+    from tiny_configs import CONFIGS, write_model
+    runner = ModelRunner(write_model(tmp_path, "A"), dtype="bfloat16", page_size=16, num_pages=64, max_requests=8, prefix_cache=False)
+    ms, spread = bench.mixed_point(runner, 3, 40, 20, 30, CONFIGS["A"][0]["vocab_size"], 3, 3, SimpleNamespace(region=lambda *span: None), repeats=1)
+    assert ms > 0 and spread["n"] == 2
