@@ -20,18 +20,18 @@
 // so the slab is copied as it lies.
 //
 // A CTA has four consumer warps (or two, or eight: launch_tma) and one producer warp.  Tiles of 64 (32, 128) keys go round
-// a 3-stage ring; every consumer warp reads every tile in turn (a parity wait tells
+// a ring of three stages (eight warps: two or three); every consumer warp reads every tile in turn (a parity wait tells
 // two phases of a barrier apart and no more, so no warp may run a whole turn of the
 // ring ahead of another: taking tiles in turn keeps them within it).  q.k^T and p.v
 // run on mma.sync.m16n8k16.  For one query token the group's heads are the (padded)
 // 16 rows of one block, each warp multiplies its own 16 keys of every tile and keeps
-// a running (max, sum, output) of its own; the four meet in shared memory at the
+// a running (max, sum, output) of its own; the warps meet in shared memory at the
 // end.  For several query tokens the rows (token, head) are spread over the warps,
 // 16 each, and every warp multiplies whole tiles.  Every wait on an mbarrier is
 // bounded: a waiter that gives up raises a status bit, tells the others and the
 // CTA returns.
 //
-// It takes items whose key range starts on a multiple of 64 and has no window, in
+// It takes items whose key range starts on a multiple of 64 (of 32, by two warps) and has no window, in
 // caches whose pages hold a power of two of at least 8 tokens; the rest is the
 // cp.async kernel's (attention_mma.cu).
 #include "common.cuh"

@@ -671,7 +671,8 @@ def rows_gemm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
 
 
 # True float32 products on the CUDA cores (csrc/gemm_f32.cu) where the library's tiles leave most of the chip idle.
-# Measured on a B200, a norm and the product behind it (us, this kernel / cuBLAS; - the library's):
+# Measured on a B200, a norm and the product behind it (us, this kernel / cuBLAS; - the library's; from 33 rows on ``linear`` asks gemm_f32_tcgen05_sizes first, so that
+# here come W of fewer than 2^20 entries or rows of fewer than 1024, and what that kernel does not take: K no multiple of eight, N none of four):
 #   rows          4            8            16           32           64           128          256
 #   1024 x 256    - 8.5 / 4.3  - 9.2 / 7.7  - 9.9 / 7.8  - 9.6 / 8.0  - 9.6 / 8.1  - 14.0/ 8.2  - 24.0/ 8.9
 #   1024 x 512    - 8.5 / 7.8  - 9.0 / 7.9  - 9.4 / 8.0  9.0 / 12.1   12.3 / 12.2  - 13.0/ 12.3 - 22.7/ 14.0
