@@ -175,7 +175,7 @@ __device__ __forceinline__ void norm_rope_row(const RowConsts<HD>& with, bool no
     }
 }
 
-template <int HD, bool KEYS_AS_ROWS, int CONSUMERS = TD_CONSUMERS, int STAGES = TD_STAGES>
+template <int HD, bool KEYS_AS_ROWS, int CONSUMERS = TD_CONSUMERS, int STAGES = TD_STAGES, bool TWO_PARTS = CONSUMERS != TD_CONSUMERS>
 __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 / CONSUMERS) attention_decode_tma_kernel(
     const bf16* q, const bf16* k_pool, const bf16* v_pool,   // written by the kernels before this one: no __restrict__
     const int* __restrict__ block_tables, const AttnWork* __restrict__ work, const int* __restrict__ n_work_ptr,
@@ -353,19 +353,25 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
     }
     asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMERS * 32));
 
-    float* o_s = reinterpret_cast<float*>(smem);          // [4][16][HD], once the ring is no longer read
-    float* ml_s = o_s + CONSUMERS * 16 * HD;           // [4][16][2]
+    float* o_s = reinterpret_cast<float*>(smem);          // [warps][16][HD], once the ring is no longer read
+    float* ml_s = o_s + CONSUMERS * 16 * HD;           // [warps][16][2]
+    // TWO_PARTS: the weights are multiplied as what bfloat16 holds of them and what it holds of the rest.  A warp's largest weight is 1 and rounds
+    // exactly, so that the distance from 64 bits of weights in one part goes with how many warps and parts share the keys (64 requests at 512, group of 2:
+    // 0.00208 by four warps, 0.00213 by two, 0.00166 in two parts, of which the result's rounding is nearly all).  With four heads at most the rest rides in
+    // the columns beyond them, whose scores are the heads' again; with more it is a product of its own.
+    const bool beside = TWO_PARTS && n_heads <= 4;
     if constexpr (KEYS_AS_ROWS) {
     // ---- consumers, one query token of at most 8 heads: the KEYS are the 16 rows of the score block --------
     // and the heads its 8 columns, S^T = K q^T and O^T = V^T P^T.  A block of 16 keys costs 8 + HD / 16
     // mma instead of twice that with the (two, four, eight) heads padded to 16 rows, the output is
     // HD / 16 x 4 registers instead of HD / 8 x 4, and the queries are 2 registers a k-step instead of 4.
+    const bool rest_here = beside && (lane & 2);
     uint32_t qb[KSTEPS][2];
     {
 #pragma unroll
         for (int kp = 0; kp < KSTEPS / 2; kp++) {
             uint32_t r[4];
-            ldsm4(r, q_s + toff<HD>(lane & 7, kp * 4 + (lane >> 3)));
+            ldsm4(r, q_s + toff<HD>(lane & (beside ? 3 : 7), kp * 4 + (lane >> 3)));
             qb[2 * kp][0] = r[0]; qb[2 * kp][1] = r[1]; qb[2 * kp + 1][0] = r[2]; qb[2 * kp + 1][1] = r[3];
         }
     }
@@ -439,7 +445,13 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
             l_run[0] += p0 + p2;
             l_run[1] += p1 + p3;
             // P^T as the second operand: (key, head pair) in this thread becomes (head, key pair)
-            const uint32_t pb0 = movmatrix_t(pack2(p0, p1)), pb1 = movmatrix_t(pack2(p2, p3));
+            uint32_t h0 = pack2(p0, p1), h1 = pack2(p2, p3), rest0 = 0, rest1 = 0;
+            if constexpr (TWO_PARTS) {
+                rest0 = pack2(p0 - __uint_as_float(h0 << 16), p1 - __uint_as_float(h0 & 0xffff0000u));
+                rest1 = pack2(p2 - __uint_as_float(h1 << 16), p3 - __uint_as_float(h1 & 0xffff0000u));
+                if (rest_here) { h0 = rest0; h1 = rest1; }
+            }
+            const uint32_t pb0 = movmatrix_t(h0), pb1 = movmatrix_t(h1);
             if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
 #pragma unroll
                 for (int d = 0; d < MT; d++) {
@@ -449,6 +461,11 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
             }
 #pragma unroll
             for (int d = 0; d < MT; d++) mma(o_acc[d], vf[d], pb0, pb1);
+            if (TWO_PARTS && !beside) {
+                const uint32_t rb0 = movmatrix_t(rest0), rb1 = movmatrix_t(rest1);
+#pragma unroll
+                for (int d = 0; d < MT; d++) mma(o_acc[d], vf[d], rb0, rb1);
+            }
         } else {
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + 8 * (STAGES + s));
@@ -679,7 +696,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, CONSUMERS == 8 ? 1 : 8 /
             const float mw = ml_s[(wi * 16 + r) * 2];
             const float f = mw == -CUDART_INF_F ? 0.f : exp2f(mw - M);
             L += ml_s[(wi * 16 + r) * 2 + 1] * f;
-            o += o_s[(size_t)(wi * 16 + r) * HD + c] * f;
+            o += (o_s[(size_t)(wi * 16 + r) * HD + c] + (beside ? o_s[(size_t)(wi * 16 + r + 4) * HD + c] : 0.f)) * f;
         }
         const int head = head0 + r;
         if (w.part_slot < 0) {
@@ -728,8 +745,10 @@ static int launch_tma(const void* q, const void* k_pool, const void* v_pool, con
         // these can be there before it is over; three where a CTA meets one on few SMs (us a step, three / two stages / four warps: 12 requests at 141
         // tokens 836 / 723 / 737, 16 at 500 862 / 797, eight at 100 677 / 653 / 671 and at 500 743 / 734 / 782, one at 300 609 / 630).
         const bool large = whole && singles > 0 && singles <= sm_count(), deep = large && 8 * singles <= sm_count();
+        // (four warps take the weights in two parts where contexts are whole that were cut: the others' results stay as they are)
         auto* kernel = small ? attention_decode_tma_kernel<HD, true, 2> : deep ? attention_decode_tma_kernel<HD, true, 8, 3>
-                     : large ? attention_decode_tma_kernel<HD, true, 8, 2> : attention_decode_tma_kernel<HD, true, TD_CONSUMERS>;
+                     : large ? attention_decode_tma_kernel<HD, true, 8, 2>
+                     : whole ? attention_decode_tma_kernel<HD, true, TD_CONSUMERS, TD_STAGES, true> : attention_decode_tma_kernel<HD, true, TD_CONSUMERS>;
         const int consumers = small ? 2 : large ? 8 : TD_CONSUMERS, stages = large && !deep ? 2 : TD_STAGES;
         const size_t smem = smem_of(consumers, stages, 16);
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

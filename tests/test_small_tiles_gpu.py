@@ -260,3 +260,33 @@ def test_many_requests_with_a_rotation(nh, nkv, hd, page):
     work, _, parts = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, 1)
     assert parts == 0
     _single_tokens(ctxs, work, nh, nkv, hd, page, True)
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 8, 128), (32, 8, 128), (8, 8, 64), (6, 2, 64), (5, 1, 128), (16, 2, 64)])
+@pytest.mark.parametrize("many", [2.0, 1.5, 0.0])
+def test_weights_in_two_parts(nh, nkv, hd, many):
+    # two, four or eight warps to a CTA (by CTAs an SM), groups of one to eight heads: only the result is rounded to bfloat16
+    B, page = int(many * ops.sm_count() / nkv + 1), 16
+    ctxs = [(97 * r) % 500 + 3 for r in range(B)]
+    g = torch.Generator(device=DEV).manual_seed(nh * hd + B)
+    width = max(ctxs) // page + 1
+    tables = torch.arange(B * width, device=DEV, dtype=torch.int32).view(B, width)
+    kp, vp = (torch.randn(B * width, nkv, page, hd, device=DEV, generator=g).bfloat16() for _ in range(2))
+    qkv = torch.randn(B, (nh + 2 * nkv) * hd, device=DEV, generator=g).bfloat16()
+    work, _, _ = attention_plan.plan_attention([(r, 1, c) for r, c in enumerate(ctxs)], 1, None, nkv, 1)
+    one = torch.zeros(1, dtype=torch.int32, device=DEV)
+    w = AttentionWork(torch.from_numpy(work).to(DEV), one + B, B, torch.zeros(1, 4, dtype=torch.int32, device=DEV), one, 0,
+                      torch.zeros(1, nh, hd, device=DEV), torch.zeros(1, nh, 2, device=DEV), kinds=1, reduces=False)
+    out, st = torch.zeros(B, nh * hd, dtype=torch.bfloat16, device=DEV), K.status()
+    ops.decode_attention_fused(qkv, None, None, 0.0, None, None, kp, vp, tables, w, out, nh, nkv, hd, hd ** -0.5, st)
+    assert st.item() == 0
+    for r, c in enumerate(ctxs):
+        n = c + 1
+        at = torch.arange(n, device=DEV) % page & 7
+        idx = (torch.arange(hd // 8, device=DEV)[None, :] ^ at[:, None])[None, :, :, None].expand(nkv, n, hd // 8, 8)
+        k, v = (p[tables[r].long()].transpose(0, 1).reshape(nkv, -1, hd)[:, :n].reshape(nkv, n, hd // 8, 8).gather(2, idx).reshape(nkv, n, hd).double()
+                for p in (kp, vp))
+        s = torch.einsum("gpd,gnd->gpn", qkv[r].double().view(-1, hd)[:nh].view(nkv, nh // nkv, hd), k) * hd ** -0.5
+        want = torch.einsum("gpn,gnd->gpd", torch.softmax(s, -1), v).reshape(-1)
+        # half a step of the result's bfloat16, and of the weights 2^-17 each (and float's roundings), of values up to 5
+        assert ((out[r].double() - want).abs() <= 2.0 ** -8 * want.abs() + 5 * 2.0 ** -16).all(), r
